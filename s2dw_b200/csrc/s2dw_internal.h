@@ -135,62 +135,95 @@ struct TwDev {
     double2 *hi = nullptr, *lo = nullptr;
 };
 
-// Tables of the plan use a padded row stride Bp = roundup(B, 32) so that
-// 32-wide tiles never read past a row.
+// Packed triangular tables of the contraction kernels, rows of R values per
+// degree.  Analysis, G: row l holds the m' < gpack_len(l) (l rounded up to 32),
+// its R rows consecutive.  Synthesis, GT: row m' holds the l >= gtpack_start(m')
+// up to the padded Lp.
+__host__ __device__ __forceinline__ int gpack_len(int l) { return 32 * ((l >> 5) + 1); }
+__host__ __device__ __forceinline__ long long gpack_row(int l, int R)
+{
+    const long long k = l >> 5;
+    return R * (512 * k * (k + 1) + 32 * (l & 31) * (k + 1));
+}
+__host__ __device__ __forceinline__ int gtpack_start(int mp) { return mp < 64 ? 0 : 64 * ((mp >> 6) - 1); }
+__host__ __device__ __forceinline__ int gtpack_len(int mp, int Lp) { return Lp - gtpack_start(mp); }
+__host__ __device__ __forceinline__ long long gtpack_row(int mp, int R, int Lp)
+{
+    const long long k = mp >> 6;
+    const long long skipped = k == 0 ? 0 : 32 * (k - 1) * (k - 2) + (mp & 63) * (k - 1);
+    return R * ((long long)mp * Lp - 64 * skipped);
+}
+
+// Tables of the plan use a padded row stride Bp = roundup(B, 32); those that
+// the analysis kernel stages have rows to a multiple of 16 and 64 values of
+// slack, so that it reads whole tiles without bounds.
 struct LwalkArgs {
-    int B, Bp, N, NP, bl, blo;
+    int B, Bp, N, NP, J;
     int nq[S2DW_NPMAX];
     const double *Acoef;  // [l*Bp + x]
     const double *Stm;    // [l0*B + k]
     const int32_t *Ste;
-    const double *G;      // [((l-blo-1)*NP + q)*Gs + m'] = Om(l,m') d^l_{m'n_q} K_j(l) s(l,n_q)
-    int Gs;               // roundup(bl, 32)
+    const double *G;      // gpack_row(l, 2 NP): Om(l,m') d^l_{m'n_q} K_j(l) s(l,n_q), row slot NP + q, slot = j & 1
     const double2 *F;     // [l*Bp + m] = Om(l,m) flm(l,m)
-    double2 *Tg;          // [g][m][m'] N x bl x bl
+    const double2 *ph;    // [g (2N-1) + n+N-1] = exp(i pi n g / N)
+    double2 *Tg;          // scale j: Tg + off[j], [g][m][m'] N x bl x bl
     const int2 *tiles;    // (p-tile, m-tile) per CTA, longest walks first
-    int ntiles;
+    int ntiles, S;        // S: m per half warp (lwalk_pairs)
+    int only;             // -1: every scale; else this scale alone
     // 0: Tg = T.  1: G holds the second real part b of S = eta (a + i b)
     // (a general complex Slm): Tg += T with the +n terms times -i and the
     // -n terms times +i (conj(S) for n >= 0, S for n < 0).
     int acc_imag;
+    short bl[S2DW_JMAX + 1], blo[S2DW_JMAX + 1];
+    long long off[S2DW_JMAX + 1];
+};
+
+// Interval lo <= l < hi whose degrees lie in the ranges of scale j and, if
+// two, of scale j + 1 (scale j's range may start at lo + 1).
+struct MwalkInterval {
+    int lo, hi, j;
+    bool two;
 };
 
 struct MwalkArgs {
-    int B, Bp, N, NP, bl, blo;
-    int nq[S2DW_NPMAX];
-    const double *Bcoef;  // [l*Bp + m']
+    int B, NP, bs, niv;
     const double *Em;     // [l*B + m]
     const int32_t *Ee;
-    const double *G;      // [((l-blo-1)*NP + q)*Gs + m'] = Gam(l,m') d^l_{m'n_q} c_j(l,n_q)
-    int Gs;               // roundup(bl, 8)
-    const double2 *V2f;   // [(q*bl + m)*Vs + m']
-    int Vs;               // roundup(bl, 8)
-    double2 *part;        // this scale's flm contribution [(l-blo-1)*bl + m], m <= l
-    // the same tables transposed for the two-l-per-thread kernel:
-    // GT[(m' (NP+1) + q) Ts + l - blo - 1], q < NP: G; q = NP: b(l, m');
-    // rows m' < roundup(bl, 8), Ts = roundup(bl - blo - 1, 64), zero padded
-    const double *GT;
-    int Ts;
-    int tile_l, tile_m;   // the plan's tile shape (mwalk_tile_l / mwalk_tile_m when it was built)
-    const int2 *tiles;    // (l-tile, m-tile) per CTA, longest walks first
+    const double *GT;     // gtpack_row(m', 2 NP + 1, Lp): Gam(l,m') d^l_{m'n_q} c_j(l,n_q), row slot NP + q; row 2 NP: b(l,m')
+    int Lp;               // roundup(B, 64) + 64
+    const double2 *V2f;   // scale j: V2f + offV[j], [(q*bl + m)*Vs + m']
+    const double2 *scoeff;
+    const double *Phi2;
+    double2 *flm;         // flm[l + B m], every value written (the scaling part added)
+    const int2 *tiles;    // (l0 | interval << 16, m0) per CTA, longest walks first
     int ntiles;
-    // 0: part = result.  1: G holds the second real part b of S = eta (a + i b)
-    // (a general complex Slm): part += i * result.
+    int2 shape;           // P x S (mwalk_shape)
+    // 0: flm = result.  1: GT holds the second real part b of S = eta (a + i b)
+    // (a general complex Slm): flm += i * result.
     int acc_imag;
+    short iv_lo[2 * S2DW_JMAX + 2], iv_hi[2 * S2DW_JMAX + 2];
+    unsigned char iv_j[2 * S2DW_JMAX + 2], iv_two[2 * S2DW_JMAX + 2];
+    short bl[S2DW_JMAX + 1], blo[S2DW_JMAX + 1], Vs[S2DW_JMAX + 1];  // Vs: roundup(bl, 8)
+    long long offV[S2DW_JMAX + 1];
 };
-// Tile lists of the contraction kernels for one scale, ordered by decreasing
-// work so that the longest walks start first.
-void build_lwalk_tiles(int bl, int blo, int ws, std::vector<int2> &t);
-void build_mwalk_tiles(int bl, int blo, int wq, int tl, std::vector<int2> &t);
-int lwalk_tile_m(int NP);  // m values per lwalk CTA tile
-int mwalk_tile_m(int NP);  // m values per mwalk CTA tile
-int mwalk_tile_l(int NP);  // l values per mwalk CTA tile: 64 for the kernel that reads GT, else 32
-struct GsTArgs {
-    int Bp, NP, bl, blo, Gs, Ts, rows;  // rows = roundup(bl, 8)
-    const double *G, *Bcoef;
+// Tile lists, ordered by decreasing work so that the longest walks start first.
+int lwalk_pairs(int B, int NP);
+void build_lwalk_tiles(int B, int S, std::vector<int2> &t);
+int2 mwalk_shape(int B, int NP);
+int build_mwalk_intervals(const std::vector<int> &bl, const std::vector<int> &blo, int B,
+                          std::vector<MwalkInterval> &iv);
+void build_mwalk_tiles(const std::vector<MwalkInterval> &iv, int2 shape, std::vector<int2> &t);
+
+// The tables G (from T = Om, kappa of the analysis) or, transposed, GT (from
+// T = Gam, kappa of the synthesis), built at set_tables time.
+struct GpackArgs {
+    int B, Bp, NP, hn, J, Lp;
+    int nq[S2DW_NPMAX];
+    const double *T, *H, *kappa, *Bcoef;  // kappa[(j*B + l)*NP + q]
     double *out;
+    short bl[S2DW_JMAX + 1], blo[S2DW_JMAX + 1];
 };
-int launch_gsyn_t(const GsTArgs &a, cudaStream_t s);
+int launch_gpack(const GpackArgs &a, bool transposed, cudaStream_t s);
 
 // flm(l,m) = sum_j part_j(l,m) + Phi2(l) scoeff(l,m), the scale sum of
 // s2dw_core_mod.f90:1228-1253 in scale order followed by :1258-1261.
@@ -204,8 +237,8 @@ struct CombineArgs {
     double2 *flm;
 };
 
-// Per-scale factor tables G (see LwalkArgs / MwalkArgs), built at
-// set_tables time: out[((l-blo-1)*NP+q)*stride + x] = T[l*Bp+x] *
+// Per-scale factor tables of the split form (see SplitArgs / SplitSynArgs),
+// built at set_tables time: out[((l-blo-1)*NP+q)*stride + x] = T[l*Bp+x] *
 // H[(l*8+nq)*B+x] * kappa[l*NP+q] for x <= l, x < bl; zero elsewhere.
 struct GprepArgs {
     int B, Bp, NP, bl, blo, stride, hn;  // hn: n rows of H
@@ -229,8 +262,10 @@ struct CztArgs {
 
 int launch_lwalk(const LwalkArgs &a, cudaStream_t s);
 int launch_gprep(const GprepArgs &a, cudaStream_t s);
-// F[l*Bp + m] = Om[l*Bp + m] * flm[l + B*m] for m <= l < B, zero for m > l.
-int launch_fprep(double2 *F, const double2 *flm, const double *Om, int B, int Bp, cudaStream_t s);
+// F[l*Bp + m] = Om[l*Bp + m] * flm[l + B*m] for m <= l < B, zero for m > l, and
+// scoeff(0:bs-1,0:bs-1) = flm(0:bs-1,0:bs-1) (s2dw_core_mod.f90:773).
+int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs,
+                 cudaStream_t s);
 int launch_mwalk(const MwalkArgs &a, cudaStream_t s);
 int launch_czt(const CztArgs &a, cudaStream_t s);
 void set_fft_values(int v);  // FFT engine variant: 8 or 16 values per thread, 0 = general engine only
@@ -244,7 +279,6 @@ void set_pfa_small(bool on);       // prime-factor alpha stages at bl = 2, 4, 8,
 // (the current device; synchronises).  Plan creation calls it, never a capture.
 int pfa_prepare();
 void set_alpha_prefetch(bool on);  // synthesis alpha / analysis beta stages: persistent kernel with prefetched input (default on)
-void set_walk_variants(int lwalk, int mwalk);  // tile shape / occupancy variants of the contraction kernels
 int launch_zero(double *p, long long n, cudaStream_t s);
 int launch_scoeff_copy(double2 *scoeff, const double2 *flm, int B, int bs, cudaStream_t s);
 int launch_scaling_add(double2 *flm, const double2 *scoeff, const double *Phi2, int B, int bs,
@@ -266,8 +300,8 @@ struct SplitArgs {
     const double *Acoef, *Om;  // [l*Bp + x]
     const double *Stm;         // [l0*B + k]
     const int32_t *Ste;
-    const double *G;           // as LwalkArgs::G
-    int Gs;
+    const double *G;           // [((l-blo-1)*NP + q)*Gs + m'] = Om(l,m') d^l_{m'n_q} K_j(l) s(l,n_q)
+    int Gs;                    // roundup(bl, 32)
     int16_t *dexp;             // [(m*bl + m')*NP + q] exponent of max_l |v|
     const int32_t *fexp;       // [m*64 + col] exponent of the map column
     const uint8_t *fdig;       // [(m*nch + chunk)*5 + digit][2048] map digits
@@ -295,8 +329,8 @@ struct SplitSynArgs {
     const double *Bcoef;       // [l*Bp + m']
     const double *Em;          // [l*B + m]
     const int32_t *Ee;
-    const double *G;           // as MwalkArgs::G
-    int Gs;
+    const double *G;           // [((l-blo-1)*NP + q)*Gs + m'] = Gam(l,m') d^l_{m'n_q} c_j(l,n_q)
+    int Gs;                    // roundup(bl, 8)
     int16_t *sexp;             // [m*bl + l] exponent of max over (m', q) of |v|
     const int32_t *vexp;       // [m*64 + col]
     const uint8_t *vdig;       // [(m*nch + chunk)*6 + digit][2048] map digits

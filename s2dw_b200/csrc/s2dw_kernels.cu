@@ -1,13 +1,7 @@
 // Device kernels of libs2dw_cuda (sm_100a, FP64).
 //
-//  * lwalk_kernel  : analysis l-contraction T(m,m',n) = sum_l d^l_{m'm} d^l_{m'n} f_lm psi_ln
-//                    (s2dw_core_mod.f90:625-673), fused with the gamma DFT
-//                    (:679-705).  d^l_{m'm}(pi/2) is generated in registers by
-//                    a three-term recurrence in l, one plane per step, never
-//                    stored.
-//  * mwalk_kernel  : synthesis contraction wig(l,m,n) = sum_m' V d^l_{m'm} d^l_{m'n}
-//                    and harmonic accumulation (:1200-1253), generating d by a
-//                    recurrence in m' at fixed (l,m).
+//  * fprep_kernel  : the analysis input scaled and transposed for the
+//                    contraction (s2dw_contract.cu)
 //  * czt_kernel    : chirp-z (Bluestein) transforms in shared memory that
 //                    replace the naive beta sums (:708-743, :1157-1198) and
 //                    the FFTW alpha transforms (:746-768, :1104-1130).
@@ -34,317 +28,8 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-// z * i^k
-__device__ __forceinline__ double2 cipow(double2 z, int k)
-{
-    switch (k & 3) {
-    case 0: return z;
-    case 1: return make_double2(-z.y, z.x);
-    case 2: return make_double2(-z.x, -z.y);
-    default: return make_double2(z.y, -z.x);
-    }
-}
-
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ int warp_max_i(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-
-// ===========================================================================
-// Asynchronous global -> shared copies (16 bytes, L2 only)
-// ===========================================================================
-__device__ __forceinline__ void cp16(void *smem, const void *gmem)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_wait()
-{
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-// ===========================================================================
-// Analysis: l-walk contraction fused with the gamma DFT
-//
-// CTA tile: 32 consecutive m' (lanes) x LW_W*S consecutive m (S per warp).
-// Each thread walks l for its S pairs (m', m); per step it needs a(l,m'),
-// G(l,m',q) (lane-distinct) and a(l,m), F(l,m) (warp-uniform broadcast),
-// staged LW_CH values of l at a time in a double-buffered cp.async pipeline.
-// ===========================================================================
-constexpr int LW_W = 4;    // warps per CTA
-constexpr int LW_CH = 16;  // l values per staged chunk (even)
-constexpr int LW_PHS = 2 * S2DW_NMAX;  // gamma-DFT phase table row: n + N - 1 < 2N - 1
-
-template <int NP, int S>
-struct LwalkSmem {
-    static constexpr int WS = LW_W * S;
-    // per buffer, in doubles: F (complex, first for 16-byte alignment), Ap, G, Am
-    static constexpr int F_OFF = 0;
-    static constexpr int AP_OFF = F_OFF + 2 * LW_CH * WS;
-    static constexpr int G_OFF = AP_OFF + LW_CH * 32;
-    static constexpr int AM_OFF = G_OFF + LW_CH * NP * 32;
-    static constexpr int BUF = AM_OFF + LW_CH * WS;
-    static constexpr size_t BYTES = 2 * BUF * sizeof(double) + S2DW_NMAX * LW_PHS * sizeof(double2);
-};
-
-template <int NP, int S>
-__device__ __forceinline__ void lwalk_body(const LwalkArgs &a)
-{
-    using L = LwalkSmem<NP, S>;
-    constexpr int WS = L::WS;
-    extern __shared__ __align__(16) double lsm[];
-    double2 *sPh = reinterpret_cast<double2 *>(lsm + 2 * L::BUF);  // [g*LW_PHS + n+N-1]
-
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int2 tile = a.tiles[blockIdx.x];
-    const int p0 = tile.x * 32, m0 = tile.y * WS;
-    const int B = a.B, Bp = a.Bp, bl = a.bl, blo = a.blo, N = a.N, Gs = a.Gs;
-    const int mp = p0 + lane;
-
-    for (int i = tid; i < N * (2 * N - 1); i += blockDim.x) {
-        const int g = i / (2 * N - 1), n = i % (2 * N - 1) - (N - 1);
-        double sn, cs;
-        sincospi((double)(n * g) / (double)N, &sn, &cs);
-        sPh[g * LW_PHS + n + N - 1] = make_double2(cs, sn);
-    }
-
-    // ---- per-pair start values; pair = (m' = mp, m = m0 + w*S + s)
-    int l0[S];
-    double st[S];
-    int maxe = INT_MIN;
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        const int m = m0 + w * S + s;
-        const bool valid = (mp < bl) && (m < bl);
-        l0[s] = valid ? max(mp, m) : INT_MAX;
-        if (valid) maxe = max(maxe, (int)a.Ste[(size_t)max(mp, m) * B + min(mp, m)]);
-    }
-    maxe = warp_max_i(maxe);
-    int Kw = (maxe != INT_MIN && maxe < S2DW_SCALE_EXP) ? -maxe : 0;
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        const int m = m0 + w * S + s;
-        st[s] = 0.0;
-        if (l0[s] != INT_MAX) {
-            const size_t o = (size_t)l0[s] * B + min(mp, m);
-            double v = ldexp(a.Stm[o], (int)a.Ste[o] + Kw);
-            if (mp >= m && ((mp - m) & 1)) v = -v;
-            st[s] = v;
-        }
-    }
-
-    double x[2][S];
-    double2 acc[2][S][NP];
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        x[0][s] = 0.0;
-        x[1][s] = 0.0;
-#pragma unroll
-        for (int q = 0; q < NP; q++) acc[0][s][q] = acc[1][s][q] = make_double2(0.0, 0.0);
-    }
-
-    const int lstart = max(p0, m0) & ~1;
-    const int rampEnd = min(max(p0 + 31, m0 + WS - 1), bl - 1);
-    const int nchunks = (bl - lstart + LW_CH - 1) / LW_CH;
-
-    // Staging: the 16-byte pieces of a chunk's rows go to the threads in a
-    // fixed pattern (piece column from the thread index, rows in passes), so
-    // that a copy costs a row bound check and one address computation.
-    static_assert(LW_W * 32 == 128 && LW_CH % 8 == 0, "staging pattern assumes 128 threads");
-    auto stage = [&](int c, int buf) {
-        const int lc = lstart + c * LW_CH;
-        double *b = lsm + buf * L::BUF;
-        const int pc = tid & 15;  // piece of a 32-double row
-        // a(l, m'): 16 pieces per row, 8 rows per pass
-#pragma unroll
-        for (int i = 0; i < LW_CH / 8; i++) {
-            const int li = (tid >> 4) + 8 * i, l = lc + li;
-            if (l < bl) cp16(b + L::AP_OFF + li * 32 + 2 * pc, a.Acoef + (size_t)l * Bp + p0 + 2 * pc);
-        }
-        // a(l, m): WS/2 pieces per row
-        constexpr int AMP = WS / 2, AMR = 128 / AMP;
-#pragma unroll
-        for (int i = 0; i < (LW_CH + AMR - 1) / AMR; i++) {
-            const int li = tid / AMP + AMR * i, l = lc + li;
-            if (li < LW_CH && l < bl)
-                cp16(b + L::AM_OFF + li * WS + 2 * (tid % AMP), a.Acoef + (size_t)l * Bp + m0 + 2 * (tid % AMP));
-        }
-        if (lc + LW_CH - 1 > blo) {
-            // G(l, m', q): rows r = li NP + q of 16 pieces, 8 rows per pass
-#pragma unroll
-            for (int i = 0; i < LW_CH * NP / 8; i++) {
-                const int r = (tid >> 4) + 8 * i, l = lc + r / NP;
-                if (l > blo && l < bl)
-                    cp16(b + L::G_OFF + r * 32 + 2 * pc,
-                         a.G + ((long long)(lc - blo - 1) * NP + r) * Gs + p0 + 2 * pc);
-            }
-            // F(l, m): WS pieces (complex values) per row
-            constexpr int FR = 128 / WS;
-#pragma unroll
-            for (int i = 0; i < (LW_CH + FR - 1) / FR; i++) {
-                const int li = tid / WS + FR * i, l = lc + li;
-                if (li < LW_CH && l > blo && l < bl)
-                    cp16(b + L::F_OFF + 2 * (li * WS + tid % WS), a.F + (size_t)l * Bp + m0 + tid % WS);
-            }
-        }
-    };
-
-    // One recurrence step at chunk row li (l parity PAR).
-    auto step = [&](const double *b, const int li, const int l, auto par_tag, const bool inj, const bool accum) {
-        constexpr int PAR = decltype(par_tag)::value;
-        const double ap = b[L::AP_OFF + li * 32 + lane];
-        double g[NP];
-        if (accum) {
-#pragma unroll
-            for (int q = 0; q < NP; q++) g[q] = b[L::G_OFF + (li * NP + q) * 32 + lane];
-        }
-        const double2 *Fr = reinterpret_cast<const double2 *>(b + L::F_OFF) + li * WS + w * S;
-        const double *Amr = b + L::AM_OFF + li * WS + w * S;
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-            if (inj && l == l0[s]) x[PAR][s] = st[s];
-            const double cur = x[PAR][s];
-            if (accum) {
-                const double2 F = Fr[s];
-                const double xr = cur * F.x, xi = cur * F.y;
-#pragma unroll
-                for (int q = 0; q < NP; q++) {
-                    acc[PAR][s][q].x = fma(xr, g[q], acc[PAR][s][q].x);
-                    acc[PAR][s][q].y = fma(xi, g[q], acc[PAR][s][q].y);
-                }
-            }
-            const double p = Amr[s] * ap;
-            x[PAR ^ 1][s] = fma(-p, cur, -x[PAR ^ 1][s]);
-        }
-    };
-    using P0 = std::integral_constant<int, 0>;
-    using P1 = std::integral_constant<int, 1>;
-
-    if (nchunks > 0) stage(0, 0);
-    cp_commit();
-    for (int c = 0; c < nchunks; c++) {
-        if (c + 1 < nchunks) stage(c + 1, (c + 1) & 1);
-        cp_commit();
-        cp_wait<1>();
-        __syncthreads();
-        const double *b = lsm + (c & 1) * L::BUF;
-        const int lc = lstart + c * LW_CH;
-        const int nl = min(LW_CH, bl - lc);
-        if (lc > rampEnd && lc > blo && nl == LW_CH) {
-            // every step accumulates, no start value enters: unrolled, so that
-            // the shared-memory reads take constant offsets
-#pragma unroll
-            for (int li = 0; li < LW_CH; li += 2) {
-                step(b, li, lc + li, P0{}, false, true);
-                step(b, li + 1, lc + li + 1, P1{}, false, true);
-            }
-        } else if (lc > rampEnd && lc + LW_CH - 1 <= blo && nl == LW_CH) {
-            // a chunk below the scale's l range: the recurrence alone (not the
-            // general path below, whose accumulation would issue predicated off)
-#pragma unroll 1
-            for (int li = 0; li < LW_CH; li += 2) {
-                step(b, li, lc + li, P0{}, false, false);
-                step(b, li + 1, lc + li + 1, P1{}, false, false);
-            }
-        } else {
-#pragma unroll 1
-            for (int li = 0; li < nl; li += 2) {
-                const int l = lc + li;
-                step(b, li, l, P0{}, l <= rampEnd, l > blo);
-                if (li + 1 < nl) step(b, li + 1, l + 1, P1{}, l + 1 <= rampEnd, l + 1 > blo);
-            }
-        }
-        if (Kw > 0) {  // keep scaled values in range (warp-uniform)
-            double mx = 0.0;
-#pragma unroll
-            for (int s = 0; s < S; s++) mx = fmax(mx, fmax(fabs(x[0][s]), fabs(x[1][s])));
-            mx = warp_max(mx);
-            if (mx > ldexp(1.0, S2DW_RENORM_EXP)) {
-                const int R = min(S2DW_RENORM_EXP, Kw);
-                const double f = ldexp(1.0, -R);
-#pragma unroll
-                for (int s = 0; s < S; s++) {
-                    x[0][s] *= f;
-                    x[1][s] *= f;
-#pragma unroll
-                    for (int q = 0; q < NP; q++) {
-                        acc[0][s][q] = cscale(acc[0][s][q], f);
-                        acc[1][s][q] = cscale(acc[1][s][q], f);
-                    }
-                }
-                Kw -= R;
-            }
-        }
-        __syncthreads();
-    }
-
-    // ---- epilogue: T(m,m',+-n) from even/odd-l sums, then the gamma DFT
-    // T(+n) = i^{n-m} conj(eta) (E+O), T(-n) = i^{-n-m} (-1)^{m'+n} eta (E-O),
-    // T(0) = i^{-m} (E+O); eta = 1 (N odd) or i (N even).
-    const double sc = ldexp(1.0, -Kw);
-    const int ev = (N % 2 == 0) ? 1 : 0;
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        if (l0[s] == INT_MAX) continue;
-        const int m = m0 + w * S + s;
-        double2 Tp[NP], Tm[NP];
-#pragma unroll
-        for (int q = 0; q < NP; q++) {
-            const int n = a.nq[q];
-            const double2 E = cscale(acc[0][s][q], sc), O = cscale(acc[1][s][q], sc);
-            const double2 sum = cadd(E, O), dif = csub(E, O);
-            // acc_imag: the b part of S enters the +n terms times -i (i^-1)
-            // and the -n terms times +i
-            const int ai = a.acc_imag ? 1 : 0;
-            if (n == 0) {
-                Tp[q] = cipow(sum, -m - ai);
-                Tm[q] = make_double2(0.0, 0.0);
-            } else {
-                Tp[q] = cipow(sum, n - m - ev - ai);
-                double2 t = cipow(dif, -n - m + ev + ai);
-                if ((mp + n) & 1) t = make_double2(-t.x, -t.y);
-                Tm[q] = t;
-            }
-        }
-        for (int gg = 0; gg < N; gg++) {
-            double2 y = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int q = 0; q < NP; q++) {
-                const int n = a.nq[q];
-                y = cadd(y, cmul(Tp[q], sPh[gg * LW_PHS + n + N - 1]));
-                if (n != 0) y = cadd(y, cmul(Tm[q], sPh[gg * LW_PHS - n + N - 1]));
-            }
-            double2 *dst = a.Tg + ((size_t)gg * bl + m) * bl + mp;
-            *dst = a.acc_imag ? cadd(*dst, y) : y;
-        }
-    }
-}
-
-// MINB = 0: no minimum-blocks bound (the compiler picks the register count)
-template <int NP, int S, int MINB>
-__global__ void __launch_bounds__(LW_W * 32) lwalk_kernel(LwalkArgs a)
-{
-    lwalk_body<NP, S>(a);
-}
-template <int NP, int S, int MINB>
-__global__ void __launch_bounds__(LW_W * 32, MINB) lwalk_kernel_minb(LwalkArgs a)
-{
-    lwalk_body<NP, S>(a);
-}
-
-// Per-scale factor tables for the contraction kernels (built once per set of
-// kernel tables).
+// Per-scale factor tables of the split form (built once per set of kernel
+// tables).
 __global__ void gprep_kernel(GprepArgs a)
 {
     const int nl = a.bl - a.blo - 1;
@@ -363,7 +48,7 @@ __global__ void gprep_kernel(GprepArgs a)
 
 // F[l*Bp + m] = Om[l*Bp+m] flm[l + B m]: transpose of the column-major flm
 // through a 32x32 shared tile.
-__global__ void fprep_kernel(double2 *F, const double2 *flm, const double *Om, int B, int Bp)
+__global__ void fprep_kernel(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs)
 {
     __shared__ double2 tile[32][33];
     const int l0 = blockIdx.x * 32, mb = blockIdx.y * 32;
@@ -371,6 +56,7 @@ __global__ void fprep_kernel(double2 *F, const double2 *flm, const double *Om, i
     for (int k = ty; k < 32; k += 8) {
         const int l = l0 + tx, m = mb + k;
         tile[k][tx] = (l < B && m < B) ? flm[(size_t)l + (size_t)B * m] : make_double2(0.0, 0.0);
+        if (l < bs && m < bs) scoeff[l + (size_t)bs * m] = tile[k][tx];
     }
     __syncthreads();
     for (int k = ty; k < 32; k += 8) {
@@ -380,434 +66,6 @@ __global__ void fprep_kernel(double2 *F, const double2 *flm, const double *Om, i
             if (m <= l && m < B) v = cscale(tile[tx][k], Om[(size_t)l * Bp + m]);
             F[(size_t)l * Bp + m] = v;
         }
-    }
-}
-
-// ===========================================================================
-// Synthesis: m'-walk contraction and harmonic accumulation
-//
-// CTA tile: 32 consecutive l (lanes) x MW_W*Q consecutive m (Q per warp).
-// Each thread walks m' down from min(l_tile_max, bl-1) to 0 for its Q pairs
-// (l, m).  Staged per chunk of MW_CH m' values (aligned to MW_CH): the
-// lane-distinct rows b(l, m') and G(l, m', q) (each thread copies its row to
-// registers) and the broadcast V2f(m, m', q).
-// ===========================================================================
-constexpr int MW_W = 4;
-constexpr int MW_CH = 8;
-constexpr int MW_RS = MW_CH + 2;  // padded row stride (conflict-free 16-byte row loads)
-
-template <int NP, int Q>
-struct MwalkSmem {
-    static constexpr int WQ = MW_W * Q;
-    static constexpr int V_OFF = 0;                          // double2 [NP][WQ][MW_CH]
-    static constexpr int B_OFF = V_OFF + 2 * NP * WQ * MW_CH;  // double [32][MW_RS]
-    static constexpr int G_OFF = B_OFF + 32 * MW_RS;           // double [NP][32][MW_RS]
-    static constexpr int BUF = G_OFF + NP * 32 * MW_RS;
-    static constexpr size_t BYTES = 2 * BUF * sizeof(double);
-};
-
-template <int NP, int Q>
-__device__ __forceinline__ void mwalk_body(const MwalkArgs &a)
-{
-    using L = MwalkSmem<NP, Q>;
-    constexpr int WQ = L::WQ;
-    extern __shared__ __align__(16) double msm[];
-
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int2 tile = a.tiles[blockIdx.x];
-    const int lt = tile.x, mt = tile.y;
-    const int B = a.B, Bp = a.Bp, bl = a.bl, blo = a.blo, Gs = a.Gs, Vs = a.Vs;
-    const int lbase = blo + 1 + lt * 32, mbase = mt * WQ;
-    const int MH = min(lbase + 31, bl - 1);
-    if (mbase > MH) return;  // tile entirely above the diagonal m <= l
-    const int l = lbase + lane;
-
-    double st[Q], mq[Q];
-    bool val[Q];
-    int maxe = INT_MIN;
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        const int m = mbase + w * Q + q;
-        val[q] = (l < bl) && (m <= l);
-        mq[q] = (double)m;
-        if (val[q]) maxe = max(maxe, (int)a.Ee[(size_t)l * B + m]);
-    }
-    maxe = warp_max_i(maxe);
-    int Kw = (maxe != INT_MIN && maxe < S2DW_SCALE_EXP) ? -maxe : 0;
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        const int m = mbase + w * Q + q;
-        st[q] = 0.0;
-        if (val[q]) {
-            const double v = ldexp(a.Em[(size_t)l * B + m], (int)a.Ee[(size_t)l * B + m] + Kw);
-            st[q] = ((l - m) & 1) ? -v : v;
-        }
-    }
-    double e[Q], ep[Q];
-    double2 acc[Q];
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        e[q] = ep[q] = 0.0;
-        acc[q] = make_double2(0.0, 0.0);
-    }
-
-    const int ctop = MH / MW_CH;  // chunks ctop, ctop-1, ..., 0 cover m' = MH .. 0
-
-    // Staging: a fixed pattern of 16-byte pieces per thread (see lwalk).  The
-    // rows of l >= bl and of m >= bl are never copied: they are zeroed once
-    // here, in both buffers, so that the idle lanes and pairs walk zeros.
-    static_assert(MW_W * 32 == 128 && MW_CH == 8, "staging pattern assumes 128 threads, 8 m' per chunk");
-    const int nt = min(32, bl - lbase), nu = min(WQ, bl - mbase);
-    if (nt < 32 || nu < WQ) {
-        for (int i = tid; i < 2 * L::BUF; i += blockDim.x) {
-            const int r = i % L::BUF;
-            bool idle;
-            if (r < L::B_OFF) idle = ((r - L::V_OFF) / (2 * MW_CH)) % WQ >= nu;
-            else if (r < L::G_OFF) idle = (r - L::B_OFF) / MW_RS >= nt;
-            else idle = ((r - L::G_OFF) / MW_RS) % 32 >= nt;
-            if (idle) msm[i] = 0.0;
-        }
-    }
-    auto stage = [&](int c, int buf) {
-        double *b = msm + buf * L::BUF;
-        const int c0 = c * MW_CH;
-        // b(l, m') and G(l, m', q): 4 pieces per row, one row per 4 threads
-        const int t = tid >> 2, k = tid & 3, ll = lbase + t;
-        if (ll < bl) {
-            cp16(b + L::B_OFF + t * MW_RS + 2 * k, a.Bcoef + (size_t)ll * Bp + c0 + 2 * k);
-#pragma unroll
-            for (int q = 0; q < NP; q++)
-                cp16(b + L::G_OFF + (q * 32 + t) * MW_RS + 2 * k,
-                     a.G + ((size_t)(ll - blo - 1) * NP + q) * Gs + c0 + 2 * k);
-        }
-        // V2f(m, m', q): MW_CH pieces (complex values) per (q, m) row
-#pragma unroll
-        for (int i = 0; i < NP * WQ * MW_CH / 128; i++) {
-            const int f = tid + 128 * i, kk = f % MW_CH, r = f / MW_CH, u = r % WQ, q = r / WQ;
-            if (mbase + u < bl)
-                cp16(b + L::V_OFF + 2 * (r * MW_CH + kk), a.V2f + ((size_t)q * bl + mbase + u) * Vs + c0 + kk);
-        }
-    };
-
-    stage(ctop, 0);
-    cp_commit();
-    for (int c = ctop, it = 0; c >= 0; c--, it++) {
-        if (c > 0) stage(c - 1, (it + 1) & 1);
-        cp_commit();
-        cp_wait<1>();
-        __syncthreads();
-        const double *b = msm + (it & 1) * L::BUF;
-        const int c0 = c * MW_CH;
-        // this thread's rows into registers
-        double br[MW_CH], gr[NP][MW_CH];
-#pragma unroll
-        for (int k = 0; k < MW_CH; k += 2) {
-            const double2 v = *reinterpret_cast<const double2 *>(b + L::B_OFF + lane * MW_RS + k);
-            br[k] = v.x;
-            br[k + 1] = v.y;
-#pragma unroll
-            for (int q = 0; q < NP; q++) {
-                const double2 u = *reinterpret_cast<const double2 *>(b + L::G_OFF + (q * 32 + lane) * MW_RS + k);
-                gr[q][k] = u.x;
-                gr[q][k + 1] = u.y;
-            }
-        }
-        const double2 *Vb = reinterpret_cast<const double2 *>(b + L::V_OFF);
-        const bool ramp = (c0 + MW_CH - 1 >= lbase);
-        // one step of the m' walk for pair q at chunk row k (the same
-        // operations in the same order on both paths below)
-        auto mstep = [&](const int k, const int q) {
-            double zr = 0.0, zi = 0.0;
-#pragma unroll
-            for (int kq = 0; kq < NP; kq++) {
-                const double2 v = Vb[(kq * WQ + w * Q + q) * MW_CH + k];
-                zr = fma(gr[kq][k], v.x, zr);
-                zi = fma(gr[kq][k], v.y, zi);
-            }
-            acc[q].x = fma(e[q], zr, acc[q].x);
-            acc[q].y = fma(e[q], zi, acc[q].y);
-            const double p = mq[q] * br[k];
-            const double en = fma(p, e[q], -ep[q]);
-            ep[q] = e[q];
-            e[q] = en;
-        };
-        if (!ramp && c0 + MW_CH - 1 <= MH) {
-            // a chunk below the tile's l rows: every step runs, no start value
-            // enters (warp-uniform)
-#pragma unroll
-            for (int k = MW_CH - 1; k >= 0; k--)
-#pragma unroll
-                for (int q = 0; q < Q; q++) mstep(k, q);
-        } else {
-#pragma unroll
-            for (int k = MW_CH - 1; k >= 0; k--) {
-                const int mpv = c0 + k;
-                if (mpv > MH) continue;  // above the top of this tile (warp-uniform)
-#pragma unroll
-                for (int q = 0; q < Q; q++) {
-                    if (ramp && mpv == l) e[q] = st[q];
-                    mstep(k, q);
-                }
-            }
-        }
-        if (Kw > 0) {
-            double mx = 0.0;
-#pragma unroll
-            for (int q = 0; q < Q; q++) mx = fmax(mx, fmax(fabs(e[q]), fabs(ep[q])));
-            mx = warp_max(mx);
-            if (mx > ldexp(1.0, S2DW_RENORM_EXP)) {
-                const int R = min(S2DW_RENORM_EXP, Kw);
-                const double f = ldexp(1.0, -R);
-#pragma unroll
-                for (int q = 0; q < Q; q++) {
-                    e[q] *= f;
-                    ep[q] *= f;
-                    acc[q] = cscale(acc[q], f);
-                }
-                Kw -= R;
-            }
-        }
-        __syncthreads();
-    }
-    // this scale's flm(l,m) = i^m * acc (the eta and i^{-n} phases are folded into G)
-    const double sc = ldexp(1.0, -Kw);
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-        if (!val[q]) continue;
-        const int m = mbase + w * Q + q;
-        double2 *dst = a.part + (size_t)(l - blo - 1) * bl + m;
-        if (a.acc_imag) *dst = cadd(*dst, cipow(cscale(acc[q], sc), m + 1));  // + i * result
-        else *dst = cipow(cscale(acc[q], sc), m);
-    }
-}
-
-template <int NP, int Q, int MINB>
-__global__ void __launch_bounds__(MW_W * 32) mwalk_kernel(MwalkArgs a)
-{
-    mwalk_body<NP, Q>(a);
-}
-template <int NP, int Q, int MINB>
-__global__ void __launch_bounds__(MW_W * 32, MINB) mwalk_kernel_minb(MwalkArgs a)
-{
-    mwalk_body<NP, Q>(a);
-}
-
-// ---------------------------------------------------------------------------
-// Synthesis m'-walk with two l per thread (NP <= 4).
-//
-// The broadcast reads of V2f(m, m', q) bound the kernel above: a 16-byte read
-// that every lane takes costs two shared-memory wavefronts, one per (m, q, m')
-// for 32 lanes' worth of FP64 work.  Here each lane walks the pairs of two l
-// (l and l + 32) with QM values of m, so that one broadcast read of V feeds
-// twice the work, and the per-l rows b(l, m') and G(l, m', q) are read per step
-// from a transposed table (GT, l fastest: conflict-free 8-byte reads) instead
-// of being held in registers.  Tile: 64 l x MW_W*QM m; the same chunks of
-// MW_CH m' values, staged by cp.async in a fixed pattern.
-// ---------------------------------------------------------------------------
-constexpr int M2_TL = 64;  // l per tile
-
-template <int NP, int QM>
-struct Mwalk2Smem {
-    static constexpr int WQ = MW_W * QM;
-    static constexpr int R = NP + 1;                               // GT rows per m'
-    static constexpr int T_OFF = 0;                                // double [MW_CH][R][64]
-    static constexpr int V_OFF = T_OFF + MW_CH * R * M2_TL;        // double2 [NP][WQ][MW_CH]
-    static constexpr int BUF = V_OFF + 2 * NP * WQ * MW_CH;
-    static constexpr size_t BYTES = 2 * BUF * sizeof(double);
-};
-
-template <int NP, int QM>
-__device__ __forceinline__ void mwalk2_body(const MwalkArgs &a)
-{
-    using L = Mwalk2Smem<NP, QM>;
-    constexpr int WQ = L::WQ, R = L::R;
-    static_assert(MW_W * 32 == 128 && MW_CH == 8 && (MW_CH * R * M2_TL / 2) % 128 == 0, "staging pattern");
-    extern __shared__ __align__(16) double msm[];
-
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int2 tile = a.tiles[blockIdx.x];
-    const int lt = tile.x, mt = tile.y;
-    const int B = a.B, bl = a.bl, blo = a.blo, Vs = a.Vs, Ts = a.Ts;
-    const int lbase = blo + 1 + lt * M2_TL, mbase = mt * WQ;
-    const int MH = min(lbase + M2_TL - 1, bl - 1);
-    if (mbase > MH) return;  // tile entirely above the diagonal m <= l
-
-    int l[2];
-    double st[2][QM], mq[QM];
-    bool val[2][QM];
-    int maxe = INT_MIN;
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        l[i] = lbase + lane + 32 * i;
-#pragma unroll
-        for (int q = 0; q < QM; q++) {
-            const int m = mbase + w * QM + q;
-            val[i][q] = (l[i] < bl) && (m <= l[i]);
-            if (val[i][q]) maxe = max(maxe, (int)a.Ee[(size_t)l[i] * B + m]);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < QM; q++) mq[q] = (double)(mbase + w * QM + q);
-    maxe = warp_max_i(maxe);
-    int Kw = (maxe != INT_MIN && maxe < S2DW_SCALE_EXP) ? -maxe : 0;
-    double e[2][QM], ep[2][QM];
-    double2 acc[2][QM];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int q = 0; q < QM; q++) {
-            const int m = mbase + w * QM + q;
-            st[i][q] = 0.0;
-            if (val[i][q]) {
-                const double v = ldexp(a.Em[(size_t)l[i] * B + m], (int)a.Ee[(size_t)l[i] * B + m] + Kw);
-                st[i][q] = ((l[i] - m) & 1) ? -v : v;
-            }
-            e[i][q] = ep[i][q] = 0.0;
-            acc[i][q] = make_double2(0.0, 0.0);
-        }
-
-    const int ctop = MH / MW_CH;  // chunks ctop, ctop-1, ..., 0 cover m' = MH .. 0
-    // V rows of m >= bl are never copied: zeroed once, in both buffers
-    const int nu = min(WQ, bl - mbase);
-    if (nu < WQ)
-        for (int i = tid; i < 2 * L::BUF; i += blockDim.x) {
-            const int r = i % L::BUF;
-            if (r >= L::V_OFF && ((r - L::V_OFF) / (2 * MW_CH)) % WQ >= nu) msm[i] = 0.0;
-        }
-    // GT rows (m', q) of a chunk are consecutive: MW_CH*R rows of 64 doubles
-    // from column lt*64 (16-byte pieces, 32 per row); V2f as in mwalk_kernel
-    const double *gsrc = a.GT + (size_t)lt * M2_TL;
-    auto stage = [&](int c, int buf) {
-        double *b = msm + buf * L::BUF;
-        const double *src = gsrc + (size_t)c * MW_CH * R * Ts;
-#pragma unroll
-        for (int i = 0; i < MW_CH * R * M2_TL / 2 / 128; i++) {
-            const int pc = tid + 128 * i, row = pc >> 5, col = pc & 31;
-            cp16(b + L::T_OFF + row * M2_TL + 2 * col, src + (size_t)row * Ts + 2 * col);
-        }
-        const int c0 = c * MW_CH;
-#pragma unroll
-        for (int i = 0; i < (NP * WQ * MW_CH + 127) / 128; i++) {
-            const int f = tid + 128 * i, kk = f % MW_CH, r = f / MW_CH, u = r % WQ, q = r / WQ;
-            if (f < NP * WQ * MW_CH && mbase + u < bl)
-                cp16(b + L::V_OFF + 2 * (r * MW_CH + kk), a.V2f + ((size_t)q * bl + mbase + u) * Vs + c0 + kk);
-        }
-    };
-
-    stage(ctop, 0);
-    cp_commit();
-    for (int c = ctop, it = 0; c >= 0; c--, it++) {
-        if (c > 0) stage(c - 1, (it + 1) & 1);
-        cp_commit();
-        cp_wait<1>();
-        __syncthreads();
-        const double *b = msm + (it & 1) * L::BUF;
-        const double *T = b + L::T_OFF;
-        const double2 *Vb = reinterpret_cast<const double2 *>(b + L::V_OFF);
-        const int c0 = c * MW_CH;
-        const bool ramp = (c0 + MW_CH - 1 >= lbase);
-        // one m' step at chunk row k for all pairs (the same operations in the
-        // same order as mwalk_kernel's step)
-        auto mstep = [&](const int k, const bool inj, const int mpv) {
-            double bk[2], gk[2][NP];
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                bk[i] = T[(k * R + NP) * M2_TL + lane + 32 * i];
-#pragma unroll
-                for (int kq = 0; kq < NP; kq++) gk[i][kq] = T[(k * R + kq) * M2_TL + lane + 32 * i];
-            }
-#pragma unroll
-            for (int q = 0; q < QM; q++) {
-                double2 v[NP];
-#pragma unroll
-                for (int kq = 0; kq < NP; kq++) v[kq] = Vb[(kq * WQ + w * QM + q) * MW_CH + k];
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    if (inj && mpv == l[i]) e[i][q] = st[i][q];
-                    double zr = 0.0, zi = 0.0;
-#pragma unroll
-                    for (int kq = 0; kq < NP; kq++) {
-                        zr = fma(gk[i][kq], v[kq].x, zr);
-                        zi = fma(gk[i][kq], v[kq].y, zi);
-                    }
-                    acc[i][q].x = fma(e[i][q], zr, acc[i][q].x);
-                    acc[i][q].y = fma(e[i][q], zi, acc[i][q].y);
-                    const double p = mq[q] * bk[i];
-                    const double en = fma(p, e[i][q], -ep[i][q]);
-                    ep[i][q] = e[i][q];
-                    e[i][q] = en;
-                }
-            }
-        };
-        if (!ramp && c0 + MW_CH - 1 <= MH) {
-            // below the tile's l rows: every step runs, no start value enters
-#pragma unroll
-            for (int k = MW_CH - 1; k >= 0; k--) mstep(k, false, 0);
-        } else {
-#pragma unroll 1
-            for (int k = MW_CH - 1; k >= 0; k--) {
-                const int mpv = c0 + k;
-                if (mpv > MH) continue;  // above the top of this tile (warp-uniform)
-                mstep(k, ramp, mpv);
-            }
-        }
-        if (Kw > 0) {
-            double mx = 0.0;
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int q = 0; q < QM; q++) mx = fmax(mx, fmax(fabs(e[i][q]), fabs(ep[i][q])));
-            mx = warp_max(mx);
-            if (mx > ldexp(1.0, S2DW_RENORM_EXP)) {
-                const int Rr = min(S2DW_RENORM_EXP, Kw);
-                const double f = ldexp(1.0, -Rr);
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int q = 0; q < QM; q++) {
-                        e[i][q] *= f;
-                        ep[i][q] *= f;
-                        acc[i][q] = cscale(acc[i][q], f);
-                    }
-                Kw -= Rr;
-            }
-        }
-        __syncthreads();
-    }
-    const double sc = ldexp(1.0, -Kw);
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int q = 0; q < QM; q++) {
-            if (!val[i][q]) continue;
-            const int m = mbase + w * QM + q;
-            double2 *dst = a.part + (size_t)(l[i] - blo - 1) * bl + m;
-            if (a.acc_imag) *dst = cadd(*dst, cipow(cscale(acc[i][q], sc), m + 1));  // + i * result
-            else *dst = cipow(cscale(acc[i][q], sc), m);
-        }
-}
-
-template <int NP, int QM>
-__global__ void __launch_bounds__(MW_W * 32, 3) mwalk2_kernel(MwalkArgs a)
-{
-    mwalk2_body<NP, QM>(a);
-}
-
-// GT[(m' (NP+1) + q) Ts + l'] from G (q < NP) and b(l, m') (q = NP), l = blo+1+l';
-// zero for l' >= bl-blo-1 or m' >= bl.
-__global__ void gsyn_t_kernel(GsTArgs a)
-{
-    const int nl = a.bl - a.blo - 1, R = a.NP + 1;
-    const long long total = (long long)a.rows * R * a.Ts;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int lp = (int)(i % a.Ts);
-        const long long r = i / a.Ts;
-        const int q = (int)(r % R), x = (int)(r / R);
-        double v = 0.0;
-        if (lp < nl && x < a.bl)
-            v = q < a.NP ? a.G[((size_t)lp * a.NP + q) * a.Gs + x] : a.Bcoef[(size_t)(a.blo + 1 + lp) * a.Bp + x];
-        a.out[i] = v;
     }
 }
 
@@ -2538,212 +1796,6 @@ __global__ void combine_kernel(CombineArgs a)
 // ===========================================================================
 // Launchers
 // ===========================================================================
-template <int NP, int S, int MINB>
-static int launch_lwalk_np(const LwalkArgs &a, cudaStream_t s)
-{
-    using L = LwalkSmem<NP, S>;
-    static bool attr[64] = {false};
-    int dev = 0;
-    S2DW_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 64 && !attr[dev]) {
-        if (MINB > 0)
-            S2DW_CUDA_TRY(cudaFuncSetAttribute(lwalk_kernel_minb<NP, S, (MINB > 0 ? MINB : 1)>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES));
-        else
-            S2DW_CUDA_TRY(cudaFuncSetAttribute(lwalk_kernel<NP, S, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)L::BYTES));
-        attr[dev] = true;
-    }
-    if (a.ntiles <= 0) return S2DWC_OK;
-    if (MINB > 0)
-        lwalk_kernel_minb<NP, S, (MINB > 0 ? MINB : 1)><<<a.ntiles, LW_W * 32, L::BYTES, s>>>(a);
-    else
-        lwalk_kernel<NP, S, 0><<<a.ntiles, LW_W * 32, L::BYTES, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-static int g_lwalk_variant = 0, g_mwalk_variant = 0;
-
-int lwalk_tile_m(int NP) { return LW_W * (NP > 4 ? 2 : 4); }  // pairs per thread: 4, or 2 for N > 8
-// the two-l-per-thread synthesis kernel (the default, variant 4), for N <= 8
-// (NP <= 4; 4 m per thread for NP <= 2, 2 for NP = 3, 4); measured on B200 at
-// B=1024, N=4: 343 -> 322 us per full-band launch, FP64 pipe 49 -> 61 %,
-// shared-memory wavefronts 61 -> 43 % of peak
-static bool mwalk2_used(int NP) { return g_mwalk_variant == 4 && NP <= 4; }
-static int mwalk2_qm(int NP) { return NP <= 2 ? 4 : 2; }
-int mwalk_tile_m(int NP)
-{
-    if (mwalk2_used(NP)) return MW_W * mwalk2_qm(NP);
-    return MW_W * (g_mwalk_variant == 1 && NP <= 4 ? 8 : 4);
-}
-int mwalk_tile_l(int NP) { return mwalk2_used(NP) ? M2_TL : 32; }
-
-void build_lwalk_tiles(int bl, int blo, int ws, std::vector<int2> &t)
-{
-    // work of tile (pt, mt): walk from max(p0, m0) to bl-1
-    t.clear();
-    const int tp = (bl + 31) / 32, tm = (bl + ws - 1) / ws;
-    for (int pt = 0; pt < tp; pt++)
-        for (int mt = 0; mt < tm; mt++) t.push_back(make_int2(pt, mt));
-    std::stable_sort(t.begin(), t.end(), [ws](int2 a, int2 b) {
-        return std::max(a.x * 32, a.y * ws) < std::max(b.x * 32, b.y * ws);
-    });
-    (void)blo;
-}
-
-void build_mwalk_tiles(int bl, int blo, int wq, int th, std::vector<int2> &t)
-{
-    // tile (lt, mt) covers l in [blo+1+th lt, +th), m in [wq mt, +wq); its
-    // walk length is ~ the largest l; tiles entirely above m <= l are dropped
-    t.clear();
-    const int nl = bl - blo - 1;
-    if (nl <= 0) return;
-    const int tl = (nl + th - 1) / th, tm = (bl + wq - 1) / wq;
-    for (int lt = tl - 1; lt >= 0; lt--) {
-        const int lmax = std::min(blo + 1 + lt * th + th - 1, bl - 1);
-        for (int mt = 0; mt < tm; mt++)
-            if (mt * wq <= lmax) t.push_back(make_int2(lt, mt));
-    }
-}
-void set_walk_variants(int lw, int mw)
-{
-    g_lwalk_variant = lw;
-    g_mwalk_variant = mw;
-}
-
-template <int S, int MINB>
-static int launch_lwalk_s(const LwalkArgs &a, cudaStream_t s)
-{
-    switch (a.NP) {
-    case 1: return launch_lwalk_np<1, S, MINB>(a, s);
-    case 2: return launch_lwalk_np<2, S, MINB>(a, s);
-    case 3: return launch_lwalk_np<3, S, MINB>(a, s);
-    case 4: return launch_lwalk_np<4, S, MINB>(a, s);
-    // N > 8: two pairs per thread keep the accumulators in registers
-    case 5: return launch_lwalk_np<5, 2, 0>(a, s);
-    case 6: return launch_lwalk_np<6, 2, 0>(a, s);
-    case 7: return launch_lwalk_np<7, 2, 0>(a, s);
-    case 8: return launch_lwalk_np<8, 2, 0>(a, s);
-    }
-    return set_error(S2DWC_ERROR_SIZE_INVALID, "lwalk: unsupported N=%d (N<=%d)", a.N, S2DW_NMAX);
-}
-
-int launch_lwalk(const LwalkArgs &a, cudaStream_t s)
-{
-    switch (g_lwalk_variant) {
-    case 1: return launch_lwalk_s<4, 4>(a, s);
-    case 2: return launch_lwalk_s<4, 3>(a, s);
-    default:
-        // more resident CTAs where the register cap costs no spills and the
-        // grid is many waves deep (bl >= 1024: 2048+ tiles); measured on
-        // B200: NP = 2, bl = 1024: 3 CTAs/SM 10 % faster than 2; NP = 1:
-        // 4 CTAs/SM 4 % faster.  Smaller grids lose more to the tail wave,
-        // and NP >= 3 spills under the caps.
-        if (a.bl >= 1024 && a.NP == 2) return launch_lwalk_np<2, 4, 3>(a, s);
-        if (a.bl >= 1024 && a.NP == 1) return launch_lwalk_np<1, 4, 4>(a, s);
-        return launch_lwalk_s<4, 0>(a, s);
-    }
-}
-
-template <int NP, int Q, int MINB>
-static int launch_mwalk_np(const MwalkArgs &a, cudaStream_t s)
-{
-    using L = MwalkSmem<NP, Q>;
-    const int nl = a.bl - a.blo - 1;
-    if (nl <= 0) return S2DWC_OK;
-    static bool attr[64] = {false};
-    int dev = 0;
-    S2DW_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 64 && !attr[dev]) {
-        if (MINB > 0)
-            S2DW_CUDA_TRY(cudaFuncSetAttribute(mwalk_kernel_minb<NP, Q, (MINB > 0 ? MINB : 1)>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES));
-        else
-            S2DW_CUDA_TRY(cudaFuncSetAttribute(mwalk_kernel<NP, Q, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)L::BYTES));
-        attr[dev] = true;
-    }
-    if (a.ntiles <= 0) return S2DWC_OK;
-    if (MINB > 0)
-        mwalk_kernel_minb<NP, Q, (MINB > 0 ? MINB : 1)><<<a.ntiles, MW_W * 32, L::BYTES, s>>>(a);
-    else
-        mwalk_kernel<NP, Q, 0><<<a.ntiles, MW_W * 32, L::BYTES, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-template <int NP, int QM>
-static int launch_mwalk2(const MwalkArgs &a, cudaStream_t s)
-{
-    using L = Mwalk2Smem<NP, QM>;
-    if (a.bl - a.blo - 1 <= 0 || a.ntiles <= 0) return S2DWC_OK;
-    if (!a.GT) return set_error(S2DWC_ERROR_ARG_INVALID, "mwalk2: transposed tables missing");
-    static bool attr[64] = {false};
-    int dev = 0;
-    S2DW_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 64 && !attr[dev]) {
-        S2DW_CUDA_TRY(cudaFuncSetAttribute(mwalk2_kernel<NP, QM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)L::BYTES));
-        attr[dev] = true;
-    }
-    mwalk2_kernel<NP, QM><<<a.ntiles, MW_W * 32, L::BYTES, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-int launch_gsyn_t(const GsTArgs &a, cudaStream_t s)
-{
-    const long long total = (long long)a.rows * (a.NP + 1) * a.Ts;
-    if (total <= 0) return S2DWC_OK;
-    long long blocks = (total + 255) / 256;
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    gsyn_t_kernel<<<(int)blocks, 256, 0, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-template <int Q, int MINB>
-static int launch_mwalk_q(const MwalkArgs &a, cudaStream_t s)
-{
-    switch (a.NP) {
-    case 1: return launch_mwalk_np<1, Q, MINB>(a, s);
-    case 2: return launch_mwalk_np<2, Q, MINB>(a, s);
-    case 3: return launch_mwalk_np<3, Q, MINB>(a, s);
-    case 4: return launch_mwalk_np<4, Q, MINB>(a, s);
-    // N > 8: no register cap (the G rows of 5-8 n values stay in registers)
-    case 5: return launch_mwalk_np<5, 4, 0>(a, s);
-    case 6: return launch_mwalk_np<6, 4, 0>(a, s);
-    case 7: return launch_mwalk_np<7, 4, 0>(a, s);
-    case 8: return launch_mwalk_np<8, 4, 0>(a, s);
-    }
-    return set_error(S2DWC_ERROR_SIZE_INVALID, "mwalk: unsupported N=%d (N<=%d)", a.N, S2DW_NMAX);
-}
-
-int launch_mwalk(const MwalkArgs &a, cudaStream_t s)
-{
-    // the kernel follows the plan's tile shape
-    if (a.tile_l == M2_TL) {
-        if (a.NP > 4 || a.tile_m != MW_W * mwalk2_qm(a.NP))
-            return set_error(S2DWC_ERROR_ARG_INVALID, "mwalk: tile shape %dx%d for NP=%d", a.tile_l, a.tile_m, a.NP);
-        switch (a.NP) {
-        case 1: return launch_mwalk2<1, 4>(a, s);
-        case 2: return launch_mwalk2<2, 4>(a, s);
-        case 3: return launch_mwalk2<3, 2>(a, s);
-        default: return launch_mwalk2<4, 2>(a, s);
-        }
-    }
-    if (a.tile_l != 32) return set_error(S2DWC_ERROR_ARG_INVALID, "mwalk: tile height %d", a.tile_l);
-    if (a.tile_m == MW_W * 8) return launch_mwalk_q<8, 0>(a, s);
-    switch (g_mwalk_variant) {
-    case 2: return launch_mwalk_q<4, 5>(a, s);
-    case 3: return launch_mwalk_q<4, 4>(a, s);
-    // 3 CTAs/SM (<= 168 registers, no spills): 3-10 % faster than 4 CTAs/SM
-    // with 128 registers and small spills, at N = 1, 3, 4, 6, 8 (B200)
-    default: return launch_mwalk_q<4, 3>(a, s);
-    }
-}
-
 int launch_gprep(const GprepArgs &a, cudaStream_t s)
 {
     const long long total = (long long)(a.bl - a.blo - 1) * a.NP * a.stride;
@@ -2755,10 +1807,11 @@ int launch_gprep(const GprepArgs &a, cudaStream_t s)
     return S2DWC_OK;
 }
 
-int launch_fprep(double2 *F, const double2 *flm, const double *Om, int B, int Bp, cudaStream_t s)
+int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs,
+                 cudaStream_t s)
 {
     dim3 grid((B + 31) / 32, (Bp + 31) / 32), block(32, 8);
-    fprep_kernel<<<grid, block, 0, s>>>(F, flm, Om, B, Bp);
+    fprep_kernel<<<grid, block, 0, s>>>(F, scoeff, flm, Om, B, Bp, bs);
     S2DW_CUDA_TRY(cudaGetLastError());
     return S2DWC_OK;
 }

@@ -45,31 +45,29 @@ struct s2dwc_plan {
     std::vector<double *> wq;  // quadrature weights per scale
     // caller tables folded into per-scale factor tables
     double *kappaA = nullptr, *kappaS = nullptr, *Phi2 = nullptr;
-    double *Ga = nullptr, *Gsyn = nullptr;       // all scales, see LwalkArgs/MwalkArgs
+    double *GA = nullptr, *GT = nullptr;         // all scales, see LwalkArgs/MwalkArgs
+    long long gpk_total = 0, gtp_total = 0;
+    int Lp = 0;                                  // MwalkArgs::Lp
+    double *Ga = nullptr, *Gsyn = nullptr;       // per scale, for the split form (SplitArgs/SplitSynArgs)
     // a general complex Slm, S = eta (a + i b) with b != 0: the tables of b
     // (built on first use); the contractions then run twice (acc_imag)
     bool slm_general = false;
-    long long ga_total = 0, gs_total = 0;
-    double *kappaA_b = nullptr, *kappaS_b = nullptr, *Ga_b = nullptr, *Gsyn_b = nullptr;
+    double *kappaA_b = nullptr, *kappaS_b = nullptr, *GA_b = nullptr, *GT_b = nullptr;
     std::vector<long long> ga_off, gs_off;       // per-scale offsets (doubles)
     std::vector<int> ga_stride, gs_stride;
-    // synthesis tables transposed for the two-l-per-thread m'-walk (MwalkArgs::GT),
-    // when the plan's tiles are 64 l high: per scale roundup(bl, 8) x (NP+1) rows
-    // of gt_ld[j] = roundup(bl-blo-1, 64) values
-    int mw_tile_l = 32, mw_tile_m = 16;
-    double *GsT = nullptr, *GsT_b = nullptr;
-    long long gt_total = 0;
-    std::vector<long long> gt_off;
-    std::vector<int> gt_ld;
     double2 *Fw = nullptr;                       // per-call F table [l*Bp + m]
     // per-scale workspaces (scales run concurrently on their own streams):
-    // A_j holds Tb / V (N x bl x 2bl), C_j holds Tg (N x bl x bl) / V2f,
-    // P_j the scale's flm rows (bl-blo-1) x bl
-    double2 *wsA = nullptr, *wsC = nullptr, *wsP = nullptr;
+    // A_j holds Tb / V (N x bl x 2bl), C_j holds Tg (N x bl x bl) / V2f; the
+    // split form's partial flm rows of scale j, (bl-blo-1) x bl, start at offP
+    double2 *wsA = nullptr, *wsC = nullptr;
     std::vector<long long> offA, offC, offP;
     std::vector<cudaStream_t> streams;
-    std::vector<int2 *> lw_tiles, mw_tiles;   // per-scale tile lists (device)
-    std::vector<int> lw_ntiles, mw_ntiles;
+    // contraction tiles of all scales (device)
+    int2 *lw_tiles = nullptr, *mw_tiles = nullptr;
+    int lw_ntiles = 0, mw_ntiles = 0, lw_pairs = 1;
+    int2 mw_shape = {1, 1};
+    std::vector<MwalkInterval> mw_iv;
+    double2 *ph = nullptr;                    // gamma-DFT phases, LwalkArgs::ph
     cudaEvent_t ev_fork = nullptr;
     std::vector<cudaEvent_t> ev_join;
     // device buffers of the host-buffer entry points (allocated on first use)
@@ -263,14 +261,16 @@ int plan_build(s2dwc_plan *p)
     // row-padded copies (stride Bp) of the tables read by 32-wide tiles
     const int Bp = (B + 31) / 32 * 32;
     p->Bp = Bp;
-    auto pad = [&](const std::vector<double> &v) {
-        std::vector<double> o((size_t)B * Bp, 0.0);
+    // a: rows to a multiple of 16 and 64 values of slack (LwalkArgs)
+    const int Br = (B + 15) / 16 * 16;
+    auto pad = [&](const std::vector<double> &v, bool a = false) {
+        std::vector<double> o(a ? (size_t)Br * Bp + 64 : (size_t)B * Bp, 0.0);
         for (int l = 0; l < B; l++)
             std::copy(v.begin() + (size_t)l * B, v.begin() + (size_t)(l + 1) * B, o.begin() + (size_t)l * Bp);
         return o;
     };
     int st;
-    if ((st = dev_upload(p, &p->Om, pad(t.Om))) || (st = dev_upload(p, &p->Acoef, pad(t.Acoef))) ||
+    if ((st = dev_upload(p, &p->Om, pad(t.Om))) || (st = dev_upload(p, &p->Acoef, pad(t.Acoef, true))) ||
         (st = dev_upload(p, &p->Stm, t.Stm)) || (st = dev_upload(p, &p->Ste, t.Ste)) ||
         (st = dev_upload(p, &p->Gam, pad(t.Gam))) || (st = dev_upload(p, &p->Bcoef, pad(t.Bcoef))) ||
         (st = dev_upload(p, &p->Em, t.Em)) || (st = dev_upload(p, &p->Ee, t.Ee)) ||
@@ -373,27 +373,17 @@ int plan_build(s2dwc_plan *p)
         na += (long long)nl * p->NP * p->ga_stride[j];
         ns += (long long)nl * p->NP * p->gs_stride[j];
     }
-    p->ga_total = na;
-    p->gs_total = ns;
-    p->mw_tile_l = mwalk_tile_l(p->NP);
-    p->mw_tile_m = mwalk_tile_m(p->NP);
-    if (p->mw_tile_l == 64) {
-        long long nt = 0;
-        for (int j = 0; j <= J; j++) {
-            const int nl = std::max(0, p->bl[j] - p->blo[j] - 1);
-            p->gt_ld.push_back((nl + 63) / 64 * 64);
-            p->gt_off.push_back(nt);
-            nt += (long long)(p->bl[j] + 7) / 8 * 8 * (p->NP + 1) * p->gt_ld[j];
-        }
-        p->gt_total = nt;
-        if ((st = dev_alloc(p, &p->GsT, (size_t)std::max(1LL, nt)))) return st;
-    }
-    if ((st = dev_alloc(p, &p->Ga, (size_t)std::max(1LL, na))) ||
-        (st = dev_alloc(p, &p->Gsyn, (size_t)std::max(1LL, ns))) ||
-        (st = dev_alloc(p, &p->Fw, (size_t)B * Bp)))
+    p->Lp = (B + 63) / 64 * 64 + 64;
+    p->gpk_total = gpack_row(32 * ((B + 31) / 32), 2 * p->NP);
+    p->gtp_total = gtpack_row((B + 7) / 8 * 8, 2 * p->NP + 1, p->Lp);
+    if ((st = dev_alloc(p, &p->GA, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT, (size_t)p->gtp_total)) ||
+        (st = dev_alloc(p, &p->Fw, (size_t)Br * Bp + 64)))
+        return st;
+    if (p->form == S2DWC_FORM_SPLIT && ((st = dev_alloc(p, &p->Ga, (size_t)std::max(1LL, na))) ||
+                                        (st = dev_alloc(p, &p->Gsyn, (size_t)std::max(1LL, ns)))))
         return st;
     // per-scale workspaces
-    long long nA = 0, nC = 0, nP = 0;
+    long long nA = 0, nC = 0, nP = 0;  // nP: split form
     for (int j = 0; j <= J; j++) {
         const long long b = p->bl[j];
         p->offA.push_back(nA);
@@ -403,22 +393,27 @@ int plan_build(s2dwc_plan *p)
         nC += std::max((long long)N * b * b, (long long)p->NP * b * p->gs_stride[j]);
         nP += (long long)std::max(0, p->bl[j] - p->blo[j] - 1) * b;
     }
-    if ((st = dev_alloc(p, &p->wsA, (size_t)nA)) || (st = dev_alloc(p, &p->wsC, (size_t)nC)) ||
-        (st = dev_alloc(p, &p->wsP, (size_t)std::max(1LL, nP))))
-        return st;
-    for (int j = 0; j <= J; j++) {
+    if ((st = dev_alloc(p, &p->wsA, (size_t)nA)) || (st = dev_alloc(p, &p->wsC, (size_t)nC))) return st;
+    {
         std::vector<int2> tl;
-        build_lwalk_tiles(p->bl[j], p->blo[j], lwalk_tile_m(p->NP), tl);
-        int2 *d = nullptr;
-        if ((st = dev_upload(p, &d, tl))) return st;
-        p->lw_tiles.push_back(d);
-        p->lw_ntiles.push_back((int)tl.size());
-        build_mwalk_tiles(p->bl[j], p->blo[j], p->mw_tile_m, p->mw_tile_l, tl);
-        d = nullptr;
-        if (tl.empty()) tl.push_back(make_int2(0, 0));  // keep a valid allocation
-        if ((st = dev_upload(p, &d, tl))) return st;
-        p->mw_tiles.push_back(d);
-        p->mw_ntiles.push_back(p->bl[j] - p->blo[j] - 1 > 0 ? (int)tl.size() : 0);
+        p->lw_pairs = lwalk_pairs(B, p->NP);
+        build_lwalk_tiles(B, p->lw_pairs, tl);
+        if ((st = dev_upload(p, &p->lw_tiles, tl))) return st;
+        p->lw_ntiles = (int)tl.size();
+        p->mw_shape = mwalk_shape(B, p->NP);
+        if ((st = build_mwalk_intervals(p->bl, p->blo, B, p->mw_iv))) return st;
+        if (p->mw_iv.size() > sizeof(MwalkArgs::iv_j))
+            return set_error(S2DWC_ERROR_SIZE_INVALID, "%zu intervals of l", p->mw_iv.size());
+        build_mwalk_tiles(p->mw_iv, p->mw_shape, tl);
+        p->mw_ntiles = (int)tl.size();
+        if ((st = dev_upload(p, &p->mw_tiles, tl))) return st;
+        std::vector<double2> ph((size_t)N * (2 * N - 1));
+        for (int g = 0; g < N; g++)
+            for (int n = -(N - 1); n <= N - 1; n++) {
+                const long double x = 3.141592653589793238462643383279502884L * (long double)(n * g) / (long double)N;
+                ph[(size_t)g * (2 * N - 1) + n + N - 1] = make_double2((double)cosl(x), (double)sinl(x));
+            }
+        if ((st = dev_upload(p, &p->ph, ph))) return st;
     }
     if (p->dry) return S2DWC_OK;
     if ((std::find(p->bl.begin(), p->bl.end(), 1024) != p->bl.end() ||
@@ -507,8 +502,72 @@ struct KernelTimer {
     }
 };
 
-// Runs the analysis: the F table on `s`, then every scale on its own stream
-// (forked from and joined back to `s`).
+// Arguments of the contraction kernels; the second pass of a general Slm sets
+// acc_imag and the tables of b.
+LwalkArgs lwalk_args(const s2dwc_plan *p, const double2 *F, double2 *Tg)
+{
+    LwalkArgs a{};
+    a.B = p->B;
+    a.Bp = p->Bp;
+    a.N = p->N;
+    a.NP = p->NP;
+    a.J = p->J;
+    std::memcpy(a.nq, p->nq, sizeof(a.nq));
+    a.Acoef = p->Acoef;
+    a.Stm = p->Stm;
+    a.Ste = p->Ste;
+    a.G = p->GA;
+    a.F = F;
+    a.ph = p->ph;
+    a.Tg = Tg;
+    a.tiles = p->lw_tiles;
+    a.ntiles = p->lw_ntiles;
+    a.S = p->lw_pairs;
+    a.only = -1;
+    for (int j = 0; j <= p->J; j++) {
+        a.bl[j] = (short)p->bl[j];
+        a.blo[j] = (short)p->blo[j];
+        a.off[j] = p->offC[j];
+    }
+    return a;
+}
+
+MwalkArgs mwalk_args(const s2dwc_plan *p, double2 *flm, const double2 *scoeff)
+{
+    MwalkArgs a{};
+    a.B = p->B;
+    a.NP = p->NP;
+    a.bs = p->bl_scoeff;
+    a.niv = (int)p->mw_iv.size();
+    a.Em = p->Em;
+    a.Ee = p->Ee;
+    a.GT = p->GT;
+    a.Lp = p->Lp;
+    a.V2f = p->wsC;
+    a.scoeff = scoeff;
+    a.Phi2 = p->Phi2;
+    a.flm = flm;
+    a.tiles = p->mw_tiles;
+    a.ntiles = p->mw_ntiles;
+    a.shape = p->mw_shape;
+    for (int v = 0; v < a.niv; v++) {
+        a.iv_lo[v] = (short)p->mw_iv[v].lo;
+        a.iv_hi[v] = (short)p->mw_iv[v].hi;
+        a.iv_j[v] = (unsigned char)p->mw_iv[v].j;
+        a.iv_two[v] = p->mw_iv[v].two;
+    }
+    for (int j = 0; j <= p->J; j++) {
+        a.bl[j] = (short)p->bl[j];
+        a.blo[j] = (short)p->blo[j];
+        a.Vs[j] = (short)p->gs_stride[j];
+        a.offV[j] = p->offC[j];
+    }
+    return a;
+}
+
+// Runs the analysis: the F table and the contraction of all scales on `s`,
+// then every scale's transforms on its own stream (forked from and joined back
+// to `s`).
 // Per-scale hook: enqueued on scale j's stream after (analysis) or before
 // (synthesis) that scale's kernels; the host-buffer entry points use it to
 // overlap each scale's host<->device copy with the other scales' kernels.
@@ -525,7 +584,18 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
     int st;
     {
         KernelTimer kt(p, S2DWC_KIND_OTHER, s);
-        if ((st = launch_fprep(p->Fw, d_flm, p->Om, p->B, p->Bp, s))) return st;
+        if ((st = launch_fprep(p->Fw, d_scoeff, d_flm, p->Om, p->B, p->Bp, p->bl_scoeff, s))) return st;
+    }
+    LwalkArgs la = lwalk_args(p, p->Fw, p->wsC);
+    {
+        KernelTimer kt(p, S2DWC_KIND_LWALK, s);
+        if ((st = launch_lwalk(la, s))) return st;
+    }
+    if (p->slm_general) {  // the b part of a general Slm, accumulated into Tg
+        la.G = p->GA_b;
+        la.acc_imag = 1;
+        KernelTimer kt(p, S2DWC_KIND_LWALK, s);
+        if ((st = launch_lwalk(la, s))) return st;
     }
     S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
     const bool serial = full_band_serial && !p->timing && (int)p->ev_done.size() == p->J + 1;
@@ -540,33 +610,6 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         const bool full = serial && bl == p->bl[p->J];
         if (full && prev_full >= 0) S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_done[prev_full], 0));
         double2 *Tg = p->wsC + p->offC[j], *Tb = p->wsA + p->offA[j];
-        LwalkArgs la{};
-        la.B = p->B;
-        la.Bp = p->Bp;
-        la.N = p->N;
-        la.NP = p->NP;
-        la.bl = bl;
-        la.blo = p->blo[j];
-        std::memcpy(la.nq, p->nq, sizeof(la.nq));
-        la.Acoef = p->Acoef;
-        la.Stm = p->Stm;
-        la.Ste = p->Ste;
-        la.G = p->Ga + p->ga_off[j];
-        la.Gs = p->ga_stride[j];
-        la.F = p->Fw;
-        la.Tg = Tg;
-        la.tiles = p->lw_tiles[j];
-        la.ntiles = p->lw_ntiles[j];
-        {
-            KernelTimer kt(p, S2DWC_KIND_LWALK, sj);
-            if ((st = launch_lwalk(la, sj))) return st;
-        }
-        if (p->slm_general) {  // the b part of a general Slm, accumulated into Tg
-            la.G = p->Ga_b + p->ga_off[j];
-            la.acc_imag = 1;
-            KernelTimer kt(p, S2DWC_KIND_LWALK, sj);
-            if ((st = launch_lwalk(la, sj))) return st;
-        }
         CztArgs ca{};
         ca.mode = p->ana_beta_mode[j];
         ca.bl = bl;
@@ -599,10 +642,6 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         }
         if (after && (st = after(j, sj))) return st;
         if (!p->timing) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j], sj));
-    }
-    {
-        KernelTimer kt(p, S2DWC_KIND_OTHER, s);
-        if ((st = launch_scoeff_copy(d_scoeff, d_flm, p->B, p->bl_scoeff, s))) return st;
     }
     if (p->timing) return S2DWC_OK;
     for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[j], 0));
@@ -652,58 +691,22 @@ int run_synthesis(s2dwc_plan *p, double2 *d_flm, const double *d_wav, const doub
             KernelTimer kt(p, S2DWC_KIND_SYN_BETA, sj);
             if ((st = launch_czt(ca, sj))) return st;
         }
-        MwalkArgs ma{};
-        ma.B = p->B;
-        ma.Bp = p->Bp;
-        ma.N = p->N;
-        ma.NP = p->NP;
-        ma.bl = bl;
-        ma.blo = p->blo[j];
-        std::memcpy(ma.nq, p->nq, sizeof(ma.nq));
-        ma.Bcoef = p->Bcoef;
-        ma.Em = p->Em;
-        ma.Ee = p->Ee;
-        ma.G = p->Gsyn + p->gs_off[j];
-        ma.Gs = p->gs_stride[j];
-        ma.V2f = V2f;
-        ma.Vs = p->gs_stride[j];
-        ma.part = p->wsP + p->offP[j];
-        ma.GT = p->GsT ? p->GsT + p->gt_off[j] : nullptr;
-        ma.Ts = p->GsT ? p->gt_ld[j] : 0;
-        ma.tile_l = p->mw_tile_l;
-        ma.tile_m = p->mw_tile_m;
-        ma.tiles = p->mw_tiles[j];
-        ma.ntiles = p->mw_ntiles[j];
-        {
-            KernelTimer kt(p, S2DWC_KIND_MWALK, sj);
-            if ((st = launch_mwalk(ma, sj))) return st;
-        }
-        if (p->slm_general) {  // the b part of a general Slm, accumulated into part
-            ma.G = p->Gsyn_b + p->gs_off[j];
-            if (p->GsT) ma.GT = p->GsT_b + p->gt_off[j];
-            ma.acc_imag = 1;
-            KernelTimer kt(p, S2DWC_KIND_MWALK, sj);
-            if ((st = launch_mwalk(ma, sj))) return st;
-        }
         if (!p->timing) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j], sj));
     }
     if (!p->timing)
         for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[j], 0));
-    CombineArgs cb{};
-    cb.B = p->B;
-    cb.J = p->J;
-    cb.bs = p->bl_scoeff;
-    for (int j = 0; j <= p->J; j++) {
-        cb.bl[j] = p->bl[j];
-        cb.blo[j] = p->blo[j];
-        cb.off[j] = p->offP[j];
+    MwalkArgs ma = mwalk_args(p, d_flm, d_scoeff);
+    {
+        KernelTimer kt(p, S2DWC_KIND_MWALK, s);
+        if ((st = launch_mwalk(ma, s))) return st;
     }
-    cb.parts = p->wsP;
-    cb.scoeff = d_scoeff;
-    cb.Phi2 = p->Phi2;
-    cb.flm = d_flm;
-    KernelTimer kt(p, S2DWC_KIND_OTHER, s);
-    return launch_combine(cb, s);
+    if (p->slm_general) {  // the b part of a general Slm, added to flm
+        ma.GT = p->GT_b;
+        ma.acc_imag = 1;
+        KernelTimer kt(p, S2DWC_KIND_MWALK, s);
+        if ((st = launch_mwalk(ma, s))) return st;
+    }
+    return S2DWC_OK;
 }
 
 // Layout of the caller-independent workspace of run_analysis_serial: the F
@@ -736,29 +739,15 @@ int run_analysis_serial(const s2dwc_plan *p, unsigned char *ws, double *d_wav, d
     double2 *F = reinterpret_cast<double2 *>(ws);
     double2 *Tg = reinterpret_cast<double2 *>(ws + L.offTg), *Tb = reinterpret_cast<double2 *>(ws + L.offTb);
     int st;
-    if ((st = launch_fprep(F, d_flm, p->Om, p->B, p->Bp, s))) return st;
+    if ((st = launch_fprep(F, d_scoeff, d_flm, p->Om, p->B, p->Bp, p->bl_scoeff, s))) return st;
     for (int j = 0; j <= p->J; j++) {
         const int bl = p->bl[j];
-        LwalkArgs la{};
-        la.B = p->B;
-        la.Bp = p->Bp;
-        la.N = p->N;
-        la.NP = p->NP;
-        la.bl = bl;
-        la.blo = p->blo[j];
-        std::memcpy(la.nq, p->nq, sizeof(la.nq));
-        la.Acoef = p->Acoef;
-        la.Stm = p->Stm;
-        la.Ste = p->Ste;
-        la.G = p->Ga + p->ga_off[j];
-        la.Gs = p->ga_stride[j];
-        la.F = F;
-        la.Tg = Tg;
-        la.tiles = p->lw_tiles[j];
-        la.ntiles = p->lw_ntiles[j];
+        LwalkArgs la = lwalk_args(p, F, Tg);
+        la.only = j;  // into the one Tg
+        la.off[j] = 0;
         if ((st = launch_lwalk(la, s))) return st;
         if (p->slm_general) {  // the b part of a general Slm, accumulated into Tg
-            la.G = p->Ga_b + p->ga_off[j];
+            la.G = p->GA_b;
             la.acc_imag = 1;
             if ((st = launch_lwalk(la, s))) return st;
         }
@@ -783,7 +772,7 @@ int run_analysis_serial(const s2dwc_plan *p, unsigned char *ws, double *d_wav, d
         ca.out_r = d_wav + p->wav_off[j];
         if ((st = launch_czt(ca, s))) return st;
     }
-    return launch_scoeff_copy(d_scoeff, d_flm, p->B, p->bl_scoeff, s);
+    return S2DWC_OK;
 }
 
 // Split form: per-scale workspaces (the scales of a batch run concurrently
@@ -1258,11 +1247,6 @@ int s2dwc_plan_create(s2dwc_plan **plan, int B, int N, double alpha, int J, int 
         const char *ap = getenv("S2DW_ALPHA_PREFETCH");
         set_alpha_prefetch(ap ? atoi(ap) != 0 : true);
     }
-    {
-        const char *lw = getenv("S2DW_LWALK_VARIANT"), *mw = getenv("S2DW_MWALK_VARIANT");
-        // default synthesis kernel: two l per thread (4; N > 8 falls back to 0)
-        set_walk_variants(lw ? atoi(lw) : 0, mw ? atoi(mw) : 4);
-    }
     auto *p = new s2dwc_plan();
     p->B = B;
     p->N = N;
@@ -1364,13 +1348,11 @@ int s2dwc_plan_set_tables(s2dwc_plan *p, const double *K_gamma, const double *Ph
     std::vector<double> kA, kS;
     factors(sa, kA, kS);
     DeviceGuard dg(p->device);
-    if (general && !p->Ga_b) {
+    if (general && !p->GA_b) {
         int st;
         if ((st = dev_alloc(p, &p->kappaA_b, (size_t)(J + 1) * B * NP)) ||
             (st = dev_alloc(p, &p->kappaS_b, (size_t)(J + 1) * B * NP)) ||
-            (st = dev_alloc(p, &p->Ga_b, (size_t)std::max(1LL, p->ga_total))) ||
-            (st = dev_alloc(p, &p->Gsyn_b, (size_t)std::max(1LL, p->gs_total))) ||
-            (p->GsT && (st = dev_alloc(p, &p->GsT_b, (size_t)std::max(1LL, p->gt_total)))))
+            (st = dev_alloc(p, &p->GA_b, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT_b, (size_t)p->gtp_total)))
             return st;
     }
     if (general) {
@@ -1385,7 +1367,34 @@ int s2dwc_plan_set_tables(s2dwc_plan *p, const double *K_gamma, const double *Ph
         S2DW_CUDA_TRY(cudaMemcpy(p->Phi2, Phi2, (size_t)B * sizeof(double), cudaMemcpyHostToDevice));
     else
         S2DW_CUDA_TRY(cudaMemset(p->Phi2, 0, (size_t)B * sizeof(double)));
-    for (int j = 0; j <= J; j++) {
+    int st;
+    {
+        GpackArgs g{};
+        g.B = B;
+        g.Bp = p->Bp;
+        g.NP = NP;
+        g.hn = p->hn;
+        g.J = J;
+        g.Lp = p->Lp;
+        std::memcpy(g.nq, p->nq, sizeof(g.nq));
+        g.H = p->H;
+        g.Bcoef = p->Bcoef;
+        for (int j = 0; j <= J; j++) {
+            g.bl[j] = (short)p->bl[j];
+            g.blo[j] = (short)p->blo[j];
+        }
+        for (int b = 0; b <= (general ? 1 : 0); b++) {
+            g.T = p->Om;
+            g.kappa = b ? p->kappaA_b : p->kappaA;
+            g.out = b ? p->GA_b : p->GA;
+            if ((st = launch_gpack(g, false, 0))) return st;
+            g.T = p->Gam;
+            g.kappa = b ? p->kappaS_b : p->kappaS;
+            g.out = b ? p->GT_b : p->GT;
+            if ((st = launch_gpack(g, true, 0))) return st;
+        }
+    }
+    for (int j = 0; j <= J && p->Ga; j++) {
         GprepArgs g{};
         g.B = B;
         g.Bp = p->Bp;
@@ -1399,44 +1408,12 @@ int s2dwc_plan_set_tables(s2dwc_plan *p, const double *K_gamma, const double *Ph
         g.kappa = p->kappaA + (size_t)j * B * NP;
         g.stride = p->ga_stride[j];
         g.out = p->Ga + p->ga_off[j];
-        int st = launch_gprep(g, 0);
-        if (st) return st;
+        if ((st = launch_gprep(g, 0))) return st;
         g.T = p->Gam;
         g.kappa = p->kappaS + (size_t)j * B * NP;
         g.stride = p->gs_stride[j];
         g.out = p->Gsyn + p->gs_off[j];
         if ((st = launch_gprep(g, 0))) return st;
-        if (general) {
-            g.T = p->Om;
-            g.kappa = p->kappaA_b + (size_t)j * B * NP;
-            g.stride = p->ga_stride[j];
-            g.out = p->Ga_b + p->ga_off[j];
-            if ((st = launch_gprep(g, 0))) return st;
-            g.T = p->Gam;
-            g.kappa = p->kappaS_b + (size_t)j * B * NP;
-            g.stride = p->gs_stride[j];
-            g.out = p->Gsyn_b + p->gs_off[j];
-            if ((st = launch_gprep(g, 0))) return st;
-        }
-        if (p->GsT) {
-            GsTArgs t{};
-            t.Bp = p->Bp;
-            t.NP = NP;
-            t.bl = p->bl[j];
-            t.blo = p->blo[j];
-            t.Gs = p->gs_stride[j];
-            t.Ts = p->gt_ld[j];
-            t.rows = (p->bl[j] + 7) / 8 * 8;
-            t.G = p->Gsyn + p->gs_off[j];
-            t.Bcoef = p->Bcoef;
-            t.out = p->GsT + p->gt_off[j];
-            if ((st = launch_gsyn_t(t, 0))) return st;
-            if (general) {
-                t.G = p->Gsyn_b + p->gs_off[j];
-                t.out = p->GsT_b + p->gt_off[j];
-                if ((st = launch_gsyn_t(t, 0))) return st;
-            }
-        }
     }
     S2DW_CUDA_TRY(cudaDeviceSynchronize());
     p->bl_scoeff = bl_scoeff;
@@ -1464,10 +1441,8 @@ int s2dwc_plan_launch_count(const s2dwc_plan *p, int *analysis, int *synthesis)
     if (!p) return set_error(S2DWC_ERROR_ARG_INVALID, "launch_count: null plan");
     // a general Slm runs each contraction twice
     const int g = p->slm_general ? 2 : 1;
-    if (analysis) *analysis = (2 + g) * (p->J + 1) + 2;
-    int ns = 1;
-    for (int j = 0; j <= p->J; j++) ns += 2 + ((p->bl[j] - p->blo[j] - 1) > 0 ? g : 0);
-    if (synthesis) *synthesis = ns;
+    if (analysis) *analysis = 2 * (p->J + 1) + 1 + g;
+    if (synthesis) *synthesis = 2 * (p->J + 1) + g;
     return S2DWC_OK;
     S2DW_API_CATCH
 }
