@@ -10,7 +10,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libs2dw_cuda.so")
-SOURCES = ["s2dw_host.cpp", "s2dw_kernels.cu", "s2dw_contract.cu", "s2dw_plan.cu", "s2dw_noalloc.cu", "s2dw_split.cu", "s2dw_stats.cu",
+SOURCES = ["s2dw_host.cpp", "s2dw_kernels.cu", "s2dw_contract.cu", "s2dw_beta.cu", "s2dw_plan.cu", "s2dw_noalloc.cu", "s2dw_split.cu", "s2dw_stats.cu",
            "s2dw_fileio.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -32,7 +32,7 @@ def _host_cxx():
 
 def build(verbose=False, force=False):
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
-    deps = srcs + [os.path.join(CSRC, "s2dw_internal.h"),
+    deps = srcs + [os.path.join(CSRC, "s2dw_internal.h"), os.path.join(CSRC, "s2dw_fft.cuh"),
                    os.path.join(HERE, "..", "include", "s2dw_cuda.h")]
     if not force and os.path.exists(OUT):
         t = os.path.getmtime(OUT)

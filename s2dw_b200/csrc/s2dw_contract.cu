@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         }
     };
     auto full_chunk = [&](const double *b) {
-        constexpr int UNR = NP <= 2 ? 4 : NP <= 4 ? 8 : 2;  // spills above
+        // more unrolling hoists loads past the register cap
+        constexpr int UNR = S == 1 || NP > 4 ? 2 : NP <= 2 ? 4 : 8;
 #pragma unroll UNR
         for (int i = 0; i < LW_CH; i += 2) {
             step(b, i, P0{}, false, 0, true, true);
@@ -829,16 +830,16 @@ int launch_lwalk(const LwalkArgs &a, cudaStream_t s)
     } else {
         switch (a.NP * 16 + a.S) {
         case 16 + 8: return launch_lwalk_t<1, 8, 2, 2>(a, s);
-        case 16 + 4: return launch_lwalk_t<1, 4, 2, 1>(a, s);
-        case 16 + 2: return launch_lwalk_t<1, 2, 2, 1>(a, s);
-        case 16 + 1: return launch_lwalk_t<1, 1, 2, 1>(a, s);
+        case 16 + 4: return launch_lwalk_t<1, 4, 2, 3>(a, s);
+        case 16 + 2: return launch_lwalk_t<1, 2, 2, 4>(a, s);
+        case 16 + 1: return launch_lwalk_t<1, 1, 2, 5>(a, s);
         case 32 + 4: return launch_lwalk_t<2, 4, 2, 2>(a, s);
-        case 32 + 2: return launch_lwalk_t<2, 2, 2, 1>(a, s);
-        case 32 + 1: return launch_lwalk_t<2, 1, 2, 1>(a, s);
+        case 32 + 2: return launch_lwalk_t<2, 2, 2, 3>(a, s);
+        case 32 + 1: return launch_lwalk_t<2, 1, 2, 4>(a, s);
         case 48 + 2: return launch_lwalk_t<3, 2, 2, 2>(a, s);
-        case 48 + 1: return launch_lwalk_t<3, 1, 2, 1>(a, s);
+        case 48 + 1: return launch_lwalk_t<3, 1, 2, 3>(a, s);
         case 64 + 2: return launch_lwalk_t<4, 2, 2, 2>(a, s);
-        case 64 + 1: return launch_lwalk_t<4, 1, 2, 1>(a, s);
+        case 64 + 1: return launch_lwalk_t<4, 1, 2, 3>(a, s);
         case 80 + 1: return launch_lwalk_t<5, 1, 2, 1>(a, s);
         case 96 + 1: return launch_lwalk_t<6, 1, 2, 1>(a, s);
         case 112 + 1: return launch_lwalk_t<7, 1, 2, 1>(a, s);
@@ -852,7 +853,7 @@ template <int NP>
 static int launch_mwalk_np(const MwalkArgs &a, cudaStream_t s)
 {
     if (a.shape.x == 2 && a.shape.y == 4) return launch_mwalk_t<NP, 2, 4, 2>(a, s);
-    if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, 1>(a, s);
+    if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, (NP <= 4 ? 5 : 3)>(a, s);
     if constexpr (NP <= 2) {
         if (a.shape.x == 1 && a.shape.y == 2) return launch_mwalk_t<NP, 1, 2, 1>(a, s);
     } else {

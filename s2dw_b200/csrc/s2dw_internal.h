@@ -260,6 +260,39 @@ struct CztArgs {
     double scale;          // (4 pi^2/N)/(2bl-1) for CZT_SYN_ALPHA
 };
 
+// One transform stage of several scales (and maps) in one launch: scale e.g.
+// of a group has the CTAs from cta0 on.  Values of map k start k * in_map
+// (out_map) values after the first's.
+struct StageEnt {
+    int cta0;
+    short kind;            // CztMode, or STAGE_PFA: prime-factor alpha
+    short lg;              // log2 of the transform length (not STAGE_PFA)
+    int bl, rows, rows_map;  // rows: of all maps; rows_map: of one
+    int out_stride;        // row stride of V2f (synthesis beta)
+    const double2 *pre, *post, *Hf;
+    const void *in;
+    void *out;
+    const double *wq;      // quadrature weights (2bl), synthesis beta
+    double scale;          // (4 pi^2/N)/(2bl-1), synthesis alpha
+    long long in_map, out_map;
+};
+constexpr int STAGE_PFA = 6;
+constexpr int STAGE_MAX = 24;  // entries per launch
+struct StageArgs {
+    int n, ncta, N, NP;
+    int nq[S2DW_NPMAX];
+    const double2 *tw;     // exp(-2 pi i k / 2048), k < 2048
+    const double2 *ph;     // LwalkArgs::ph
+    StageEnt e[STAGE_MAX];
+};
+enum Stage { STAGE_ANA_BETA, STAGE_ANA_ALPHA, STAGE_SYN_ALPHA, STAGE_SYN_BETA };
+// Fills kind, lg and the CTA count of an entry whose mode, bl and transform
+// length M are given; false where the stage kernels have no transform of that
+// size (it then runs through launch_czt).
+bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta);
+int launch_stage(Stage st, const StageArgs &a, cudaStream_t s);
+int launch_stage_beta(Stage st, const StageArgs &a, cudaStream_t s);
+
 int launch_lwalk(const LwalkArgs &a, cudaStream_t s);
 int launch_gprep(const GprepArgs &a, cudaStream_t s);
 // F[l*Bp + m] = Om[l*Bp + m] * flm[l + B*m] for m <= l < B, zero for m > l, and
@@ -268,14 +301,8 @@ int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *
                  cudaStream_t s);
 int launch_mwalk(const MwalkArgs &a, cudaStream_t s);
 int launch_czt(const CztArgs &a, cudaStream_t s);
-void set_fft_values(int v);  // FFT engine variant: 8 or 16 values per thread, 0 = general engine only
-void set_large_2048(bool on);  // M = 2048 transforms on the one-row-per-CTA engines (default on)
-void set_pfa(bool on);  // prime-factor alpha stages at bl = 2048 and 1024 (default on)
-void set_pfa2047_threads(int n);  // threads per CTA of the length-2047 kernel (128 or 256)
-void set_pfa1023(bool on);         // prime-factor alpha stages at bl = 512
-void set_pfa511(bool on);          // prime-factor alpha stages at bl = 256
-void set_pfa_small(bool on);       // prime-factor alpha stages at bl = 2, 4, 8, 16, 32, 128
-// Builds, once per device, the constant table of the length-2047 alpha stages
+void set_pfa(bool on);  // prime-factor alpha stages (default on; off: Bluestein)
+// Builds, once per device, the constant tables of the length-2047 and -511 alpha stages
 // (the current device; synchronises).  Plan creation calls it, never a capture.
 int pfa_prepare();
 void set_alpha_prefetch(bool on);  // synthesis alpha / analysis beta stages: persistent kernel with prefetched input (default on)

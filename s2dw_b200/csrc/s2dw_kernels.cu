@@ -2,9 +2,10 @@
 //
 //  * fprep_kernel  : the analysis input scaled and transposed for the
 //                    contraction (s2dw_contract.cu)
-//  * czt_kernel    : chirp-z (Bluestein) transforms in shared memory that
-//                    replace the naive beta sums (:708-743, :1157-1198) and
-//                    the FFTW alpha transforms (:746-768, :1104-1130).
+//  * fft_large / fft_pf : FFTs of 2048 to 8192 points of the large scales'
+//                    beta and (Bluestein) alpha stages (:708-768, :1104-1198)
+//  * pfa*          : prime-factor alpha stages of the power-of-two band limits
+//  * alpha_kernel  : alpha stages of a group of scales of up to 512
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -13,21 +14,11 @@
 #include <cstdio>
 #include <type_traits>
 
+#include "s2dw_fft.cuh"
 #include "s2dw_internal.h"
 
 namespace s2dw {
 
-// ---------------------------------------------------------------------------
-// Complex helpers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b)
-{
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-__device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 // Per-scale factor tables of the split form (built once per set of kernel
 // tables).
 __global__ void gprep_kernel(GprepArgs a)
@@ -73,481 +64,12 @@ __global__ void fprep_kernel(double2 *F, double2 *scoeff, const double2 *flm, co
 // Chirp-z transform engine: power-of-two FFTs in shared memory
 // ===========================================================================
 
-// exp(SIGN * 2 pi i k / 16) for k in [0, 8)
-template <int SIGN>
-__device__ __forceinline__ double2 w16(int k)
-{
-    const double C[8] = {1.0, 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173,
-                         0.0, -0.38268343236508977173, -0.70710678118654752440, -0.92387953251128675613};
-    const double Sn[8] = {0.0, 0.38268343236508977173, 0.70710678118654752440, 0.92387953251128675613,
-                          1.0, 0.92387953251128675613, 0.70710678118654752440, 0.38268343236508977173};
-    return make_double2(C[k], SIGN * Sn[k]);
-}
-
-// In-register DFT of size R (R = 1, 2, 4, 8, 16), radix-2 decimation in time.
-template <int R, int SIGN>
-struct Dft {
-    __device__ __forceinline__ static void run(double2 *v)
-    {
-        double2 ev[R / 2], od[R / 2];
-#pragma unroll
-        for (int i = 0; i < R / 2; i++) {
-            ev[i] = v[2 * i];
-            od[i] = v[2 * i + 1];
-        }
-        Dft<R / 2, SIGN>::run(ev);
-        Dft<R / 2, SIGN>::run(od);
-#pragma unroll
-        for (int k = 0; k < R / 2; k++) {
-            double2 t;
-            if (k == 0) t = od[k];
-            else if (4 * k == R) t = (SIGN < 0) ? make_double2(od[k].y, -od[k].x) : make_double2(-od[k].y, od[k].x);
-            else t = cmul(od[k], w16<SIGN>(k * (16 / R)));
-            v[k] = cadd(ev[k], t);
-            v[k + R / 2] = csub(ev[k], t);
-        }
-    }
-};
-template <int SIGN>
-struct Dft<1, SIGN> {
-    __device__ __forceinline__ static void run(double2 *) {}
-};
-
 __host__ __device__ __forceinline__ int padix(int i) { return i + (i >> 4); }
 
 // W_M^x (forward) from the two-level tables.
 __device__ __forceinline__ double2 twid(const double2 *twh, const double2 *twl, int x)
 {
     return cmul(twh[x >> 6], twl[x & 63]);
-}
-
-// Stockham passes with the data of each pass in registers.  A CTA of T
-// threads holds E = V*T complex values (V per thread): E/M transforms of size
-// M (a power of two).  In a pass of radix R (R <= V) each thread owns V/R
-// butterflies; butterfly (t,u) reads positions r*M + j + s*(M/R) and, after
-// twiddles exp(SIGN 2 pi i (j mod Ns) s/(Ns R)) and a radix-R DFT, writes
-// r*M + (j/Ns)*Ns*R + j%Ns + s*Ns.  The last pass (Ns = M/R) therefore writes
-// exactly the positions the first pass of the same radix reads, so a forward
-// FFT followed by an inverse FFT whose radices run in reverse order keeps the
-// data in registers across the boundary.
-template <int V, int R>
-__device__ __forceinline__ int in_pos(int t, int u, int s, int lgM)
-{
-    constexpr int NB = V / R, LR = (R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : 4);
-    const int b = t * NB + u, lper = lgM - LR, r = b >> lper, j = b & ((1 << lper) - 1);
-    return (r << lgM) + j + (s << lper);
-}
-
-template <int V, int R, int SIGN>
-__device__ __forceinline__ void bfly(double2 (&v)[V], int t, int lgM, int lNs, const double2 *twh,
-                                     const double2 *twl)
-{
-    constexpr int NB = V / R, LR = (R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : 4);
-#pragma unroll
-    for (int u = 0; u < NB; u++) {
-        if (lNs > 0) {
-            const int b = t * NB + u, j = b & ((1 << (lgM - LR)) - 1), k = j & ((1 << lNs) - 1);
-            const int step = k << (lgM - lNs - LR);
-#pragma unroll
-            for (int s = 1; s < R; s++) {
-                double2 w = twid(twh, twl, step * s);
-                if (SIGN > 0) w = cconj(w);
-                v[u * R + s] = cmul(v[u * R + s], w);
-            }
-        }
-        Dft<R, SIGN>::run(&v[u * R]);
-    }
-}
-
-template <int V, int R>
-__device__ __forceinline__ void store_pass(const double2 (&v)[V], double2 *buf, int t, int lgM, int lNs)
-{
-    constexpr int NB = V / R, LR = (R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : 4);
-#pragma unroll
-    for (int u = 0; u < NB; u++) {
-        const int b = t * NB + u, lper = lgM - LR, r = b >> lper, j = b & ((1 << lper) - 1);
-        const int idx = (r << lgM) + ((j >> lNs) << (lNs + LR)) + (j & ((1 << lNs) - 1));
-#pragma unroll
-        for (int s = 0; s < R; s++) buf[padix(idx + (s << lNs))] = v[u * R + s];
-    }
-}
-
-template <int V, int R>
-__device__ __forceinline__ void load_pass(double2 (&v)[V], const double2 *buf, int t, int lgM)
-{
-    constexpr int NB = V / R;
-#pragma unroll
-    for (int u = 0; u < NB; u++)
-#pragma unroll
-        for (int s = 0; s < R; s++) v[u * R + s] = buf[padix(in_pos<V, R>(t, u, s, lgM))];
-}
-
-// Radix plans for M = 2^k: forward [V,...,V,2^(k mod log2 V)], inverse in
-// reverse order.  The radix of pass p is computed, not stored, so that no
-// plan array is indexed dynamically.
-struct RadixPlan {
-    int np, nv, rem;
-    bool rev;
-    __device__ __forceinline__ int r(int p) const
-    {
-        if (rev) return (rem && p == 0) ? (1 << rem) : nv_radix;
-        return (p < nv) ? nv_radix : (1 << rem);
-    }
-    int nv_radix;
-};
-template <int V>
-__device__ __forceinline__ RadixPlan radix_plan(int lgM, bool reversed)
-{
-    constexpr int LV = (V == 8 ? 3 : 4);
-    RadixPlan p;
-    p.nv = lgM / LV;
-    p.rem = lgM % LV;
-    p.np = p.nv + (p.rem ? 1 : 0);
-    p.rev = reversed;
-    p.nv_radix = V;
-    return p;
-}
-
-template <int V, int SIGN>
-__device__ __forceinline__ void bfly_any(double2 (&v)[V], int R, int t, int lgM, int lNs, const double2 *twh,
-                                         const double2 *twl)
-{
-    if (V == 16 && R == 16) bfly<V, (V >= 16 ? 16 : 2), SIGN>(v, t, lgM, lNs, twh, twl);
-    else if (R == 8) bfly<V, 8, SIGN>(v, t, lgM, lNs, twh, twl);
-    else if (R == 4) bfly<V, 4, SIGN>(v, t, lgM, lNs, twh, twl);
-    else bfly<V, 2, SIGN>(v, t, lgM, lNs, twh, twl);
-}
-template <int V>
-__device__ __forceinline__ void store_any(const double2 (&v)[V], int R, double2 *buf, int t, int lgM, int lNs)
-{
-    if (V == 16 && R == 16) store_pass<V, (V >= 16 ? 16 : 2)>(v, buf, t, lgM, lNs);
-    else if (R == 8) store_pass<V, 8>(v, buf, t, lgM, lNs);
-    else if (R == 4) store_pass<V, 4>(v, buf, t, lgM, lNs);
-    else store_pass<V, 2>(v, buf, t, lgM, lNs);
-}
-template <int V>
-__device__ __forceinline__ void load_any(double2 (&v)[V], int R, const double2 *buf, int t, int lgM)
-{
-    if (V == 16 && R == 16) load_pass<V, (V >= 16 ? 16 : 2)>(v, buf, t, lgM);
-    else if (R == 8) load_pass<V, 8>(v, buf, t, lgM);
-    else if (R == 4) load_pass<V, 4>(v, buf, t, lgM);
-    else load_pass<V, 2>(v, buf, t, lgM);
-}
-
-template <int V, int SIGN>
-__device__ __forceinline__ void fft_run(double2 (&v)[V], double2 *buf, int t, int lgM, const RadixPlan &P,
-                                        const double2 *twh, const double2 *twl)
-{
-    int lNs = 0;
-    for (int p = 0; p < P.np; p++) {
-        const int R = P.r(p), LR = 31 - __clz(R);
-        bfly_any<V, SIGN>(v, R, t, lgM, lNs, twh, twl);
-        if (p + 1 < P.np) {
-            store_any<V>(v, R, buf, t, lgM, lNs);
-            __syncthreads();
-            load_any<V>(v, P.r(p + 1), buf, t, lgM);
-            __syncthreads();
-        }
-        lNs += LR;
-    }
-}
-
-// Position (within the CTA buffer) of value i = u*R + s a thread holds for a
-// pass of radix R.
-template <int V>
-__device__ __forceinline__ int pos_of(int i, int R, int t, int lgM)
-{
-    const int LR = 31 - __clz(R), u = i >> LR, s = i & (R - 1);
-    const int b = t * (V / R) + u, lper = lgM - LR, r = b >> lper, j = b & ((1 << lper) - 1);
-    return (r << lgM) + j + (s << lper);
-}
-
-// 32-byte accesses of the alpha stages (the two b columns of a b pair at
-// one (g, m)): one 256-bit access instead of two 128-bit ones halves the
-// L1 wavefronts of these row-strided loads and stores.  The streamed input
-// is not kept in L1, which holds the chirp tables.
-__device__ __forceinline__ void ld_pair(const double2 *p, double2 &a, double2 &b)
-{
-    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
-        : "l"(p));
-}
-__device__ __forceinline__ void st_pair(double2 *p, double2 a, double2 b)
-{
-    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y)
-                 : "memory");
-}
-
-// Filter spectrum entry k of a Bluestein transform.  The alpha stages' filter
-// h(d) = conj(chirp(d)) is even in d (no offsets), so its spectrum is even:
-// Hf[k] = Hf[M - k]; reading only k <= M/2 halves the table's cache
-// footprint (32 KB instead of 64 KB at M = 4096).
-template <int MODE>
-__device__ __forceinline__ double2 hf_at(const double2 *Hf, int k, int M)
-{
-    if (MODE == CZT_ANA_ALPHA || MODE == CZT_SYN_ALPHA) return Hf[k <= (M >> 1) ? k : M - k];
-    return Hf[k];
-}
-
-// ---- beta transforms as FFTs of length L = 2 bl (Makhoul's algorithm) ----
-// Analysis (s2dw_core_mod.f90:708-743), one row X(p), p < bl:
-//   cos rows (m+N-1 even): Y(b) = sum_p c_p X(p) cos(p beta_b), c_0 = 1, c_p = 2,
-//   sin rows (m+N-1 odd):  Y(b) = X(0) + sum_{p>=1} 2i X(p) sin(p beta_b),
-// beta_b = pi (2b+1)/(2L), b < L.  The cos sum is a DCT-III of length L:
-//   V_0 = X(0), V_k = e_k X(k) (0 < k < bl), V_bl = 0, V_k = conj(e_{L-k}) X(L-k) (k > bl),
-//   v = sum_k V_k e^{+2 pi i k n/L},  Y(2n) = v_n, Y(2n+1) = v_{L-1-n}  (n < bl),
-// e_k = exp(i pi k/(2L)) (the czt.pre table).  The sin sum is the same DCT-III
-// of the reversed input times i(-1)^b, which moves factors -i (k < bl) and +i
-// (k > bl) onto V and i, -i onto the two output halves; its V_0 is 0 and the
-// reference's m' = 0 term X(0) (eta = 1) is added to every output.
-// Synthesis (:1157-1198), one row u_b, b < L, folded over +-m':
-//   cos rows (m+n even): V'(0) = sum_b u_b, V'(m') = 2 sum_b u_b cos(m' beta_b),
-//   sin rows (m+n odd):  V'(m') = -2i sum_b u_b sin(m' beta_b),
-// a DCT-II of length L: permute v_n = u_{2n}, v_{L-1-n} = u_{2n+1} (n < bl),
-// V = sum_n v_n e^{-2 pi i k n/L}, V'(m') = conj(e_m') V_m' +- e_m' V_{L-m'}
-// (+ cos, - sin; the sin rows' input carries (-1)^b).  A sin row's V'(0)
-// multiplies d^l_{0m}(pi/2) d^l_{0n}(pi/2), which is zero for every l when m+n
-// is odd, so it is stored as 0.
-
-// Position b of the beta grid whose value sits at FFT index k in the
-// DCT-II / DCT-III reordering (k < bl: b = 2k; k >= bl: b = 2L-1-2k).
-__device__ __forceinline__ int beta_src(int k, int bl) { return k < bl ? 2 * k : 4 * bl - 1 - 2 * k; }
-
-// DCT-III input V_k of the analysis beta transform of row X (bl values).
-__device__ __forceinline__ double2 ana_beta_in(const double2 *X, int k, int bl, bool sn, const double2 *e)
-{
-    if (k == 0) return sn ? make_double2(0.0, 0.0) : X[0];
-    if (k < bl) {
-        const double2 x = cmul(X[k], e[k]);
-        return sn ? make_double2(x.y, -x.x) : x;  // -i x
-    }
-    if (k == bl) return make_double2(0.0, 0.0);
-    const int p = 2 * bl - k;
-    const double2 x = cmul(X[p], cconj(e[p]));
-    return sn ? make_double2(-x.y, x.x) : x;  // i x
-}
-
-// Output of the analysis beta transform held at FFT index j: its b, and the
-// value (the sin rows' factor i or -i and the m' = 0 term x0 applied).
-__device__ __forceinline__ double2 ana_beta_out(double2 y, int j, int bl, bool sn, double2 x0, int *b)
-{
-    if (j < bl) {
-        *b = 2 * j;
-        if (sn) y = make_double2(-y.y + x0.x, y.x + x0.y);  // i y + x0
-    } else {
-        *b = 4 * bl - 1 - 2 * j;
-        if (sn) y = make_double2(y.y + x0.x, -y.x + x0.y);  // -i y + x0
-    }
-    return y;
-}
-
-// Folded synthesis beta output V'(m') from the FFT values at m' and L-m'.
-__device__ __forceinline__ double2 syn_beta_out(double2 vk, double2 vlk, int mpv, bool sn, const double2 *e)
-{
-    if (mpv == 0) return sn ? make_double2(0.0, 0.0) : vk;
-    const double2 y = cmul(vk, cconj(e[mpv])), z = cmul(vlk, e[mpv]);
-    return sn ? csub(y, z) : cadd(y, z);
-}
-
-// Input element k of transform `row` of a MODE transform (pre-chirp or
-// pre-twiddle applied); zero outside the transform's input range.
-template <int MODE>
-__device__ __forceinline__ double2 fft_load(const CztArgs &a, int row, int k, const double2 *ph)
-{
-    const int bl = a.bl, n = 2 * bl - 1, N = a.N;
-    const double2 zero = make_double2(0.0, 0.0);
-    if (MODE == CZT_ANA_ALPHA) {  // row = (g, b pair); Hermitian completion in m
-        if (k >= n) return zero;
-        const int g = row / bl, bp = row % bl;
-        const bool lo = k < bl;
-        const double2 *p = a.in_c + ((size_t)g * bl + (lo ? k : n - k)) * (2 * bl) + 2 * bp;
-        double2 x1, x2;
-        ld_pair(p, x1, x2);
-        const double2 pr = a.czt.pre[k];
-        if (!lo) { x1 = cconj(x1); x2 = cconj(x2); }
-        if (k == 0) { x1.y = 0.0; x2.y = 0.0; }
-        return cmul(make_double2(x1.x - x2.y, x1.y + x2.x), pr);
-    } else if (MODE == CZT_SYN_ALPHA) {  // row = (g, b pair); z = w(:,b1) + i w(:,b2)
-        if (k >= n) return zero;
-        const int g = row / bl, bp = row % bl;
-        const double *p = a.in_r + (size_t)k + (size_t)n * (2 * bp + (size_t)2 * bl * g);
-        return cmul(make_double2(p[0], p[n]), a.czt.pre[k]);
-    } else if (MODE == CZT_ANA_BETA) {  // row = (g, m); k <-> m' = k-(bl-1)
-        if (k >= a.czt.spec.K) return zero;
-        const int g = row / bl, m = row % bl, mpv = k - (bl - 1), ab = mpv < 0 ? -mpv : mpv;
-        double2 x = a.in_c[((size_t)g * bl + m) * bl + ab];
-        if (((m + N - 1) & 1) && mpv < 0) x = make_double2(-x.x, -x.y);
-        return cmul(x, a.czt.pre[k]);
-    } else if (MODE == FFT_ANA_BETA) {  // row = (g, m); DCT-III input V_k, k < L = 2bl
-        const int g = row / bl, m = row % bl;
-        return ana_beta_in(a.in_c + ((size_t)g * bl + m) * bl, k, bl, (m + N - 1) & 1, a.czt.pre);
-    } else if (MODE == FFT_SYN_BETA) {  // row = (q, m); DCT-II input: u at b = beta_src(k), gamma DFT on the fly
-        const int q = row / bl, m = row % bl, b = beta_src(k, bl);
-        double2 u = zero;
-        for (int g = 0; g < N; g++) u = cadd(u, cmul(a.in_c[((size_t)g * bl + m) * (2 * bl) + b], ph[q * N + g]));
-        u = cscale(u, a.wq[b]);
-        return (((m + a.nq[q]) & 1) && (b & 1)) ? make_double2(-u.x, -u.y) : u;
-    } else {  // CZT_SYN_BETA: row = (q, m); k = b; gamma DFT on the fly
-        if (k >= 2 * bl) return zero;
-        const int q = row / bl, m = row % bl;
-        double2 u = zero;
-        for (int g = 0; g < N; g++) u = cadd(u, cmul(a.in_c[((size_t)g * bl + m) * (2 * bl) + k], ph[q * N + g]));
-        u = cscale(u, a.wq[k]);
-        return cmul(u, a.czt.pre[k]);
-    }
-}
-
-template <int V, int THREADS, int MODE>
-__global__ void __launch_bounds__(THREADS, (V * THREADS <= 4096 ? 2 : 1)) fft_kernel(CztArgs a)
-{
-    extern __shared__ double2 smem[];
-    constexpr int E = V * THREADS;
-    constexpr bool CHIRP = (MODE != FFT_ANA_BETA && MODE != FFT_SYN_BETA);
-    constexpr bool SYNB = (MODE == CZT_SYN_BETA || MODE == FFT_SYN_BETA);
-    const int M = a.czt.M, lgM = 31 - __clz(M), R = E / M;
-    double2 *buf = smem;
-    double2 *twh = smem + padix(E) + 1;
-    const int nhi = (M + 63) / 64;
-    double2 *twl = twh + nhi;
-    double2 *ph = twl + 64;  // [q][g] exp(-i pi n_q g / N) for the synthesis beta modes
-    const int t = threadIdx.x;
-    const int bl = a.bl, n = 2 * bl - 1, N = a.N, Bout = a.czt.spec.Bout;
-    const int row0 = blockIdx.x * R;
-
-    for (int i = t; i < nhi; i += THREADS) twh[i] = a.tw.hi[i];
-    for (int i = t; i < 64; i += THREADS) twl[i] = a.tw.lo[i];
-    if (SYNB)
-        for (int i = t; i < a.NP * N; i += THREADS) {
-            const int q = i / N, g = i % N;
-            double sn, cs;
-            sincospi(-(double)(a.nq[q] * g) / (double)N, &sn, &cs);
-            ph[i] = make_double2(cs, sn);
-        }
-    __syncthreads();
-
-    const RadixPlan Pf = radix_plan<V>(lgM, false), Pi = radix_plan<V>(lgM, true);
-    const int R0 = (MODE == FFT_ANA_BETA) ? Pi.r(0) : Pf.r(0);
-
-    double2 v[V];
-    if (MODE == FFT_SYN_BETA) {
-        // the gamma DFT one sample (row of V) at a time, so that a thread's V
-        // loads of one sample are in flight together (as fft_load, reordered)
-        int src[V];
-#pragma unroll
-        for (int i = 0; i < V; i++) {
-            const int pos = pos_of<V>(i, R0, t, lgM), row = row0 + (pos >> lgM);
-            src[i] = row < a.rows ? (row % bl) * (2 * bl) + beta_src(pos & (M - 1), bl) : -1;
-            v[i] = make_double2(0.0, 0.0);
-        }
-        for (int gg = 0; gg < N; gg++) {
-            const double2 *Vg = a.in_c + (size_t)gg * bl * (2 * bl);
-#pragma unroll
-            for (int i = 0; i < V; i++) {
-                if (src[i] < 0) continue;
-                const int pos = pos_of<V>(i, R0, t, lgM), q = (row0 + (pos >> lgM)) / bl;
-                v[i] = cadd(v[i], cmul(Vg[src[i]], ph[q * N + gg]));
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < V; i++) {
-            if (src[i] < 0) continue;
-            const int pos = pos_of<V>(i, R0, t, lgM), row = row0 + (pos >> lgM), q = row / bl, m = row % bl;
-            const int b = beta_src(pos & (M - 1), bl);
-            const double2 u = cscale(v[i], a.wq[b]);
-            v[i] = (((m + a.nq[q]) & 1) && (b & 1)) ? make_double2(-u.x, -u.y) : u;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < V; i++) {
-            const int pos = pos_of<V>(i, R0, t, lgM), r = pos >> lgM, k = pos & (M - 1), row = row0 + r;
-            v[i] = (row < a.rows) ? fft_load<MODE>(a, row, k, ph) : make_double2(0.0, 0.0);
-        }
-    }
-
-    int RL;  // radix of the last pass run
-    if (MODE == FFT_ANA_BETA) {
-        fft_run<V, +1>(v, buf, t, lgM, Pi, twh, twl);
-        RL = Pi.r(Pi.np - 1);
-    } else if (MODE == FFT_SYN_BETA) {
-        fft_run<V, -1>(v, buf, t, lgM, Pf, twh, twl);
-        RL = Pf.r(Pf.np - 1);
-    } else {
-        fft_run<V, -1>(v, buf, t, lgM, Pf, twh, twl);
-        const int RF = Pf.r(Pf.np - 1);
-#pragma unroll
-        for (int i = 0; i < V; i++) v[i] = cmul(v[i], hf_at<MODE>(a.czt.Hf, pos_of<V>(i, RF, t, lgM) & (M - 1), M));
-        fft_run<V, +1>(v, buf, t, lgM, Pi, twh, twl);
-        RL = Pi.r(Pi.np - 1);
-    }
-
-    // ---- store
-    if (MODE == CZT_ANA_BETA || MODE == FFT_ANA_BETA || MODE == CZT_ANA_ALPHA) {
-#pragma unroll
-        for (int i = 0; i < V; i++) {
-            const int pos = pos_of<V>(i, RL, t, lgM), r = pos >> lgM, b = pos & (M - 1), row = row0 + r;
-            if (row >= a.rows || b >= Bout) continue;
-            if (MODE == FFT_ANA_BETA) {
-                const int g = row / bl, m = row % bl;
-                const bool sn = (m + N - 1) & 1;
-                const double2 *X = a.in_c + ((size_t)g * bl + m) * bl;
-                int bo;
-                const double2 y = ana_beta_out(v[i], b, bl, sn, sn ? X[0] : make_double2(0.0, 0.0), &bo);
-                a.out_c[((size_t)g * bl + m) * (2 * bl) + bo] = y;
-                continue;
-            }
-            const double2 y = CHIRP ? cmul(v[i], a.czt.post[b]) : v[i];
-            if (MODE == CZT_ANA_ALPHA) {
-                const int g = row / bl, bp = row % bl;
-                double *p = a.out_r + (size_t)b + (size_t)n * (2 * bp + (size_t)2 * bl * g);
-                p[0] = y.x;
-                p[n] = y.y;
-            } else {
-                const int g = row / bl, m = row % bl;
-                a.out_c[((size_t)g * bl + m) * (2 * bl) + b] = y;
-            }
-        }
-        return;
-    }
-    // pair stores go through shared memory
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < V; i++) buf[padix(pos_of<V>(i, RL, t, lgM))] = v[i];
-    __syncthreads();
-    if (MODE == CZT_SYN_ALPHA) {
-        for (int i = t; i < R * bl; i += THREADS) {
-            const int r = i / bl, m = i % bl, row = row0 + r;
-            if (row >= a.rows) continue;
-            const int g = row / bl, bp = row % bl;
-            const int mc = (m == 0) ? 0 : n - m;
-            const double2 Z = cmul(buf[padix((r << lgM) + m)], a.czt.post[m]);
-            const double2 Zc = cconj(cmul(buf[padix((r << lgM) + mc)], a.czt.post[mc]));
-            const double2 sm = cadd(Z, Zc), d = csub(Z, Zc);
-            const double hh = 0.5 * a.scale;
-            st_pair(a.out_c + ((size_t)g * bl + m) * (2 * bl) + 2 * bp, make_double2(sm.x * hh, sm.y * hh),
-                    make_double2(d.y * hh, -d.x * hh));
-        }
-        return;
-    }
-    // synthesis beta: V2(m') for m' in (-bl, bl), folded to m' >= 0
-    for (int i = t; i < R * bl; i += THREADS) {
-        const int r = i / bl, mpv = i % bl, row = row0 + r;
-        if (row >= a.rows) continue;
-        const int q = row / bl, m = row % bl;
-        double2 y, z;
-        if (MODE == CZT_SYN_BETA) {
-            const int t0 = bl - 1 + mpv, t1 = bl - 1 - mpv;
-            y = cmul(buf[padix((r << lgM) + t0)], a.czt.post[t0]);
-            z = cmul(buf[padix((r << lgM) + t1)], a.czt.post[t1]);
-            if (mpv > 0) {
-                if ((m + a.nq[q]) & 1) z = make_double2(-z.x, -z.y);
-                y = cadd(y, z);
-            }
-        } else {
-            y = syn_beta_out(buf[padix((r << lgM) + mpv)], buf[padix((r << lgM) + ((M - mpv) & (M - 1)))], mpv,
-                             (m + a.nq[q]) & 1, a.czt.pre);
-        }
-        a.out_c[((size_t)q * bl + m) * a.out_stride + mpv] = y;
-    }
 }
 
 // ===========================================================================
@@ -560,30 +82,6 @@ __global__ void __launch_bounds__(THREADS, (V * THREADS <= 4096 ? 2 : 1)) fft_ke
 // keeps shared-memory traffic to the data exchanges.  The row (g, m) or
 // (g, b pair) comes from the 2-D grid, so no integer division is needed.
 // ===========================================================================
-template <int SIGN>
-__device__ __forceinline__ void twiddle_powers16(double2 (&v)[16], double2 w)
-{
-    if (SIGN > 0) w = cconj(w);
-    const double2 w2 = cmul(w, w), w4 = cmul(w2, w2), w8 = cmul(w4, w4);
-    const double2 w3 = cmul(w2, w), w5 = cmul(w4, w), w6 = cmul(w4, w2), w7 = cmul(w4, w3);
-    v[1] = cmul(v[1], w);
-    v[2] = cmul(v[2], w2);
-    v[3] = cmul(v[3], w3);
-    v[4] = cmul(v[4], w4);
-    v[5] = cmul(v[5], w5);
-    v[6] = cmul(v[6], w6);
-    v[7] = cmul(v[7], w7);
-    v[8] = cmul(v[8], w8);
-    v[9] = cmul(v[9], cmul(w8, w));
-    v[10] = cmul(v[10], cmul(w8, w2));
-    v[11] = cmul(v[11], cmul(w8, w3));
-    v[12] = cmul(v[12], cmul(w8, w4));
-    v[13] = cmul(v[13], cmul(w8, w5));
-    v[14] = cmul(v[14], cmul(w8, w6));
-    v[15] = cmul(v[15], cmul(w8, w7));
-}
-
-// One radix-16 pass (16 values per thread, thread t = butterfly j).
 template <int LGM, int LNS, int SIGN>
 __device__ __forceinline__ void pass16(double2 (&v)[16], int t, const double2 *twh, const double2 *twl)
 {
@@ -1078,79 +576,6 @@ __device__ __forceinline__ void pfa_load(const CztArgs &a, double2 *X, Pos pos)
 
 constexpr int PFA_N = 4095, PFA_THREADS = 256;
 
-// cos(2 pi j / R) and sin(2 pi j / R), j < R (local constant tables: with j
-// known after unrolling they fold into immediates)
-template <int R>
-__device__ __forceinline__ void pfa_cs(int j, double &c, double &s);
-template <>
-__device__ __forceinline__ void pfa_cs<5>(int j, double &c, double &s)
-{
-    constexpr double C[5] = {1.0, 0.309016994374947424102, -0.809016994374947424102, -0.809016994374947424102, 0.309016994374947424102};
-    constexpr double S[5] = {0.0, 0.951056516295153572116, 0.587785252292473129169, -0.587785252292473129169, -0.951056516295153572116};
-    c = C[j];
-    s = S[j];
-}
-template <>
-__device__ __forceinline__ void pfa_cs<7>(int j, double &c, double &s)
-{
-    constexpr double C[7] = {1.0, 0.623489801858733530525, -0.222520933956314404289, -0.900968867902419126236, -0.900968867902419126236, -0.222520933956314404289, 0.623489801858733530525};
-    constexpr double S[7] = {0.0, 0.781831482468029808708, 0.974927912181823607018, 0.433883739117558120476, -0.433883739117558120476, -0.974927912181823607018, -0.781831482468029808708};
-    c = C[j];
-    s = S[j];
-}
-template <>
-__device__ __forceinline__ void pfa_cs<9>(int j, double &c, double &s)
-{
-    constexpr double C[9] = {1.0, 0.766044443118978035202, 0.173648177666930348852, -0.5, -0.939692620785908384054, -0.939692620785908384054, -0.5, 0.173648177666930348852, 0.766044443118978035202};
-    constexpr double S[9] = {0.0, 0.642787609686539326323, 0.984807753012208059367, 0.866025403784438646764, 0.342020143325668733044, -0.342020143325668733044, -0.866025403784438646764, -0.984807753012208059367, -0.642787609686539326323};
-    c = C[j];
-    s = S[j];
-}
-template <>
-__device__ __forceinline__ void pfa_cs<13>(int j, double &c, double &s)
-{
-    constexpr double C[13] = {1.0, 0.885456025653209895900, 0.568064746731155802512, 0.120536680255323053349, -0.354604887042535625970, -0.748510748171101098635, -0.970941817426052027157, -0.970941817426052027157, -0.748510748171101098635, -0.354604887042535625970, 0.120536680255323053349, 0.568064746731155802512, 0.885456025653209895900};
-    constexpr double S[13] = {0.0, 0.464723172043768545656, 0.822983865893656394580, 0.992708874098053992801, 0.935016242685414823440, 0.663122658240795202377, 0.239315664287557767149, -0.239315664287557767149, -0.663122658240795202377, -0.935016242685414823440, -0.992708874098053992801, -0.822983865893656394580, -0.464723172043768545656};
-    c = C[j];
-    s = S[j];
-}
-
-// In-place DFT of length R (odd) with exp(SIGN 2 pi i k m / R):
-// y_m = x_0 + sum_k (x_k + x_{R-k}) cos + SIGN i sum_k (x_k - x_{R-k}) sin.
-template <int R, int SIGN>
-__device__ __forceinline__ void pfa_dft(double2 (&x)[R])
-{
-    constexpr int H = (R - 1) / 2;
-    double2 ap[H], am[H];
-    double2 y0 = x[0];
-#pragma unroll
-    for (int k = 1; k <= H; k++) {
-        ap[k - 1] = cadd(x[k], x[R - k]);
-        am[k - 1] = csub(x[k], x[R - k]);
-        y0 = cadd(y0, ap[k - 1]);
-    }
-    const double2 x0 = x[0];
-    x[0] = y0;
-#pragma unroll
-    for (int m = 1; m <= H; m++) {
-        double2 P = x0, Q = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int k = 1; k <= H; k++) {
-            double c, sn;
-            pfa_cs<R>((k * m) % R, c, sn);
-            P.x = fma(ap[k - 1].x, c, P.x);
-            P.y = fma(ap[k - 1].y, c, P.y);
-            Q.x = fma(am[k - 1].x, sn, Q.x);
-            Q.y = fma(am[k - 1].y, sn, Q.y);
-        }
-        // SIGN i Q
-        const double2 iq = SIGN > 0 ? make_double2(-Q.y, Q.x) : make_double2(Q.y, -Q.x);
-        x[m] = cadd(P, iq);
-        x[R - m] = csub(P, iq);
-    }
-}
-
-// DFTs of length R along the dimension of stride S of the 4-D layout.
 template <int R, int S, int SIGN>
 __device__ __forceinline__ void pfa_stage(double2 *sm, int t)
 {
@@ -1207,76 +632,6 @@ __global__ void __launch_bounds__(PFA_THREADS, 3) pfa_alpha_kernel(CztArgs a)
             st_pair(a.out_c + ((size_t)g * bl + m) * (2 * bl) + 2 * rr, make_double2(sm.x * hh, sm.y * hh),
                     make_double2(d.y * hh, -d.x * hh));
         }
-    }
-}
-
-template <>
-__device__ __forceinline__ void pfa_cs<11>(int j, double &c, double &s)
-{
-    constexpr double C[11] = {
-        1.00000000000000000000, 0.841253532831181168862, 0.415415013001886425529, -0.142314838273285140444,
-        -0.654860733945285064057, -0.959492973614497389890, -0.959492973614497389890, -0.654860733945285064057,
-        -0.142314838273285140444, 0.415415013001886425529, 0.841253532831181168862};
-    constexpr double S[11] = {
-        0.0, 0.540640817455597582108, 0.909631995354518371412, 0.989821441880932732376, 0.755749574354258283774,
-        0.281732556841429697711, -0.281732556841429697711, -0.755749574354258283774, -0.989821441880932732376,
-        -0.909631995354518371412, -0.540640817455597582108};
-    c = C[j];
-    s = S[j];
-}
-template <>
-__device__ __forceinline__ void pfa_cs<23>(int j, double &c, double &s)
-{
-    constexpr double C[23] = {
-        1.00000000000000000000, 0.962917287347799295015, 0.854419404546488552548, 0.682553143218654082875,
-        0.460065037731152126042, 0.203456013052633789878, -0.0682424133646709759212, -0.334879612170986151958,
-        -0.576680322114867141251, -0.775711290704419807041, -0.917211301505453017844, -0.990685946036330752342,
-        -0.990685946036330752342, -0.917211301505453017844, -0.775711290704419807041, -0.576680322114867141251,
-        -0.334879612170986151958, -0.0682424133646709759212, 0.203456013052633789878, 0.460065037731152126042,
-        0.682553143218654082875, 0.854419404546488552548, 0.962917287347799295015};
-    constexpr double S[23] = {
-        0.0, 0.269796771157024271245, 0.519583950035433578133, 0.730835964278124101651, 0.887885218402375234984,
-        0.979084087682322875633, 0.997668769190539198454, 0.942260922118820495618, 0.816969893010442016973,
-        0.631087944326052789367, 0.398401089846241457998, 0.136166649096246590761, -0.136166649096246590761,
-        -0.398401089846241457998, -0.631087944326052789367, -0.816969893010442016973, -0.942260922118820495618,
-        -0.997668769190539198454, -0.979084087682322875633, -0.887885218402375234984, -0.730835964278124101651,
-        -0.519583950035433578133, -0.269796771157024271245};
-    c = C[j];
-    s = S[j];
-}
-
-// In-place-input DFT of length R (odd), outputs written to out[base + m S]:
-// the symmetric pairs overwrite x (x_k <- x_k + x_{R-k}, x_{R-k} <- x_k - x_{R-k}),
-// which keeps the registers of a long DFT (R = 23) to about R complex values.
-template <int R, int SIGN>
-__device__ __forceinline__ void pfa_dft_out(double2 (&x)[R], double2 *out, int base, int S)
-{
-    constexpr int H = (R - 1) / 2;
-    const double2 x0 = x[0];
-    double2 y0 = x0;
-#pragma unroll
-    for (int k = 1; k <= H; k++) {
-        const double2 p = cadd(x[k], x[R - k]), q = csub(x[k], x[R - k]);
-        x[k] = p;
-        x[R - k] = q;
-        y0 = cadd(y0, p);
-    }
-    out[base] = y0;
-#pragma unroll
-    for (int m = 1; m <= H; m++) {
-        double2 P = x0, Q = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int k = 1; k <= H; k++) {
-            double c, sn;
-            pfa_cs<R>((k * m) % R, c, sn);
-            P.x = fma(x[k].x, c, P.x);
-            P.y = fma(x[k].y, c, P.y);
-            Q.x = fma(x[R - k].x, sn, Q.x);
-            Q.y = fma(x[R - k].y, sn, Q.y);
-        }
-        const double2 iq = SIGN > 0 ? make_double2(-Q.y, Q.x) : make_double2(Q.y, -Q.x);
-        out[base + m * S] = cadd(P, iq);
-        out[base + (R - m) * S] = csub(P, iq);
     }
 }
 
@@ -1420,41 +775,145 @@ __global__ void __launch_bounds__(NT, (NT == 128 ? 3 : 2)) pfa2047_alpha_kernel(
     }
 }
 
-template <>
-__device__ __forceinline__ void pfa_cs<3>(int j, double &c, double &s)
+// ---------------------------------------------------------------------------
+// Row pairs of an alpha stage into and out of shared memory: RP pairs (g, rr)
+// of the transform of odd length N = 2 bl - 1, value m of pair r at at(r, m).
+// Consecutive threads take consecutive pairs of one m where the rows are
+// strided (32 bytes per pair: RP pairs are one contiguous piece), consecutive
+// values where they are contiguous.
+// ---------------------------------------------------------------------------
+template <int MODE, int N, int RP, typename At>
+__device__ __forceinline__ void alpha_rows_in(const StageEnt &e, int cta, At at)
 {
-    constexpr double C[3] = {
-        1.00000000000000000000, -0.500000000000000000000, -0.500000000000000000000};
-    constexpr double S[3] = {
-        0.0, 0.866025403784438646764, -0.866025403784438646764};
-    c = C[j];
-    s = S[j];
+    constexpr int BL = (N + 1) / 2, NT = ST_THREADS;
+    const int t = threadIdx.x, row0 = cta * RP, per = e.rows_map;
+    if (MODE == CZT_ANA_ALPHA) {  // rows m < bl; the Hermitian half from the same values
+        constexpr int IT = (RP * BL + NT - 1) / NT, U = IT < 4 ? IT : 4;
+        for (int i0 = t; i0 < RP * BL; i0 += U * NT) {
+            double2 x1[U], x2[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int i = i0 + u * NT, r = i % RP, m = i / RP, row = row0 + r;
+                if (m >= BL || row >= e.rows) continue;
+                const int k = row / per, gr = row - k * per, g = gr / BL, rr = gr - g * BL;
+                ld_pair(static_cast<const double2 *>(e.in) + k * e.in_map + ((size_t)g * BL + m) * (2 * BL) + 2 * rr,
+                        x1[u], x2[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int i = i0 + u * NT, r = i % RP, m = i / RP;
+                if (m >= BL || row0 + r >= e.rows) continue;
+                if (m == 0) { x1[u].y = 0.0; x2[u].y = 0.0; }
+                at(r, m) = make_double2(x1[u].x - x2[u].y, x1[u].y + x2[u].x);
+                if (m > 0) at(r, N - m) = make_double2(x1[u].x + x2[u].y, x2[u].x - x1[u].y);
+            }
+        }
+    } else {  // the two real rows of a pair, z = w(:, b1) + i w(:, b2)
+        constexpr int IT = (RP * N + NT - 1) / NT, U = IT < 4 ? IT : 4;
+        for (int i0 = t; i0 < RP * N; i0 += U * NT) {
+            double z0[U], z1[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int i = i0 + u * NT, r = i / N, m = i - r * N, row = row0 + r;
+                if (i >= RP * N || row >= e.rows) continue;
+                const int k = row / per, gr = row - k * per;
+                const double *p = static_cast<const double *>(e.in) + k * e.in_map + (size_t)(2 * N) * gr + m;
+                z0[u] = __ldg(p);
+                z1[u] = __ldg(p + N);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int i = i0 + u * NT, r = i / N, m = i - r * N;
+                if (i < RP * N && row0 + r < e.rows) at(r, m) = make_double2(z0[u], z1[u]);
+            }
+        }
+    }
 }
-template <>
-__device__ __forceinline__ void pfa_cs<31>(int j, double &c, double &s)
+
+template <int MODE, int N, int RP, typename At>
+__device__ __forceinline__ void alpha_rows_out(const StageEnt &e, int cta, At at)
 {
-    constexpr double C[31] = {
-        1.00000000000000000000, 0.979529941252494493938, 0.918957811620230629127, 0.820763441207276326364,
-        0.688966919075686567801, 0.528964010326962457365, 0.347305252844820285542, 0.151427777504576663657,
-        -0.050649168838712712279, -0.250652532258720539315, -0.440394151557634309516,
-        -0.612105982547662844147, -0.758758122692790901913, -0.874346616144582118827,
-        -0.954139256400048851476, -0.994869323391895146321, -0.994869323391895146321,
-        -0.954139256400048851476, -0.874346616144582118827, -0.758758122692790901913,
-        -0.612105982547662844147, -0.440394151557634309516, -0.250652532258720539315,
-        -0.050649168838712712279, 0.151427777504576663657, 0.347305252844820285542, 0.528964010326962457365,
-        0.688966919075686567801, 0.820763441207276326364, 0.918957811620230629127, 0.979529941252494493938};
-    constexpr double S[31] = {
-        0.0, 0.201298520088660079142, 0.394355855113318580102, 0.571268215094792279157,
-        0.724792787229119958865, 0.848644257494750950464, 0.937752132147080458429, 0.988468324328111399162,
-        0.998716507171052807146, 0.968077118866204305153, 0.897804539570741657137, 0.790775736937698582078,
-        0.651372482722222207454, 0.485301962531081025215, 0.299363122973357954008, 0.101168321987432177786,
-        -0.101168321987432177786, -0.299363122973357954008, -0.485301962531081025215,
-        -0.651372482722222207454, -0.790775736937698582078, -0.897804539570741657137,
-        -0.968077118866204305153, -0.998716507171052807146, -0.988468324328111399162,
-        -0.937752132147080458429, -0.848644257494750950464, -0.724792787229119958865,
-        -0.571268215094792279157, -0.394355855113318580102, -0.201298520088660079142};
-    c = C[j];
-    s = S[j];
+    constexpr int BL = (N + 1) / 2, NT = ST_THREADS;
+    const int t = threadIdx.x, row0 = cta * RP, per = e.rows_map;
+    if (MODE == CZT_ANA_ALPHA) {
+        for (int i = t; i < RP * N; i += NT) {
+            const int r = i / N, m = i - r * N, row = row0 + r;
+            if (row >= e.rows) continue;
+            const int k = row / per, gr = row - k * per;
+            const double2 y = at(r, m);
+            double *p = static_cast<double *>(e.out) + k * e.out_map + (size_t)(2 * N) * gr + m;
+            p[0] = y.x;
+            p[N] = y.y;
+        }
+    } else {
+        const double hh = 0.5 * e.scale;
+        for (int i = t; i < RP * BL; i += NT) {
+            const int r = i % RP, m = i / RP, row = row0 + r;
+            if (row >= e.rows) continue;
+            const int k = row / per, gr = row - k * per, g = gr / BL, rr = gr - g * BL;
+            const double2 Z = at(r, m), Zc = cconj(at(r, m == 0 ? 0 : N - m));
+            const double2 sm = cadd(Z, Zc), d = csub(Z, Zc);
+            st_pair(static_cast<double2 *>(e.out) + k * e.out_map + ((size_t)g * BL + m) * (2 * BL) + 2 * rr,
+                    make_double2(sm.x * hh, sm.y * hh), make_double2(d.y * hh, -d.x * hh));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Prime-factor alpha stages of the small scales: n = 2bl - 1 = R1 R2 R3 with
+// small pairwise coprime factors (bl = 2: 3; 4: 7; 8: 3 * 5; 32: 7 * 9;
+// 128: 3 * 5 * 17; bl = 16 and 64, whose n is prime, are Bluestein transforms), Good-Thomas with direct symmetric-pair DFTs (factors of 1
+// are skipped), RP row pairs per CTA.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr int pfs_inv(int a, int r)
+{
+    int x = 1;
+    while (r > 1 && (a * x) % r != 1) x++;
+    return x;
+}
+// row pairs per CTA: about a thousand values
+__host__ __device__ constexpr int pfs_rows(int n) { return n >= 255 ? 4 : n >= 63 ? 8 : n >= 15 ? 16 : 32; }
+
+template <int N, int R, int S, int RP, int SIGN>
+__device__ __forceinline__ void pfs_stage(double2 *sm, int t)
+{
+    for (int i = t; i < RP * (N / R); i += ST_THREADS) {
+        const int d = i % (N / R), base = (i / (N / R)) * N + (d % S) + (d / S) * (S * R);
+        double2 x[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) x[r] = sm[base + r * S];
+        pfa_dft<R, SIGN>(x);
+#pragma unroll
+        for (int r = 0; r < R; r++) sm[base + r * S] = x[r];
+    }
+}
+
+template <int R1, int R2, int R3, int MODE>
+__device__ __forceinline__ void pfs_rows_run(const StageEnt &e, int cta, double2 *smem)
+{
+    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1;
+    constexpr int N = R1 * R2 * R3, RP = pfs_rows(N);
+    constexpr int U1 = pfs_inv((N / R1) % R1, R1), U2 = pfs_inv((N / R2) % R2, R2), U3 = pfs_inv((N / R3) % R3, R3);
+    const int t = threadIdx.x;
+    alpha_rows_in<MODE, N, RP>(e, cta, [&](int r, int m) -> double2 & {
+        return smem[r * N + (m * U1) % R1 + R1 * ((m * U2) % R2) + R1 * R2 * ((m * U3) % R3)];
+    });
+    __syncthreads();
+    if constexpr (R1 > 1) {
+        pfs_stage<N, R1, 1, RP, SIGN>(smem, t);
+        __syncthreads();
+    }
+    if constexpr (R2 > 1) {
+        pfs_stage<N, R2, R1, RP, SIGN>(smem, t);
+        __syncthreads();
+    }
+    if constexpr (R3 > 1) {
+        pfs_stage<N, R3, R1 * R2, RP, SIGN>(smem, t);
+        __syncthreads();
+    }
+    alpha_rows_out<MODE, N, RP>(e, cta, [&](int r, int k) -> double2 {
+        return smem[r * N + k % R1 + R1 * (k % R2) + R1 * R2 * (k % R3)];
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1472,7 +931,6 @@ constexpr int PFD_N = 511;
 constexpr int PFD_P = 9;               // pitch of d2 in the shared row
 constexpr int PFD_XS = PFD_P * 73;
 constexpr int PFD_SP = 83;             // pitch of a Rader column (positions i + 9 j, i < 8, j < 9)
-constexpr int PFD_THREADS = 128;
 
 __constant__ int c_rader73_src[72] = {
     1, 22, 46, 63, 72, 51, 27, 10, 37, 11, 23, 68, 36, 62, 50, 5, 55, 42, 48, 34, 18, 31, 25, 39, 64, 21, 24, 17,
@@ -1504,19 +962,17 @@ __global__ void rader73_init_kernel()
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(PFD_THREADS) pfa511_alpha_kernel(CztArgs a)
+__device__ __forceinline__ void pfa511_row(const StageEnt &e, int cta, double2 *smem)
 {
-    static_assert(MODE == CZT_ANA_ALPHA || MODE == CZT_SYN_ALPHA, "alpha stages only");
     constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1;
-    constexpr int NT = PFD_THREADS;
-    extern __shared__ double2 smem[];
+    constexpr int NT = ST_THREADS;
     double2 *X = smem;
     double2 *Sc = smem + PFD_XS;
     double2 *X0 = Sc + 7 * PFD_SP;
     const int t = threadIdx.x;
-    const int bl = a.bl, n = PFD_N;  // n = 2 bl - 1
-    const int g = blockIdx.y, rr = blockIdx.x;
-    pfa_load<MODE, NT, PFD_N>(a, X, [](int m) { return (m * 5) % 7 + PFD_P * ((m * 21) % 73); });
+    alpha_rows_in<MODE, PFD_N, 1>(e, cta, [&](int, int m) -> double2 & {
+        return X[(m * 5) % 7 + PFD_P * ((m * 21) % 73)];
+    });
     __syncthreads();
     // length-7 DFTs along d1
     for (int d2 = t; d2 < 73; d2 += NT) {
@@ -1565,24 +1021,7 @@ __global__ void __launch_bounds__(PFD_THREADS) pfa511_alpha_kernel(CztArgs a)
         for (int i = 0; i < 8; i++) X[c1 + PFD_P * c_rader73_dst[i + 8 * j]] = cadd(x0, v[i]);
     }
     __syncthreads();
-    if (MODE == CZT_ANA_ALPHA) {
-        for (int k = t; k < n; k += NT) {
-            const double2 y = X[k % 7 + PFD_P * (k % 73)];
-            double *p = a.out_r + (size_t)k + (size_t)n * (2 * rr + (size_t)2 * bl * g);
-            p[0] = y.x;
-            p[n] = y.y;
-        }
-    } else {
-        const double hh = 0.5 * a.scale;
-        for (int m = t; m < bl; m += NT) {
-            const int mc = m == 0 ? 0 : n - m;
-            const double2 Z = X[m % 7 + PFD_P * (m % 73)];
-            const double2 Zc = cconj(X[mc % 7 + PFD_P * (mc % 73)]);
-            const double2 sm = cadd(Z, Zc), d = csub(Z, Zc);
-            st_pair(a.out_c + ((size_t)g * bl + m) * (2 * bl) + 2 * rr, make_double2(sm.x * hh, sm.y * hh),
-                    make_double2(d.y * hh, -d.x * hh));
-        }
-    }
+    alpha_rows_out<MODE, PFD_N, 1>(e, cta, [&](int, int k) -> double2 { return X[k % 7 + PFD_P * (k % 73)]; });
 }
 
 // ---------------------------------------------------------------------------
@@ -1595,158 +1034,145 @@ __global__ void __launch_bounds__(PFD_THREADS) pfa511_alpha_kernel(CztArgs a)
 // registers to about 31 complex values).  About 45 FP64 operations per point
 // against ~220 for the 2048-point Bluestein convolution.
 // ---------------------------------------------------------------------------
-constexpr int PFC_N = 1023, PFC_THREADS = 128;
+constexpr int PFC_N = 1023;
 
 __device__ __forceinline__ int pfc_in_pos(int n) { return (n * 2) % 3 + 3 * ((n * 9) % 11) + 33 * ((n * 16) % 31); }
 __device__ __forceinline__ int pfc_out_pos(int k) { return k % 3 + 3 * (k % 11) + 33 * (k % 31); }
 
-// in-place DFTs of length R along stride S of the 1023-point layout
-template <int R, int S, int SIGN>
-__device__ __forceinline__ void pfc_stage(double2 *sm, int t)
-{
-    for (int d = t; d < PFC_N / R; d += PFC_THREADS) {
-        const int base = (d % S) + (d / S) * (S * R);
-        double2 x[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) x[r] = sm[base + r * S];
-        pfa_dft<R, SIGN>(x);
-#pragma unroll
-        for (int r = 0; r < R; r++) sm[base + r * S] = x[r];
-    }
-}
-
+// Two row pairs per CTA; the length-31 DFTs run with a column's real and
+// imaginary parts in two lanes, so that 132 lanes work on them with half the
+// registers (one thread per column: 33 of 128 threads per row pair, 168
+// registers, three CTAs per SM).
 template <int MODE>
-__global__ void __launch_bounds__(PFC_THREADS, 3) pfa1023_alpha_kernel(CztArgs a)
+__device__ __forceinline__ void pfa1023_rows(const StageEnt &e, int cta, double2 *smem)
 {
-    static_assert(MODE == CZT_ANA_ALPHA || MODE == CZT_SYN_ALPHA, "alpha stages only");
-    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1;
-    extern __shared__ double2 smem[];
+    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1, RP = 2;
     const int t = threadIdx.x;
-    const int bl = a.bl, n = PFC_N;  // n = 2 bl - 1
-    const int g = blockIdx.y, rr = blockIdx.x;
-    pfa_load<MODE, PFC_THREADS, PFC_N>(a, smem, [](int m) { return pfc_in_pos(m); });
+    alpha_rows_in<MODE, PFC_N, RP>(e, cta, [&](int r, int m) -> double2 & { return smem[r * PFC_N + pfc_in_pos(m)]; });
     __syncthreads();
-    pfc_stage<3, 1, SIGN>(smem, t);
+    pfs_stage<PFC_N, 3, 1, RP, SIGN>(smem, t);
     __syncthreads();
-    pfc_stage<11, 3, SIGN>(smem, t);
+    pfs_stage<PFC_N, 11, 3, RP, SIGN>(smem, t);
     __syncthreads();
     // length-31 DFTs along d3 (stride 33), in registers, back to the same positions
-    for (int d = t; d < 33; d += PFC_THREADS) {
-        double2 x[31];
+    double *sd = reinterpret_cast<double *>(smem) + (t & 1);
+    for (int i = t >> 1; (i & ~15) < RP * 33; i += ST_THREADS / 2) {  // warps whole
+        const bool live = i < RP * 33;
+        const int d = live ? (i / 33) * PFC_N + i % 33 : 0;
+        double x[31];
 #pragma unroll
-        for (int r = 0; r < 31; r++) x[r] = smem[d + 33 * r];
-        pfa_dft_out<31, SIGN>(x, smem, d, 33);
+        for (int r = 0; r < 31; r++) x[r] = sd[2 * (d + 33 * r)];
+        pfa_dft_part<31, SIGN>(x, sd, d, 33, live);
     }
     __syncthreads();
-    if (MODE == CZT_ANA_ALPHA) {
-        for (int k = t; k < n; k += PFC_THREADS) {
-            const double2 y = smem[pfc_out_pos(k)];
-            double *p = a.out_r + (size_t)k + (size_t)n * (2 * rr + (size_t)2 * bl * g);
-            p[0] = y.x;
-            p[n] = y.y;
-        }
-    } else {
-        const double hh = 0.5 * a.scale;
-        for (int m = t; m < bl; m += PFC_THREADS) {
-            const double2 Z = smem[pfc_out_pos(m)];
-            const double2 Zc = cconj(smem[pfc_out_pos(m == 0 ? 0 : n - m)]);
-            const double2 sm = cadd(Z, Zc), d = csub(Z, Zc);
-            st_pair(a.out_c + ((size_t)g * bl + m) * (2 * bl) + 2 * rr, make_double2(sm.x * hh, sm.y * hh),
-                    make_double2(d.y * hh, -d.x * hh));
-        }
-    }
-}
-
-template <>
-__device__ __forceinline__ void pfa_cs<17>(int j, double &c, double &s)
-{
-    constexpr double C[17] = {
-        1.00000000000000000000, 0.932472229404355804573, 0.739008917220659115925, 0.445738355776538267396,
-        0.092268359463301995240, -0.273662990072082863539, -0.602634636379256389179, -0.850217135729614152134,
-        -0.982973099683901778282, -0.982973099683901778282, -0.850217135729614152134, -0.602634636379256389179,
-        -0.273662990072082863539, 0.092268359463301995240, 0.445738355776538267396, 0.739008917220659115925,
-        0.932472229404355804573};
-    constexpr double S[17] = {
-        0.0, 0.361241666187152948745, 0.673695643646557211713, 0.895163291355062322067, 0.995734176295034521871,
-        0.961825643172819070409, 0.798017227280239503333, 0.526432162877355800245, 0.183749517816570331574,
-        -0.183749517816570331574, -0.526432162877355800245, -0.798017227280239503333, -0.961825643172819070409,
-        -0.995734176295034521871, -0.895163291355062322067, -0.673695643646557211713, -0.361241666187152948745};
-    c = C[j];
-    s = S[j];
+    alpha_rows_out<MODE, PFC_N, RP>(e, cta, [&](int r, int k) -> double2 { return smem[r * PFC_N + pfc_out_pos(k)]; });
 }
 
 // ---------------------------------------------------------------------------
-// Prime-factor alpha stages of the small scales: n = 2bl - 1 = R1 R2 R3 with
-// small pairwise coprime factors (bl = 2: 3; 4: 7; 8: 3 * 5; 16: 31; 32: 7 * 9;
-// 128: 3 * 5 * 17), Good-Thomas with direct symmetric-pair DFTs (factors of 1
-// are skipped), one CTA per row pair as the kernels above.
+// Bluestein alpha stages of up to 2048 points (bl <= 512): one row pair per
+// RowFft row
 // ---------------------------------------------------------------------------
-__host__ __device__ constexpr int pfs_inv(int a, int r)
+template <int MODE, int LG, int VMAX>
+__device__ __forceinline__ void czt_alpha(const StageArgs &a, const StageEnt &e, int cta, double2 *smem)
 {
-    int x = 1;
-    while (r > 1 && (a * x) % r != 1) x++;
-    return x;
-}
-
-template <int N, int R, int S>
-__device__ __forceinline__ void pfs_stage(double2 *sm, int t, int nt, int sign)
-{
-    for (int d = t; d < N / R; d += nt) {
-        const int base = (d % S) + (d / S) * (S * R);
-        double2 x[R];
+    using F = RowFft<LG, VMAX>;
+    constexpr int M = F::M, V = F::V, TPR = F::TPR;
+    const int t = threadIdx.x % TPR, r = threadIdx.x / TPR, bl = e.bl, n = 2 * bl - 1;
+    const int row = cta * F::ROWS + r, per = e.rows_map;
+    const bool valid = row < e.rows;
+    const int k = valid ? row / per : 0, gr = valid ? row - k * per : 0, g = gr / bl, rr = gr - g * bl;
+    double2 *buf = smem + r * F::PITCH;
+    double2 v[V];
+    if (MODE == CZT_ANA_ALPHA) {  // Hermitian completion in m
+        const double2 *p = static_cast<const double2 *>(e.in) + k * e.in_map + (size_t)g * bl * (2 * bl) + 2 * rr;
 #pragma unroll
-        for (int r = 0; r < R; r++) x[r] = sm[base + r * S];
-        if (sign > 0) pfa_dft<R, +1>(x);
-        else pfa_dft<R, -1>(x);
-#pragma unroll
-        for (int r = 0; r < R; r++) sm[base + r * S] = x[r];
-    }
-}
-
-constexpr int PFS_THREADS = 64;
-
-template <int R1, int R2, int R3, int MODE>
-__global__ void __launch_bounds__(PFS_THREADS) pfs_alpha_kernel(CztArgs a)
-{
-    static_assert(MODE == CZT_ANA_ALPHA || MODE == CZT_SYN_ALPHA, "alpha stages only");
-    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1;
-    constexpr int N = R1 * R2 * R3, NT = PFS_THREADS;
-    constexpr int U1 = pfs_inv((N / R1) % R1, R1), U2 = pfs_inv((N / R2) % R2, R2), U3 = pfs_inv((N / R3) % R3, R3);
-    extern __shared__ double2 smem[];
-    const int t = threadIdx.x;
-    const int bl = a.bl, n = N;  // n = 2 bl - 1
-    const int g = blockIdx.y, rr = blockIdx.x;
-    pfa_load<MODE, NT, N>(a, smem, [](int m) {
-        return (m * U1) % R1 + R1 * ((m * U2) % R2) + R1 * R2 * ((m * U3) % R3);
-    });
-    __syncthreads();
-    if constexpr (R1 > 1) pfs_stage<N, R1, 1>(smem, t, NT, SIGN);
-    __syncthreads();
-    if constexpr (R2 > 1) {
-        pfs_stage<N, R2, R1>(smem, t, NT, SIGN);
-        __syncthreads();
-    }
-    if constexpr (R3 > 1) {
-        pfs_stage<N, R3, R1 * R2>(smem, t, NT, SIGN);
-        __syncthreads();
-    }
-    auto opos = [](int k) { return k % R1 + R1 * (k % R2) + R1 * R2 * (k % R3); };
-    if (MODE == CZT_ANA_ALPHA) {
-        for (int k = t; k < n; k += NT) {
-            const double2 y = smem[opos(k)];
-            double *p = a.out_r + (size_t)k + (size_t)n * (2 * rr + (size_t)2 * bl * g);
-            p[0] = y.x;
-            p[n] = y.y;
+        for (int i = 0; i < V; i++) {
+            const int m = t + i * TPR;
+            v[i] = make_double2(0.0, 0.0);
+            if (m >= n) continue;
+            const bool lo = m < bl;
+            double2 x1, x2;
+            ld_pair(p + (size_t)(lo ? m : n - m) * (2 * bl), x1, x2);
+            if (!lo) { x1 = cconj(x1); x2 = cconj(x2); }
+            if (m == 0) { x1.y = 0.0; x2.y = 0.0; }
+            v[i] = cmul(make_double2(x1.x - x2.y, x1.y + x2.x), __ldg(e.pre + m));
         }
     } else {
-        const double hh = 0.5 * a.scale;
-        for (int m = t; m < bl; m += NT) {
-            const double2 Z = smem[opos(m)];
-            const double2 Zc = cconj(smem[opos(m == 0 ? 0 : n - m)]);
-            const double2 sm = cadd(Z, Zc), d = csub(Z, Zc);
-            st_pair(a.out_c + ((size_t)g * bl + m) * (2 * bl) + 2 * rr, make_double2(sm.x * hh, sm.y * hh),
-                    make_double2(d.y * hh, -d.x * hh));
+        const double *p = static_cast<const double *>(e.in) + k * e.in_map + (size_t)(2 * n) * gr;
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            const int m = t + i * TPR;
+            v[i] = m < n ? cmul(make_double2(__ldg(p + m), __ldg(p + n + m)), __ldg(e.pre + m)) : make_double2(0.0, 0.0);
         }
+    }
+    F::template run<-1>(v, buf, t, a.tw);
+#pragma unroll
+    for (int i = 0; i < V; i++) v[i] = cmul(v[i], hf_at<MODE>(e.Hf, t + i * TPR, M));
+    F::template run<+1>(v, buf, t, a.tw);
+    if (MODE == CZT_ANA_ALPHA) {
+        if (!valid) return;
+        double *p = static_cast<double *>(e.out) + k * e.out_map + (size_t)(2 * n) * gr;
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            const int b = t + i * TPR;
+            if (b >= n) continue;
+            const double2 y = cmul(v[i], __ldg(e.post + b));
+            p[b] = y.x;
+            p[n + b] = y.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; i++) buf[F::pad(t + i * TPR)] = v[i];
+        F::sync();
+        if (!valid) return;
+        const double hh = 0.5 * e.scale;
+        double2 *p = static_cast<double2 *>(e.out) + k * e.out_map + (size_t)g * bl * (2 * bl) + 2 * rr;
+        for (int m = t; m < bl; m += TPR) {
+            const int mc = m == 0 ? 0 : n - m;
+            const double2 Z = cmul(buf[F::pad(m)], __ldg(e.post + m));
+            const double2 Zc = cconj(cmul(buf[F::pad(mc)], __ldg(e.post + mc)));
+            const double2 sm = cadd(Z, Zc), d = csub(Z, Zc);
+            st_pair(p + (size_t)m * (2 * bl), make_double2(sm.x * hh, sm.y * hh), make_double2(d.y * hh, -d.x * hh));
+        }
+    }
+}
+
+// Alpha stages of the scales of a group, one launch (bl <= 512).  Two kernels:
+// without the 1024- and 2048-point transforms and the length-1023 rows 80
+// registers are enough and six CTAs fit on an SM.
+template <int MODE, bool BIG>
+__global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __grid_constant__ StageArgs a)
+{
+    extern __shared__ __align__(16) double2 smem[];
+    int cta;
+    const StageEnt &e = stage_entry(a, cta);
+    if (e.kind == STAGE_PFA) {
+        switch (e.bl) {
+        case 2: pfs_rows_run<3, 1, 1, MODE>(e, cta, smem); break;
+        case 4: pfs_rows_run<7, 1, 1, MODE>(e, cta, smem); break;
+        case 8: pfs_rows_run<3, 5, 1, MODE>(e, cta, smem); break;
+        case 32: pfs_rows_run<7, 9, 1, MODE>(e, cta, smem); break;
+        case 128: pfs_rows_run<3, 5, 17, MODE>(e, cta, smem); break;
+        case 256: pfa511_row<MODE>(e, cta, smem); break;
+        case 512:
+            if constexpr (BIG) pfa1023_rows<MODE>(e, cta, smem);
+            break;
+        }
+        return;
+    }
+    switch (e.lg) {
+    case 4: czt_alpha<MODE, 4, 8>(a, e, cta, smem); break;
+    case 5: czt_alpha<MODE, 5, 8>(a, e, cta, smem); break;
+    case 6: czt_alpha<MODE, 6, 8>(a, e, cta, smem); break;
+    case 7: czt_alpha<MODE, 7, 8>(a, e, cta, smem); break;
+    case 8: czt_alpha<MODE, 8, 8>(a, e, cta, smem); break;
+    case 9: czt_alpha<MODE, 9, 8>(a, e, cta, smem); break;
+    case 10:
+        if constexpr (BIG) czt_alpha<MODE, 10, 16>(a, e, cta, smem);
+        break;
+    case 11:
+        if constexpr (BIG) czt_alpha<MODE, 11, 16>(a, e, cta, smem);
+        break;
     }
 }
 
@@ -1816,42 +1242,6 @@ int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *
     return S2DWC_OK;
 }
 
-template <int V, int THREADS, int MODE>
-static int launch_fft_t(const CztArgs &a, cudaStream_t s)
-{
-    constexpr int E = V * THREADS;
-    const int M = a.czt.M, R = E / M;
-    const int nhi = (M + 63) / 64;
-    const size_t smem = sizeof(double2) * ((size_t)padix(E) + 1 + nhi + 64 + S2DW_NPMAX * S2DW_NMAX);  // + ph[q][g]
-    static bool attr[64] = {false};
-    int dev = 0;
-    S2DW_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 64 && !attr[dev]) {
-        S2DW_CUDA_TRY(cudaFuncSetAttribute(fft_kernel<V, THREADS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)(sizeof(double2) * ((size_t)padix(E) + 1 + 128 + 64 + S2DW_NPMAX * S2DW_NMAX))));
-        attr[dev] = true;
-    }
-    const int grid = (a.rows + R - 1) / R;
-    if (grid == 0) return S2DWC_OK;
-    fft_kernel<V, THREADS, MODE><<<grid, THREADS, smem, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-template <int V, int THREADS>
-static int launch_fft_mode(const CztArgs &a, cudaStream_t s)
-{
-    switch (a.mode) {
-    case CZT_ANA_BETA: return launch_fft_t<V, THREADS, CZT_ANA_BETA>(a, s);
-    case CZT_ANA_ALPHA: return launch_fft_t<V, THREADS, CZT_ANA_ALPHA>(a, s);
-    case CZT_SYN_ALPHA: return launch_fft_t<V, THREADS, CZT_SYN_ALPHA>(a, s);
-    case CZT_SYN_BETA: return launch_fft_t<V, THREADS, CZT_SYN_BETA>(a, s);
-    case FFT_ANA_BETA: return launch_fft_t<V, THREADS, FFT_ANA_BETA>(a, s);
-    case FFT_SYN_BETA: return launch_fft_t<V, THREADS, FFT_SYN_BETA>(a, s);
-    }
-    return set_error(S2DWC_ERROR_ARG_INVALID, "unknown transform mode %d", a.mode);
-}
-
 template <int MODE, int LGM>
 static int launch_large_t(const CztArgs &a, cudaStream_t s)
 {
@@ -1878,50 +1268,20 @@ template <int LGM>
 static int launch_large(const CztArgs &a, cudaStream_t s)
 {
     switch (a.mode) {
-    case CZT_ANA_BETA: return launch_large_t<CZT_ANA_BETA, LGM>(a, s);
-    case CZT_ANA_ALPHA: return launch_large_t<CZT_ANA_ALPHA, LGM>(a, s);
-    case CZT_SYN_ALPHA: return launch_large_t<CZT_SYN_ALPHA, LGM>(a, s);
-    case CZT_SYN_BETA: return launch_large_t<CZT_SYN_BETA, LGM>(a, s);
     case FFT_ANA_BETA: return launch_large_t<FFT_ANA_BETA, LGM>(a, s);
     case FFT_SYN_BETA: return launch_large_t<FFT_SYN_BETA, LGM>(a, s);
+    default: break;
     }
-    return set_error(S2DWC_ERROR_ARG_INVALID, "unknown transform mode %d", a.mode);
-}
-
-template <int R1, int R2, int R3, int MODE>
-static int launch_pfs(const CztArgs &a, cudaStream_t s)
-{
-    const size_t smem = sizeof(double2) * (R1 * R2 * R3);
-    const dim3 grid(a.bl, a.rows / a.bl);  // (b pair, g)
-    pfs_alpha_kernel<R1, R2, R3, MODE><<<grid, PFS_THREADS, smem, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-template <int R1, int R2, int R3>
-static int launch_pfs_m(const CztArgs &a, cudaStream_t s)
-{
-    return a.mode == CZT_ANA_ALPHA ? launch_pfs<R1, R2, R3, CZT_ANA_ALPHA>(a, s)
-                                   : launch_pfs<R1, R2, R3, CZT_SYN_ALPHA>(a, s);
-}
-
-template <int MODE>
-static int launch_pfa511(const CztArgs &a, cudaStream_t s)
-{
-    const size_t smem = sizeof(double2) * (PFD_XS + 7 * PFD_SP + 7);  // 20 KB: no opt-in needed
-    const dim3 grid(a.bl, a.rows / a.bl);                              // (b pair, g)
-    pfa511_alpha_kernel<MODE><<<grid, PFD_THREADS, smem, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-template <int MODE>
-static int launch_pfa1023(const CztArgs &a, cudaStream_t s)
-{
-    const size_t smem = sizeof(double2) * PFC_N;  // 16 KB: no opt-in needed
-    const dim3 grid(a.bl, a.rows / a.bl);          // (b pair, g)
-    pfa1023_alpha_kernel<MODE><<<grid, PFC_THREADS, smem, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
+    if constexpr (LGM > 11) {  // chirp-z transforms of 2048 points: the stage kernels
+        switch (a.mode) {
+        case CZT_ANA_BETA: return launch_large_t<CZT_ANA_BETA, LGM>(a, s);
+        case CZT_ANA_ALPHA: return launch_large_t<CZT_ANA_ALPHA, LGM>(a, s);
+        case CZT_SYN_ALPHA: return launch_large_t<CZT_SYN_ALPHA, LGM>(a, s);
+        case CZT_SYN_BETA: return launch_large_t<CZT_SYN_BETA, LGM>(a, s);
+        default: break;
+        }
+    }
+    return set_error(S2DWC_ERROR_ARG_INVALID, "transform mode %d of %d points", a.mode, 1 << LGM);
 }
 
 template <int MODE>
@@ -1977,19 +1337,9 @@ int pfa_prepare()
     return S2DWC_OK;
 }
 
-static bool g_pfa = true;  // prime-factor alpha stages at bl = 2048, 1024, 512 and 256
-static bool g_pfa1023 = true;  // bl = 512 (measurement switch)
-static bool g_pfa511 = true;   // bl = 256 (measurement switch)
-static bool g_pfa_small = true;  // bl = 2 .. 128 except 64 (measurement switch)
-void set_pfa_small(bool on) { g_pfa_small = on; }
-void set_pfa1023(bool on) { g_pfa1023 = on; }
-void set_pfa511(bool on) { g_pfa511 = on; }
-static int g_pfa2047_threads = 128;
+static bool g_pfa = true;  // prime-factor alpha stages
 void set_pfa(bool on) { g_pfa = on; }
-void set_pfa2047_threads(int n) { g_pfa2047_threads = n == 256 ? 256 : 128; }
 
-static int g_fft_values = 8;  // values per thread of the general FFT engine (8 or 16)
-static bool g_large_2048 = true;  // M = 2048 transforms on the one-row-per-CTA engines
 static bool g_alpha_prefetch = true;  // contiguous-input stages: persistent kernel with prefetched input
 
 // Persistent launch of the prefetching stages: as many CTAs as fit on the
@@ -2026,75 +1376,92 @@ void set_alpha_prefetch(bool on) { g_alpha_prefetch = on; }
 
 int launch_czt(const CztArgs &a, cudaStream_t s)
 {
-    if (g_pfa && g_pfa_small && (a.mode == CZT_ANA_ALPHA || a.mode == CZT_SYN_ALPHA) && a.rows % a.bl == 0) {
-        switch (a.bl) {
-        case 2: return launch_pfs_m<3, 1, 1>(a, s);
-        case 4: return launch_pfs_m<7, 1, 1>(a, s);
-        case 8: return launch_pfs_m<3, 5, 1>(a, s);
-        case 16: return launch_pfs_m<31, 1, 1>(a, s);
-        case 32: return launch_pfs_m<7, 9, 1>(a, s);
-        case 128: return launch_pfs_m<3, 5, 17>(a, s);
-        default: break;
-        }
-    }
-    if (g_pfa && g_pfa511 && a.bl == 256 && 2 * a.bl - 1 == PFD_N && a.rows % a.bl == 0) {
-        int dev = 0;
-        S2DW_CUDA_TRY(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
-            return set_error(S2DWC_ERROR_NOT_INIT, "the length-511 alpha tables are not built on device %d", dev);
-        if (a.mode == CZT_ANA_ALPHA) return launch_pfa511<CZT_ANA_ALPHA>(a, s);
-        if (a.mode == CZT_SYN_ALPHA) return launch_pfa511<CZT_SYN_ALPHA>(a, s);
-    }
-    if (g_pfa && g_pfa1023 && a.bl == 512 && 2 * a.bl - 1 == PFC_N && a.rows % a.bl == 0) {
-        if (a.mode == CZT_ANA_ALPHA) return launch_pfa1023<CZT_ANA_ALPHA>(a, s);
-        if (a.mode == CZT_SYN_ALPHA) return launch_pfa1023<CZT_SYN_ALPHA>(a, s);
-    }
-    if (g_pfa && a.bl == 2048 && 2 * a.bl - 1 == PFA_N && a.rows % a.bl == 0) {
+    if (a.rows % a.bl) return set_error(S2DWC_ERROR_ARG_INVALID, "transform of %d rows at bl=%d", a.rows, a.bl);
+    if (g_pfa && a.bl == 2048) {
         if (a.mode == CZT_ANA_ALPHA) return launch_pfa<CZT_ANA_ALPHA>(a, s);
         if (a.mode == CZT_SYN_ALPHA) return launch_pfa<CZT_SYN_ALPHA>(a, s);
     }
-    if (g_pfa && a.bl == 1024 && 2 * a.bl - 1 == PFB_N && a.rows % a.bl == 0) {
+    if (g_pfa && a.bl == 1024 && (a.mode == CZT_ANA_ALPHA || a.mode == CZT_SYN_ALPHA)) {
         int dev = 0;
         S2DW_CUDA_TRY(cudaGetDevice(&dev));
         if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
             return set_error(S2DWC_ERROR_NOT_INIT, "the length-2047 alpha tables are not built on device %d", dev);
-        if (g_pfa2047_threads == 128) {
-            if (a.mode == CZT_ANA_ALPHA) return launch_pfa2047<CZT_ANA_ALPHA, 128>(a, s);
-            if (a.mode == CZT_SYN_ALPHA) return launch_pfa2047<CZT_SYN_ALPHA, 128>(a, s);
-        } else {
-            if (a.mode == CZT_ANA_ALPHA) return launch_pfa2047<CZT_ANA_ALPHA, 256>(a, s);
-            if (a.mode == CZT_SYN_ALPHA) return launch_pfa2047<CZT_SYN_ALPHA, 256>(a, s);
-        }
+        return a.mode == CZT_ANA_ALPHA ? launch_pfa2047<CZT_ANA_ALPHA, 128>(a, s)
+                                       : launch_pfa2047<CZT_SYN_ALPHA, 128>(a, s);
     }
+    // Stages whose input row is contiguous: persistent kernel with the next
+    // row prefetched (synthesis alpha 4% faster than one row per CTA at
+    // bl = 1024).  The analysis alpha stage stays one row per CTA: its
+    // row-strided input gathered by cp.async gave no gain over 256-bit loads
+    // (the chirp-table loads from L2, not the input, dominate its remaining
+    // memory stalls).
     const int M = a.czt.M;
-    if (M < 16 || M > 8192 || (M & (M - 1)))
-        return set_error(S2DWC_ERROR_SIZE_INVALID, "transform size %d unsupported", M);
-    if (a.rows % a.bl == 0 && g_fft_values != 0) {
-        // Stages whose input row is contiguous: persistent kernel with the
-        // next row prefetched (synthesis alpha 4% faster than one row per
-        // CTA at bl = 1024).  The analysis alpha stage stays one row per
-        // CTA: its row-strided input gathered by cp.async gave no gain over
-        // 256-bit loads (the chirp-table loads from L2, not the input,
-        // dominate its remaining memory stalls).
-        if (g_alpha_prefetch && a.mode == CZT_SYN_ALPHA && ((uintptr_t)a.in_r & 15) == 0) {
-            if (M == 2048 && g_large_2048) return launch_pf<CZT_SYN_ALPHA, 11>(a, s);
-            if (M == 4096) return launch_pf<CZT_SYN_ALPHA, 12>(a, s);
-            if (M == 8192) return launch_pf<CZT_SYN_ALPHA, 13>(a, s);
-        }
-        if (g_alpha_prefetch && a.mode == FFT_ANA_BETA && ((uintptr_t)a.in_c & 15) == 0) {
-            if (M == 2048 && g_large_2048) return launch_pf<FFT_ANA_BETA, 11>(a, s);
-            if (M == 4096) return launch_pf<FFT_ANA_BETA, 12>(a, s);
-        }
-        if (M == 2048 && g_large_2048) return launch_large<11>(a, s);
-        if (M == 4096) return launch_large<12>(a, s);
-        if (M == 8192) return launch_large<13>(a, s);
+    if (g_alpha_prefetch && a.mode == CZT_SYN_ALPHA && ((uintptr_t)a.in_r & 15) == 0) {
+        if (M == 4096) return launch_pf<CZT_SYN_ALPHA, 12>(a, s);
+        if (M == 8192) return launch_pf<CZT_SYN_ALPHA, 13>(a, s);
     }
-    if (g_fft_values == 16) return M <= 4096 ? launch_fft_mode<16, 256>(a, s) : launch_fft_mode<16, 512>(a, s);
-    return M <= 4096 ? launch_fft_mode<8, 512>(a, s) : launch_fft_mode<8, 1024>(a, s);
+    if (g_alpha_prefetch && a.mode == FFT_ANA_BETA && ((uintptr_t)a.in_c & 15) == 0) {
+        if (M == 2048) return launch_pf<FFT_ANA_BETA, 11>(a, s);
+        if (M == 4096) return launch_pf<FFT_ANA_BETA, 12>(a, s);
+    }
+    if (M == 2048) return launch_large<11>(a, s);
+    if (M == 4096) return launch_large<12>(a, s);
+    if (M == 8192) return launch_large<13>(a, s);
+    return set_error(S2DWC_ERROR_SIZE_INVALID, "transform size %d unsupported", M);
 }
 
-void set_fft_values(int v) { g_fft_values = (v == 16) ? 16 : (v == 0 ? 0 : 8); }
-void set_large_2048(bool on) { g_large_2048 = on; }
+bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta)
+{
+    const bool alpha = mode == CZT_ANA_ALPHA || mode == CZT_SYN_ALPHA;
+    int per = 0;  // rows per CTA
+    if (alpha && g_pfa && bl <= 512 && bl >= 2 && (bl & (bl - 1)) == 0 && bl != 64 && bl != 16) {
+        e->kind = STAGE_PFA;
+        e->lg = 0;
+        per = bl == 512 ? 2 : bl == 256 ? 1 : pfs_rows(2 * bl - 1);
+    } else {
+        // the 2048-point beta transforms of bl = 1024 keep their own kernels
+        if (M < 16 || M > 2048 || (M & (M - 1)) || bl > 512) return false;
+        int lg = 4;
+        while ((1 << lg) < M) lg++;
+        e->kind = (short)mode;
+        e->lg = (short)lg;
+        per = ST_THREADS * row_fft_v(lg, alpha && lg < 10 ? 8 : 16) / M;
+    }
+    *ncta = (rows + per - 1) / per;
+    return true;
+}
+
+int launch_stage(Stage st, const StageArgs &a, cudaStream_t s)
+{
+    if (st == STAGE_ANA_BETA || st == STAGE_SYN_BETA) return launch_stage_beta(st, a, s);
+    if (a.ncta <= 0) return S2DWC_OK;
+    size_t smem = 0;  // of the group's largest row set
+    bool big = false;
+    for (int i = 0; i < a.n; i++) {
+        const StageEnt &e = a.e[i];
+        size_t n;
+        if (e.kind != STAGE_PFA) n = ST_THREADS * row_fft_v(e.lg, e.lg < 10 ? 8 : 16) * 5 / 4 + 32;
+        else if (e.bl == 512) n = 2 * PFC_N;
+        else if (e.bl == 256) {
+            int dev = 0;
+            S2DW_CUDA_TRY(cudaGetDevice(&dev));
+            if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
+                return set_error(S2DWC_ERROR_NOT_INIT, "the length-511 alpha tables are not built on device %d", dev);
+            n = PFD_XS + 7 * PFD_SP + 7;
+        } else n = (size_t)pfs_rows(2 * e.bl - 1) * (2 * e.bl - 1);
+        smem = std::max(smem, n * sizeof(double2));
+        big = big || e.lg >= 10 || (e.kind == STAGE_PFA && e.bl == 512);
+    }
+    if (st == STAGE_ANA_ALPHA) {
+        if (big) alpha_kernel<CZT_ANA_ALPHA, true><<<a.ncta, ST_THREADS, smem, s>>>(a);
+        else alpha_kernel<CZT_ANA_ALPHA, false><<<a.ncta, ST_THREADS, smem, s>>>(a);
+    } else {
+        if (big) alpha_kernel<CZT_SYN_ALPHA, true><<<a.ncta, ST_THREADS, smem, s>>>(a);
+        else alpha_kernel<CZT_SYN_ALPHA, false><<<a.ncta, ST_THREADS, smem, s>>>(a);
+    }
+    S2DW_CUDA_TRY(cudaGetLastError());
+    return S2DWC_OK;
+}
 
 int launch_combine(const CombineArgs &a, cudaStream_t s)
 {

@@ -42,6 +42,7 @@ struct s2dwc_plan {
     std::vector<std::array<CztDev, 6>> czt;
     std::vector<int> ana_beta_mode, syn_beta_mode;
     std::map<int, TwDev> tw;
+    double2 *tw2048 = nullptr;  // StageArgs::tw
     std::vector<double *> wq;  // quadrature weights per scale
     // caller tables folded into per-scale factor tables
     double *kappaA = nullptr, *kappaS = nullptr, *Phi2 = nullptr;
@@ -357,6 +358,14 @@ int plan_build(s2dwc_plan *p)
         p->ana_beta_mode.push_back(fftb ? FFT_ANA_BETA : CZT_ANA_BETA);
         p->syn_beta_mode.push_back(fftb ? FFT_SYN_BETA : CZT_SYN_BETA);
     }
+    {
+        std::vector<double2> t(2048);
+        for (int k = 0; k < 2048; k++) {
+            const long double x = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / 2048.0L;
+            t[k] = make_double2((double)cosl(x), (double)sinl(x));
+        }
+        if ((st = dev_upload(p, &p->tw2048, t))) return st;
+    }
     // kernel-table factors
     if ((st = dev_alloc(p, &p->kappaA, (size_t)(J + 1) * B * p->NP)) ||
         (st = dev_alloc(p, &p->kappaS, (size_t)(J + 1) * B * p->NP)) ||
@@ -565,19 +574,169 @@ MwalkArgs mwalk_args(const s2dwc_plan *p, double2 *flm, const double2 *scoeff)
     return a;
 }
 
-// Runs the analysis: the F table and the contraction of all scales on `s`,
-// then every scale's transforms on its own stream (forked from and joined back
-// to `s`).
+// The transform stages of scale j as CztArgs: the tables and sizes of a stage,
+// with the given input and output (of one map).
+int stage_mode(const s2dwc_plan *p, int j, Stage st)
+{
+    return st == STAGE_ANA_BETA   ? p->ana_beta_mode[j]
+           : st == STAGE_ANA_ALPHA ? CZT_ANA_ALPHA
+           : st == STAGE_SYN_ALPHA ? CZT_SYN_ALPHA
+                                   : p->syn_beta_mode[j];
+}
+
+int stage_rows(const s2dwc_plan *p, int j, Stage st) { return (st == STAGE_SYN_BETA ? p->NP : p->N) * p->bl[j]; }
+
+double syn_alpha_scale(const s2dwc_plan *p, int j)
+{
+    return (4.0 * (M_PI * M_PI) / (double)p->N) / (2.0 * p->bl[j] - 1.0);
+}
+
+int stage_kind(Stage st)
+{
+    return st == STAGE_ANA_BETA   ? S2DWC_KIND_ANA_BETA
+           : st == STAGE_ANA_ALPHA ? S2DWC_KIND_ANA_ALPHA
+           : st == STAGE_SYN_ALPHA ? S2DWC_KIND_SYN_ALPHA
+                                   : S2DWC_KIND_SYN_BETA;
+}
+
+// Whether the stage kernels (s2dw_beta.cu, alpha_kernel) have scale j's transform.
+bool stage_small(const s2dwc_plan *p, int j, Stage st)
+{
+    StageEnt e{};
+    int n = 0;
+    const int mode = stage_mode(p, j, st);
+    return stage_plan(mode, p->bl[j], p->czt[j][mode].M, 1, &e, &n);
+}
+
+// One stage of scales `js` for `maps` maps on stream s, in as few launches as
+// their transforms allow: the large ones one launch each (per map), the rest
+// together.  in(j) and out(j): the first map's input and output of scale j;
+// im(j), om(j): values between maps.
+template <typename In, typename Out, typename Im, typename Om>
+int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In in, Out out, Im im, Om om,
+              cudaStream_t s)
+{
+    int st;
+    StageArgs sa{};
+    sa.N = p->N;
+    sa.NP = p->NP;
+    std::memcpy(sa.nq, p->nq, sizeof(sa.nq));
+    sa.tw = p->tw2048;
+    sa.ph = p->ph;
+    auto flush = [&]() -> int {
+        if (sa.n == 0) return S2DWC_OK;
+        KernelTimer kt(p, stage_kind(stg), s);
+        const int e = launch_stage(stg, sa, s);
+        sa.n = sa.ncta = 0;
+        return e;
+    };
+    for (int j : js) {
+        const int mode = stage_mode(p, j, stg), rows = stage_rows(p, j, stg);
+        const CztDev &c = p->czt[j][mode];
+        if (!stage_small(p, j, stg)) {
+            CztArgs ca{};
+            ca.mode = mode;
+            ca.bl = p->bl[j];
+            ca.N = p->N;
+            ca.NP = p->NP;
+            std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
+            ca.rows = rows;
+            ca.czt = c;
+            if ((st = plan_tw(p, c.M, &ca.tw))) return st;
+            ca.out_stride = p->gs_stride[j];
+            ca.wq = p->wq[j];
+            ca.scale = syn_alpha_scale(p, j);
+            const void *pi = in(j);
+            void *po = out(j);
+            for (int k = 0; k < maps; k++) {
+                const bool rin = stg == STAGE_SYN_ALPHA, rout = stg == STAGE_ANA_ALPHA;
+                if (rin) ca.in_r = static_cast<const double *>(pi) + k * im(j);
+                else ca.in_c = static_cast<const double2 *>(pi) + k * im(j);
+                if (rout) ca.out_r = static_cast<double *>(po) + k * om(j);
+                else ca.out_c = static_cast<double2 *>(po) + k * om(j);
+                KernelTimer kt(p, stage_kind(stg), s);
+                if ((st = launch_czt(ca, s))) return st;
+            }
+            continue;
+        }
+        if (sa.n == STAGE_MAX && (st = flush())) return st;
+        StageEnt &e = sa.e[sa.n];
+        e = StageEnt{};
+        int n = 0;
+        stage_plan(mode, p->bl[j], c.M, rows * maps, &e, &n);
+        e.cta0 = sa.ncta;
+        e.bl = p->bl[j];
+        e.rows = rows * maps;
+        e.rows_map = rows;
+        e.out_stride = p->gs_stride[j];
+        e.pre = c.pre;
+        e.post = c.post;
+        e.Hf = c.Hf;
+        e.in = in(j);
+        e.out = out(j);
+        e.wq = p->wq[j];
+        e.scale = syn_alpha_scale(p, j);
+        e.in_map = im(j);
+        e.out_map = om(j);
+        sa.ncta += n;
+        sa.n++;
+    }
+    return flush();
+}
+
+// The scales as groups, each run on one stream: a scale with a transform of
+// more than 2048 points (or the 2048-point beta of bl = 1024) fills the GPU and
+// is a group of its own, the rest are one.  Without the former there is one
+// group and everything runs on the caller's stream.  `each`: every scale by
+// itself (the host-buffer entry points, whose copies follow each scale).
+std::vector<std::vector<int>> scale_groups(const s2dwc_plan *p, Stage a, Stage b, bool each)
+{
+    std::vector<std::vector<int>> g;
+    std::vector<int> rest;
+    for (int j = 0; j <= p->J; j++) {
+        if (each || !stage_small(p, j, a) || !stage_small(p, j, b)) g.push_back({j});
+        else rest.push_back(j);
+    }
+    if (!rest.empty()) g.push_back(rest);
+    return g;
+}
+
+// Runs f(group, stream) for every group: on `s` if there is one group or in
+// timing mode, else on the streams of the groups' first scales, forked from
+// and joined back to `s`.
+template <typename F>
+int for_groups(s2dwc_plan *p, const std::vector<std::vector<int>> &g, cudaStream_t s, F &&f)
+{
+    int st;
+    if (p->timing || g.size() == 1) {
+        for (const auto &js : g)
+            if ((st = f(js, s))) return st;
+        return S2DWC_OK;
+    }
+    S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
+    for (const auto &js : g) {
+        cudaStream_t sj = p->streams[js[0]];
+        S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_fork, 0));
+        if ((st = f(js, sj))) return st;
+        S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[js[0]], sj));
+    }
+    for (const auto &js : g) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[js[0]], 0));
+    return S2DWC_OK;
+}
+
 // Per-scale hook: enqueued on scale j's stream after (analysis) or before
 // (synthesis) that scale's kernels; the host-buffer entry points use it to
 // overlap each scale's host<->device copy with the other scales' kernels.
 using ScaleHook = std::function<int(int, cudaStream_t)>;
 
-// full_band_serial (host-buffer entry points): the scales of the largest band
-// limit, which hold most of the coefficients, run one after another, the
-// last scale first, so that the first one's device-to-host copy overlaps the
-// next one's kernels instead of all of them finishing together at the end.
-// (Queuing the smaller scales ahead of them measured 2 % slower end to end.)
+constexpr auto one_map = [](int) { return 0LL; };
+
+// Runs the analysis: the F table and the contraction of all scales on `s`,
+// then the beta and alpha stages of the scales' groups.
+// full_band_serial (host-buffer entry points): the scales one by one, those of
+// the last scale's band limit one after another, the last scale first, so that
+// the first one's device-to-host copy overlaps the next one's kernels instead
+// of all of them finishing together at the end.
 int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 *d_flm, cudaStream_t s,
                  const ScaleHook &after = ScaleHook(), bool full_band_serial = false)
 {
@@ -597,104 +756,53 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         KernelTimer kt(p, S2DWC_KIND_LWALK, s);
         if ((st = launch_lwalk(la, s))) return st;
     }
-    S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
     const bool serial = full_band_serial && !p->timing && (int)p->ev_done.size() == p->J + 1;
+    auto groups = scale_groups(p, STAGE_ANA_BETA, STAGE_ANA_ALPHA, (bool)after);
+    if (serial) std::reverse(groups.begin(), groups.end());
     int prev_full = -1;
-    for (int jj = 0; jj <= p->J; jj++) {
-        const int j = serial ? p->J - jj : jj;
-        // per-kernel timing runs every launch on the caller's stream so that
-        // each event pair brackets one kernel running alone
-        cudaStream_t sj = p->timing ? s : p->streams[j];
-        if (!p->timing) S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_fork, 0));
-        const int bl = p->bl[j];
-        const bool full = serial && bl == p->bl[p->J];
+    return for_groups(p, groups, s, [&](const std::vector<int> &js, cudaStream_t sj) -> int {
+        int e;
+        const int j0 = js[0];
+        const bool full = serial && p->bl[j0] == p->bl[p->J];
         if (full && prev_full >= 0) S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_done[prev_full], 0));
-        double2 *Tg = p->wsC + p->offC[j], *Tb = p->wsA + p->offA[j];
-        CztArgs ca{};
-        ca.mode = p->ana_beta_mode[j];
-        ca.bl = bl;
-        ca.N = p->N;
-        ca.NP = p->NP;
-        std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
-        ca.rows = p->N * bl;
-        ca.czt = p->czt[j][ca.mode];
-        if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-        ca.in_c = Tg;
-        ca.out_c = Tb;
-        {
-            KernelTimer kt(p, S2DWC_KIND_ANA_BETA, sj);
-            if ((st = launch_czt(ca, sj))) return st;
-        }
-        ca.mode = CZT_ANA_ALPHA;
-        ca.rows = p->N * bl;  // (g, b pair)
-        ca.czt = p->czt[j][CZT_ANA_ALPHA];
-        if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-        ca.in_c = Tb;
-        ca.out_c = nullptr;
-        ca.out_r = d_wav + p->wav_off[j];
-        {
-            KernelTimer kt(p, S2DWC_KIND_ANA_ALPHA, sj);
-            if ((st = launch_czt(ca, sj))) return st;
-        }
+        auto Tg = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
+        auto Tb = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
+        auto wav = [&](int j) -> double * { return d_wav + p->wav_off[j]; };
+        if ((e = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj))) return e;
+        if ((e = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj))) return e;
         if (full) {
-            S2DW_CUDA_TRY(cudaEventRecord(p->ev_done[j], sj));
-            prev_full = j;
+            S2DW_CUDA_TRY(cudaEventRecord(p->ev_done[j0], sj));
+            prev_full = j0;
         }
-        if (after && (st = after(j, sj))) return st;
-        if (!p->timing) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j], sj));
-    }
-    if (p->timing) return S2DWC_OK;
-    for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[j], 0));
-    return S2DWC_OK;
+        if (after)
+            for (int j : js)
+                if ((e = after(j, sj))) return e;
+        return S2DWC_OK;
+    });
 }
 
-// largest_first: scales queued from the last (largest) down, the order in
-// which the host-buffer entry points bring the coefficients in.
+// Runs the synthesis: the alpha and beta stages of the scales' groups, then
+// the contraction of all scales on `s`.  largest_first: scales queued from the
+// last one down, the order in which the host-buffer entry points bring the
+// coefficients in.
 int run_synthesis(s2dwc_plan *p, double2 *d_flm, const double *d_wav, const double2 *d_scoeff,
                   cudaStream_t s, const ScaleHook &before = ScaleHook(), bool largest_first = false)
 {
     int st;
-    S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
-    for (int jj = 0; jj <= p->J; jj++) {
-        const int j = largest_first ? p->J - jj : jj;
-        cudaStream_t sj = p->timing ? s : p->streams[j];
-        if (!p->timing) S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_fork, 0));
-        if (before && (st = before(j, sj))) return st;
-        const int bl = p->bl[j];
-        double2 *Vw = p->wsA + p->offA[j], *V2f = p->wsC + p->offC[j];
-        CztArgs ca{};
-        ca.mode = CZT_SYN_ALPHA;
-        ca.bl = bl;
-        ca.N = p->N;
-        ca.NP = p->NP;
-        std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
-        ca.rows = p->N * bl;
-        ca.czt = p->czt[j][CZT_SYN_ALPHA];
-        if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-        ca.in_r = d_wav + p->wav_off[j];
-        ca.out_c = Vw;
-        ca.scale = (4.0 * (M_PI * M_PI) / (double)p->N) / (2.0 * bl - 1.0);
-        {
-            KernelTimer kt(p, S2DWC_KIND_SYN_ALPHA, sj);
-            if ((st = launch_czt(ca, sj))) return st;
-        }
-        ca.mode = p->syn_beta_mode[j];
-        ca.rows = p->NP * bl;
-        ca.czt = p->czt[j][ca.mode];
-        if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-        ca.in_c = Vw;
-        ca.in_r = nullptr;
-        ca.out_c = V2f;
-        ca.out_stride = p->gs_stride[j];
-        ca.wq = p->wq[j];
-        {
-            KernelTimer kt(p, S2DWC_KIND_SYN_BETA, sj);
-            if ((st = launch_czt(ca, sj))) return st;
-        }
-        if (!p->timing) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j], sj));
-    }
-    if (!p->timing)
-        for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[j], 0));
+    auto groups = scale_groups(p, STAGE_SYN_ALPHA, STAGE_SYN_BETA, (bool)before);
+    if (largest_first) std::reverse(groups.begin(), groups.end());
+    st = for_groups(p, groups, s, [&](const std::vector<int> &js, cudaStream_t sj) -> int {
+        int e;
+        if (before)
+            for (int j : js)
+                if ((e = before(j, sj))) return e;
+        auto wav = [&](int j) -> const double * { return d_wav + p->wav_off[j]; };
+        auto V = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
+        auto V2f = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
+        if ((e = run_stage(p, STAGE_SYN_ALPHA, js, 1, wav, V, one_map, one_map, sj))) return e;
+        return run_stage(p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj);
+    });
+    if (st) return st;
     MwalkArgs ma = mwalk_args(p, d_flm, d_scoeff);
     {
         KernelTimer kt(p, S2DWC_KIND_MWALK, s);
@@ -732,7 +840,7 @@ SerialLayout serial_layout(const s2dwc_plan *p)
 // scales one after another, so that each scale reuses the same Tg and Tb.
 // Every element a kernel reads here is written earlier in the same call, so
 // `ws` needs no initial contents.
-int run_analysis_serial(const s2dwc_plan *p, unsigned char *ws, double *d_wav, double2 *d_scoeff,
+int run_analysis_serial(s2dwc_plan *p, unsigned char *ws, double *d_wav, double2 *d_scoeff,
                         const double2 *d_flm, cudaStream_t s)
 {
     const SerialLayout L = serial_layout(p);
@@ -751,26 +859,12 @@ int run_analysis_serial(const s2dwc_plan *p, unsigned char *ws, double *d_wav, d
             la.acc_imag = 1;
             if ((st = launch_lwalk(la, s))) return st;
         }
-        CztArgs ca{};
-        ca.mode = p->ana_beta_mode[j];
-        ca.bl = bl;
-        ca.N = p->N;
-        ca.NP = p->NP;
-        std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
-        ca.rows = p->N * bl;
-        ca.czt = p->czt[j][ca.mode];
-        if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-        ca.in_c = Tg;
-        ca.out_c = Tb;
-        if ((st = launch_czt(ca, s))) return st;
-        ca.mode = CZT_ANA_ALPHA;
-        ca.rows = p->N * bl;
-        ca.czt = p->czt[j][CZT_ANA_ALPHA];
-        if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-        ca.in_c = Tb;
-        ca.out_c = nullptr;
-        ca.out_r = d_wav + p->wav_off[j];
-        if ((st = launch_czt(ca, s))) return st;
+        const std::vector<int> js{j};
+        auto tg = [&](int) { return Tg; };
+        auto tb = [&](int) { return Tb; };
+        auto wav = [&](int) { return d_wav + p->wav_off[j]; };
+        if ((st = run_stage(p, STAGE_ANA_BETA, js, 1, tg, tb, one_map, one_map, s))) return st;
+        if ((st = run_stage(p, STAGE_ANA_ALPHA, js, 1, tb, wav, one_map, one_map, s))) return st;
     }
     return S2DWC_OK;
 }
@@ -1002,32 +1096,13 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
                 KernelTimer kt(p, S2DWC_KIND_LWALK, sj);
                 if ((st2 = launch_split(a, sj))) return st2;
             }
+            const std::vector<int> js{j};
             for (int k = 0; k < nk; k++) {
-                CztArgs ca{};
-                ca.mode = p->ana_beta_mode[j];
-                ca.bl = bl;
-                ca.N = p->N;
-                ca.NP = p->NP;
-                std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
-                ca.rows = p->N * bl;
-                ca.czt = p->czt[j][ca.mode];
-                if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-                ca.in_c = p->sp_Tg + p->sp_cap * S.tg_off + (long long)k * p->N * bl * bl;
-                ca.out_c = p->sp_Tb + S.tb_off;
-                {
-                    KernelTimer kt(p, S2DWC_KIND_ANA_BETA, sj);
-                    if ((st2 = launch_czt(ca, sj))) return st2;
-                }
-                ca.mode = CZT_ANA_ALPHA;
-                ca.czt = p->czt[j][CZT_ANA_ALPHA];
-                if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-                ca.in_c = p->sp_Tb + S.tb_off;
-                ca.out_c = nullptr;
-                ca.out_r = d_wav + (g0 + k) * wtot + p->wav_off[j];
-                {
-                    KernelTimer kt(p, S2DWC_KIND_ANA_ALPHA, sj);
-                    if ((st2 = launch_czt(ca, sj))) return st2;
-                }
+                auto Tg = [&](int) { return p->sp_Tg + p->sp_cap * S.tg_off + (long long)k * p->N * bl * bl; };
+                auto Tb = [&](int) { return p->sp_Tb + S.tb_off; };
+                auto wav = [&](int) { return d_wav + (g0 + k) * wtot + p->wav_off[j]; };
+                if ((st2 = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj))) return st2;
+                if ((st2 = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj))) return st2;
             }
             return S2DWC_OK;
         });
@@ -1061,36 +1136,13 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
             int st2;
             const int bl = p->bl[j];
             const auto &S = p->sp[j];
+            const std::vector<int> js{j};
             for (int k = 0; k < nk; k++) {
-                CztArgs ca{};
-                ca.mode = CZT_SYN_ALPHA;
-                ca.bl = bl;
-                ca.N = p->N;
-                ca.NP = p->NP;
-                std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
-                ca.rows = p->N * bl;
-                ca.czt = p->czt[j][CZT_SYN_ALPHA];
-                if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-                ca.in_r = d_wav + (g0 + k) * wtot + p->wav_off[j];
-                ca.out_c = p->sp_Tb + S.tb_off;
-                ca.scale = (4.0 * (M_PI * M_PI) / (double)p->N) / (2.0 * bl - 1.0);
-                {
-                    KernelTimer kt(p, S2DWC_KIND_SYN_ALPHA, sj);
-                    if ((st2 = launch_czt(ca, sj))) return st2;
-                }
-                ca.mode = p->syn_beta_mode[j];
-                ca.rows = p->NP * bl;
-                ca.czt = p->czt[j][ca.mode];
-                if ((st = plan_tw(p, ca.czt.M, &ca.tw))) return st;
-                ca.in_c = p->sp_Tb + S.tb_off;
-                ca.in_r = nullptr;
-                ca.out_c = p->sp_V2f + p->sp_cap * S.v2f_off + k * S.vstride;
-                ca.out_stride = p->gs_stride[j];
-                ca.wq = p->wq[j];
-                {
-                    KernelTimer kt(p, S2DWC_KIND_SYN_BETA, sj);
-                    if ((st2 = launch_czt(ca, sj))) return st2;
-                }
+                auto wav = [&](int) -> const double * { return d_wav + (g0 + k) * wtot + p->wav_off[j]; };
+                auto V = [&](int) { return p->sp_Tb + S.tb_off; };
+                auto V2f = [&](int) { return p->sp_V2f + p->sp_cap * S.v2f_off + k * S.vstride; };
+                if ((st2 = run_stage(p, STAGE_SYN_ALPHA, js, 1, wav, V, one_map, one_map, sj))) return st2;
+                if ((st2 = run_stage(p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj))) return st2;
             }
             if (bl - p->blo[j] - 1 <= 0) return S2DWC_OK;
             VdigArgs va{};
@@ -1228,20 +1280,9 @@ int s2dwc_plan_create(s2dwc_plan **plan, int B, int N, double alpha, int J, int 
     if (device < 0 || device >= ndev)
         return set_error(S2DWC_ERROR_ARG_INVALID, "device %d out of range (%d devices)", device, ndev);
     DeviceGuard dg(device);
-    if (const char *fv = getenv("S2DW_FFT_VALUES")) set_fft_values(atoi(fv));
     {
-        const char *l2 = getenv("S2DW_LARGE_2048");
-        set_large_2048(l2 ? atoi(l2) != 0 : true);
         const char *pf = getenv("S2DW_PFA");
         set_pfa(pf ? atoi(pf) != 0 : true);
-        const char *pt = getenv("S2DW_PFA2047_THREADS");
-        set_pfa2047_threads(pt ? atoi(pt) : 128);
-        const char *p3 = getenv("S2DW_PFA1023");
-        set_pfa1023(p3 ? atoi(p3) != 0 : true);
-        const char *p5 = getenv("S2DW_PFA511");
-        set_pfa511(p5 ? atoi(p5) != 0 : true);
-        const char *ps = getenv("S2DW_PFA_SMALL");
-        set_pfa_small(ps ? atoi(ps) != 0 : true);
     }
     {
         const char *ap = getenv("S2DW_ALPHA_PREFETCH");
@@ -1441,8 +1482,18 @@ int s2dwc_plan_launch_count(const s2dwc_plan *p, int *analysis, int *synthesis)
     if (!p) return set_error(S2DWC_ERROR_ARG_INVALID, "launch_count: null plan");
     // a general Slm runs each contraction twice
     const int g = p->slm_general ? 2 : 1;
-    if (analysis) *analysis = 2 * (p->J + 1) + 1 + g;
-    if (synthesis) *synthesis = 2 * (p->J + 1) + g;
+    auto stages = [&](Stage a, Stage b) {  // run_stage's launches of scale_groups
+        int n = 0;
+        for (const auto &js : scale_groups(p, a, b, false))
+            for (Stage st : {a, b}) {
+                int small = 0;
+                for (int j : js) (stage_small(p, j, st) ? small : n)++;
+                n += (small + STAGE_MAX - 1) / STAGE_MAX;
+            }
+        return n;
+    };
+    if (analysis) *analysis = stages(STAGE_ANA_BETA, STAGE_ANA_ALPHA) + 1 + g;
+    if (synthesis) *synthesis = stages(STAGE_SYN_ALPHA, STAGE_SYN_BETA) + g;
     return S2DWC_OK;
     S2DW_API_CATCH
 }
@@ -1773,7 +1824,8 @@ int s2dwc_plan_analysis_noalloc(const s2dwc_plan *p, double *d_wav, double *d_sc
     void *ws = nullptr;
     int st = noalloc_scratch(p->device, &ws);
     if (st) return st;
-    return run_analysis_serial(p, static_cast<unsigned char *>(ws), d_wav, reinterpret_cast<double2 *>(d_scoeff),
+    // run_stage only writes the plan's timing records, and only with timing on
+    return run_analysis_serial(const_cast<s2dwc_plan *>(p), static_cast<unsigned char *>(ws), d_wav, reinterpret_cast<double2 *>(d_scoeff),
                                reinterpret_cast<const double2 *>(d_flm), (cudaStream_t)stream);
     S2DW_API_CATCH
 }
