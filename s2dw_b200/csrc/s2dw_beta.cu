@@ -28,10 +28,33 @@ __device__ __forceinline__ void ana_beta(const StageArgs &a, const StageEnt &e, 
     const bool sn = (m + N - 1) & 1;
     double2 *buf = smem + r * F::PITCH;
     double2 v[V];
-    if (MODE == FFT_ANA_BETA) {  // DCT-III input, M = 2 bl
-        const double2 x0 = X[0];
+    if (MODE == FFT_ANA_BETA) {
+        // DCT-III input (see s2dw_fft.cuh), M = 2 bl: X(k) e_k at k < bl and
+        // X(k) conj(e_k) at M - k, which its reader takes from shared memory,
+        // so that every X and e is loaded once, all loads of a thread together
+        constexpr int BL = M / 2;
+        double2 xe[V / 2], w[V / 2];
 #pragma unroll
-        for (int i = 0; i < V; i++) v[i] = ana_beta_in(X, t + i * TPR, bl, sn, e.pre);
+        for (int i = 0; i < V / 2; i++) xe[i] = X[t + i * TPR];
+#pragma unroll
+        for (int i = 0; i < V / 2; i++) w[i] = __ldg(e.pre + t + i * TPR);
+        double2 x0 = make_double2(0.0, 0.0);
+        if (sn) x0 = X[0];
+#pragma unroll
+        for (int i = 0; i < V / 2; i++) {
+            const int k = t + i * TPR;
+            const double2 y = cmul(xe[i], w[i]), z = cmul(xe[i], cconj(w[i]));
+            v[i] = sn ? make_double2(y.y, -y.x) : y;  // -i y
+            if (k > 0) buf[F::pad(M - k)] = sn ? make_double2(-z.y, z.x) : z;  // i z
+            else {
+                if (sn) v[i] = make_double2(0.0, 0.0);
+                buf[F::pad(BL)] = make_double2(0.0, 0.0);
+            }
+        }
+        F::sync();
+#pragma unroll
+        for (int i = V / 2; i < V; i++) v[i] = buf[F::pad(t + i * TPR)];
+        F::sync();
         F::template run<+1>(v, buf, t, a.tw);
         // even and odd b from the two halves: through shared memory, so that
         // the stores are contiguous

@@ -255,33 +255,34 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         for (int s = 0; s < S; s++) {
             const int m = mb + s;
             if (mp < bl && m < bl) {
-                double2 Tp[NP], Tm[NP];
+                // gamma DFT of the pair (n, -n): sum cos(n g) + i dif sin(n g)
+                double2 Ts[NP], Td[NP];
 #pragma unroll
                 for (int q = 0; q < NP; q++) {
                     const int n = a.nq[q];
                     const double2 E = cscale(acc[K][0][s][q], sc), O = cscale(acc[K][1][s][q], sc);
-                    const double2 sum = cadd(E, O), dif = csub(E, O);
                     // acc_imag: the b part of S enters the +n terms times -i (i^-1)
                     // and the -n terms times +i
                     if (n == 0) {
-                        Tp[q] = cipow(sum, -m - ai);
-                        Tm[q] = make_double2(0.0, 0.0);
+                        Ts[q] = cipow(cadd(E, O), -m - ai);
+                        Td[q] = make_double2(0.0, 0.0);
                     } else {
-                        Tp[q] = cipow(sum, n - m - ev - ai);
-                        double2 t = cipow(dif, -n - m + ev + ai);
-                        if ((mp + n) & 1) t = make_double2(-t.x, -t.y);
-                        Tm[q] = t;
+                        const double2 tp = cipow(cadd(E, O), n - m - ev - ai);
+                        double2 tm = cipow(csub(E, O), -n - m + ev + ai);
+                        if ((mp + n) & 1) tm = make_double2(-tm.x, -tm.y);
+                        Ts[q] = cadd(tp, tm);
+                        Td[q] = make_double2(tm.y - tp.y, tp.x - tm.x);  // i (tp - tm)
                     }
                 }
                 double2 *dst = a.Tg + a.off[j] + (size_t)m * bl + mp;
-                for (int gg = 0; gg < N; gg++, dst += (size_t)bl * bl) {
-                    const double2 *ph = a.ph + gg * (2 * N - 1) + N - 1;
+                const double2 *ph = a.ph + N - 1;
+                for (int gg = 0; gg < N; gg++, dst += (size_t)bl * bl, ph += 2 * N - 1) {
                     double2 y = make_double2(0.0, 0.0);
 #pragma unroll
                     for (int q = 0; q < NP; q++) {
-                        const int n = a.nq[q];
-                        y = cadd(y, cmul(Tp[q], __ldg(ph + n)));
-                        if (n != 0) y = cadd(y, cmul(Tm[q], __ldg(ph - n)));
+                        const double2 w = __ldg(ph + a.nq[q]);
+                        y.x = fma(Ts[q].x, w.x, fma(Td[q].x, w.y, y.x));
+                        y.y = fma(Ts[q].y, w.x, fma(Td[q].y, w.y, y.y));
                     }
                     *dst = a.acc_imag ? cadd(*dst, y) : y;
                 }

@@ -290,6 +290,9 @@ enum Stage { STAGE_ANA_BETA, STAGE_ANA_ALPHA, STAGE_SYN_ALPHA, STAGE_SYN_BETA };
 // length M are given; false where the stage kernels have no transform of that
 // size (it then runs through launch_czt).
 bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta);
+// The length-1023 alpha rows have a kernel of their own: a launch holds only
+// such entries or none.
+bool stage_alone(const StageEnt &e);
 int launch_stage(Stage st, const StageArgs &a, cudaStream_t s);
 int launch_stage_beta(Stage st, const StageArgs &a, cudaStream_t s);
 

@@ -782,13 +782,13 @@ __global__ void __launch_bounds__(NT, (NT == 128 ? 3 : 2)) pfa2047_alpha_kernel(
 // strided (32 bytes per pair: RP pairs are one contiguous piece), consecutive
 // values where they are contiguous.
 // ---------------------------------------------------------------------------
-template <int MODE, int N, int RP, typename At>
+template <int MODE, int N, int RP, int NT = ST_THREADS, typename At>
 __device__ __forceinline__ void alpha_rows_in(const StageEnt &e, int cta, At at)
 {
-    constexpr int BL = (N + 1) / 2, NT = ST_THREADS;
+    constexpr int BL = (N + 1) / 2;
     const int t = threadIdx.x, row0 = cta * RP, per = e.rows_map;
     if (MODE == CZT_ANA_ALPHA) {  // rows m < bl; the Hermitian half from the same values
-        constexpr int IT = (RP * BL + NT - 1) / NT, U = IT < 4 ? IT : 4;
+        constexpr int IT = (RP * BL + NT - 1) / NT, U = IT < 6 ? IT : 6;  // loads in flight
         for (int i0 = t; i0 < RP * BL; i0 += U * NT) {
             double2 x1[U], x2[U];
 #pragma unroll
@@ -809,7 +809,7 @@ __device__ __forceinline__ void alpha_rows_in(const StageEnt &e, int cta, At at)
             }
         }
     } else {  // the two real rows of a pair, z = w(:, b1) + i w(:, b2)
-        constexpr int IT = (RP * N + NT - 1) / NT, U = IT < 4 ? IT : 4;
+        constexpr int IT = (RP * N + NT - 1) / NT, U = IT < 8 ? IT : 8;
         for (int i0 = t; i0 < RP * N; i0 += U * NT) {
             double z0[U], z1[U];
 #pragma unroll
@@ -830,10 +830,10 @@ __device__ __forceinline__ void alpha_rows_in(const StageEnt &e, int cta, At at)
     }
 }
 
-template <int MODE, int N, int RP, typename At>
+template <int MODE, int N, int RP, int NT = ST_THREADS, typename At>
 __device__ __forceinline__ void alpha_rows_out(const StageEnt &e, int cta, At at)
 {
-    constexpr int BL = (N + 1) / 2, NT = ST_THREADS;
+    constexpr int BL = (N + 1) / 2;
     const int t = threadIdx.x, row0 = cta * RP, per = e.rows_map;
     if (MODE == CZT_ANA_ALPHA) {
         for (int i = t; i < RP * N; i += NT) {
@@ -874,10 +874,10 @@ __host__ __device__ constexpr int pfs_inv(int a, int r)
 // row pairs per CTA: about a thousand values
 __host__ __device__ constexpr int pfs_rows(int n) { return n >= 255 ? 4 : n >= 63 ? 8 : n >= 15 ? 16 : 32; }
 
-template <int N, int R, int S, int RP, int SIGN>
+template <int N, int R, int S, int RP, int SIGN, int NT = ST_THREADS>
 __device__ __forceinline__ void pfs_stage(double2 *sm, int t)
 {
-    for (int i = t; i < RP * (N / R); i += ST_THREADS) {
+    for (int i = t; i < RP * (N / R); i += NT) {
         const int d = i % (N / R), base = (i / (N / R)) * N + (d % S) + (d / S) * (S * R);
         double2 x[R];
 #pragma unroll
@@ -1039,33 +1039,38 @@ constexpr int PFC_N = 1023;
 __device__ __forceinline__ int pfc_in_pos(int n) { return (n * 2) % 3 + 3 * ((n * 9) % 11) + 33 * ((n * 16) % 31); }
 __device__ __forceinline__ int pfc_out_pos(int k) { return k % 3 + 3 * (k % 11) + 33 * (k % 31); }
 
-// Two row pairs per CTA; the length-31 DFTs run with a column's real and
-// imaginary parts in two lanes, so that 132 lanes work on them with half the
-// registers (one thread per column: 33 of 128 threads per row pair, 168
-// registers, three CTAs per SM).
+// A row pair per CTA of 96 threads: 93 length-11 DFTs are one pass, and so are
+// the 33 length-31 DFTs with a column's real and imaginary parts in two lanes
+// (66 lanes; one thread per column took 168 registers and left 95 of 128 threads
+// waiting).
+constexpr int PFC_THREADS = 96;
+
 template <int MODE>
-__device__ __forceinline__ void pfa1023_rows(const StageEnt &e, int cta, double2 *smem)
+__global__ void __launch_bounds__(PFC_THREADS, 6) pfa1023_kernel(const __grid_constant__ StageArgs a)
 {
-    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1, RP = 2;
+    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1, NT = PFC_THREADS;
+    extern __shared__ __align__(16) double2 smem[];
+    int cta;
+    const StageEnt &e = stage_entry(a, cta);
     const int t = threadIdx.x;
-    alpha_rows_in<MODE, PFC_N, RP>(e, cta, [&](int r, int m) -> double2 & { return smem[r * PFC_N + pfc_in_pos(m)]; });
+    alpha_rows_in<MODE, PFC_N, 1, NT>(e, cta, [&](int, int m) -> double2 & { return smem[pfc_in_pos(m)]; });
     __syncthreads();
-    pfs_stage<PFC_N, 3, 1, RP, SIGN>(smem, t);
+    pfs_stage<PFC_N, 3, 1, 1, SIGN, NT>(smem, t);
     __syncthreads();
-    pfs_stage<PFC_N, 11, 3, RP, SIGN>(smem, t);
+    pfs_stage<PFC_N, 11, 3, 1, SIGN, NT>(smem, t);
     __syncthreads();
     // length-31 DFTs along d3 (stride 33), in registers, back to the same positions
-    double *sd = reinterpret_cast<double *>(smem) + (t & 1);
-    for (int i = t >> 1; (i & ~15) < RP * 33; i += ST_THREADS / 2) {  // warps whole
-        const bool live = i < RP * 33;
-        const int d = live ? (i / 33) * PFC_N + i % 33 : 0;
+    {
+        double *sd = reinterpret_cast<double *>(smem) + (t & 1);
+        const bool live = t < 66;
+        const int d = live ? t >> 1 : 0;
         double x[31];
 #pragma unroll
         for (int r = 0; r < 31; r++) x[r] = sd[2 * (d + 33 * r)];
         pfa_dft_part<31, SIGN>(x, sd, d, 33, live);
     }
     __syncthreads();
-    alpha_rows_out<MODE, PFC_N, RP>(e, cta, [&](int r, int k) -> double2 { return smem[r * PFC_N + pfc_out_pos(k)]; });
+    alpha_rows_out<MODE, PFC_N, 1, NT>(e, cta, [&](int, int k) -> double2 { return smem[pfc_out_pos(k)]; });
 }
 
 // ---------------------------------------------------------------------------
@@ -1138,8 +1143,8 @@ __device__ __forceinline__ void czt_alpha(const StageArgs &a, const StageEnt &e,
 }
 
 // Alpha stages of the scales of a group, one launch (bl <= 512).  Two kernels:
-// without the 1024- and 2048-point transforms and the length-1023 rows 80
-// registers are enough and six CTAs fit on an SM.
+// without the 1024- and 2048-point transforms 80 registers are enough and six
+// CTAs fit on an SM.
 template <int MODE, bool BIG>
 __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __grid_constant__ StageArgs a)
 {
@@ -1154,9 +1159,6 @@ __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __
         case 32: pfs_rows_run<7, 9, 1, MODE>(e, cta, smem); break;
         case 128: pfs_rows_run<3, 5, 17, MODE>(e, cta, smem); break;
         case 256: pfa511_row<MODE>(e, cta, smem); break;
-        case 512:
-            if constexpr (BIG) pfa1023_rows<MODE>(e, cta, smem);
-            break;
         }
         return;
     }
@@ -1417,7 +1419,7 @@ bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta)
     if (alpha && g_pfa && bl <= 512 && bl >= 2 && (bl & (bl - 1)) == 0 && bl != 64 && bl != 16) {
         e->kind = STAGE_PFA;
         e->lg = 0;
-        per = bl == 512 ? 2 : bl == 256 ? 1 : pfs_rows(2 * bl - 1);
+        per = bl >= 256 ? 1 : pfs_rows(2 * bl - 1);
     } else {
         // the 2048-point beta transforms of bl = 1024 keep their own kernels
         if (M < 16 || M > 2048 || (M & (M - 1)) || bl > 512) return false;
@@ -1431,26 +1433,36 @@ bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta)
     return true;
 }
 
+bool stage_alone(const StageEnt &e) { return e.kind == STAGE_PFA && e.bl == 512; }
+
 int launch_stage(Stage st, const StageArgs &a, cudaStream_t s)
 {
     if (st == STAGE_ANA_BETA || st == STAGE_SYN_BETA) return launch_stage_beta(st, a, s);
     if (a.ncta <= 0) return S2DWC_OK;
+    if (stage_alone(a.e[0])) {
+        if (st == STAGE_ANA_ALPHA) pfa1023_kernel<CZT_ANA_ALPHA><<<a.ncta, PFC_THREADS, sizeof(double2) * PFC_N, s>>>(a);
+        else pfa1023_kernel<CZT_SYN_ALPHA><<<a.ncta, PFC_THREADS, sizeof(double2) * PFC_N, s>>>(a);
+        S2DW_CUDA_TRY(cudaGetLastError());
+        return S2DWC_OK;
+    }
     size_t smem = 0;  // of the group's largest row set
     bool big = false;
     for (int i = 0; i < a.n; i++) {
         const StageEnt &e = a.e[i];
         size_t n;
-        if (e.kind != STAGE_PFA) n = ST_THREADS * row_fft_v(e.lg, e.lg < 10 ? 8 : 16) * 5 / 4 + 32;
-        else if (e.bl == 512) n = 2 * PFC_N;
-        else if (e.bl == 256) {
+        if (e.kind != STAGE_PFA) {
+            n = ST_THREADS * row_fft_v(e.lg, e.lg < 10 ? 8 : 16) * 5 / 4 + 32;
+        } else if (e.bl == 256) {
             int dev = 0;
             S2DW_CUDA_TRY(cudaGetDevice(&dev));
             if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
                 return set_error(S2DWC_ERROR_NOT_INIT, "the length-511 alpha tables are not built on device %d", dev);
             n = PFD_XS + 7 * PFD_SP + 7;
-        } else n = (size_t)pfs_rows(2 * e.bl - 1) * (2 * e.bl - 1);
+        } else {
+            n = (size_t)pfs_rows(2 * e.bl - 1) * (2 * e.bl - 1);
+        }
         smem = std::max(smem, n * sizeof(double2));
-        big = big || e.lg >= 10 || (e.kind == STAGE_PFA && e.bl == 512);
+        big = big || e.lg >= 10;
     }
     if (st == STAGE_ANA_ALPHA) {
         if (big) alpha_kernel<CZT_ANA_ALPHA, true><<<a.ncta, ST_THREADS, smem, s>>>(a);

@@ -659,13 +659,12 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
             }
             continue;
         }
-        if (sa.n == STAGE_MAX && (st = flush())) return st;
-        StageEnt &e = sa.e[sa.n];
-        e = StageEnt{};
+        StageEnt e{};
         int n = 0;
         stage_plan(mode, p->bl[j], c.M, rows * maps, &e, &n);
-        e.cta0 = sa.ncta;
         e.bl = p->bl[j];
+        if ((sa.n == STAGE_MAX || (sa.n > 0 && stage_alone(sa.e[0]) != stage_alone(e))) && (st = flush())) return st;
+        e.cta0 = sa.ncta;
         e.rows = rows * maps;
         e.rows_map = rows;
         e.out_stride = p->gs_stride[j];
@@ -678,8 +677,8 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
         e.scale = syn_alpha_scale(p, j);
         e.in_map = im(j);
         e.out_map = om(j);
+        sa.e[sa.n++] = e;
         sa.ncta += n;
-        sa.n++;
     }
     return flush();
 }
@@ -1486,9 +1485,16 @@ int s2dwc_plan_launch_count(const s2dwc_plan *p, int *analysis, int *synthesis)
         int n = 0;
         for (const auto &js : scale_groups(p, a, b, false))
             for (Stage st : {a, b}) {
-                int small = 0;
-                for (int j : js) (stage_small(p, j, st) ? small : n)++;
-                n += (small + STAGE_MAX - 1) / STAGE_MAX;
+                int small = 0, alone = 0;
+                for (int j : js) {
+                    StageEnt e{};
+                    e.bl = p->bl[j];
+                    int c = 0;
+                    const int mode = stage_mode(p, j, st);
+                    if (!stage_plan(mode, p->bl[j], p->czt[j][mode].M, 1, &e, &c)) n++;
+                    else (stage_alone(e) ? alone : small)++;
+                }
+                n += (small + STAGE_MAX - 1) / STAGE_MAX + (alone + STAGE_MAX - 1) / STAGE_MAX;
             }
         return n;
     };
