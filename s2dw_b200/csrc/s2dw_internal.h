@@ -231,6 +231,8 @@ struct CombineArgs {
     int B, J, bs;
     int bl[S2DW_JMAX + 1], blo[S2DW_JMAX + 1];
     long long off[S2DW_JMAX + 1];  // offset of part_j in `parts` (complex values)
+    int maps;                      // map k: parts + k*pstride, scoeff + k*bs^2, flm + k*B^2
+    long long pstride;
     const double2 *parts;
     const double2 *scoeff;
     const double *Phi2;
@@ -309,10 +311,8 @@ void set_pfa(bool on);  // prime-factor alpha stages (default on; off: Bluestein
 // (the current device; synchronises).  Plan creation calls it, never a capture.
 int pfa_prepare();
 void set_alpha_prefetch(bool on);  // synthesis alpha / analysis beta stages: persistent kernel with prefetched input (default on)
-int launch_zero(double *p, long long n, cudaStream_t s);
-int launch_scoeff_copy(double2 *scoeff, const double2 *flm, int B, int bs, cudaStream_t s);
-int launch_scaling_add(double2 *flm, const double2 *scoeff, const double *Phi2, int B, int bs,
-                       cudaStream_t s);
+// scoeff (bs x bs) of `maps` maps
+int launch_scoeff_copy(double2 *scoeff, const double2 *flm, int B, int bs, int maps, cudaStream_t s);
 int launch_combine(const CombineArgs &a, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
@@ -396,14 +396,15 @@ int launch_split(const SplitArgs &a, cudaStream_t s);
 // ---------------------------------------------------------------------------
 // Moments of the wavelet coefficients per scale (s2dw_stats.cu)
 // ---------------------------------------------------------------------------
-constexpr int STAT_P = 64;  // blocks per (map, scale) in the reduction passes
+constexpr int STAT_P = 96;  // blocks per (map, scale) in the reduction passes
+constexpr int STAT_W = 8;   // partial sums per block: 2 of pass 1, 6 of pass 2
 struct StatArgs {
     int J, nmaps;
     long long wtot;            // doubles per map in the packed layout
     long long off[S2DW_JMAX + 2];  // scale offsets (J+2 entries)
     const double *wav;         // map k at wav + k*wtot
     const double *mask;        // packed layout of one map, or null
-    double *part;              // nmaps*(J+1)*STAT_P*6 partial sums
+    double *part, *part2;      // nmaps*(J+1)*STAT_P x 2 and x 6 partial sums
     double *mean_nj;           // nmaps*(J+1)*2
     double *out;               // nmaps*(J+1)*6: mean, var, skew, kur, five, six
     int *flags;                // nmaps*(J+1): 1 zero variance, 2 fewer than two samples

@@ -1178,46 +1178,28 @@ __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __
     }
 }
 
-// ===========================================================================
-// Small kernels
-// ===========================================================================
-__global__ void zero_kernel(double *p, long long n)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        p[i] = 0.0;
-}
-
 // scoeff(0:bs-1,0:bs-1) = flm(0:bs-1,0:bs-1), s2dw_core_mod.f90:773
 __global__ void scoeff_copy_kernel(double2 *sc, const double2 *flm, int B, int bs)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < bs * bs) sc[i] = flm[(i % bs) + (size_t)B * (i / bs)];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+    if (i < bs * bs) sc[(size_t)k * bs * bs + i] = flm[(size_t)k * B * B + (i % bs) + (size_t)B * (i / bs)];
 }
 
-// flm(l,0:bs-1) += Phi2(l) scoeff(l,0:bs-1), s2dw_core_mod.f90:1258-1261
-__global__ void scaling_add_kernel(double2 *flm, const double2 *sc, const double *Phi2, int B, int bs)
+__global__ void combine_kernel(const __grid_constant__ CombineArgs a)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < bs * bs) {
-        const int l = i % bs, m = i / bs;
-        double2 *f = flm + l + (size_t)B * m;
-        *f = cadd(*f, cscale(sc[i], Phi2[l]));
-    }
-}
-
-__global__ void combine_kernel(CombineArgs a)
-{
-    const int B = a.B;
+    const int B = a.B, k = blockIdx.y;
+    const double2 *parts = a.parts + k * a.pstride, *scoeff = a.scoeff + (size_t)k * a.bs * a.bs;
+    double2 *flm = a.flm + (size_t)k * B * B;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)B * B;
          i += (long long)gridDim.x * blockDim.x) {
         const int l = (int)(i % B), m = (int)(i / B);
         double2 f = make_double2(0.0, 0.0);
         if (m <= l) {
             for (int j = 0; j <= a.J; j++)
-                if (l > a.blo[j] && l < a.bl[j]) f = cadd(f, a.parts[a.off[j] + (size_t)(l - a.blo[j] - 1) * a.bl[j] + m]);
+                if (l > a.blo[j] && l < a.bl[j]) f = cadd(f, parts[a.off[j] + (size_t)(l - a.blo[j] - 1) * a.bl[j] + m]);
         }
-        if (l < a.bs && m < a.bs) f = cadd(f, cscale(a.scoeff[l + (size_t)a.bs * m], a.Phi2[l]));
-        a.flm[i] = f;
+        if (l < a.bs && m < a.bs) f = cadd(f, cscale(scoeff[l + (size_t)a.bs * m], a.Phi2[l]));
+        flm[i] = f;
     }
 }
 
@@ -1479,36 +1461,16 @@ int launch_combine(const CombineArgs &a, cudaStream_t s)
 {
     long long n = (long long)a.B * a.B, blocks = (n + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    combine_kernel<<<(int)blocks, 256, 0, s>>>(a);
+    combine_kernel<<<dim3((int)blocks, a.maps), 256, 0, s>>>(a);
     S2DW_CUDA_TRY(cudaGetLastError());
     return S2DWC_OK;
 }
 
-int launch_zero(double *p, long long n, cudaStream_t s)
-{
-    if (n <= 0) return S2DWC_OK;
-    long long blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    zero_kernel<<<(int)blocks, 256, 0, s>>>(p, n);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-int launch_scoeff_copy(double2 *scoeff, const double2 *flm, int B, int bs, cudaStream_t s)
+int launch_scoeff_copy(double2 *scoeff, const double2 *flm, int B, int bs, int maps, cudaStream_t s)
 {
     const int n = bs * bs;
-    if (n <= 0) return S2DWC_OK;
-    scoeff_copy_kernel<<<(n + 255) / 256, 256, 0, s>>>(scoeff, flm, B, bs);
-    S2DW_CUDA_TRY(cudaGetLastError());
-    return S2DWC_OK;
-}
-
-int launch_scaling_add(double2 *flm, const double2 *scoeff, const double *Phi2, int B, int bs,
-                       cudaStream_t s)
-{
-    const int n = bs * bs;
-    if (n <= 0) return S2DWC_OK;
-    scaling_add_kernel<<<(n + 255) / 256, 256, 0, s>>>(flm, scoeff, Phi2, B, bs);
+    if (n <= 0 || maps <= 0) return S2DWC_OK;
+    scoeff_copy_kernel<<<dim3((n + 255) / 256, maps), 256, 0, s>>>(scoeff, flm, B, bs);
     S2DW_CUDA_TRY(cudaGetLastError());
     return S2DWC_OK;
 }

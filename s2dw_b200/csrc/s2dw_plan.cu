@@ -121,11 +121,15 @@ struct s2dwc_plan {
     // maps the map-proportional workspaces (Tg, V2f, part) hold: grown on
     // demand up to the 32 maps of one tensor-core pass
     int sp_cap = 0;
+    // scales whose transform stages take sp_chunk maps in one launch (Tb of a
+    // map below 16 MB); the others run map by map in their FP64 workspace
+    std::vector<int> sp_small;
+    int sp_chunk = 1;
     long long sp_tg_map = 0, sp_v2f_map = 0;
     int *sp_err = nullptr;
     unsigned long long sp_wait_ns = 2000000000ull;  // bound on every split-kernel pipeline wait (2 s)
     int sp_min_batch = 1;  // split-form batches smaller than this run the FP64 path
-    // moments of the coefficients (built on first use): 32 maps per pass
+    // moments of the coefficients (built on first use): 16 maps per pass
     double *st_part = nullptr, *st_mean = nullptr;
     int *st_flags = nullptr;
     std::vector<void *> allocs;
@@ -900,8 +904,8 @@ int split_prepare(s2dwc_plan *p, int nmaps, cudaStream_t s)
             fexp += (long long)bl * 64;
             S.tg_off = tg;
             tg += (long long)p->N * bl * bl;
-            S.tb_off = tb;
             tb += (long long)p->N * bl * 2 * bl;
+            if ((long long)p->N * bl * 2 * bl * (long long)sizeof(double2) < (16LL << 20)) p->sp_small.push_back(j);
             S.vstride = (long long)NP * bl * Vs;
             S.v2f_off = v2f;
             v2f += S.vstride;
@@ -931,8 +935,25 @@ int split_prepare(s2dwc_plan *p, int nmaps, cudaStream_t s)
         if ((st = dev_alloc(p, &p->sp_dexp, (size_t)nd)) || (st = dev_alloc(p, &p->sp_sexp, (size_t)ns)) ||
             (st = dev_alloc(p, &p->sp_fexp, (size_t)fexp)) || (st = dev_alloc(p, &p->sp_vexp, (size_t)fexp)) ||
             (st = dev_alloc(p, &p->sp_fdig, (size_t)fdig)) || (st = dev_alloc(p, &p->sp_vdig, (size_t)vdig)) ||
-            (st = dev_alloc(p, &p->sp_Tb, (size_t)tb)) || (st = dev_alloc(p, &p->sp_err, 1)))
+            (st = dev_alloc(p, &p->sp_err, 1)))
             return st;
+        // Tb of the small scales for a chunk of maps: about 64 MB, which stay
+        // in L2 between the beta and the alpha stage, or one map's Tb of every
+        // scale where a memory limit leaves no more
+        long long one = 0;
+        for (int j : p->sp_small) one += (long long)p->N * p->bl[j] * 2 * p->bl[j];
+        auto chunk = [&](long long values) { return (int)std::max(1LL, std::min((long long)MAPS, one ? values / one : 1)); };
+        p->sp_chunk = chunk((64LL << 20) / (long long)sizeof(double2));
+        if (one && (p->sp_chunk * one <= tb || dev_alloc(p, &p->sp_Tb, (size_t)(p->sp_chunk * one)))) {
+            cudaGetLastError();  // of a failed allocation
+            p->sp_chunk = std::min(p->sp_chunk, chunk(tb));
+            if ((st = dev_alloc(p, &p->sp_Tb, (size_t)tb))) return st;
+        }
+        long long off = 0;
+        for (int j : p->sp_small) {
+            p->sp[j].tb_off = off;
+            off += (long long)p->sp_chunk * p->N * p->bl[j] * 2 * p->bl[j];
+        }
         p->sp_tg_map = tg;
         p->sp_v2f_map = v2f;
         S2DW_CUDA_TRY(cudaMemsetAsync(p->sp_err, 0, sizeof(int), s));
@@ -1011,24 +1032,47 @@ int split_prepare(s2dwc_plan *p, int nmaps, cudaStream_t s)
     return S2DWC_OK;
 }
 
-// Runs f(j, stream) for every scale: on the plan's per-scale streams forked
-// from and joined back to `s`, or all on `s` in timing mode.
-template <typename F>
-int for_scales(s2dwc_plan *p, cudaStream_t s, F &&f)
+// One group of maps of the split form: digits(j, stream) (digits and
+// contraction of scale j) and the transform stages, which follow it (analysis)
+// or go before it.  Each scale has its stream, forked from and joined back to
+// `s` (all on `s` in timing mode): large(j, stream) runs the stages of a large
+// scale there; small(stream) those of all small scales together on the first
+// one's stream.
+template <typename D, typename L, typename S>
+int split_scales(s2dwc_plan *p, cudaStream_t s, bool analysis, D &&digits, L &&large, S &&small)
 {
     int st;
-    if (p->timing) {
-        for (int j = 0; j <= p->J; j++)
-            if ((st = f(j, s))) return st;
-        return S2DWC_OK;
+    const bool par = !p->timing;
+    auto stream = [&](int j) { return par ? p->streams[j] : s; };
+    auto is_small = [&](int j) { return std::find(p->sp_small.begin(), p->sp_small.end(), j) != p->sp_small.end(); };
+    const int j0 = p->sp_small.empty() ? -1 : p->sp_small[0];  // the small scales' stream
+    if (par) {
+        S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
+        for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j], p->ev_fork, 0));
     }
-    S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
+    if (!analysis && j0 >= 0) {
+        if ((st = small(stream(j0)))) return st;
+        if (par) {
+            S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j0], p->streams[j0]));
+            for (int j : p->sp_small)
+                if (j != j0) S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j], p->ev_join[j0], 0));
+        }
+    }
     for (int j = 0; j <= p->J; j++) {
-        S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j], p->ev_fork, 0));
-        if ((st = f(j, p->streams[j]))) return st;
-        S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j], p->streams[j]));
+        if (!analysis && !is_small(j) && (st = large(j, stream(j)))) return st;
+        if ((st = digits(j, stream(j)))) return st;
+        if (analysis && !is_small(j) && (st = large(j, stream(j)))) return st;
+        if (par) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j], p->streams[j]));
     }
-    for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[j], 0));
+    if (analysis && j0 >= 0) {
+        if (par)
+            for (int j : p->sp_small)
+                if (j != j0) S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j0], p->ev_join[j], 0));
+        if ((st = small(stream(j0)))) return st;
+        if (par) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j0], p->streams[j0]));
+    }
+    if (par)
+        for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_join[j], 0));
     return S2DWC_OK;
 }
 
@@ -1047,7 +1091,7 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
     const long long bs2 = (long long)p->bl_scoeff * p->bl_scoeff;
     for (int g0 = 0; g0 < nmaps; g0 += MAPS) {
         const int nk = std::min(MAPS, nmaps - g0);
-        st = for_scales(p, s, [&](int j, cudaStream_t sj) -> int {
+        auto digits = [&](int j, cudaStream_t sj) -> int {
             int st2;
             const int bl = p->bl[j];
             const auto &S = p->sp[j];
@@ -1095,23 +1139,34 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
                 KernelTimer kt(p, S2DWC_KIND_LWALK, sj);
                 if ((st2 = launch_split(a, sj))) return st2;
             }
-            const std::vector<int> js{j};
-            for (int k = 0; k < nk; k++) {
-                auto Tg = [&](int) { return p->sp_Tg + p->sp_cap * S.tg_off + (long long)k * p->N * bl * bl; };
-                auto Tb = [&](int) { return p->sp_Tb + S.tb_off; };
-                auto wav = [&](int) { return d_wav + (g0 + k) * wtot + p->wav_off[j]; };
-                if ((st2 = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj))) return st2;
-                if ((st2 = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj))) return st2;
-            }
             return S2DWC_OK;
-        });
+        };
+        auto stages = [&](const std::vector<int> &js, int k, int maps, bool shared, cudaStream_t sj) -> int {
+            auto Tg = [&](int j) { return p->sp_Tg + p->sp_cap * p->sp[j].tg_off + (long long)k * p->N * p->bl[j] * p->bl[j]; };
+            auto Tb = [&](int j) { return shared ? p->sp_Tb + p->sp[j].tb_off : p->wsA + p->offA[j]; };
+            auto wav = [&](int j) { return d_wav + (g0 + k) * wtot + p->wav_off[j]; };
+            auto tg_map = [&](int j) { return (long long)p->N * p->bl[j] * p->bl[j]; };
+            auto tb_map = [&](int j) { return 2 * tg_map(j); };
+            auto wav_map = [&](int) { return wtot; };
+            if (int e = run_stage(p, STAGE_ANA_BETA, js, maps, Tg, Tb, tg_map, tb_map, sj)) return e;
+            return run_stage(p, STAGE_ANA_ALPHA, js, maps, Tb, wav, tb_map, wav_map, sj);
+        };
+        st = split_scales(
+            p, s, true, digits,
+            [&](int j, cudaStream_t sj) -> int {
+                for (int k = 0; k < nk; k++)
+                    if (int e = stages({j}, k, 1, false, sj)) return e;
+                return S2DWC_OK;
+            },
+            [&](cudaStream_t sj) -> int {
+                for (int k = 0; k < nk; k += p->sp_chunk)
+                    if (int e = stages(p->sp_small, k, std::min(p->sp_chunk, nk - k), true, sj)) return e;
+                return S2DWC_OK;
+            });
         if (st) return st;
-        for (int k = 0; k < nk; k++) {
-            KernelTimer kt(p, S2DWC_KIND_OTHER, s);
-            if ((st = launch_scoeff_copy(d_scoeff ? d_scoeff + (g0 + k) * bs2 : nullptr, d_flm + (g0 + k) * B2, p->B,
-                                         p->bl_scoeff, s)))
-                return st;
-        }
+        KernelTimer kt(p, S2DWC_KIND_OTHER, s);
+        if ((st = launch_scoeff_copy(d_scoeff ? d_scoeff + g0 * bs2 : nullptr, d_flm + g0 * B2, p->B, p->bl_scoeff, nk, s)))
+            return st;
     }
     return S2DWC_OK;
 }
@@ -1131,18 +1186,10 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
     const long long bs2 = (long long)p->bl_scoeff * p->bl_scoeff;
     for (int g0 = 0; g0 < nmaps; g0 += MAPS) {
         const int nk = std::min(MAPS, nmaps - g0);
-        st = for_scales(p, s, [&](int j, cudaStream_t sj) -> int {
+        auto digits = [&](int j, cudaStream_t sj) -> int {
             int st2;
             const int bl = p->bl[j];
             const auto &S = p->sp[j];
-            const std::vector<int> js{j};
-            for (int k = 0; k < nk; k++) {
-                auto wav = [&](int) -> const double * { return d_wav + (g0 + k) * wtot + p->wav_off[j]; };
-                auto V = [&](int) { return p->sp_Tb + S.tb_off; };
-                auto V2f = [&](int) { return p->sp_V2f + p->sp_cap * S.v2f_off + k * S.vstride; };
-                if ((st2 = run_stage(p, STAGE_SYN_ALPHA, js, 1, wav, V, one_map, one_map, sj))) return st2;
-                if ((st2 = run_stage(p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj))) return st2;
-            }
             if (bl - p->blo[j] - 1 <= 0) return S2DWC_OK;
             VdigArgs va{};
             va.bl = bl;
@@ -1183,25 +1230,47 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
             b.wait_ns = p->sp_wait_ns;
             KernelTimer kt(p, S2DWC_KIND_MWALK, sj);
             return launch_split_syn(b, sj);
-        });
+        };
+        auto stages = [&](const std::vector<int> &js, int k, int maps, bool shared, cudaStream_t sj) -> int {
+            auto wav = [&](int j) -> const double * { return d_wav + (g0 + k) * wtot + p->wav_off[j]; };
+            auto V = [&](int j) { return shared ? p->sp_Tb + p->sp[j].tb_off : p->wsA + p->offA[j]; };
+            auto V2f = [&](int j) { return p->sp_V2f + p->sp_cap * p->sp[j].v2f_off + k * p->sp[j].vstride; };
+            auto wav_map = [&](int) { return wtot; };
+            auto v_map = [&](int j) { return (long long)p->N * p->bl[j] * 2 * p->bl[j]; };
+            auto v2f_map = [&](int j) { return p->sp[j].vstride; };
+            if (int e = run_stage(p, STAGE_SYN_ALPHA, js, maps, wav, V, wav_map, v_map, sj)) return e;
+            return run_stage(p, STAGE_SYN_BETA, js, maps, V, V2f, v_map, v2f_map, sj);
+        };
+        st = split_scales(
+            p, s, false, digits,
+            [&](int j, cudaStream_t sj) -> int {
+                for (int k = 0; k < nk; k++)
+                    if (int e = stages({j}, k, 1, false, sj)) return e;
+                return S2DWC_OK;
+            },
+            [&](cudaStream_t sj) -> int {
+                for (int k = 0; k < nk; k += p->sp_chunk)
+                    if (int e = stages(p->sp_small, k, std::min(p->sp_chunk, nk - k), true, sj)) return e;
+                return S2DWC_OK;
+            });
         if (st) return st;
-        for (int k = 0; k < nk; k++) {
-            CombineArgs cb{};
-            cb.B = p->B;
-            cb.J = p->J;
-            cb.bs = p->bl_scoeff;
-            for (int j = 0; j <= p->J; j++) {
-                cb.bl[j] = p->bl[j];
-                cb.blo[j] = p->blo[j];
-                cb.off[j] = p->offP[j];
-            }
-            cb.parts = p->sp_part + k * p->sp_pstride;
-            cb.scoeff = d_scoeff ? d_scoeff + (g0 + k) * bs2 : nullptr;
-            cb.Phi2 = p->Phi2;
-            cb.flm = d_flm + (g0 + k) * B2;
-            KernelTimer kt(p, S2DWC_KIND_OTHER, s);
-            if ((st = launch_combine(cb, s))) return st;
+        CombineArgs cb{};
+        cb.B = p->B;
+        cb.J = p->J;
+        cb.bs = p->bl_scoeff;
+        for (int j = 0; j <= p->J; j++) {
+            cb.bl[j] = p->bl[j];
+            cb.blo[j] = p->blo[j];
+            cb.off[j] = p->offP[j];
         }
+        cb.maps = nk;
+        cb.pstride = p->sp_pstride;
+        cb.parts = p->sp_part;
+        cb.scoeff = d_scoeff ? d_scoeff + g0 * bs2 : nullptr;
+        cb.Phi2 = p->Phi2;
+        cb.flm = d_flm + g0 * B2;
+        KernelTimer kt(p, S2DWC_KIND_OTHER, s);
+        if ((st = launch_combine(cb, s))) return st;
     }
     return S2DWC_OK;
 }
@@ -1620,11 +1689,11 @@ int s2dwc_plan_stat_moments(s2dwc_plan *p, int nmaps, const double *d_wav, const
     if (!p || !d_wav || !d_moments) return set_error(S2DWC_ERROR_ARG_INVALID, "plan_stat_moments: null pointer");
     if (nmaps < 0) return set_error(S2DWC_ERROR_ARG_INVALID, "plan_stat_moments: nmaps=%d", nmaps);
     DeviceGuard dg(p->device);
-    constexpr int G = 32;
+    constexpr int G = 16;
     int st;
     if (!p->st_part) {
         const size_t ny = (size_t)G * (p->J + 1);
-        if ((st = dev_alloc(p, &p->st_part, ny * STAT_P * 6)) || (st = dev_alloc(p, &p->st_mean, ny * 2)) ||
+        if ((st = dev_alloc(p, &p->st_part, ny * STAT_P * STAT_W)) || (st = dev_alloc(p, &p->st_mean, ny * 2)) ||
             (st = dev_alloc(p, &p->st_flags, ny)))
             return st;
     }
@@ -1638,6 +1707,7 @@ int s2dwc_plan_stat_moments(s2dwc_plan *p, int nmaps, const double *d_wav, const
         a.wav = d_wav + (size_t)g0 * wtot;
         a.mask = d_mask;
         a.part = p->st_part;
+        a.part2 = p->st_part + (size_t)G * (p->J + 1) * STAT_P * 2;
         a.mean_nj = p->st_mean;
         a.out = d_moments + (size_t)g0 * (p->J + 1) * 6;
         a.flags = p->st_flags;
@@ -1671,14 +1741,14 @@ int s2dwc_stat_moments(double *const *wav_scales, int J, int B, int N, double al
     const size_t ny = (size_t)J + 1;
     // one device block for everything this call needs, freed before return
     const size_t nw = (size_t)a.wtot, nm = mask_scales ? nw : 0;
-    const size_t bytes = 8 * (nw + nm + ny * STAT_P * 6 + ny * 2 + ny * 6) + 4 * ny + 256;
+    const size_t bytes = 8 * (nw + nm + ny * STAT_P * STAT_W + ny * 2 + ny * 6) + 4 * ny + 256;
     char *blk = nullptr;
     cudaError_t e = cudaMalloc(&blk, bytes);
     if (e != cudaSuccess)
         return set_error(S2DWC_ERROR_MEM_ALLOC_FAIL, "stat_moments: cudaMalloc of %zu bytes failed: %s", bytes,
                          cudaGetErrorString(e));
     std::unique_ptr<char, void (*)(char *)> guard(blk, [](char *q) { cudaFree(q); });
-    double *dw = reinterpret_cast<double *>(blk), *dm = dw + nw, *dpart = dm + nm, *dmean = dpart + ny * STAT_P * 6,
+    double *dw = reinterpret_cast<double *>(blk), *dm = dw + nw, *dpart = dm + nm, *dmean = dpart + ny * STAT_P * STAT_W,
            *dout = dmean + ny * 2;
     int *dflags = reinterpret_cast<int *>(dout + ny * 6);
     for (int j = 0; j <= J; j++) {
@@ -1689,6 +1759,7 @@ int s2dwc_stat_moments(double *const *wav_scales, int J, int B, int N, double al
     a.wav = dw;
     a.mask = mask_scales ? dm : nullptr;
     a.part = dpart;
+    a.part2 = dpart + ny * STAT_P * 2;
     a.mean_nj = dmean;
     a.out = dout;
     a.flags = dflags;

@@ -7,8 +7,16 @@
 //           mask is 1 (all samples without a mask);
 // then the reference's normalisations (n-1 variance, standardised skewness,
 // excess kurtosis, fifth and excess sixth moments; zero variance -> zeros).
-// Every reduction runs in a fixed order (per-block shared-memory trees, then
-// the STAT_P block partials in index order), so results are bit-reproducible.
+// Every reduction runs in a fixed order (per-thread sums, shuffle and
+// shared-memory trees, then the STAT_P block partials in a warp's tree), so
+// results are bit-reproducible.
+//
+// Bound by HBM: two reads of the coefficients (and mask).  Each thread has
+// eight 8-byte loads in flight (four 16-byte ones where the arrays allow it),
+// and the partials are summed by a warp at the start of the pass that needs
+// them: 4 maps at B=512, N=4 with a mask (626 MB through the two passes, with
+// the mask's re-reads) took 245 us with one load in flight, 64 blocks per scale
+// and single threads summing the partials.
 #include <cuda_runtime.h>
 
 #include "s2dw_internal.h"
@@ -19,22 +27,39 @@ namespace {
 constexpr int STAT_T = 256;
 constexpr double TOL_ZERO = 1e-12;
 
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double (*sh)[STAT_T])
+__device__ __forceinline__ double warp_sum(double v)
 {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Sums of v over the block, in thread 0.
+template <int K>
+__device__ __forceinline__ void block_sum(double (&v)[K])
+{
+    __shared__ double sh[K][STAT_T / 32];
     const int t = threadIdx.x;
 #pragma unroll
-    for (int k = 0; k < K; k++) sh[k][t] = v[k];
-    __syncthreads();
-    for (int o = STAT_T / 2; o > 0; o >>= 1) {
-        if (t < o) {
-#pragma unroll
-            for (int k = 0; k < K; k++) sh[k][t] += sh[k][t + o];
-        }
-        __syncthreads();
+    for (int k = 0; k < K; k++) {
+        v[k] = warp_sum(v[k]);
+        if ((t & 31) == 0) sh[k][t >> 5] = v[k];
     }
+    __syncthreads();
+    if (t == 0)
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k] = sh[k][0];
+        for (int k = 0; k < K; k++) {
+            v[k] = sh[k][0];
+            for (int w = 1; w < STAT_T / 32; w++) v[k] += sh[k][w];
+        }
+}
+
+// Sum over the STAT_P block partials of pass 1's value k of row y, by one warp.
+__device__ __forceinline__ double partial_sum(const StatArgs &a, int y, int k)
+{
+    double s = 0.0;
+    for (int x = threadIdx.x & 31; x < STAT_P; x += 32) s += a.part[((size_t)y * STAT_P + x) * 2 + k];
+    return warp_sum(s);
 }
 
 // (map, scale) of blockIdx.y and its coefficient block
@@ -52,58 +77,84 @@ __device__ __forceinline__ StatBlock stat_block(const StatArgs &a)
     return b;
 }
 
-__global__ void __launch_bounds__(STAT_T) stat_pass1(StatArgs a)
+// Calls f(w, mask) for the block's share of the (map, scale) block's values,
+// eight per thread at a time.
+template <typename F>
+__device__ __forceinline__ void stat_values(const StatBlock &b, F &&f)
 {
-    __shared__ double sh[2][STAT_T];
+    constexpr int U = 4;
+    const long long step = (long long)STAT_P * STAT_T;
+    const long long t = (long long)blockIdx.x * STAT_T + threadIdx.x;
+    if ((((uintptr_t)b.w | (uintptr_t)b.mk) & 15) == 0) {  // pairs (an even number of values)
+        const double2 *w = reinterpret_cast<const double2 *>(b.w), *m = reinterpret_cast<const double2 *>(b.mk);
+        const long long n = b.n / 2;
+        for (long long i0 = t; i0 < n; i0 += U * step) {
+            double2 x[U], y[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const long long i = i0 + u * step;
+                if (i < n) {
+                    x[u] = w[i];
+                    y[u] = m ? m[i] : make_double2(1.0, 1.0);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (i0 + u * step < n) {
+                    f(x[u].x, y[u].x);
+                    f(x[u].y, y[u].y);
+                }
+        }
+        return;
+    }
+    for (long long i = t; i < b.n; i += step) f(b.w[i], b.mk ? b.mk[i] : 1.0);
+}
+
+__global__ void __launch_bounds__(STAT_T) stat_pass1(const __grid_constant__ StatArgs a)
+{
     const StatBlock b = stat_block(a);
     double v[2] = {0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * STAT_T + threadIdx.x; i < b.n; i += (long long)STAT_P * STAT_T) {
-        if (b.mk) {
-            const double m = b.mk[i];
-            if (fabs(m - 1.0) < TOL_ZERO) v[0] += b.w[i] * m;
-            v[1] += m;
-        } else {
-            v[0] += b.w[i];
-        }
-    }
-    block_sum<2>(v, sh);
+    stat_values(b, [&](double w, double m) {
+        if (fabs(m - 1.0) < TOL_ZERO) v[0] += w * m;
+        v[1] += m;
+    });
+    block_sum<2>(v);
     if (threadIdx.x == 0) {
-        double *p = a.part + ((size_t)blockIdx.y * STAT_P + blockIdx.x) * 6;
+        double *p = a.part + ((size_t)blockIdx.y * STAT_P + blockIdx.x) * 2;
         p[0] = v[0];
         p[1] = v[1];
     }
 }
 
-// mean and nj per (map, scale): the STAT_P partials in index order
-__global__ void stat_mean(StatArgs a)
+// mean and nj of row y, by one warp
+__device__ __forceinline__ double2 stat_mean(const StatArgs &a, int y)
 {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= a.nmaps * (a.J + 1)) return;
     const int j = y % (a.J + 1);
-    double s = 0.0, c = 0.0;
-    for (int x = 0; x < STAT_P; x++) {
-        s += a.part[((size_t)y * STAT_P + x) * 6];
-        c += a.part[((size_t)y * STAT_P + x) * 6 + 1];
-    }
+    const double s = partial_sum(a, y, 0), c = partial_sum(a, y, 1);
     const double nj = a.mask ? rint(c) : (double)(a.off[j + 1] - a.off[j]);
-    a.mean_nj[2 * y] = s / nj;
-    a.mean_nj[2 * y + 1] = nj;
+    return make_double2(s / nj, nj);
 }
 
-__global__ void __launch_bounds__(STAT_T) stat_pass2(StatArgs a)
+__global__ void __launch_bounds__(STAT_T) stat_pass2(const __grid_constant__ StatArgs a)
 {
-    __shared__ double sh[6][STAT_T];
+    __shared__ double smu;
     const StatBlock b = stat_block(a);
-    const double mu = a.mean_nj[2 * blockIdx.y];
-    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (long long i = (long long)blockIdx.x * STAT_T + threadIdx.x; i < b.n; i += (long long)STAT_P * STAT_T) {
-        double w = b.w[i];
-        if (b.mk) {
-            const double m = b.mk[i];
-            if (!(fabs(m - 1.0) < TOL_ZERO)) continue;
-            w *= m;
+    if (threadIdx.x < 32) {
+        const double2 m = stat_mean(a, blockIdx.y);
+        if (threadIdx.x == 0) {
+            smu = m.x;
+            if (blockIdx.x == 0) {
+                a.mean_nj[2 * blockIdx.y] = m.x;
+                a.mean_nj[2 * blockIdx.y + 1] = m.y;
+            }
         }
-        const double s = w - mu;
+    }
+    __syncthreads();
+    const double mu = smu;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    stat_values(b, [&](double w, double m) {
+        if (!(fabs(m - 1.0) < TOL_ZERO)) return;
+        const double s = w * m - mu;
         double p = s * s;
         v[0] += s;
         v[1] += p;
@@ -115,21 +166,29 @@ __global__ void __launch_bounds__(STAT_T) stat_pass2(StatArgs a)
         v[4] += p;
         p *= s;
         v[5] += p;
+    });
+    block_sum<6>(v);
+    if (threadIdx.x == 0) {
+        double *p = a.part2 + ((size_t)blockIdx.y * STAT_P + blockIdx.x) * 6;
+#pragma unroll
+        for (int k = 0; k < 6; k++) p[k] = v[k];
     }
-    block_sum<6>(v, sh);
-    if (threadIdx.x < 6) a.part[((size_t)blockIdx.y * STAT_P + blockIdx.x) * 6 + threadIdx.x] = v[threadIdx.x];
 }
 
-// moments per (map, scale): out[y*6 + {mean, var, skew, kur, five, six}],
-// flags[y] = 1 zero variance, 2 fewer than two samples
-__global__ void stat_final(StatArgs a)
+// moments per (map, scale), a warp each: out[y*6 + {mean, var, skew, kur,
+// five, six}], flags[y] = 1 zero variance, 2 fewer than two samples
+__global__ void __launch_bounds__(128) stat_final(const __grid_constant__ StatArgs a)
 {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (y >= a.nmaps * (a.J + 1)) return;
-    double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int x = 0; x < STAT_P; x++)
+    double s[6];
 #pragma unroll
-        for (int k = 0; k < 6; k++) s[k] += a.part[((size_t)y * STAT_P + x) * 6 + k];
+    for (int k = 0; k < 6; k++) {
+        double t = 0.0;
+        for (int x = threadIdx.x & 31; x < STAT_P; x += 32) t += a.part2[((size_t)y * STAT_P + x) * 6 + k];
+        s[k] = warp_sum(t);
+    }
+    if (threadIdx.x & 31) return;
     const double mu = a.mean_nj[2 * y], nj = a.mean_nj[2 * y + 1];
     double *o = a.out + (size_t)y * 6;
     o[0] = mu;
@@ -161,9 +220,8 @@ int launch_stat_moments(const StatArgs &a, cudaStream_t s)
     if (ny <= 0) return S2DWC_OK;
     dim3 grid(STAT_P, ny);
     stat_pass1<<<grid, STAT_T, 0, s>>>(a);
-    stat_mean<<<(ny + 127) / 128, 128, 0, s>>>(a);
     stat_pass2<<<grid, STAT_T, 0, s>>>(a);
-    stat_final<<<(ny + 127) / 128, 128, 0, s>>>(a);
+    stat_final<<<(ny + 3) / 4, 128, 0, s>>>(a);
     S2DW_CUDA_TRY(cudaGetLastError());
     return S2DWC_OK;
 }
