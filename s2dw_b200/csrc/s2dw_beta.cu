@@ -35,9 +35,10 @@ __device__ __forceinline__ void ana_beta(const StageArgs &a, const StageEnt &e, 
         constexpr int BL = M / 2;
         double2 xe[V / 2], w[V / 2];
 #pragma unroll
-        for (int i = 0; i < V / 2; i++) xe[i] = X[t + i * TPR];
-#pragma unroll
         for (int i = 0; i < V / 2; i++) w[i] = __ldg(e.pre + t + i * TPR);
+        pdl_wait();
+#pragma unroll
+        for (int i = 0; i < V / 2; i++) xe[i] = X[t + i * TPR];
         double2 x0 = make_double2(0.0, 0.0);
         if (sn) x0 = X[0];
 #pragma unroll
@@ -70,6 +71,7 @@ __device__ __forceinline__ void ana_beta(const StageArgs &a, const StageEnt &e, 
         for (int i = 0; i < V; i++) Y[t + i * TPR] = buf[F::pad(t + i * TPR)];
     } else {  // k <-> m' = k - (bl - 1)
         const int K = 2 * bl - 1;
+        pdl_wait();
 #pragma unroll
         for (int i = 0; i < V; i++) {
             const int kk = t + i * TPR, mpv = kk - (bl - 1);
@@ -112,13 +114,14 @@ __device__ __forceinline__ void syn_beta(const StageArgs &a, const StageEnt &e, 
     double2 v[V];
 #pragma unroll
     for (int i = 0; i < V; i++) v[i] = make_double2(0.0, 0.0);
+    pdl_wait();
     // gamma DFT, one sample at a time: its loads are in flight together
     for (int g = 0; g < N; g++, X += (size_t)bl * (2 * bl)) {
         const double2 w = __ldg(ph + g * (2 * N - 1));
 #pragma unroll
         for (int i = 0; i < V; i++) {
             const int b = t + i * TPR;
-            if (MODE == FFT_SYN_BETA || b < 2 * bl) v[i] = cadd(v[i], cmul(__ldg(X + b), w));
+            if (MODE == FFT_SYN_BETA || b < 2 * bl) v[i] = cadd(v[i], cmul(X[b], w));
         }
     }
     if (MODE == FFT_SYN_BETA) {
@@ -190,6 +193,7 @@ template <int FFT, int CZT>
 __global__ void __launch_bounds__(ST_THREADS, 4) beta_kernel(const __grid_constant__ StageArgs a)
 {
     extern __shared__ __align__(16) double2 smem[];
+    pdl_start();
     int cta;
     const StageEnt &e = stage_entry(a, cta);
     if (e.kind == FFT) beta_size<FFT>(a, e, cta, smem);
@@ -201,12 +205,11 @@ constexpr size_t BETA_SMEM = sizeof(double2) * (2048 + 2048 / 4 + 32);
 
 }  // namespace
 
-int launch_stage_beta(Stage st, const StageArgs &a, cudaStream_t s)
+int launch_stage_beta(Stage st, const StageArgs &a, bool dep, cudaStream_t s)
 {
     if (a.ncta <= 0) return S2DWC_OK;
-    if (st == STAGE_ANA_BETA) beta_kernel<FFT_ANA_BETA, CZT_ANA_BETA><<<a.ncta, ST_THREADS, BETA_SMEM, s>>>(a);
-    else beta_kernel<FFT_SYN_BETA, CZT_SYN_BETA><<<a.ncta, ST_THREADS, BETA_SMEM, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
+    auto *k = st == STAGE_ANA_BETA ? beta_kernel<FFT_ANA_BETA, CZT_ANA_BETA> : beta_kernel<FFT_SYN_BETA, CZT_SYN_BETA>;
+    S2DW_CUDA_TRY(launch_dep(k, a.ncta, ST_THREADS, BETA_SMEM, s, dep, a));
     return S2DWC_OK;
 }
 

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
     using L = LwalkSmem<NP, S, NS>;
     constexpr int MT = L::MT, NR = NS * NP;
     extern __shared__ __align__(16) double lsm[];
+    pdl_start();
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, lp = lane & 15;
     const int B = a.B, Bp = a.Bp, N = a.N;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
     // tables have rows to a multiple of 16 l and slack behind the last one;
     // values of m or l past the band limit are read but belong to pairs that
     // stay at zero and are not stored.
-    auto stage = [&](int c) {
+    auto stage_tables = [&](int c) {
         const int lc = lstart + c * LW_CH;
         double *b = lsm + (c % LW_ST) * L::BUF;
         {
@@ -163,19 +164,21 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
             if (LW_CH * AP % THREADS == 0 || f < LW_CH * AP)
                 cp16(b + L::AM_OFF + li * MT + pc, a.Acoef + (size_t)(lc + li) * Bp + m0 + pc);
         }
+    };
+    auto stage_f = [&](int c) {
+        const int lc = lstart + c * LW_CH;
+        double *b = lsm + (c % LW_ST) * L::BUF;
 #pragma unroll
         for (int i = 0; i < LW_CH * MT / THREADS; i++) {
             const int f = tid + THREADS * i, li = f / MT, pc = f % MT;
             cp16(b + L::F_OFF + 2 * (li * MT + pc), a.F + (size_t)(lc + li) * Bp + m0 + pc);
         }
     };
-
-    // the first chunks are on their way while the start values are read
+    // the first chunks' tables are on their way while the start values are
+    // read (and the kernel that writes F ends)
 #pragma unroll
-    for (int c = 0; c < LW_ST - 1; c++) {
-        if (c < nchunks) stage(c);
-        cp_commit();
-    }
+    for (int c = 0; c < LW_ST - 1; c++)
+        if (c < nchunks) stage_tables(c);
 
     // ---- start values of the pairs (m', m = mb + s), all in the domain scaled by 2^Kw
     double st[S];
@@ -194,6 +197,12 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
             const double v = ldexp(a.Stm[o], (int)a.Ste[o] + Kw);
             st[s] = (mp >= m && ((mp - m) & 1)) ? -v : v;
         }
+    }
+    pdl_wait();
+#pragma unroll
+    for (int c = 0; c < LW_ST - 1; c++) {
+        if (c < nchunks) stage_f(c);
+        cp_commit();
     }
     double x[2][S];
     double2 acc[NS][2][S][NP];
@@ -333,7 +342,10 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         if (c < nchunks) {
             cp_wait<LW_ST - 2>();
             __syncthreads();  // chunk c in shared memory, buffer of chunk c - 1 free
-            if (c + LW_ST - 1 < nchunks) stage(c + LW_ST - 1);
+            if (c + LW_ST - 1 < nchunks) {
+                stage_tables(c + LW_ST - 1);
+                stage_f(c + LW_ST - 1);
+            }
             cp_commit();
         }
         for (int li = 0;;) {
@@ -444,7 +456,9 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
     using L = MwalkSmem<NP, P, S>;
     constexpr int TL = L::TL, MT = L::MT, R = L::R, NST = L::ST;
     extern __shared__ __align__(16) double msm[];
+    pdl_start();
     if ((int)blockIdx.x >= a.ntiles) {
+        pdl_wait();
         mwalk_fill(a, (int)blockIdx.x - a.ntiles, (int)gridDim.x - a.ntiles);
         return;
     }
@@ -472,7 +486,7 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
     const int actA = a.blo[jA];
     const bool edge = l0 <= actA;
 
-    auto stage = [&](int c, int buf) {
+    auto stage_tables = [&](int c, int buf) {
         double *b = msm + buf * L::BUF;
         const int c0 = c * MW_CH, len = gtpack_len(c0, a.Lp);
         const double *src = a.GT + gtpack_row(c0, R, a.Lp) + (l0 - gtpack_start(c0));
@@ -482,6 +496,10 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
             const int f = tid + THREADS * i, row = f / TP, pc = 2 * (f % TP);
             if (NT % THREADS == 0 || f < NT) cp16(b + L::T_OFF + row * TL + pc, src + (size_t)row * len + pc);
         }
+    };
+    auto stage_v = [&](int c, int buf) {
+        double *b = msm + buf * L::BUF;
+        const int c0 = c * MW_CH;
         constexpr int NV = 2 * NP * MT * MW_CH;
 #pragma unroll
         for (int i = 0; i < (NV + THREADS - 1) / THREADS; i++) {
@@ -496,10 +514,8 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
 
     const int ctop = MH / MW_CH;
 #pragma unroll
-    for (int i = 0; i < NST - 1; i++) {
-        if (ctop - i >= 0) stage(ctop - i, i);
-        cp_commit();
-    }
+    for (int i = 0; i < NST - 1; i++)
+        if (ctop - i >= 0) stage_tables(ctop - i, i);
 
     double st[P][S], mq[S];
     int maxe = INT_MIN;
@@ -530,10 +546,19 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
             acc[i][s] = make_double2(0.0, 0.0);
         }
 
+    pdl_wait();
+#pragma unroll
+    for (int i = 0; i < NST - 1; i++) {
+        if (ctop - i >= 0) stage_v(ctop - i, i);
+        cp_commit();
+    }
     for (int c = ctop, it = 0; c >= 0; c--, it++) {
         cp_wait<NST - 2>();
         __syncthreads();  // chunk c in shared memory, the previous chunk's buffer free
-        if (c - (NST - 1) >= 0) stage(c - (NST - 1), (it + NST - 1) % NST);
+        if (c - (NST - 1) >= 0) {
+            stage_tables(c - (NST - 1), (it + NST - 1) % NST);
+            stage_v(c - (NST - 1), (it + NST - 1) % NST);
+        }
         cp_commit();
         const double *b = msm + (it % NST) * L::BUF;
         const double *T = b + L::T_OFF + lp;
@@ -693,7 +718,7 @@ __global__ void gtpack_kernel(GpackArgs a)
 constexpr int lwalk_smax(int NP) { return NP == 1 ? 8 : NP == 2 ? 4 : NP <= 4 ? 2 : 1; }
 
 template <int NP, int S, int NS, int MINB>
-int launch_lwalk_t(const LwalkArgs &a, cudaStream_t s)
+int launch_lwalk_t(const LwalkArgs &a, bool dep, cudaStream_t s)
 {
     using L = LwalkSmem<NP, S, NS>;
     static bool attr[64] = {false};
@@ -707,13 +732,12 @@ int launch_lwalk_t(const LwalkArgs &a, cudaStream_t s)
     const int bl = a.bl[std::max(0, a.only)];
     const int grid = NS == 1 ? ((bl + 15) / 16) * ((bl + L::MT - 1) / L::MT) : a.ntiles;
     if (grid <= 0) return S2DWC_OK;
-    lwalk_kernel<NP, S, NS, MINB><<<grid, THREADS, L::BYTES, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
+    S2DW_CUDA_TRY(launch_dep(lwalk_kernel<NP, S, NS, MINB>, grid, THREADS, L::BYTES, s, dep, a));
     return S2DWC_OK;
 }
 
 template <int NP, int P, int S, int MINB>
-int launch_mwalk_t(const MwalkArgs &a, cudaStream_t s)
+int launch_mwalk_t(const MwalkArgs &a, bool dep, cudaStream_t s)
 {
     using L = MwalkSmem<NP, P, S>;
     static bool attr[64] = {false};
@@ -726,8 +750,7 @@ int launch_mwalk_t(const MwalkArgs &a, cudaStream_t s)
     }
     const int fill = a.acc_imag ? 0 : std::min(148, (a.B * a.B + 8 * THREADS - 1) / (8 * THREADS));
     if (a.ntiles + fill <= 0) return S2DWC_OK;
-    mwalk_kernel<NP, P, S, MINB><<<a.ntiles + fill, THREADS, L::BYTES, s>>>(a);
-    S2DW_CUDA_TRY(cudaGetLastError());
+    S2DW_CUDA_TRY(launch_dep(mwalk_kernel<NP, P, S, MINB>, a.ntiles + fill, THREADS, L::BYTES, s, dep, a));
     return S2DWC_OK;
 }
 
@@ -815,65 +838,65 @@ void build_mwalk_tiles(const std::vector<MwalkInterval> &iv, int2 shape, std::ve
     std::stable_sort(t.begin(), t.end(), [](int2 a, int2 b) { return (a.x & 0xffff) > (b.x & 0xffff); });
 }
 
-int launch_lwalk(const LwalkArgs &a, cudaStream_t s)
+int launch_lwalk(const LwalkArgs &a, bool dep, cudaStream_t s)
 {
     if (a.only >= 0) {
         switch (a.NP) {
-        case 1: return launch_lwalk_t<1, 2, 1, 1>(a, s);
-        case 2: return launch_lwalk_t<2, 2, 1, 1>(a, s);
-        case 3: return launch_lwalk_t<3, 2, 1, 1>(a, s);
-        case 4: return launch_lwalk_t<4, 2, 1, 1>(a, s);
-        case 5: return launch_lwalk_t<5, 2, 1, 1>(a, s);
-        case 6: return launch_lwalk_t<6, 2, 1, 1>(a, s);
-        case 7: return launch_lwalk_t<7, 2, 1, 1>(a, s);
-        case 8: return launch_lwalk_t<8, 2, 1, 1>(a, s);
+        case 1: return launch_lwalk_t<1, 2, 1, 1>(a, dep, s);
+        case 2: return launch_lwalk_t<2, 2, 1, 1>(a, dep, s);
+        case 3: return launch_lwalk_t<3, 2, 1, 1>(a, dep, s);
+        case 4: return launch_lwalk_t<4, 2, 1, 1>(a, dep, s);
+        case 5: return launch_lwalk_t<5, 2, 1, 1>(a, dep, s);
+        case 6: return launch_lwalk_t<6, 2, 1, 1>(a, dep, s);
+        case 7: return launch_lwalk_t<7, 2, 1, 1>(a, dep, s);
+        case 8: return launch_lwalk_t<8, 2, 1, 1>(a, dep, s);
         }
     } else {
         switch (a.NP * 16 + a.S) {
-        case 16 + 8: return launch_lwalk_t<1, 8, 2, 2>(a, s);
-        case 16 + 4: return launch_lwalk_t<1, 4, 2, 3>(a, s);
-        case 16 + 2: return launch_lwalk_t<1, 2, 2, 4>(a, s);
-        case 16 + 1: return launch_lwalk_t<1, 1, 2, 5>(a, s);
-        case 32 + 4: return launch_lwalk_t<2, 4, 2, 2>(a, s);
-        case 32 + 2: return launch_lwalk_t<2, 2, 2, 3>(a, s);
-        case 32 + 1: return launch_lwalk_t<2, 1, 2, 4>(a, s);
-        case 48 + 2: return launch_lwalk_t<3, 2, 2, 2>(a, s);
-        case 48 + 1: return launch_lwalk_t<3, 1, 2, 3>(a, s);
-        case 64 + 2: return launch_lwalk_t<4, 2, 2, 2>(a, s);
-        case 64 + 1: return launch_lwalk_t<4, 1, 2, 3>(a, s);
-        case 80 + 1: return launch_lwalk_t<5, 1, 2, 1>(a, s);
-        case 96 + 1: return launch_lwalk_t<6, 1, 2, 1>(a, s);
-        case 112 + 1: return launch_lwalk_t<7, 1, 2, 1>(a, s);
-        case 128 + 1: return launch_lwalk_t<8, 1, 2, 1>(a, s);
+        case 16 + 8: return launch_lwalk_t<1, 8, 2, 2>(a, dep, s);
+        case 16 + 4: return launch_lwalk_t<1, 4, 2, 3>(a, dep, s);
+        case 16 + 2: return launch_lwalk_t<1, 2, 2, 4>(a, dep, s);
+        case 16 + 1: return launch_lwalk_t<1, 1, 2, 5>(a, dep, s);
+        case 32 + 4: return launch_lwalk_t<2, 4, 2, 2>(a, dep, s);
+        case 32 + 2: return launch_lwalk_t<2, 2, 2, 3>(a, dep, s);
+        case 32 + 1: return launch_lwalk_t<2, 1, 2, 4>(a, dep, s);
+        case 48 + 2: return launch_lwalk_t<3, 2, 2, 2>(a, dep, s);
+        case 48 + 1: return launch_lwalk_t<3, 1, 2, 3>(a, dep, s);
+        case 64 + 2: return launch_lwalk_t<4, 2, 2, 2>(a, dep, s);
+        case 64 + 1: return launch_lwalk_t<4, 1, 2, 3>(a, dep, s);
+        case 80 + 1: return launch_lwalk_t<5, 1, 2, 1>(a, dep, s);
+        case 96 + 1: return launch_lwalk_t<6, 1, 2, 1>(a, dep, s);
+        case 112 + 1: return launch_lwalk_t<7, 1, 2, 1>(a, dep, s);
+        case 128 + 1: return launch_lwalk_t<8, 1, 2, 1>(a, dep, s);
         }
     }
     return set_error(S2DWC_ERROR_SIZE_INVALID, "lwalk: unsupported N=%d (N<=%d)", a.N, S2DW_NMAX);
 }
 
 template <int NP>
-static int launch_mwalk_np(const MwalkArgs &a, cudaStream_t s)
+static int launch_mwalk_np(const MwalkArgs &a, bool dep, cudaStream_t s)
 {
-    if (a.shape.x == 2 && a.shape.y == 4) return launch_mwalk_t<NP, 2, 4, 2>(a, s);
-    if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, (NP <= 4 ? 5 : 3)>(a, s);
+    if (a.shape.x == 2 && a.shape.y == 4) return launch_mwalk_t<NP, 2, 4, 2>(a, dep, s);
+    if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, (NP <= 4 ? 5 : 3)>(a, dep, s);
     if constexpr (NP <= 2) {
-        if (a.shape.x == 1 && a.shape.y == 2) return launch_mwalk_t<NP, 1, 2, 1>(a, s);
+        if (a.shape.x == 1 && a.shape.y == 2) return launch_mwalk_t<NP, 1, 2, 1>(a, dep, s);
     } else {
-        if (a.shape.x == 2 && a.shape.y == 2) return launch_mwalk_t<NP, 2, 2, 2>(a, s);
+        if (a.shape.x == 2 && a.shape.y == 2) return launch_mwalk_t<NP, 2, 2, 2>(a, dep, s);
     }
     return set_error(S2DWC_ERROR_ARG_INVALID, "mwalk: tile shape %d x %d", a.shape.x, a.shape.y);
 }
 
-int launch_mwalk(const MwalkArgs &a, cudaStream_t s)
+int launch_mwalk(const MwalkArgs &a, bool dep, cudaStream_t s)
 {
     switch (a.NP) {
-    case 1: return launch_mwalk_np<1>(a, s);
-    case 2: return launch_mwalk_np<2>(a, s);
-    case 3: return launch_mwalk_np<3>(a, s);
-    case 4: return launch_mwalk_np<4>(a, s);
-    case 5: return launch_mwalk_np<5>(a, s);
-    case 6: return launch_mwalk_np<6>(a, s);
-    case 7: return launch_mwalk_np<7>(a, s);
-    case 8: return launch_mwalk_np<8>(a, s);
+    case 1: return launch_mwalk_np<1>(a, dep, s);
+    case 2: return launch_mwalk_np<2>(a, dep, s);
+    case 3: return launch_mwalk_np<3>(a, dep, s);
+    case 4: return launch_mwalk_np<4>(a, dep, s);
+    case 5: return launch_mwalk_np<5>(a, dep, s);
+    case 6: return launch_mwalk_np<6>(a, dep, s);
+    case 7: return launch_mwalk_np<7>(a, dep, s);
+    case 8: return launch_mwalk_np<8>(a, dep, s);
     }
     return set_error(S2DWC_ERROR_SIZE_INVALID, "mwalk: unsupported number of n values %d (N<=%d)", a.NP, S2DW_NMAX);
 }

@@ -90,7 +90,7 @@ __device__ __forceinline__ void twiddle_powers16(double2 (&v)[16], double2 w)
 // is not kept in L1, which holds the chirp tables.
 __device__ __forceinline__ void ld_pair(const double2 *p, double2 &a, double2 &b)
 {
-    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
         : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
         : "l"(p));
 }

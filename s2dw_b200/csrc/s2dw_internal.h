@@ -7,6 +7,7 @@
 #include <exception>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/s2dw_cuda.h"
@@ -44,6 +45,34 @@ int set_error(int code, const char *fmt, ...);
     catch (...) {                                                                             \
         return ::s2dw::set_error(S2DWC_ERROR_ARG_INVALID, "%s: unexpected exception", __func__); \
     }
+
+// Programmatic dependent launch: the kernels of a call that follow one another
+// on one stream are launched with it (`dep`), so that a kernel's CTAs are in
+// place, and its tables on their way, when its predecessor ends.  Every such
+// kernel calls pdl_start() first and pdl_wait() before it touches anything a
+// kernel before it reads or writes; launched without the attribute both do
+// nothing.  A kernel whose predecessor on the stream is not one of this call is
+// launched without it.
+template <typename... P, typename... A>
+inline cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool dep,
+                              A &&...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = dep ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
 
 // ---------------------------------------------------------------------------
 // Host helpers restating the reference's scalar routines.
@@ -292,19 +321,19 @@ enum Stage { STAGE_ANA_BETA, STAGE_ANA_ALPHA, STAGE_SYN_ALPHA, STAGE_SYN_BETA };
 // length M are given; false where the stage kernels have no transform of that
 // size (it then runs through launch_czt).
 bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta);
+int launch_stage(Stage st, const StageArgs &a, bool dep, cudaStream_t s);
+int launch_stage_beta(Stage st, const StageArgs &a, bool dep, cudaStream_t s);
 // The length-1023 alpha rows have a kernel of their own: a launch holds only
 // such entries or none.
 bool stage_alone(const StageEnt &e);
-int launch_stage(Stage st, const StageArgs &a, cudaStream_t s);
-int launch_stage_beta(Stage st, const StageArgs &a, cudaStream_t s);
 
-int launch_lwalk(const LwalkArgs &a, cudaStream_t s);
+int launch_lwalk(const LwalkArgs &a, bool dep, cudaStream_t s);
 int launch_gprep(const GprepArgs &a, cudaStream_t s);
 // F[l*Bp + m] = Om[l*Bp + m] * flm[l + B*m] for m <= l < B, zero for m > l, and
 // scoeff(0:bs-1,0:bs-1) = flm(0:bs-1,0:bs-1) (s2dw_core_mod.f90:773).
 int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs,
                  cudaStream_t s);
-int launch_mwalk(const MwalkArgs &a, cudaStream_t s);
+int launch_mwalk(const MwalkArgs &a, bool dep, cudaStream_t s);
 int launch_czt(const CztArgs &a, cudaStream_t s);
 void set_pfa(bool on);  // prime-factor alpha stages (default on; off: Bluestein)
 // Builds, once per device, the constant tables of the length-2047 and -511 alpha stages

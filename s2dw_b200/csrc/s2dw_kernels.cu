@@ -42,6 +42,7 @@ __global__ void gprep_kernel(GprepArgs a)
 __global__ void fprep_kernel(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs)
 {
     __shared__ double2 tile[32][33];
+    pdl_start();
     const int l0 = blockIdx.x * 32, mb = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
     for (int k = ty; k < 32; k += 8) {
@@ -1050,8 +1051,10 @@ __global__ void __launch_bounds__(PFC_THREADS, 6) pfa1023_kernel(const __grid_co
 {
     constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1, NT = PFC_THREADS;
     extern __shared__ __align__(16) double2 smem[];
+    pdl_start();
     int cta;
     const StageEnt &e = stage_entry(a, cta);
+    pdl_wait();
     const int t = threadIdx.x;
     alpha_rows_in<MODE, PFC_N, 1, NT>(e, cta, [&](int, int m) -> double2 & { return smem[pfc_in_pos(m)]; });
     __syncthreads();
@@ -1149,8 +1152,10 @@ template <int MODE, bool BIG>
 __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __grid_constant__ StageArgs a)
 {
     extern __shared__ __align__(16) double2 smem[];
+    pdl_start();
     int cta;
     const StageEnt &e = stage_entry(a, cta);
+    pdl_wait();
     if (e.kind == STAGE_PFA) {
         switch (e.bl) {
         case 2: pfs_rows_run<3, 1, 1, MODE>(e, cta, smem); break;
@@ -1417,14 +1422,13 @@ bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta)
 
 bool stage_alone(const StageEnt &e) { return e.kind == STAGE_PFA && e.bl == 512; }
 
-int launch_stage(Stage st, const StageArgs &a, cudaStream_t s)
+int launch_stage(Stage st, const StageArgs &a, bool dep, cudaStream_t s)
 {
-    if (st == STAGE_ANA_BETA || st == STAGE_SYN_BETA) return launch_stage_beta(st, a, s);
+    if (st == STAGE_ANA_BETA || st == STAGE_SYN_BETA) return launch_stage_beta(st, a, dep, s);
     if (a.ncta <= 0) return S2DWC_OK;
     if (stage_alone(a.e[0])) {
-        if (st == STAGE_ANA_ALPHA) pfa1023_kernel<CZT_ANA_ALPHA><<<a.ncta, PFC_THREADS, sizeof(double2) * PFC_N, s>>>(a);
-        else pfa1023_kernel<CZT_SYN_ALPHA><<<a.ncta, PFC_THREADS, sizeof(double2) * PFC_N, s>>>(a);
-        S2DW_CUDA_TRY(cudaGetLastError());
+        auto *k = st == STAGE_ANA_ALPHA ? pfa1023_kernel<CZT_ANA_ALPHA> : pfa1023_kernel<CZT_SYN_ALPHA>;
+        S2DW_CUDA_TRY(launch_dep(k, a.ncta, PFC_THREADS, sizeof(double2) * PFC_N, s, dep, a));
         return S2DWC_OK;
     }
     size_t smem = 0;  // of the group's largest row set
@@ -1446,14 +1450,9 @@ int launch_stage(Stage st, const StageArgs &a, cudaStream_t s)
         smem = std::max(smem, n * sizeof(double2));
         big = big || e.lg >= 10;
     }
-    if (st == STAGE_ANA_ALPHA) {
-        if (big) alpha_kernel<CZT_ANA_ALPHA, true><<<a.ncta, ST_THREADS, smem, s>>>(a);
-        else alpha_kernel<CZT_ANA_ALPHA, false><<<a.ncta, ST_THREADS, smem, s>>>(a);
-    } else {
-        if (big) alpha_kernel<CZT_SYN_ALPHA, true><<<a.ncta, ST_THREADS, smem, s>>>(a);
-        else alpha_kernel<CZT_SYN_ALPHA, false><<<a.ncta, ST_THREADS, smem, s>>>(a);
-    }
-    S2DW_CUDA_TRY(cudaGetLastError());
+    auto *k = st == STAGE_ANA_ALPHA ? (big ? alpha_kernel<CZT_ANA_ALPHA, true> : alpha_kernel<CZT_ANA_ALPHA, false>)
+                                    : (big ? alpha_kernel<CZT_SYN_ALPHA, true> : alpha_kernel<CZT_SYN_ALPHA, false>);
+    S2DW_CUDA_TRY(launch_dep(k, a.ncta, ST_THREADS, smem, s, dep, a));
     return S2DWC_OK;
 }
 

@@ -615,10 +615,11 @@ bool stage_small(const s2dwc_plan *p, int j, Stage st)
 // One stage of scales `js` for `maps` maps on stream s, in as few launches as
 // their transforms allow: the large ones one launch each (per map), the rest
 // together.  in(j) and out(j): the first map's input and output of scale j;
-// im(j), om(j): values between maps.
+// im(j), om(j): values between maps.  dep: the launch before on `s` is one of
+// the same call (launch_dep).
 template <typename In, typename Out, typename Im, typename Om>
 int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In in, Out out, Im im, Om om,
-              cudaStream_t s)
+              cudaStream_t s, bool dep = false)
 {
     int st;
     StageArgs sa{};
@@ -630,7 +631,7 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
     auto flush = [&]() -> int {
         if (sa.n == 0) return S2DWC_OK;
         KernelTimer kt(p, stage_kind(stg), s);
-        const int e = launch_stage(stg, sa, s);
+        const int e = launch_stage(stg, sa, dep && !p->timing, s);
         sa.n = sa.ncta = 0;
         return e;
     };
@@ -751,13 +752,13 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
     LwalkArgs la = lwalk_args(p, p->Fw, p->wsC);
     {
         KernelTimer kt(p, S2DWC_KIND_LWALK, s);
-        if ((st = launch_lwalk(la, s))) return st;
+        if ((st = launch_lwalk(la, !p->timing, s))) return st;
     }
     if (p->slm_general) {  // the b part of a general Slm, accumulated into Tg
         la.G = p->GA_b;
         la.acc_imag = 1;
         KernelTimer kt(p, S2DWC_KIND_LWALK, s);
-        if ((st = launch_lwalk(la, s))) return st;
+        if ((st = launch_lwalk(la, !p->timing, s))) return st;
     }
     const bool serial = full_band_serial && !p->timing && (int)p->ev_done.size() == p->J + 1;
     auto groups = scale_groups(p, STAGE_ANA_BETA, STAGE_ANA_ALPHA, (bool)after);
@@ -771,8 +772,8 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         auto Tg = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
         auto Tb = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
         auto wav = [&](int j) -> double * { return d_wav + p->wav_off[j]; };
-        if ((e = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj))) return e;
-        if ((e = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj))) return e;
+        if ((e = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj, sj == s))) return e;
+        if ((e = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj, true))) return e;
         if (full) {
             S2DW_CUDA_TRY(cudaEventRecord(p->ev_done[j0], sj));
             prev_full = j0;
@@ -803,19 +804,24 @@ int run_synthesis(s2dwc_plan *p, double2 *d_flm, const double *d_wav, const doub
         auto V = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
         auto V2f = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
         if ((e = run_stage(p, STAGE_SYN_ALPHA, js, 1, wav, V, one_map, one_map, sj))) return e;
-        return run_stage(p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj);
+        return run_stage(p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj, true);
     });
     if (st) return st;
     MwalkArgs ma = mwalk_args(p, d_flm, d_scoeff);
+    // CTAs placed while the beta stage still runs pile up on the SMs that are
+    // free first: harmless up to one tile per SM, where the launch is bound by
+    // its longest walk (B=128 N=1 synthesis 35 -> 27 us), but more tiles need an
+    // even spread (B=256 N=5: 80 us, placed early 112)
+    const bool dep = !p->timing && groups.size() == 1 && ma.ntiles <= 148;
     {
         KernelTimer kt(p, S2DWC_KIND_MWALK, s);
-        if ((st = launch_mwalk(ma, s))) return st;
+        if ((st = launch_mwalk(ma, dep, s))) return st;
     }
     if (p->slm_general) {  // the b part of a general Slm, added to flm
         ma.GT = p->GT_b;
         ma.acc_imag = 1;
         KernelTimer kt(p, S2DWC_KIND_MWALK, s);
-        if ((st = launch_mwalk(ma, s))) return st;
+        if ((st = launch_mwalk(ma, dep, s))) return st;
     }
     return S2DWC_OK;
 }
@@ -856,11 +862,11 @@ int run_analysis_serial(s2dwc_plan *p, unsigned char *ws, double *d_wav, double2
         LwalkArgs la = lwalk_args(p, F, Tg);
         la.only = j;  // into the one Tg
         la.off[j] = 0;
-        if ((st = launch_lwalk(la, s))) return st;
+        if ((st = launch_lwalk(la, true, s))) return st;
         if (p->slm_general) {  // the b part of a general Slm, accumulated into Tg
             la.G = p->GA_b;
             la.acc_imag = 1;
-            if ((st = launch_lwalk(la, s))) return st;
+            if ((st = launch_lwalk(la, true, s))) return st;
         }
         const std::vector<int> js{j};
         auto tg = [&](int) { return Tg; };
