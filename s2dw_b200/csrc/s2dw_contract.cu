@@ -251,12 +251,27 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
     using P0 = std::integral_constant<int, 0>;
     using P1 = std::integral_constant<int, 1>;
 
-    // Scale j ends: T(m, m', +-n) from the even- and odd-l sums of its slot
-    // K, then the gamma DFT.
+    // Scale j ends: T(m, m', +-n) from the even- and odd-l sums of its slot,
+    // then the gamma DFT, and the slot restarts at zero.
     // T(+n) = i^{n-m} conj(eta) (E+O), T(-n) = i^{-n-m} (-1)^{m'+n} eta (E-O),
-    // T(0) = i^{-m} (E+O); eta = 1 (N odd) or i (N even).
-    auto flush = [&](auto slot_tag, const int j) {
-        constexpr int K = decltype(slot_tag)::value;
+    // T(0) = i^{-m} (E+O); eta = 1 (N odd) or i (N even); F carries the i^{-m}.
+    // One copy of the code, for slot 0, between exchanges of the slots: small
+    // transforms meet most of this kernel's code once, cold.
+    auto flush = [&](const int j) {
+        const bool odd = NS == 2 && (j & 1);
+        auto exchange = [&]() {
+#pragma unroll
+            for (int s = 0; s < S; s++)
+#pragma unroll
+                for (int q = 0; q < NP; q++)
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        const double2 u = acc[0][p][s][q], v = acc[NS - 1][p][s][q];
+                        acc[0][p][s][q] = odd ? v : u;
+                        acc[NS - 1][p][s][q] = odd ? u : v;
+                    }
+        };
+        if (NS == 2) exchange();
         const int bl = a.bl[j];
         const double sc = ldexp(1.0, -Kw);
         const int ev = (N % 2 == 0) ? 1 : 0, ai = a.acc_imag ? 1 : 0;
@@ -269,15 +284,15 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
 #pragma unroll
                 for (int q = 0; q < NP; q++) {
                     const int n = a.nq[q];
-                    const double2 E = cscale(acc[K][0][s][q], sc), O = cscale(acc[K][1][s][q], sc);
+                    const double2 E = cscale(acc[0][0][s][q], sc), O = cscale(acc[0][1][s][q], sc);
                     // acc_imag: the b part of S enters the +n terms times -i (i^-1)
                     // and the -n terms times +i
                     if (n == 0) {
-                        Ts[q] = cipow(cadd(E, O), -m - ai);
+                        Ts[q] = cipow(cadd(E, O), -ai);
                         Td[q] = make_double2(0.0, 0.0);
                     } else {
-                        const double2 tp = cipow(cadd(E, O), n - m - ev - ai);
-                        double2 tm = cipow(csub(E, O), -n - m + ev + ai);
+                        const double2 tp = cipow(cadd(E, O), n - ev - ai);
+                        double2 tm = cipow(csub(E, O), -n + ev + ai);
                         if ((mp + n) & 1) tm = make_double2(-tm.x, -tm.y);
                         Ts[q] = cadd(tp, tm);
                         Td[q] = make_double2(tm.y - tp.y, tp.x - tm.x);  // i (tp - tm)
@@ -297,8 +312,9 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
                 }
             }
 #pragma unroll
-            for (int q = 0; q < NP; q++) acc[K][0][s][q] = acc[K][1][s][q] = make_double2(0.0, 0.0);
+            for (int q = 0; q < NP; q++) acc[0][0][s][q] = acc[0][1][s][q] = make_double2(0.0, 0.0);
         }
+        if (NS == 2) exchange();
     };
 
     // in the scaled domain: keep the values in range (warp-uniform)
@@ -335,6 +351,20 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         }
     };
 
+    // the next end, and the l up to which a slot has no scale in range yet
+    int nextb, b0, b1, btop;
+    auto next_scale = [&]() {
+        nextb = INT_MAX;
+        b0 = b1 = btop = INT_MAX;
+        if (jd < jlast) return;
+        nextb = a.bl[jd];
+        const int bD = a.blo[jd], bM = NS == 2 && jd > 0 ? a.blo[jd - 1] : INT_MAX;
+        const bool odd = NS == 2 && (jd & 1);
+        b0 = odd ? bM : bD;
+        b1 = odd ? bD : bM;
+        btop = NS == 1 ? b0 : max(b0, b1);
+    };
+    next_scale();
     for (int c = 0; c <= nchunks; c++) {
         const int lc = lstart + c * LW_CH;
         const int nl = c < nchunks ? min(LW_CH, bend - lc) : 0;
@@ -350,33 +380,31 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         }
         for (int li = 0;;) {
             // the scales that end here (the walk's last ones at l = bend)
-            while (jd >= jlast && lc + li >= a.bl[jd]) {
-                if (NS == 2 && (jd & 1)) flush(std::integral_constant<int, NS - 1>{}, jd);
-                else flush(P0{}, jd);
+            while (lc + li >= nextb) {
+                flush(jd);
                 jd--;
+                next_scale();
             }
             if (li >= nl) break;
             // run to the next scale's end
-            int le = min(nl, a.bl[jd] - lc);
-            const int bD = a.blo[jd], bM = NS == 2 && jd > 0 ? a.blo[jd - 1] : INT_MAX;
-            const int b0 = NS == 2 && (jd & 1) ? bM : bD, b1 = NS == 2 && (jd & 1) ? bD : bM;
+            int le = min(nl, nextb - lc);
             const int lo = lc + li;
-            if (li == 0 && le == LW_CH && lc > rampEnd && lc > b0 && (NS == 1 || lc > b1)) {
+            if (li == 0 && le == LW_CH && lc > rampEnd && lc > btop) {
                 // both slots accumulate at every step, no start value enters
-                if (NP <= 2 && Kw == 0) {
+                if (NP <= 2 && S > 1 && Kw == 0) {
                     full_chunk(b);
                     li = le;
                     continue;
                 }
                 full_chunk(b);
-            } else if (li == 0 && le == LW_CH && lc > rampEnd && lc + LW_CH - 1 <= min(b0, b1)) {
+            } else if (S > 1 && li == 0 && le == LW_CH && lc > rampEnd && lc + LW_CH - 1 <= min(b0, b1)) {
                 // below every scale's range: the recurrence alone
 #pragma unroll 1
                 for (int i = 0; i < LW_CH; i += 2) {
                     step(b, i, P0{}, false, 0, false, false);
                     step(b, i + 1, P1{}, false, 0, false, false);
                 }
-            } else if (lo > b0 && (NS == 1 || lo > b1)) {
+            } else if (S > 1 && lo > btop) {
                 // start values enter, or a part of a chunk
                 int l = lo;
                 if ((l & 1) && l < lc + le) {
@@ -390,17 +418,12 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
                 }
                 if (l < lc + le) step(b, l - lc, P0{}, true, l, true, true);
             } else {
-                // a slot without a scale in range: only up to where both are
-                const int top = max(b0, NS == 1 ? b0 : b1);
-                if (top < lc + le) le = top + 1 - lc;
-                int l = lo;
-                if ((l & 1) && l < lc + le) {
-                    step(b, l - lc, P1{}, true, l, l > b0, l > b1);
-                    l++;
-                }
+                // any l (for S > 1: a slot without a scale in range, only up to
+                // where both are)
+                if (S > 1 && btop < lc + le) le = btop + 1 - lc;
 #pragma unroll 1
-                for (; l < lc + le; l += 2) {
-                    step(b, l - lc, P0{}, true, l, l > b0, l > b1);
+                for (int l = lo & ~1; l < lc + le; l += 2) {
+                    if (l >= lo) step(b, l - lc, P0{}, true, l, l > b0, l > b1);
                     if (l + 1 < lc + le) step(b, l + 1 - lc, P1{}, true, l + 1, l + 1 > b0, l + 1 > b1);
                 }
             }

@@ -193,7 +193,7 @@ struct LwalkArgs {
     const double *Stm;    // [l0*B + k]
     const int32_t *Ste;
     const double *G;      // gpack_row(l, 2 NP): Om(l,m') d^l_{m'n_q} K_j(l) s(l,n_q), row slot NP + q, slot = j & 1
-    const double2 *F;     // [l*Bp + m] = Om(l,m) flm(l,m)
+    const double2 *F;     // [l*Bp + m] = i^{-m} Om(l,m) flm(l,m)
     const double2 *ph;    // [g (2N-1) + n+N-1] = exp(i pi n g / N)
     double2 *Tg;          // scale j: Tg + off[j], [g][m][m'] N x bl x bl
     const int2 *tiles;    // (p-tile, m-tile) per CTA, longest walks first
@@ -329,7 +329,7 @@ bool stage_alone(const StageEnt &e);
 
 int launch_lwalk(const LwalkArgs &a, bool dep, cudaStream_t s);
 int launch_gprep(const GprepArgs &a, cudaStream_t s);
-// F[l*Bp + m] = Om[l*Bp + m] * flm[l + B*m] for m <= l < B, zero for m > l, and
+// F[l*Bp + m] = i^{-m} Om[l*Bp + m] * flm[l + B*m] for m <= l < B, zero for m > l, and
 // scoeff(0:bs-1,0:bs-1) = flm(0:bs-1,0:bs-1) (s2dw_core_mod.f90:773).
 int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs,
                  cudaStream_t s);

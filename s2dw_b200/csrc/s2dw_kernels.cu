@@ -37,7 +37,7 @@ __global__ void gprep_kernel(GprepArgs a)
     }
 }
 
-// F[l*Bp + m] = Om[l*Bp+m] flm[l + B m]: transpose of the column-major flm
+// F[l*Bp + m] = i^{-m} Om[l*Bp+m] flm[l + B m]: transpose of the column-major flm
 // through a 32x32 shared tile.
 __global__ void fprep_kernel(double2 *F, double2 *scoeff, const double2 *flm, const double *Om, int B, int Bp, int bs)
 {
@@ -55,7 +55,11 @@ __global__ void fprep_kernel(double2 *F, double2 *scoeff, const double2 *flm, co
         const int l = l0 + k, m = mb + tx;
         if (l < B && m < Bp) {
             double2 v = make_double2(0.0, 0.0);
-            if (m <= l && m < B) v = cscale(tile[tx][k], Om[(size_t)l * Bp + m]);
+            if (m <= l && m < B) {
+                v = cscale(tile[tx][k], Om[(size_t)l * Bp + m]);
+                if (m & 1) v = make_double2(v.y, -v.x);  // i^{-m}
+                if (m & 2) v = make_double2(-v.x, -v.y);
+            }
             F[(size_t)l * Bp + m] = v;
         }
     }
