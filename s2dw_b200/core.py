@@ -120,9 +120,10 @@ def s2dw_core_analysis_flm2wav_dynamic(flm, K_gamma, Slm, J, B, N, bl_scoeff, al
     f = _f64(flm, (B, B), True)
     K = _f64(K_gamma, (J + 1, B))
     S = _f64(Slm, (B, N), True)
-    wavdyn = [np.zeros(wav_scale_shape(j, B, N, alpha), order="F") for j in range(J + 1)]
+    # every value is written by the library (J and the sizes are checked there)
+    wavdyn = [np.empty(wav_scale_shape(j, B, N, alpha), order="F") for j in range(J + 1)]
     ptrs = (_dp * (J + 1))(*[_p(w) for w in wavdyn])
-    sc = np.zeros((max(bl_scoeff, 0), max(bl_scoeff, 0)), dtype=np.complex128, order="F")
+    sc = np.empty((max(bl_scoeff, 0), max(bl_scoeff, 0)), dtype=np.complex128, order="F")
     check(lib().s2dwc_analysis_flm2wav_dynamic(ptrs, _p(sc), _p(f), _p(K), _p(S), int(J), int(B), int(N),
                                                int(bl_scoeff), float(alpha)))
     return wavdyn, sc

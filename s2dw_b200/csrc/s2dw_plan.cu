@@ -75,9 +75,10 @@ struct s2dwc_plan {
     double *hbWav = nullptr;
     double2 *hbFlm = nullptr, *hbSc = nullptr;
     int hbSc_n = 0;
-    // two page-locked staging buffers for pageable caller arrays (first use)
-    char *stage[2] = {nullptr, nullptr};
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+    // page-locked staging buffers for pageable caller arrays (first use)
+    static constexpr int STAGES = 2, STAGE_EVENTS = 16;
+    char *stage[STAGES] = {};
+    cudaEvent_t stage_ev[STAGE_EVENTS] = {};
     // host-buffer entry points: the caller's tables last folded in (compared
     // by content, so that repeated calls with the same K_gamma and Slm keep
     // the device tables), a copy stream, and per-scale events that order the
@@ -156,10 +157,10 @@ struct s2dwc_plan {
         if (ev_host) cudaEventDestroy(ev_host);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         for (void *p : allocs) cudaFree(p);
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < STAGES; i++)
             if (stage[i]) cudaFreeHost(stage[i]);
-            if (stage_ev[i]) cudaEventDestroy(stage_ev[i]);
-        }
+        for (auto ev : stage_ev)
+            if (ev) cudaEventDestroy(ev);
         cudaSetDevice(cur);
     }
 };
@@ -691,14 +692,16 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
 // The scales as groups, each run on one stream: a scale with a transform of
 // more than 2048 points (or the 2048-point beta of bl = 1024) fills the GPU and
 // is a group of its own, the rest are one.  Without the former there is one
-// group and everything runs on the caller's stream.  `each`: every scale by
-// itself (the host-buffer entry points, whose copies follow each scale).
+// group and everything runs on the caller's stream.  `each`: also the scales
+// with an eighth of the coefficients or more by themselves (the host-buffer
+// entry points, whose copies follow the groups).
 std::vector<std::vector<int>> scale_groups(const s2dwc_plan *p, Stage a, Stage b, bool each)
 {
     std::vector<std::vector<int>> g;
     std::vector<int> rest;
     for (int j = 0; j <= p->J; j++) {
-        if (each || !stage_small(p, j, a) || !stage_small(p, j, b)) g.push_back({j});
+        const bool alone = each && 8 * (p->wav_off[j + 1] - p->wav_off[j]) >= p->wav_off[p->J + 1];
+        if (alone || !stage_small(p, j, a) || !stage_small(p, j, b)) g.push_back({j});
         else rest.push_back(j);
     }
     if (!rest.empty()) g.push_back(rest);
@@ -737,10 +740,10 @@ constexpr auto one_map = [](int) { return 0LL; };
 
 // Runs the analysis: the F table and the contraction of all scales on `s`,
 // then the beta and alpha stages of the scales' groups.
-// full_band_serial (host-buffer entry points): the scales one by one, those of
-// the last scale's band limit one after another, the last scale first, so that
-// the first one's device-to-host copy overlaps the next one's kernels instead
-// of all of them finishing together at the end.
+// full_band_serial (host-buffer entry points): the groups from the last scale
+// to the first, the two full-band scales one after the other, so that the first
+// one's device-to-host copy overlaps the next one's kernels instead of both
+// finishing together at the end.
 int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 *d_flm, cudaStream_t s,
                  const ScaleHook &after = ScaleHook(), bool full_band_serial = false)
 {
@@ -767,7 +770,7 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
     return for_groups(p, groups, s, [&](const std::vector<int> &js, cudaStream_t sj) -> int {
         int e;
         const int j0 = js[0];
-        const bool full = serial && p->bl[j0] == p->bl[p->J];
+        const bool full = serial && p->bl[j0] == p->bl[0];
         if (full && prev_full >= 0) S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_done[prev_full], 0));
         auto Tg = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
         auto Tb = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
@@ -797,9 +800,9 @@ int run_synthesis(s2dwc_plan *p, double2 *d_flm, const double *d_wav, const doub
     if (largest_first) std::reverse(groups.begin(), groups.end());
     st = for_groups(p, groups, s, [&](const std::vector<int> &js, cudaStream_t sj) -> int {
         int e;
-        if (before)
-            for (int j : js)
-                if ((e = before(j, sj))) return e;
+        if (before)  // the last scale first, as the copies come in
+            for (auto it = js.rbegin(); it != js.rend(); ++it)
+                if ((e = before(*it, sj))) return e;
         auto wav = [&](int j) -> const double * { return d_wav + p->wav_off[j]; };
         auto V = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
         auto V2f = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
@@ -1996,20 +1999,24 @@ static int host_prepare(int B, int N, double alpha, int J, int bl_scoeff, const 
 }
 
 // Copies between pageable caller memory and the device through the plan's
-// two page-locked staging buffers: the DMA of one chunk overlaps the host
-// copy (OpenMP threads) of the other.  The driver's own pageable copies run
-// at about a third of the page-locked rate, which made the host entry points
-// three times slower for callers with ordinary (Fortran, numpy) arrays.
+// page-locked staging buffers: the DMA of some chunks overlaps the host copy
+// (OpenMP threads) of another.  The driver's own pageable copies run at about a
+// third of the page-locked rate.  Up to 32 MB in all the chunks are 4 MB (16 of
+// them in the two buffers): a chunk's DMA is 80 us, so that the parts of a call
+// without overlap, the first copy in and the last one out, stay short.  Larger
+// copies take 32 MB: their destination is often fresh memory, and then every
+// thread should have huge pages of its own to touch (B=512 N=4 analysis 5.0 ms
+// with 32 MB, 5.7 with 4 MB; B=256 N=4 1.57 ms with 32 MB, 0.71 with 4 MB).
 struct HostSeg {
     char *host;
     char *dev;
     size_t bytes;
 };
-constexpr size_t STAGE_BYTES = 32u << 20;
+constexpr size_t STAGE_BYTES = 32u << 20;  // of a buffer
 
-static void host_copy(char *dst, const char *src, size_t n)
+static void host_copy(char *dst, const char *src, size_t n, size_t chunk)
 {
-    const long long blk = 1 << 20, nb = (long long)((n + blk - 1) / blk);
+    const long long blk = (long long)chunk / 32, nb = (long long)((n + blk - 1) / blk);
 #pragma omp parallel for schedule(static)
     for (long long i = 0; i < nb; i++) {
         const size_t o = (size_t)(i * blk);
@@ -2025,9 +2032,13 @@ class StagedCopy {
   public:
     StagedCopy(s2dwc_plan *p, const std::vector<HostSeg> &segs, cudaStream_t s) : p_(p), s_(s)
     {
+        size_t total = 0;
+        for (const auto &g : segs) total += g.bytes;
+        chunk_ = total <= STAGE_BYTES ? STAGE_BYTES / (s2dwc_plan::STAGE_EVENTS / 2) : STAGE_BYTES;
+        NB = s2dwc_plan::STAGES * (STAGE_BYTES / chunk_);
         for (const auto &g : segs) {
-            for (size_t o = 0; o < g.bytes; o += STAGE_BYTES)
-                ch_.push_back({g.host + o, g.dev + o, std::min(STAGE_BYTES, g.bytes - o)});
+            for (size_t o = 0; o < g.bytes; o += chunk_)
+                ch_.push_back({g.host + o, g.dev + o, std::min(chunk_, g.bytes - o)});
             seg_end_.push_back(ch_.size());
         }
     }
@@ -2035,14 +2046,14 @@ class StagedCopy {
     // call's DMA on them.
     int start()
     {
-        for (int i = 0; i < 2; i++) {
-            if (!p_->stage[i]) {
-                S2DW_CUDA_TRY(
-                    cudaHostAlloc(reinterpret_cast<void **>(&p_->stage[i]), STAGE_BYTES, cudaHostAllocDefault));
-                S2DW_CUDA_TRY(cudaEventCreateWithFlags(&p_->stage_ev[i], cudaEventDisableTiming));
-                S2DW_CUDA_TRY(cudaEventRecord(p_->stage_ev[i], s_));
+        for (auto &buf : p_->stage)
+            if (!buf) S2DW_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&buf), STAGE_BYTES, cudaHostAllocDefault));
+        for (auto &ev : p_->stage_ev) {
+            if (!ev) {
+                S2DW_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+                S2DW_CUDA_TRY(cudaEventRecord(ev, s_));
             }
-            S2DW_CUDA_TRY(cudaEventSynchronize(p_->stage_ev[i]));
+            S2DW_CUDA_TRY(cudaEventSynchronize(ev));
         }
         return S2DWC_OK;
     }
@@ -2051,10 +2062,10 @@ class StagedCopy {
     {
         for (; next_ < seg_end_[k]; next_++) {
             const size_t i = next_;
-            const int b = (int)(i & 1);
-            if (i >= 2) S2DW_CUDA_TRY(cudaEventSynchronize(p_->stage_ev[b]));  // chunk i-2's DMA done
-            host_copy(p_->stage[b], ch_[i].host, ch_[i].n);
-            S2DW_CUDA_TRY(cudaMemcpyAsync(ch_[i].dev, p_->stage[b], ch_[i].n, cudaMemcpyHostToDevice, s_));
+            const int b = (int)(i % NB);
+            if (i >= NB) S2DW_CUDA_TRY(cudaEventSynchronize(p_->stage_ev[b]));  // chunk i-NB's DMA done
+            host_copy(buf(b), ch_[i].host, ch_[i].n, chunk_);
+            S2DW_CUDA_TRY(cudaMemcpyAsync(ch_[i].dev, buf(b), ch_[i].n, cudaMemcpyHostToDevice, s_));
             S2DW_CUDA_TRY(cudaEventRecord(p_->stage_ev[b], s_));
         }
         return S2DWC_OK;
@@ -2067,17 +2078,17 @@ class StagedCopy {
         size_t k = 0;  // segment of chunk i
         for (size_t i = 0; i < ch_.size(); i++) {
             while (seg_end_[k] <= i) k++;
-            const int b = (int)(i & 1);
+            const int b = (int)(i % NB);
             if (wait && i == (k ? seg_end_[k - 1] : 0))  // segment k's first chunk
                 S2DW_CUDA_TRY(cudaStreamWaitEvent(s_, wait[k], 0));
-            S2DW_CUDA_TRY(cudaMemcpyAsync(p_->stage[b], ch_[i].dev, ch_[i].n, cudaMemcpyDeviceToHost, s_));
+            S2DW_CUDA_TRY(cudaMemcpyAsync(buf(b), ch_[i].dev, ch_[i].n, cudaMemcpyDeviceToHost, s_));
             S2DW_CUDA_TRY(cudaEventRecord(p_->stage_ev[b], s_));
-            if (i >= 1) {  // the previous chunk, while this one's DMA runs
-                if (int st = drain(i - 1, seg_done)) return st;
+            if (i + 1 >= NB) {  // an earlier chunk, while the DMA of the next ones runs
+                if (int st = drain(i + 1 - NB, seg_done)) return st;
             }
         }
-        if (!ch_.empty())
-            if (int st = drain(ch_.size() - 1, seg_done)) return st;
+        for (size_t i = ch_.size() < NB ? 0 : ch_.size() + 1 - NB; i < ch_.size(); i++)
+            if (int st = drain(i, seg_done)) return st;
         // segments without chunks (empty scales) are complete at once
         if (seg_done)
             for (size_t q = 0; q < seg_end_.size(); q++)
@@ -2086,15 +2097,17 @@ class StagedCopy {
     }
 
   private:
+    char *buf(int b) { return p_->stage[b / (STAGE_BYTES / chunk_)] + (b % (STAGE_BYTES / chunk_)) * chunk_; }
+    size_t chunk_ = STAGE_BYTES, NB = s2dwc_plan::STAGES;  // buffers of chunk_ bytes
     struct Chunk {
         char *host, *dev;
         size_t n;
     };
     int drain(size_t i, const std::function<void(size_t)> &seg_done)
     {
-        const int b = (int)(i & 1);
+        const int b = (int)(i % NB);
         S2DW_CUDA_TRY(cudaEventSynchronize(p_->stage_ev[b]));
-        host_copy(ch_[i].host, p_->stage[b], ch_[i].n);
+        host_copy(ch_[i].host, buf(b), ch_[i].n, chunk_);
         if (seg_done)
             for (size_t q = 0; q < seg_end_.size(); q++)
                 if (seg_end_[q] == i + 1 && seg_end_[q] != (q ? seg_end_[q - 1] : 0)) seg_done(q);
@@ -2122,6 +2135,23 @@ static bool all_pinned(const void *const *ptrs, int n)
     return true;
 }
 
+// flm between the caller and the device on the legacy stream: queued (to the
+// device) or complete (to the host) on return.
+static int copy_flm(s2dwc_plan *p, double *host, double2 *dev, bool to_device)
+{
+    const size_t n = sizeof(double2) * (size_t)p->B * p->B;
+    const void *ptr = host;
+    if (all_pinned(&ptr, 1)) {
+        S2DW_CUDA_TRY(cudaMemcpyAsync(to_device ? (void *)dev : host, to_device ? (void *)host : dev, n,
+                                      to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, 0));
+        if (!to_device) S2DW_CUDA_TRY(cudaStreamSynchronize(0));
+        return S2DWC_OK;
+    }
+    StagedCopy c(p, {{reinterpret_cast<char *>(host), reinterpret_cast<char *>(dev), n}}, 0);
+    if (int st = c.start()) return st;
+    return to_device ? c.to_device_through(0) : c.to_host();
+}
+
 static int analysis_host(double *wav_static, double *const *wav_scales, double *scoeff, const double *flm,
                          const double *K_gamma, const double *Slm, int J, int B, int N, int bl_scoeff,
                          double alpha)
@@ -2134,7 +2164,7 @@ static int analysis_host(double *wav_static, double *const *wav_scales, double *
     int st = host_prepare(B, N, alpha, J, bl_scoeff, K_gamma, nullptr, Slm, &p, hb, lk);
     if (st) return st;
     DeviceGuard dg(p->device);
-    S2DW_CUDA_TRY(cudaMemcpy(hb.flm, flm, sizeof(double2) * (size_t)B * B, cudaMemcpyHostToDevice));
+    if ((st = copy_flm(p, const_cast<double *>(flm), hb.flm, true))) return st;
     // The scales' device-to-host copies overlap the other scales' kernels,
     // with the full-band scales run one after another.  Pinned per-scale
     // outputs: each copy follows its scale's kernels on the scale's stream.
@@ -2281,8 +2311,7 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
         cudaStreamSynchronize(p->copy_stream);  // no read of the caller's arrays outlives the call
         return st;
     }
-    S2DW_CUDA_TRY(cudaMemcpy(flm, hb.flm, sizeof(double2) * (size_t)B * B, cudaMemcpyDeviceToHost));
-    return S2DWC_OK;
+    return copy_flm(p, flm, hb.flm, false);
 }
 
 int s2dwc_synthesis_wav2flm(double *flm, const double *wav, const double *scoeff, const double *K_gamma,
