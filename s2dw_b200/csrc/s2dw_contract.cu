@@ -439,18 +439,26 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
 // CTA tile: TL = 16 P values of l by MT = 8 S values of m; a thread walks m'
 // from the largest l of the tile down to 0 for its P S pairs (l, m), l = l0 +
 // lane % 16 + 16 i.  Per step it reads b(l, m') and G(l, slot, q, m') of its l
-// by lane and V_j(m, m', q) of the two scales by broadcast, staged 4 values of
-// m' at a time.  The sum over the scales is in the accumulator, so flm is
+// by lane and V_j(m, m', q) of the two scales by broadcast, staged 4 to 16
+// values of m' at a time.  The sum over the scales is in the accumulator, so flm is
 // written directly (with the scaling part), without partial rows per scale.
 // P = 2, S = 4, NP = 2: 48 FP64-pipe cycles per step against 42 of shared
 // memory.  Tiles lie in one interval of l with the same two scales (MwalkArgs).
 // ===========================================================================
-constexpr int MW_CH = 4;
-
 template <int NP, int P, int S>
 struct MwalkSmem {
     static constexpr int TL = 16 * P, MT = 2 * WARPS * S, R = 2 * NP + 1;
-    static constexpr int ST = NP > 4 ? 2 : 3;                   // staging buffers
+    // m' per chunk: a barrier and the staging per chunk against shared memory.
+    // Measured on B200 (us): 2 x 4, N = 4: 4 510, 8 461; N = 8: 4 788, 8 932;
+    // 1 x 1 at B = 256, N = 2: 4 31, 8 23, 16 21; 2 x 2 at B = 512, N = 8: 4 171, 8
+    // 163; 1 x 2 at B = 512, N = 4: 4 101, 8 107
+    static constexpr int MW_CH = P * S == 8   ? (NP <= 2 ? 8 : 4)
+                                 : P * S == 4 ? 8
+                                 : P * S == 2 ? 4
+                                 : NP == 1    ? 16
+                                 : NP == 2    ? 8
+                                              : 4;
+    static constexpr int ST = NP > 4 ? 2 : 3;                // staging buffers
     static constexpr int T_OFF = 0;                             // [CH][R][TL]
     static constexpr int V_OFF = T_OFF + MW_CH * R * TL;        // double2 [2][NP][MT][CH]
     static constexpr int BUF = V_OFF + 2 * 2 * NP * MT * MW_CH;
@@ -477,7 +485,7 @@ template <int NP, int P, int S, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_constant__ MwalkArgs a)
 {
     using L = MwalkSmem<NP, P, S>;
-    constexpr int TL = L::TL, MT = L::MT, R = L::R, NST = L::ST;
+    constexpr int TL = L::TL, MT = L::MT, R = L::R, NST = L::ST, MW_CH = L::MW_CH;
     extern __shared__ __align__(16) double msm[];
     pdl_start();
     if ((int)blockIdx.x >= a.ntiles) {
@@ -529,7 +537,8 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
             const int f = tid + THREADS * i, k = f % MW_CH, r = f / MW_CH, u = r % MT, sq = r / MT;
             const bool isB = sq >= NP;
             const int q = isB ? sq - NP : sq, bl = isB ? blB : blA;
-            if ((NV % THREADS == 0 || f < NV) && m0 + u < bl)
+            // (chunks of 16 m' pass the end of a V row, padded to 8)
+            if ((NV % THREADS == 0 || f < NV) && m0 + u < bl && (MW_CH <= 8 || c0 + k < (isB ? VsB : VsA)))
                 cp16(b + L::V_OFF + 2 * f,
                      (isB ? VB : VA) + ((size_t)q * bl + m0 + u) * (isB ? VsB : VsA) + c0 + k);
         }
@@ -930,7 +939,7 @@ int launch_gpack(const GpackArgs &a, bool transposed, cudaStream_t s)
         const long long total = gpack_row(32 * ((a.B + 31) / 32), 2 * a.NP);
         gpack_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 32), 256, 0, s>>>(a);
     } else {
-        const dim3 grid(std::max(1, std::min(8, a.Lp / 256)), (a.B + 7) / 8 * 8);
+        const dim3 grid(std::max(1, std::min(8, a.Lp / 256)), (a.B + 15) / 16 * 16);
         gtpack_kernel<<<grid, 256, 0, s>>>(a);
     }
     S2DW_CUDA_TRY(cudaGetLastError());

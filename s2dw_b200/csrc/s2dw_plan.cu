@@ -299,7 +299,12 @@ int plan_build(s2dwc_plan *p)
                 {n, n, n, -1, 0, 0, 0},                              // CZT_SYN_ALPHA
                 {2 * b, 2 * b - 1, 4 * b, -1, 1, -2 * (b - 1), 0},  // CZT_SYN_BETA
             };
+            // beta transforms as one power-of-two FFT of length L = 2 bl (a
+            // DCT-III / DCT-II pair of that length) when 2 bl is a power of two
+            const int L2 = 2 * b;
+            const bool fft_beta = L2 >= 16 && L2 <= 4096 && (L2 & (L2 - 1)) == 0;
             for (int md = 0; md < 4; md++) {
+                if (fft_beta && (md == CZT_ANA_BETA || md == CZT_SYN_BETA)) continue;
                 CztSpec c = specs[md];
                 c.M = czt_size(c.K, c.Bout);
                 std::vector<double2> pre, post, Hf;
@@ -326,10 +331,7 @@ int plan_build(s2dwc_plan *p)
                     p->tw[c.M] = tw;
                 }
             }
-            // beta transforms as one power-of-two FFT of length L = 2 bl (a
-            // DCT-III / DCT-II pair of that length) when 2 bl is a power of two
-            const int L2 = 2 * b;
-            if (L2 >= 16 && L2 <= 4096 && (L2 & (L2 - 1)) == 0) {
+            if (fft_beta) {
                 std::vector<double2> twb;
                 build_beta_twiddles(b, twb);
                 for (int md : {(int)FFT_ANA_BETA, (int)FFT_SYN_BETA}) {
@@ -364,11 +366,14 @@ int plan_build(s2dwc_plan *p)
         p->syn_beta_mode.push_back(fftb ? FFT_SYN_BETA : CZT_SYN_BETA);
     }
     {
-        std::vector<double2> t(2048);
-        for (int k = 0; k < 2048; k++) {
-            const long double x = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / 2048.0L;
-            t[k] = make_double2((double)cosl(x), (double)sinl(x));
-        }
+        static const std::vector<double2> t = [] {  // built once per process
+            std::vector<double2> v(2048);
+            for (int k = 0; k < 2048; k++) {
+                const long double x = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / 2048.0L;
+                v[k] = make_double2((double)cosl(x), (double)sinl(x));
+            }
+            return v;
+        }();
         if ((st = dev_upload(p, &p->tw2048, t))) return st;
     }
     // kernel-table factors
@@ -389,7 +394,7 @@ int plan_build(s2dwc_plan *p)
     }
     p->Lp = (B + 63) / 64 * 64 + 64;
     p->gpk_total = gpack_row(32 * ((B + 31) / 32), 2 * p->NP);
-    p->gtp_total = gtpack_row((B + 7) / 8 * 8, 2 * p->NP + 1, p->Lp);
+    p->gtp_total = gtpack_row((B + 15) / 16 * 16, 2 * p->NP + 1, p->Lp);  // whole chunks of m'
     if ((st = dev_alloc(p, &p->GA, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT, (size_t)p->gtp_total)) ||
         (st = dev_alloc(p, &p->Fw, (size_t)Br * Bp + 64)))
         return st;
