@@ -111,18 +111,29 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, lp = lane & 15;
     const int B = a.B, Bp = a.Bp, N = a.N;
-    const int jlast = NS == 1 ? a.only : 0;
-    const int bend = a.bl[jlast];  // the largest band limit of the walk
     int2 tile;
-    if (NS == 1) tile = make_int2((int)blockIdx.x / ((bend + MT - 1) / MT), (int)blockIdx.x % ((bend + MT - 1) / MT));
-    else tile = a.tiles[blockIdx.x];
+    int jlast = 0, jfirst = a.J;  // the scales of this CTA: jlast <= j <= jfirst
+    if (NS == 1) {
+        jlast = jfirst = a.only;
+        const int tm = (a.bl[jlast] + MT - 1) / MT;
+        tile = make_int2((int)blockIdx.x / tm, (int)blockIdx.x % tm);
+    } else {
+        tile = a.tiles[blockIdx.x];
+        if (S == 1) {  // see lwalk_split
+            if (tile.x >> 16) jlast = a.jsplit;
+            else if (tile.y >> 16) jfirst = a.jsplit - 1;
+            tile.x &= 0xffff;
+            tile.y &= 0xffff;
+        }
+    }
+    const int bend = a.bl[jlast];  // the largest band limit of the walk
     const int p0 = tile.x * 16, m0 = tile.y * MT;
     const int mp = p0 + lp, mi = (w * 2 + (lane >> 4)) * S, mb = m0 + mi;
 
     // the scale that ends next: the last one that holds pairs of this tile
     int jd = jlast;
     if (NS == 2)
-        while (jd < a.J && a.bl[jd + 1] > max(p0, m0)) jd++;
+        while (jd < jfirst && a.bl[jd + 1] > max(p0, m0)) jd++;
 
     const int lstart = max(p0, m0) & ~(LW_CH - 1);
     const int rampEnd = min(max(p0 + 15, m0 + MT - 1), bend - 1);
@@ -341,11 +352,11 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
             Kw -= R;
         }
     };
-    auto full_chunk = [&](const double *b) {
+    auto full_chunk = [&](const double *b, int first) {
         // more unrolling hoists loads past the register cap
         constexpr int UNR = S == 1 || NP > 4 ? 2 : NP <= 2 ? 4 : 8;
 #pragma unroll UNR
-        for (int i = 0; i < LW_CH; i += 2) {
+        for (int i = first; i < LW_CH; i += 2) {
             step(b, i, P0{}, false, 0, true, true);
             step(b, i + 1, P1{}, false, 0, true, true);
         }
@@ -358,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         b0 = b1 = btop = INT_MAX;
         if (jd < jlast) return;
         nextb = a.bl[jd];
-        const int bD = a.blo[jd], bM = NS == 2 && jd > 0 ? a.blo[jd - 1] : INT_MAX;
+        const int bD = a.blo[jd], bM = NS == 2 && jd > jlast ? a.blo[jd - 1] : INT_MAX;
         const bool odd = NS == 2 && (jd & 1);
         b0 = odd ? bM : bD;
         b1 = odd ? bD : bM;
@@ -392,11 +403,16 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
             if (li == 0 && le == LW_CH && lc > rampEnd && lc > btop) {
                 // both slots accumulate at every step, no start value enters
                 if (NP <= 2 && S > 1 && Kw == 0) {
-                    full_chunk(b);
+                    full_chunk(b, 0);
                     li = le;
                     continue;
                 }
-                full_chunk(b);
+                full_chunk(b, 0);
+            } else if (S == 1 && li == 0 && le == LW_CH && lc > rampEnd && lc == btop) {
+                // one slot's scale starts after the first row
+                step(b, 0, P0{}, false, 0, lc > b0, lc > b1);
+                step(b, 1, P1{}, false, 0, true, true);
+                full_chunk(b, 2);
             } else if (S > 1 && li == 0 && le == LW_CH && lc > rampEnd && lc + LW_CH - 1 <= min(b0, b1)) {
                 // below every scale's range: the recurrence alone
 #pragma unroll 1
@@ -800,16 +816,35 @@ int lwalk_pairs(int B, int NP)
     return S;
 }
 
-void build_lwalk_tiles(int B, int S, std::vector<int2> &t)
+// Where the launch is bound by its longest walk (S = 1), the tiles that hold
+// pairs of the small scales (bl <= B/4) are two CTAs: one walks the small
+// scales' l and ends them (their many short ranges are cold code and flushes),
+// the other leaves them out.  B=256 N=4: 60,000 cycles in the longest CTA, half
+// of them before l = 64.
+int lwalk_split(const std::vector<int> &bl, int S)
 {
-    // work of tile (pt, mt): the walk from max(p0, m0) up; longest first
+    int j = 0;
+    while (j < (int)bl.size() && bl[j] > (bl[0] + 3) / 4) j++;
+    return S == 1 && j >= 2 && j < (int)bl.size() ? j : 0;
+}
+
+void build_lwalk_tiles(const std::vector<int> &bl, int S, int jsplit, std::vector<int2> &t)
+{
+    // work of tile (pt, mt): the walk from max(p0, m0) up; longest first.
+    // Bit 16 of y: without the small scales; of x: these alone
     t.clear();
-    const int MT = 2 * WARPS * S, tp = (B + 15) / 16, tm = (B + MT - 1) / MT;
+    const int B = bl[0], MT = 2 * WARPS * S, tp = (B + 15) / 16, tm = (B + MT - 1) / MT;
+    const int small = jsplit ? bl[jsplit] : 0;
     for (int pt = 0; pt < tp; pt++)
-        for (int mt = 0; mt < tm; mt++) t.push_back(make_int2(pt, mt));
-    std::stable_sort(t.begin(), t.end(), [MT](int2 a, int2 b) {
-        return std::max(a.x * 16, a.y * MT) < std::max(b.x * 16, b.y * MT);
-    });
+        for (int mt = 0; mt < tm; mt++) {
+            const bool both = std::max(pt * 16, mt * MT) < small;
+            t.push_back(make_int2(pt, mt | (both ? 1 << 16 : 0)));
+            if (both) t.push_back(make_int2(pt | 1 << 16, mt));
+        }
+    auto length = [&](int2 a) {
+        return (a.x >> 16 ? small : B) - std::max((a.x & 0xffff) * 16, (a.y & 0xffff) * MT);
+    };
+    std::stable_sort(t.begin(), t.end(), [&](int2 a, int2 b) { return length(a) > length(b); });
 }
 
 // P and S of the synthesis kernel by band limit.  Measured on B200 (us per

@@ -198,6 +198,7 @@ struct LwalkArgs {
     double2 *Tg;          // scale j: Tg + off[j], [g][m][m'] N x bl x bl
     const int2 *tiles;    // (p-tile, m-tile) per CTA, longest walks first
     int ntiles, S;        // S: m per half warp (lwalk_pairs)
+    int jsplit;           // first of the small scales with CTAs of their own (lwalk_split)
     int only;             // -1: every scale; else this scale alone
     // 0: Tg = T.  1: G holds the second real part b of S = eta (a + i b)
     // (a general complex Slm): Tg += T with the +n terms times -i and the
@@ -237,7 +238,8 @@ struct MwalkArgs {
 };
 // Tile lists, ordered by decreasing work so that the longest walks start first.
 int lwalk_pairs(int B, int NP);
-void build_lwalk_tiles(int B, int S, std::vector<int2> &t);
+int lwalk_split(const std::vector<int> &bl, int S);
+void build_lwalk_tiles(const std::vector<int> &bl, int S, int jsplit, std::vector<int2> &t);
 int2 mwalk_shape(int B, int NP);
 int build_mwalk_intervals(const std::vector<int> &bl, const std::vector<int> &blo, int B,
                           std::vector<MwalkInterval> &iv);

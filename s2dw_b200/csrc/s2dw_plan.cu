@@ -65,7 +65,7 @@ struct s2dwc_plan {
     std::vector<cudaStream_t> streams;
     // contraction tiles of all scales (device)
     int2 *lw_tiles = nullptr, *mw_tiles = nullptr;
-    int lw_ntiles = 0, mw_ntiles = 0, lw_pairs = 1;
+    int lw_ntiles = 0, mw_ntiles = 0, lw_pairs = 1, lw_split = 0;
     int2 mw_shape = {1, 1};
     std::vector<MwalkInterval> mw_iv;
     double2 *ph = nullptr;                    // gamma-DFT phases, LwalkArgs::ph
@@ -416,7 +416,8 @@ int plan_build(s2dwc_plan *p)
     {
         std::vector<int2> tl;
         p->lw_pairs = lwalk_pairs(B, p->NP);
-        build_lwalk_tiles(B, p->lw_pairs, tl);
+        p->lw_split = lwalk_split(p->bl, p->lw_pairs);
+        build_lwalk_tiles(p->bl, p->lw_pairs, p->lw_split, tl);
         if ((st = dev_upload(p, &p->lw_tiles, tl))) return st;
         p->lw_ntiles = (int)tl.size();
         p->mw_shape = mwalk_shape(B, p->NP);
@@ -542,6 +543,7 @@ LwalkArgs lwalk_args(const s2dwc_plan *p, const double2 *F, double2 *Tg)
     a.tiles = p->lw_tiles;
     a.ntiles = p->lw_ntiles;
     a.S = p->lw_pairs;
+    a.jsplit = p->lw_split;
     a.only = -1;
     for (int j = 0; j <= p->J; j++) {
         a.bl[j] = (short)p->bl[j];
