@@ -466,13 +466,13 @@ struct MwalkSmem {
     static constexpr int TL = 16 * P, MT = 2 * WARPS * S, R = 2 * NP + 1;
     // m' per chunk: a barrier and the staging per chunk against shared memory.
     // Measured on B200 (us): 2 x 4, N = 4: 4 510, 8 461; N = 8: 4 788, 8 932;
-    // 1 x 1 at B = 256, N = 2: 4 31, 8 23, 16 21; 2 x 2 at B = 512, N = 8: 4 171, 8
+    // 1 x 1 at B = 256, N = 2: 4 31, 8 23, 16 21, N = 5: 4 43, 8 38; 2 x 2 at B = 512, N = 8: 4 171, 8
     // 163; 1 x 2 at B = 512, N = 4: 4 101, 8 107
     static constexpr int MW_CH = P * S == 8   ? (NP <= 2 ? 8 : 4)
                                  : P * S == 4 ? 8
                                  : P * S == 2 ? 4
-                                 : NP == 1    ? 16
-                                 : NP == 2    ? 8
+                                 : NP <= 2    ? 16
+                                 : NP <= 4    ? 8
                                               : 4;
     static constexpr int ST = NP > 4 ? 2 : 3;                // staging buffers
     static constexpr int T_OFF = 0;                             // [CH][R][TL]
@@ -944,7 +944,7 @@ template <int NP>
 static int launch_mwalk_np(const MwalkArgs &a, bool dep, cudaStream_t s)
 {
     if (a.shape.x == 2 && a.shape.y == 4) return launch_mwalk_t<NP, 2, 4, 2>(a, dep, s);
-    if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, (NP <= 4 ? 5 : 3)>(a, dep, s);
+    if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, 3>(a, dep, s);
     if constexpr (NP <= 2) {
         if (a.shape.x == 1 && a.shape.y == 2) return launch_mwalk_t<NP, 1, 2, 1>(a, dep, s);
     } else {

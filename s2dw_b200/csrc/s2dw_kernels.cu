@@ -966,42 +966,48 @@ __global__ void rader73_init_kernel()
     g_rader73_w[blockIdx.x][k % 8 + 8 * (k % 9)] = make_double2(re / 72.0, im / 72.0);
 }
 
+// Two row pairs per CTA: 126 or 112 threads of 128 work in the convolution's
+// phases, and five CTAs hold ten rows on an SM (one row pair per CTA: 63 or 56
+// threads, six rows).
+constexpr int PFD_RP = 2;
+constexpr int PFD_ROW = PFD_XS + 7 * PFD_SP + 7;  // shared values of a row
+
 template <int MODE>
-__device__ __forceinline__ void pfa511_row(const StageEnt &e, int cta, double2 *smem)
+__device__ __forceinline__ void pfa511_rows(const StageEnt &e, int cta, double2 *smem)
 {
     constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1;
-    constexpr int NT = ST_THREADS;
-    double2 *X = smem;
-    double2 *Sc = smem + PFD_XS;
-    double2 *X0 = Sc + 7 * PFD_SP;
+    constexpr int NT = ST_THREADS, RP = PFD_RP;
     const int t = threadIdx.x;
-    alpha_rows_in<MODE, PFD_N, 1>(e, cta, [&](int, int m) -> double2 & {
-        return X[(m * 5) % 7 + PFD_P * ((m * 21) % 73)];
+    alpha_rows_in<MODE, PFD_N, RP>(e, cta, [&](int r, int m) -> double2 & {
+        return smem[r * PFD_ROW + (m * 5) % 7 + PFD_P * ((m * 21) % 73)];
     });
     __syncthreads();
     // length-7 DFTs along d1
-    for (int d2 = t; d2 < 73; d2 += NT) {
+    for (int i = t; i < RP * 73; i += NT) {
+        double2 *X = smem + (i / 73) * PFD_ROW + PFD_P * (i % 73);
         double2 x[7];
 #pragma unroll
-        for (int r = 0; r < 7; r++) x[r] = X[PFD_P * d2 + r];
-        pfa_dft_out<7, SIGN>(x, X, PFD_P * d2, 1);
+        for (int r = 0; r < 7; r++) x[r] = X[r];
+        pfa_dft_out<7, SIGN>(x, X, 0, 1);
     }
     __syncthreads();
     // length-73 DFTs along d2 (column c1) by Rader: forward length-8 DFTs
-    for (int u = t; u < 7 * 9; u += NT) {
-        const int c1 = u % 7, j = u / 7;
+    for (int i = t; i < RP * 7 * 9; i += NT) {
+        double2 *X = smem + (i / 63) * PFD_ROW, *Sc = X + PFD_XS, *X0 = Sc + 7 * PFD_SP;
+        const int u = i % 63, c1 = u % 7, j = u / 7;
         double2 v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = X[c1 + PFD_P * c_rader73_src[i + 8 * j]];
+        for (int k = 0; k < 8; k++) v[k] = X[c1 + PFD_P * c_rader73_src[k + 8 * j]];
         Dft<8, -1>::run(v);
 #pragma unroll
-        for (int i = 0; i < 8; i++) Sc[c1 * PFD_SP + i + 9 * j] = v[i];
+        for (int k = 0; k < 8; k++) Sc[c1 * PFD_SP + k + 9 * j] = v[k];
         if (j == 0) X0[c1] = X[c1];
     }
     __syncthreads();
     // forward length-9 DFTs, product with the DFT of w, inverse length-9
-    for (int u = t; u < 7 * 8; u += NT) {
-        const int c1 = u / 8, i = u % 8;
+    for (int k = t; k < RP * 7 * 8; k += NT) {
+        double2 *X = smem + (k / 56) * PFD_ROW, *Sc = X + PFD_XS, *X0 = Sc + 7 * PFD_SP;
+        const int u = k % 56, c1 = u / 8, i = u % 8;
         double2 v[9];
 #pragma unroll
         for (int jj = 0; jj < 9; jj++) v[jj] = Sc[c1 * PFD_SP + i + 9 * jj];
@@ -1015,18 +1021,21 @@ __device__ __forceinline__ void pfa511_row(const StageEnt &e, int cta, double2 *
     }
     __syncthreads();
     // inverse length-8 DFTs; y_{g^q} = x_0 + convolution
-    for (int u = t; u < 7 * 9; u += NT) {
-        const int c1 = u % 7, j = u / 7;
+    for (int i = t; i < RP * 7 * 9; i += NT) {
+        double2 *X = smem + (i / 63) * PFD_ROW, *Sc = X + PFD_XS, *X0 = Sc + 7 * PFD_SP;
+        const int u = i % 63, c1 = u % 7, j = u / 7;
         double2 v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = Sc[c1 * PFD_SP + i + 9 * j];
+        for (int k = 0; k < 8; k++) v[k] = Sc[c1 * PFD_SP + k + 9 * j];
         Dft<8, +1>::run(v);
         const double2 x0 = X0[c1];
 #pragma unroll
-        for (int i = 0; i < 8; i++) X[c1 + PFD_P * c_rader73_dst[i + 8 * j]] = cadd(x0, v[i]);
+        for (int k = 0; k < 8; k++) X[c1 + PFD_P * c_rader73_dst[k + 8 * j]] = cadd(x0, v[k]);
     }
     __syncthreads();
-    alpha_rows_out<MODE, PFD_N, 1>(e, cta, [&](int, int k) -> double2 { return X[k % 7 + PFD_P * (k % 73)]; });
+    alpha_rows_out<MODE, PFD_N, RP>(e, cta, [&](int r, int k) -> double2 {
+        return smem[r * PFD_ROW + k % 7 + PFD_P * (k % 73)];
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1167,7 +1176,7 @@ __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __
         case 8: pfs_rows_run<3, 5, 1, MODE>(e, cta, smem); break;
         case 32: pfs_rows_run<7, 9, 1, MODE>(e, cta, smem); break;
         case 128: pfs_rows_run<3, 5, 17, MODE>(e, cta, smem); break;
-        case 256: pfa511_row<MODE>(e, cta, smem); break;
+        case 256: pfa511_rows<MODE>(e, cta, smem); break;
         }
         return;
     }
@@ -1410,7 +1419,7 @@ bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta)
     if (alpha && g_pfa && bl <= 512 && bl >= 2 && (bl & (bl - 1)) == 0 && bl != 64 && bl != 16) {
         e->kind = STAGE_PFA;
         e->lg = 0;
-        per = bl >= 256 ? 1 : pfs_rows(2 * bl - 1);
+        per = bl == 512 ? 1 : bl == 256 ? PFD_RP : pfs_rows(2 * bl - 1);
     } else {
         // the 2048-point beta transforms of bl = 1024 keep their own kernels
         if (M < 16 || M > 2048 || (M & (M - 1)) || bl > 512) return false;
@@ -1447,7 +1456,7 @@ int launch_stage(Stage st, const StageArgs &a, bool dep, cudaStream_t s)
             S2DW_CUDA_TRY(cudaGetDevice(&dev));
             if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
                 return set_error(S2DWC_ERROR_NOT_INIT, "the length-511 alpha tables are not built on device %d", dev);
-            n = PFD_XS + 7 * PFD_SP + 7;
+            n = PFD_RP * PFD_ROW;
         } else {
             n = (size_t)pfs_rows(2 * e.bl - 1) * (2 * e.bl - 1);
         }
