@@ -313,6 +313,7 @@ constexpr int STAGE_PFA = 6;
 constexpr int STAGE_MAX = 24;  // entries per launch
 struct StageArgs {
     int n, ncta, N, NP;
+    int late;              // length-1023 alpha rows: does not depend on the launch before
     int nq[S2DW_NPMAX];
     const double2 *tw;     // exp(-2 pi i k / 2048), k < 2048
     const double2 *ph;     // LwalkArgs::ph

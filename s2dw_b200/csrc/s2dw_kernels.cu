@@ -780,6 +780,20 @@ __global__ void __launch_bounds__(NT, (NT == 128 ? 3 : 2)) pfa2047_alpha_kernel(
     }
 }
 
+// Alpha launches of one stage do not depend on one another: a second one
+// (late) starts while the first still runs and waits for it at its end instead.
+// That is safe as an alpha kernel lets its successor start only after its own
+// wait: what came before the first launch is then complete.
+__device__ __forceinline__ void alpha_begin(const StageArgs &a)
+{
+    if (!a.late) pdl_wait();
+    pdl_start();
+}
+__device__ __forceinline__ void alpha_end(const StageArgs &a)
+{
+    if (a.late) pdl_wait();
+}
+
 // ---------------------------------------------------------------------------
 // Row pairs of an alpha stage into and out of shared memory: RP pairs (g, rr)
 // of the transform of odd length N = 2 bl - 1, value m of pair r at at(r, m).
@@ -1064,10 +1078,9 @@ __global__ void __launch_bounds__(PFC_THREADS, 6) pfa1023_kernel(const __grid_co
 {
     constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1, NT = PFC_THREADS;
     extern __shared__ __align__(16) double2 smem[];
-    pdl_start();
     int cta;
     const StageEnt &e = stage_entry(a, cta);
-    pdl_wait();
+    alpha_begin(a);
     const int t = threadIdx.x;
     alpha_rows_in<MODE, PFC_N, 1, NT>(e, cta, [&](int, int m) -> double2 & { return smem[pfc_in_pos(m)]; });
     __syncthreads();
@@ -1087,6 +1100,7 @@ __global__ void __launch_bounds__(PFC_THREADS, 6) pfa1023_kernel(const __grid_co
     }
     __syncthreads();
     alpha_rows_out<MODE, PFC_N, 1, NT>(e, cta, [&](int, int k) -> double2 { return smem[pfc_out_pos(k)]; });
+    alpha_end(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1165,10 +1179,9 @@ template <int MODE, bool BIG>
 __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __grid_constant__ StageArgs a)
 {
     extern __shared__ __align__(16) double2 smem[];
-    pdl_start();
     int cta;
     const StageEnt &e = stage_entry(a, cta);
-    pdl_wait();
+    alpha_begin(a);
     if (e.kind == STAGE_PFA) {
         switch (e.bl) {
         case 2: pfs_rows_run<3, 1, 1, MODE>(e, cta, smem); break;
