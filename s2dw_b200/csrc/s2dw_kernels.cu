@@ -477,8 +477,24 @@ __global__ void __launch_bounds__((1 << LGM) / 16, (LGM == 11 ? 4 : LGM == 12 ? 
         } else {  // DCT-III input, as fft_large_kernel's FFT_ANA_BETA load
             sn = (rr + N - 1) & 1;
             x0 = stg[0];
+            // ana_beta_in with M = 2 bl and the half of each k known from i: no
+            // conditions between the twiddle loads, which are in flight together
+            double2 w[16];
 #pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = ana_beta_in(stg, lpos<LGM, R0>(t, i), bl, sn, a.czt.pre);
+            for (int i = 0; i < 16; i++) {
+                const int k = lpos<LGM, R0>(t, i);
+                const bool up = R0 == 8 ? (i & 7) >= 4 : i >= 8;
+                w[i] = __ldg(a.czt.pre + (up ? (M - k) & (M / 2 - 1) : k));
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const int k = lpos<LGM, R0>(t, i);
+                const bool up = R0 == 8 ? (i & 7) >= 4 : i >= 8;
+                const double2 x = stg[up ? (M - k) & (M / 2 - 1) : k];
+                const double2 y = cmul(x, up ? cconj(w[i]) : w[i]);
+                v[i] = !sn ? y : up ? make_double2(-y.y, y.x) : make_double2(y.y, -y.x);
+                if (up ? k == M / 2 : (sn && k == 0)) v[i] = zero;
+            }
         }
         __syncthreads();  // staging free: copy the next row while this one runs
         if (r + (int)gridDim.x < rows) pf_prefetch<MODE, THREADS>(a, r + gridDim.x, stg, t);
