@@ -252,6 +252,14 @@ struct RowFft {
     }
 };
 
+// Asynchronous 16-byte copies of values that the copying thread itself reads.
+__device__ __forceinline__ void cp16_own(double2 *smem, const double2 *gmem)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_own_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The entry (scale) of this CTA, and the CTA's index within it.
 __device__ __forceinline__ const StageEnt &stage_entry(const StageArgs &a, int &cta)
 {

@@ -267,16 +267,30 @@ __global__ void __launch_bounds__((1 << LGM) / 16, (LGM == 11 ? 4 : LGM == 12 ? 
         // threads), then the DCT-II reordering through shared memory: the
         // value of b goes to FFT index b/2 (b even) or (4bl-1-b)/2 (b odd)
         const bool sn = (rr + a.nq[g]) & 1;
-        // one gamma sample (row of V) at a time: its 16 loads per thread are
-        // independent, so they are all in flight together
 #pragma unroll
         for (int i = 0; i < 16; i++) v[i] = zero;
-        for (int gg = 0; gg < N; gg++) {
+        // Two rows of V at a time, the second through this transform's shared
+        // memory, each thread its own values: both are in flight together (B=2048
+        // N=8: 1.36 -> 1.21 ms per synthesis; in the stage kernels' smaller CTAs it
+        // was slower)
+        for (int gg = 0; gg < N; gg += 2) {
             const double2 *row = a.in_c + ((size_t)gg * bl + rr) * (2 * bl);
+            const bool two = gg + 1 < N;
+            if (two)
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    cp16_own(buf + t + i * THREADS, row + (size_t)bl * (2 * bl) + t + i * THREADS);
             const double2 w = ph[gg];
 #pragma unroll
             for (int i = 0; i < 16; i++) v[i] = cadd(v[i], cmul(row[t + i * THREADS], w));
+            if (two) {
+                cp_own_wait();
+                const double2 w1 = ph[gg + 1];
+#pragma unroll
+                for (int i = 0; i < 16; i++) v[i] = cadd(v[i], cmul(buf[t + i * THREADS], w1));
+            }
         }
+        __syncthreads();
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             const int b = t + i * THREADS;
