@@ -731,7 +731,7 @@ __global__ void gpack_kernel(GpackArgs a)
             int j = slot;
             while (j <= a.J && !(a.blo[j] < l && l < a.bl[j])) j += 2;
             if (j <= a.J)
-                v = a.T[(size_t)l * a.Bp + x] * a.H[((size_t)l * a.hn + a.nq[q]) * a.B + x] *
+                v = a.T[(size_t)l * a.Bp + x] * a.H[((size_t)l * NP + q) * a.B + x] *
                     a.kappa[((size_t)j * a.B + l) * NP + q];
         }
         a.out[i] = v;
@@ -754,7 +754,7 @@ __global__ void gtpack_kernel(GpackArgs a)
                 int j = r / NP;
                 while (j <= a.J && !(a.blo[j] < l && l < a.bl[j])) j += 2;
                 if (j <= a.J)
-                    v = a.T[(size_t)l * a.Bp + mp] * a.H[((size_t)l * a.hn + a.nq[q]) * a.B + mp] *
+                    v = a.T[(size_t)l * a.Bp + mp] * a.H[((size_t)l * NP + q) * a.B + mp] *
                         a.kappa[((size_t)j * a.B + l) * NP + q];
             }
         }

@@ -174,13 +174,15 @@ __host__ __device__ __forceinline__ long long gpack_row(int l, int R)
     const long long k = l >> 5;
     return R * (512 * k * (k + 1) + 32 * (l & 31) * (k + 1));
 }
-__host__ __device__ __forceinline__ int gtpack_start(int mp) { return mp < 64 ? 0 : 64 * ((mp >> 6) - 1); }
+// (a tile of at most 32 l reads the chunks of up to 16 m' that start at or
+// below its last l, so 32 values before the chunk's own m' are kept)
+__host__ __device__ __forceinline__ int gtpack_start(int mp) { return mp < 32 ? 0 : 16 * ((mp >> 4) - 2); }
 __host__ __device__ __forceinline__ int gtpack_len(int mp, int Lp) { return Lp - gtpack_start(mp); }
 __host__ __device__ __forceinline__ long long gtpack_row(int mp, int R, int Lp)
 {
-    const long long k = mp >> 6;
-    const long long skipped = k == 0 ? 0 : 32 * (k - 1) * (k - 2) + (mp & 63) * (k - 1);
-    return R * ((long long)mp * Lp - 64 * skipped);
+    const long long k = mp < 32 ? 0 : (mp >> 4) - 2;
+    const long long skipped = 8 * k * (k - 1) + (mp & 15) * k;  // /16
+    return R * ((long long)mp * Lp - 16 * skipped);
 }
 
 // Tables of the plan use a padded row stride Bp = roundup(B, 32); those that
@@ -220,7 +222,7 @@ struct MwalkArgs {
     const double *Em;     // [l*B + m]
     const int32_t *Ee;
     const double *GT;     // gtpack_row(m', 2 NP + 1, Lp): Gam(l,m') d^l_{m'n_q} c_j(l,n_q), row slot NP + q; row 2 NP: b(l,m')
-    int Lp;               // roundup(B, 64) + 64
+    int Lp;               // roundup(B, 8) + the tiles' l
     const double2 *V2f;   // scale j: V2f + offV[j], [(q*bl + m)*Vs + m']
     const double2 *scoeff;
     const double *Phi2;
@@ -248,9 +250,8 @@ void build_mwalk_tiles(const std::vector<MwalkInterval> &iv, int2 shape, std::ve
 // The tables G (from T = Om, kappa of the analysis) or, transposed, GT (from
 // T = Gam, kappa of the synthesis), built at set_tables time.
 struct GpackArgs {
-    int B, Bp, NP, hn, J, Lp;
-    int nq[S2DW_NPMAX];
-    const double *T, *H, *kappa, *Bcoef;  // kappa[(j*B + l)*NP + q]
+    int B, Bp, NP, J, Lp;
+    const double *T, *H, *kappa, *Bcoef;  // H[(l*NP + q)*B + m'], kappa[(j*B + l)*NP + q]
     double *out;
     short bl[S2DW_JMAX + 1], blo[S2DW_JMAX + 1];
 };
@@ -272,10 +273,9 @@ struct CombineArgs {
 
 // Per-scale factor tables of the split form (see SplitArgs / SplitSynArgs),
 // built at set_tables time: out[((l-blo-1)*NP+q)*stride + x] = T[l*Bp+x] *
-// H[(l*8+nq)*B+x] * kappa[l*NP+q] for x <= l, x < bl; zero elsewhere.
+// H[(l*NP+q)*B+x] * kappa[l*NP+q] for x <= l, x < bl; zero elsewhere.
 struct GprepArgs {
-    int B, Bp, NP, bl, blo, stride, hn;  // hn: n rows of H
-    int nq[S2DW_NPMAX];
+    int B, Bp, NP, bl, blo, stride;
     const double *T, *H, *kappa;
     double *out;
 };
@@ -339,9 +339,12 @@ int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *
 int launch_mwalk(const MwalkArgs &a, bool dep, cudaStream_t s);
 int launch_czt(const CztArgs &a, cudaStream_t s);
 void set_pfa(bool on);  // prime-factor alpha stages (default on; off: Bluestein)
-// Builds, once per device, the constant tables of the length-2047 and -511 alpha stages
+// Builds, once per device, the constant tables of the length-2047 and -511
+// alpha stages and the stages' twiddles
 // (the current device; synchronises).  Plan creation calls it, never a capture.
 int pfa_prepare();
+// The current device's table exp(-2 pi i k/2048) (built by pfa_prepare).
+int stage_twiddles(const double2 **tw);
 void set_alpha_prefetch(bool on);  // synthesis alpha / analysis beta stages: persistent kernel with prefetched input (default on)
 // scoeff (bs x bs) of `maps` maps
 int launch_scoeff_copy(double2 *scoeff, const double2 *flm, int B, int bs, int maps, cudaStream_t s);

@@ -10,6 +10,8 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
+#include <mutex>
 #include <vector>
 #include <cstdio>
 #include <type_traits>
@@ -32,7 +34,7 @@ __global__ void gprep_kernel(GprepArgs a)
         const int q = (int)(r % a.NP), l = a.blo + 1 + (int)(r / a.NP);
         double v = 0.0;
         if (x <= l && x < a.bl)
-            v = a.T[(size_t)l * a.Bp + x] * a.H[((size_t)l * a.hn + a.nq[q]) * a.B + x] * a.kappa[(size_t)l * a.NP + q];
+            v = a.T[(size_t)l * a.Bp + x] * a.H[((size_t)l * a.NP + q) * a.B + x] * a.kappa[(size_t)l * a.NP + q];
         a.out[i] = v;
     }
 }
@@ -1366,19 +1368,39 @@ static int launch_pfa2047(const CztArgs &a, cudaStream_t s)
 }
 
 static bool g_rader_ready[64] = {false};
+static __device__ double2 g_tw[ST_TW];
 
 int pfa_prepare()
 {
     int dev = 0;
     S2DW_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return set_error(S2DWC_ERROR_ARG_INVALID, "device index %d", dev);
+    static std::mutex mu;
+    std::lock_guard<std::mutex> g(mu);
     if (g_rader_ready[dev]) return S2DWC_OK;
+    static const std::vector<double2> tw = [] {
+        std::vector<double2> v(ST_TW);
+        for (int k = 0; k < ST_TW; k++) {
+            const long double x = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / (long double)ST_TW;
+            v[k] = make_double2((double)cosl(x), (double)sinl(x));
+        }
+        return v;
+    }();
+    S2DW_CUDA_TRY(cudaMemcpyToSymbol(g_tw, tw.data(), sizeof(double2) * ST_TW));
     rader_init_kernel<<<2, 96>>>();
     S2DW_CUDA_TRY(cudaGetLastError());
     rader73_init_kernel<<<2, 96>>>();
     S2DW_CUDA_TRY(cudaGetLastError());
     S2DW_CUDA_TRY(cudaStreamSynchronize(0));
     g_rader_ready[dev] = true;
+    return S2DWC_OK;
+}
+
+int stage_twiddles(const double2 **tw)
+{
+    void *p = nullptr;
+    S2DW_CUDA_TRY(cudaGetSymbolAddress(&p, g_tw));
+    *tw = static_cast<const double2 *>(p);
     return S2DWC_OK;
 }
 

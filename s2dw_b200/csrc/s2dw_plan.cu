@@ -29,7 +29,6 @@ struct s2dwc_plan {
     int B = 0, Bp = 0, N = 0, J = 0, device = 0, form = 0, NP = 0;
     double alpha = 0.0;
     int nq[S2DW_NPMAX] = {};
-    int hn = 8;  // n rows of H
     int bl_scoeff = 0;
     bool tables_set = false;
     std::vector<int> bl, blo;
@@ -42,7 +41,7 @@ struct s2dwc_plan {
     std::vector<std::array<CztDev, 6>> czt;
     std::vector<int> ana_beta_mode, syn_beta_mode;
     std::map<int, TwDev> tw;
-    double2 *tw2048 = nullptr;  // StageArgs::tw
+    const double2 *tw2048 = nullptr;  // StageArgs::tw, of the device
     std::vector<double *> wq;  // quadrature weights per scale
     // caller tables folded into per-scale factor tables
     double *kappaA = nullptr, *kappaS = nullptr, *Phi2 = nullptr;
@@ -262,7 +261,6 @@ int plan_build(s2dwc_plan *p)
             tp = it->second;
         }
     }
-    p->hn = hn;
     const RecTables &t = *tp;
     // row-padded copies (stride Bp) of the tables read by 32-wide tiles
     const int Bp = (B + 31) / 32 * 32;
@@ -279,9 +277,15 @@ int plan_build(s2dwc_plan *p)
     if ((st = dev_upload(p, &p->Om, pad(t.Om))) || (st = dev_upload(p, &p->Acoef, pad(t.Acoef, true))) ||
         (st = dev_upload(p, &p->Stm, t.Stm)) || (st = dev_upload(p, &p->Ste, t.Ste)) ||
         (st = dev_upload(p, &p->Gam, pad(t.Gam))) || (st = dev_upload(p, &p->Bcoef, pad(t.Bcoef))) ||
-        (st = dev_upload(p, &p->Em, t.Em)) || (st = dev_upload(p, &p->Ee, t.Ee)) ||
-        (st = dev_upload(p, &p->H, t.H)))
+        (st = dev_upload(p, &p->Em, t.Em)) || (st = dev_upload(p, &p->Ee, t.Ee)))
         return st;
+    {  // d^l_{m'n}(pi/2) of the plan's n alone: [(l*NP + q)*B + m']
+        std::vector<double> h((size_t)B * p->NP * B);
+        for (int l = 0; l < B; l++)
+            for (int q = 0; q < p->NP; q++)
+                std::copy_n(t.H.begin() + ((size_t)l * hn + p->nq[q]) * B, B, h.begin() + ((size_t)l * p->NP + q) * B);
+        if ((st = dev_upload(p, &p->H, h))) return st;
+    }
 
     // chirp-z tables per scale and mode
     p->czt.resize(J + 1);
@@ -365,17 +369,6 @@ int plan_build(s2dwc_plan *p)
         p->ana_beta_mode.push_back(fftb ? FFT_ANA_BETA : CZT_ANA_BETA);
         p->syn_beta_mode.push_back(fftb ? FFT_SYN_BETA : CZT_SYN_BETA);
     }
-    {
-        static const std::vector<double2> t = [] {  // built once per process
-            std::vector<double2> v(2048);
-            for (int k = 0; k < 2048; k++) {
-                const long double x = -2.0L * 3.141592653589793238462643383279502884L * (long double)k / 2048.0L;
-                v[k] = make_double2((double)cosl(x), (double)sinl(x));
-            }
-            return v;
-        }();
-        if ((st = dev_upload(p, &p->tw2048, t))) return st;
-    }
     // kernel-table factors
     if ((st = dev_alloc(p, &p->kappaA, (size_t)(J + 1) * B * p->NP)) ||
         (st = dev_alloc(p, &p->kappaS, (size_t)(J + 1) * B * p->NP)) ||
@@ -392,7 +385,8 @@ int plan_build(s2dwc_plan *p)
         na += (long long)nl * p->NP * p->ga_stride[j];
         ns += (long long)nl * p->NP * p->gs_stride[j];
     }
-    p->Lp = (B + 63) / 64 * 64 + 64;
+    p->mw_shape = mwalk_shape(B, p->NP);
+    p->Lp = (B + 7) / 8 * 8 + 16 * p->mw_shape.x;
     p->gpk_total = gpack_row(32 * ((B + 31) / 32), 2 * p->NP);
     p->gtp_total = gtpack_row((B + 15) / 16 * 16, 2 * p->NP + 1, p->Lp);  // whole chunks of m'
     if ((st = dev_alloc(p, &p->GA, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT, (size_t)p->gtp_total)) ||
@@ -420,7 +414,6 @@ int plan_build(s2dwc_plan *p)
         build_lwalk_tiles(p->bl, p->lw_pairs, p->lw_split, tl);
         if ((st = dev_upload(p, &p->lw_tiles, tl))) return st;
         p->lw_ntiles = (int)tl.size();
-        p->mw_shape = mwalk_shape(B, p->NP);
         if ((st = build_mwalk_intervals(p->bl, p->blo, B, p->mw_iv))) return st;
         if (p->mw_iv.size() > sizeof(MwalkArgs::iv_j))
             return set_error(S2DWC_ERROR_SIZE_INVALID, "%zu intervals of l", p->mw_iv.size());
@@ -436,10 +429,7 @@ int plan_build(s2dwc_plan *p)
         if ((st = dev_upload(p, &p->ph, ph))) return st;
     }
     if (p->dry) return S2DWC_OK;
-    if ((std::find(p->bl.begin(), p->bl.end(), 1024) != p->bl.end() ||
-         std::find(p->bl.begin(), p->bl.end(), 256) != p->bl.end()) &&
-        (st = pfa_prepare()))
-        return st;
+    if ((st = pfa_prepare()) || (st = stage_twiddles(&p->tw2048))) return st;
     p->streams.resize(J + 1);
     p->ev_join.resize(J + 1);
     for (int j = 0; j <= J; j++) {
@@ -1511,10 +1501,8 @@ int s2dwc_plan_set_tables(s2dwc_plan *p, const double *K_gamma, const double *Ph
         g.B = B;
         g.Bp = p->Bp;
         g.NP = NP;
-        g.hn = p->hn;
         g.J = J;
         g.Lp = p->Lp;
-        std::memcpy(g.nq, p->nq, sizeof(g.nq));
         g.H = p->H;
         g.Bcoef = p->Bcoef;
         for (int j = 0; j <= J; j++) {
@@ -1539,9 +1527,7 @@ int s2dwc_plan_set_tables(s2dwc_plan *p, const double *K_gamma, const double *Ph
         g.NP = NP;
         g.bl = p->bl[j];
         g.blo = p->blo[j];
-        std::memcpy(g.nq, p->nq, sizeof(g.nq));
         g.H = p->H;
-        g.hn = p->hn;
         g.T = p->Om;
         g.kappa = p->kappaA + (size_t)j * B * NP;
         g.stride = p->ga_stride[j];
