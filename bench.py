@@ -46,15 +46,15 @@ HBM_GBS = _hbm_gbs()
 UNIT = "pairs/s"
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of each
-# kernel kind, averaged over the 11 launches of each kind in one
+# kernel kind, averaged over the launches of each kind in one
 # analysis+synthesis pair at B=1024 N=4 alpha=2 J=10, from the ncu launch list
 # of `python -m s2dw_b200.workload 1024 4 1` (profiles/launches_B1024_N4.md).
 # Used only for the roofline "traffic" entry of that workload.
-NCU_TRAFFIC = {(1024, 4, 2.0): {"lwalk": 7.18e6, "mwalk": 10.89e6, "ana_beta": 27.22e6,
-                                "ana_alpha": 44.23e6, "syn_alpha": 44.30e6, "syn_beta": 31.00e6}}
+NCU_TRAFFIC = {(1024, 4, 2.0): {"lwalk": 130.63e6, "mwalk": 111.90e6, "ana_beta": 99.55e6,
+                                "ana_alpha": 121.71e6, "syn_alpha": 121.80e6, "syn_beta": 113.62e6}}
 NCU_TRAFFIC_SOURCE = ("ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum "
-                      "--clock-control none of `python -m s2dw_b200.workload 1024 4 1` (one pair, 11 launches of "
-                      "each kind), profiles/launches_B1024_N4.md")
+                      "--clock-control none of `python -m s2dw_b200.workload 1024 4 1` (one pair), "
+                      "profiles/launches_B1024_N4.md")
 
 
 def parse():

@@ -15,6 +15,13 @@
 // distinct doubles is one shared-memory cycle where 32 distinct ones are two
 // (measured: 1.00 and 2.00 cycles per warp read on B200; a 16-byte read that
 // all lanes of a half-warp share costs two in either layout).
+//
+// Against a launch per scale (us per pair, B200): B = 1024, N = 4 analysis 787
+// -> 430 (26.7 TFLOP/s algorithmic, FP64 pipe 60 %), synthesis 869 -> 465
+// (12.3 TFLOP/s, 58 %); B = 2048, N = 8 7110 -> 5990 and 7720 -> 5600.  What is
+// left: two CTAs of 250 registers per SM (eight warps) cover the dependent FP64
+// chain only in part, and an FP64 instruction with three distinct operands
+// issues every 0.565 cycles per SM instead of 0.5.
 #include <cuda_runtime.h>
 
 #include <algorithm>
