@@ -265,13 +265,15 @@ int s2dwc_plan_check(s2dwc_plan *plan);
  * No counterpart in the reference. */
 int s2dwc_plan_set_split_min_batch(s2dwc_plan *plan, int nmaps);
 
-/* CUDA stream priority of the plan's per-scale streams (CUDA's convention:
+/* CUDA stream priority of the plan's own streams (CUDA's convention:
  * lower values run first; clamped to cudaDeviceGetStreamPriorityRange).  The
  * plan's kernels, and those of CUDA graphs captured from its calls after
  * this one, then take SMs ahead of work of lower priority: a server gives
  * its small, latency-bound transforms precedence over the full-band scales
  * of large ones.  Waits for the plan's streams to drain; call it between
- * transforms, outside stream capture.  No counterpart in the reference. */
+ * transforms, outside stream capture.  A transform called on a stream of
+ * another priority is forked from that stream to the plan's own and joined
+ * back to it.  No counterpart in the reference. */
 int s2dwc_plan_set_priority(s2dwc_plan *plan, int priority);
 
 /* Bound, in nanoseconds, on every wait of the split-form kernels' pipeline

@@ -56,7 +56,7 @@ struct s2dwc_plan {
     std::vector<long long> ga_off, gs_off;       // per-scale offsets (doubles)
     std::vector<int> ga_stride, gs_stride;
     double2 *Fw = nullptr;                       // per-call F table [l*Bp + m]
-    // per-scale workspaces (scales run concurrently on their own streams):
+    // per-scale workspaces (the groups of scales run concurrently on streams):
     // A_j holds Tb / V (N x bl x 2bl), C_j holds Tg (N x bl x bl) / V2f; the
     // split form's partial flm rows of scale j, (bl-blo-1) x bl, start at offP
     double2 *wsA = nullptr, *wsC = nullptr;
@@ -69,6 +69,8 @@ struct s2dwc_plan {
     std::vector<MwalkInterval> mw_iv;
     double2 *ph = nullptr;                    // gamma-DFT phases, LwalkArgs::ph
     cudaEvent_t ev_fork = nullptr;
+    cudaStream_t prio_stream = nullptr;  // set_priority: where the FP64 form's transforms run
+    int prio = 0;                        // its priority
     std::vector<cudaEvent_t> ev_join;
     // device buffers of the host-buffer entry points (allocated on first use)
     double *hbWav = nullptr;
@@ -149,6 +151,7 @@ struct s2dwc_plan {
             cudaEventDestroy(std::get<2>(t));
         }
         for (auto st : streams) cudaStreamDestroy(st);
+        if (prio_stream) cudaStreamDestroy(prio_stream);
         for (auto ev : ev_join) cudaEventDestroy(ev);
         if (ev_fork) cudaEventDestroy(ev_fork);
         for (auto ev : ev_done) cudaEventDestroy(ev);
@@ -741,6 +744,34 @@ int for_groups(s2dwc_plan *p, const std::vector<std::vector<int>> &g, cudaStream
     return S2DWC_OK;
 }
 
+// True when a transform called on `s` runs on the plan's own stream: the plan
+// has a priority (s2dwc_plan_set_priority) that `s` does not have.  st: status.
+bool leaves_stream(s2dwc_plan *p, cudaStream_t s, int &st)
+{
+    st = S2DWC_OK;
+    if (!p->prio_stream || p->timing || s == p->prio_stream) return false;
+    int prio = 0;
+    const cudaError_t e = cudaStreamGetPriority(s, &prio);
+    if (e != cudaSuccess) {
+        st = set_error(S2DWC_ERROR_CUDA, "cudaStreamGetPriority: %s", cudaGetErrorString(e));
+        return true;
+    }
+    return prio != p->prio;
+}
+
+// Runs f on the plan's stream of its priority, forked from and joined to `s`.
+template <typename F>
+int at_priority(s2dwc_plan *p, cudaStream_t s, F &&f)
+{
+    int st;
+    S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
+    S2DW_CUDA_TRY(cudaStreamWaitEvent(p->prio_stream, p->ev_fork, 0));
+    if ((st = f(p->prio_stream))) return st;
+    S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, p->prio_stream));
+    S2DW_CUDA_TRY(cudaStreamWaitEvent(s, p->ev_fork, 0));
+    return S2DWC_OK;
+}
+
 // Per-scale hook: enqueued on scale j's stream after (analysis) or before
 // (synthesis) that scale's kernels; the host-buffer entry points use it to
 // overlap each scale's host<->device copy with the other scales' kernels.
@@ -758,6 +789,10 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
                  const ScaleHook &after = ScaleHook(), bool full_band_serial = false)
 {
     int st;
+    if (leaves_stream(p, s, st))
+        return st ? st : at_priority(p, s, [&](cudaStream_t q) {
+            return run_analysis(p, d_wav, d_scoeff, d_flm, q, after, full_band_serial);
+        });
     {
         KernelTimer kt(p, S2DWC_KIND_OTHER, s);
         if ((st = launch_fprep(p->Fw, d_scoeff, d_flm, p->Om, p->B, p->Bp, p->bl_scoeff, s))) return st;
@@ -806,6 +841,10 @@ int run_synthesis(s2dwc_plan *p, double2 *d_flm, const double *d_wav, const doub
                   cudaStream_t s, const ScaleHook &before = ScaleHook(), bool largest_first = false)
 {
     int st;
+    if (leaves_stream(p, s, st))
+        return st ? st : at_priority(p, s, [&](cudaStream_t q) {
+            return run_synthesis(p, d_flm, d_wav, d_scoeff, q, before, largest_first);
+        });
     auto groups = scale_groups(p, STAGE_SYN_ALPHA, STAGE_SYN_BETA, (bool)before);
     if (largest_first) std::reverse(groups.begin(), groups.end());
     st = for_groups(p, groups, s, [&](const std::vector<int> &js, cudaStream_t sj) -> int {
@@ -1850,6 +1889,13 @@ int s2dwc_plan_set_priority(s2dwc_plan *p, int priority)
     int least = 0, greatest = 0;
     S2DW_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     const int prio = std::min(least, std::max(greatest, priority));
+    if (p->prio_stream) {
+        S2DW_CUDA_TRY(cudaStreamSynchronize(p->prio_stream));
+        S2DW_CUDA_TRY(cudaStreamDestroy(p->prio_stream));
+        p->prio_stream = nullptr;
+    }
+    S2DW_CUDA_TRY(cudaStreamCreateWithPriority(&p->prio_stream, cudaStreamNonBlocking, prio));
+    p->prio = prio;
     for (auto &st : p->streams) {
         S2DW_CUDA_TRY(cudaStreamSynchronize(st));
         S2DW_CUDA_TRY(cudaStreamDestroy(st));

@@ -187,7 +187,7 @@ class Plan:
         check(lib().s2dwc_plan_set_split_min_batch(self._h, int(nmaps)))
 
     def set_priority(self, priority):
-        """CUDA stream priority of the plan's per-scale streams (lower runs
+        """CUDA stream priority of the plan's own streams (lower runs
         first); graphs captured afterwards keep it."""
         check(lib().s2dwc_plan_set_priority(self._h, int(priority)))
 
