@@ -474,10 +474,9 @@ struct MwalkSmem {
     // m' per chunk: a barrier and the staging per chunk against shared memory.
     // Measured on B200 (us): 2 x 4, N = 4: 4 510, 8 461; N = 8: 4 788, 8 932;
     // 1 x 1 at B = 256, N = 2: 4 31, 8 23, 16 21, N = 5: 4 43, 8 38; 2 x 2 at B = 512, N = 8: 4 171, 8
-    // 163; 1 x 2 at B = 512, N = 4: 4 101, 8 107
+    // 163
     static constexpr int MW_CH = P * S == 8   ? (NP <= 2 ? 8 : 4)
                                  : P * S == 4 ? 8
-                                 : P * S == 2 ? 4
                                  : NP <= 2    ? 16
                                  : NP <= 4    ? 8
                                               : 4;
@@ -854,15 +853,19 @@ void build_lwalk_tiles(const std::vector<int> &bl, int S, int jsplit, std::vecto
     std::stable_sort(t.begin(), t.end(), [&](int2 a, int2 b) { return length(a) > length(b); });
 }
 
-// P and S of the synthesis kernel by band limit.  Measured on B200 (us per
-// synthesis): B = 1024, N = 8: 2 x 4 783, 4 x 2 828, 2 x 2 916, 1 x 1 1636;
-// B = 512, N = 4: 1 x 2 99, 2 x 2 107, 2 x 4 120, 1 x 1 135 (N = 8: 2 x 2 169,
-// 1 x 2 185); B = 256, N = 5: 1 x 1 41, 1 x 2 46, 2 x 4 81 (few CTAs: the
-// longest walk bounds the launch).
+// P and S of the synthesis kernel by band limit: the smallest tile while there
+// are fewer tiles than CTA slots (the longest walk bounds the launch), larger
+// ones as the shared reads per pair begin to.  Measured on B200 (us per
+// synthesis of N = 4, 1 x 1, 2 x 2, 2 x 4): B = 384 61, 70, 86; 416 74, 77, 91;
+// 448 89, 83, 98; 512 121, 97, 113; 640 214, 162, 193; 768 356, 233, 272;
+// 896 556, 353, 324; 1024 824, 513, 465.  N = 2: 448 51, 58, 68; 480 60, 65,
+// 70; 512 72, 69, 76; 768 210, 157, 186; 896 326, 225, 218.  N = 8: 448 158,
+// 136, 162; 512 218, 160, 183; 896 1029, 602, 558.  (One l and two m per
+// thread lay between: N = 4 at 384 69, 512 100, 768 304.)
 int2 mwalk_shape(int B, int NP)
 {
-    if (B >= 768) return make_int2(2, 4);
-    if (B >= 384) return NP >= 3 ? make_int2(2, 2) : make_int2(1, 2);
+    if (B >= 832) return make_int2(2, 4);
+    if (B >= (NP == 1 ? 496 : 432)) return make_int2(2, 2);
     return make_int2(1, 1);
 }
 
@@ -952,11 +955,7 @@ static int launch_mwalk_np(const MwalkArgs &a, bool dep, cudaStream_t s)
 {
     if (a.shape.x == 2 && a.shape.y == 4) return launch_mwalk_t<NP, 2, 4, 2>(a, dep, s);
     if (a.shape.x == 1 && a.shape.y == 1) return launch_mwalk_t<NP, 1, 1, 3>(a, dep, s);
-    if constexpr (NP <= 2) {
-        if (a.shape.x == 1 && a.shape.y == 2) return launch_mwalk_t<NP, 1, 2, 1>(a, dep, s);
-    } else {
-        if (a.shape.x == 2 && a.shape.y == 2) return launch_mwalk_t<NP, 2, 2, 2>(a, dep, s);
-    }
+    if (a.shape.x == 2 && a.shape.y == 2) return launch_mwalk_t<NP, 2, 2, 2>(a, dep, s);
     return set_error(S2DWC_ERROR_ARG_INVALID, "mwalk: tile shape %d x %d", a.shape.x, a.shape.y);
 }
 

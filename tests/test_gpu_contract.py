@@ -16,7 +16,8 @@ from s2dw_b200.workload import gaussian_flm, transform_setup
 CASES = [
     (15, 4, 2.0, None), (16, 4, 2.0, None), (17, 4, 2.0, None), (31, 2, 1.5, None), (33, 3, 3.0, None),
     (48, 5, 1.7, None), (63, 7, 2.0, 3), (64, 8, 2.0, 1), (65, 1, 2.0, 2), (96, 6, 2.5, None), (130, 4, 3.0, 2),
-    (40, 12, 2.0, None), (34, 16, 1.3, None),
+    (40, 12, 2.0, None), (34, 16, 1.3, None), (431, 3, 2.0, None), (433, 4, 3.0, None), (495, 2, 2.0, None),
+    (497, 1, 2.0, None), (450, 10, 2.0, 1),
 ]
 
 
