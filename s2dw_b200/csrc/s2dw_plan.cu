@@ -189,14 +189,32 @@ int dev_alloc(s2dwc_plan *p, T **ptr, size_t count)
                          "plan memory limit: %zu more bytes would take the plan to %lld bytes, above the "
                          "limit of %lld", count * sizeof(T), p->ws_bytes + (long long)(count * sizeof(T)), lim);
     cudaError_t e = cudaMalloc(&v, count * sizeof(T));
-    if (e != cudaSuccess)
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here: not the next launch's error
         return set_error(S2DWC_ERROR_MEM_ALLOC_FAIL, "cudaMalloc of %zu bytes failed: %s",
                          count * sizeof(T), cudaGetErrorString(e));
+    }
     p->allocs.push_back(v);
     p->ws_bytes += (long long)(count * sizeof(T));
     *ptr = static_cast<T *>(v);
     return S2DWC_OK;
 }
+
+// Several allocations as one: what dev_alloc gave the plan since the
+// construction is taken back at the end of the scope unless `keep` is set.
+struct AllocGroup {
+    s2dwc_plan *p;
+    size_t n;
+    long long bytes;
+    bool keep = false;
+    explicit AllocGroup(s2dwc_plan *p_) : p(p_), n(p_->allocs.size()), bytes(p_->ws_bytes) {}
+    ~AllocGroup()
+    {
+        if (keep) return;
+        for (; p->allocs.size() > n; p->allocs.pop_back()) cudaFree(p->allocs.back());
+        p->ws_bytes = bytes;
+    }
+};
 
 // Frees a buffer of `count` elements allocated by dev_alloc.
 template <typename T>
@@ -931,100 +949,113 @@ int run_analysis_serial(s2dwc_plan *p, unsigned char *ws, double *d_wav, double2
 }
 
 // Split form: per-scale workspaces (the scales of a batch run concurrently
-// on the plan's streams), tile lists and the per-row exponent tables (the
-// latter depend on the kernel tables and are rebuilt after set_tables).
+// on the plan's streams) and tile lists, all or none of them.
+int split_alloc(s2dwc_plan *p, cudaStream_t s)
+{
+    int st;
+    AllocGroup mem(p);
+    const int NP = p->NP, CH = split_chains(NP), MAPS = split_maps_per_pass(), MC = split_syn_mc(NP);
+    p->sp.assign(p->J + 1, {});
+    p->sp_small.clear();
+    p->sp_err = nullptr;
+    int *err = nullptr;
+    long long nd = 0, ns = 0, fdig = 0, fexp = 0, tg = 0, tb = 0, v2f = 0, vdig = 0;
+    for (int j = 0; j <= p->J; j++) {
+        auto &S = p->sp[j];
+        const int bl = p->bl[j], blo = p->blo[j], nl = bl - blo - 1;
+        const long long Vs = p->gs_stride[j];
+        S.c0 = (blo + 1) / 32;
+        S.nch = (bl - 1) / 32 - S.c0 + 1;
+        S.snch = (bl + MC - 1) / MC;
+        S.dexp_off = nd;
+        nd += (long long)bl * bl * NP;
+        S.sexp_off = ns;
+        ns += (long long)bl * bl;
+        S.fdig_off = fdig;
+        fdig += (split_fdig_bytes(bl, S.nch) + 255) / 256 * 256;
+        S.vdig_off = vdig;
+        vdig += (split_vdig_bytes(bl, S.snch) + 255) / 256 * 256;
+        S.fexp_off = fexp;
+        fexp += (long long)bl * 64;
+        S.tg_off = tg;
+        tg += (long long)p->N * bl * bl;
+        tb += (long long)p->N * bl * 2 * bl;
+        if ((long long)p->N * bl * 2 * bl * (long long)sizeof(double2) < (16LL << 20)) p->sp_small.push_back(j);
+        S.vstride = (long long)NP * bl * Vs;
+        S.v2f_off = v2f;
+        v2f += S.vstride;
+        // analysis tiles (m, chain tile), longest walks (smallest first row) first
+        std::vector<int2> tl;
+        const int np = (bl + CH - 1) / CH;
+        for (int m = 0; m < bl; m++)
+            for (int pt = 0; pt < np; pt++) tl.push_back(make_int2(m, pt));
+        std::stable_sort(tl.begin(), tl.end(), [CH](int2 a, int2 b) {
+            return std::max(a.x, a.y * CH) < std::max(b.x, b.y * CH);
+        });
+        S.ntiles = (int)tl.size();
+        if ((st = dev_upload(p, &S.tiles, tl))) return st;
+        // synthesis tiles (m, 128-row l tile), m-major so that the tiles of
+        // one m share its map digits in L2
+        tl.clear();
+        for (int m = 0; m < bl; m++)
+            for (int lt = 0; lt * 128 < nl; lt++) {
+                const int lbase = blo + 1 + lt * 128;
+                if (m <= std::min(lbase + 127, bl - 1)) tl.push_back(make_int2(m, lt));
+            }
+        S.sntiles = (int)tl.size();
+        if (tl.empty()) tl.push_back(make_int2(0, 0));
+        if ((st = dev_upload(p, &S.stiles, tl))) return st;
+    }
+    p->sp_pstride = std::max(1LL, p->offP.back() + (long long)std::max(0, p->bl[p->J] - p->blo[p->J] - 1) * p->bl[p->J]);
+    if ((st = dev_alloc(p, &p->sp_dexp, (size_t)nd)) || (st = dev_alloc(p, &p->sp_sexp, (size_t)ns)) ||
+        (st = dev_alloc(p, &p->sp_fexp, (size_t)fexp)) || (st = dev_alloc(p, &p->sp_vexp, (size_t)fexp)) ||
+        (st = dev_alloc(p, &p->sp_fdig, (size_t)fdig)) || (st = dev_alloc(p, &p->sp_vdig, (size_t)vdig)) ||
+        (st = dev_alloc(p, &err, 1)))
+        return st;
+    // Tb of the small scales for a chunk of maps: about 64 MB, which stay
+    // in L2 between the beta and the alpha stage, or one map's Tb of every
+    // scale where a memory limit leaves no more
+    long long one = 0;
+    for (int j : p->sp_small) one += (long long)p->N * p->bl[j] * 2 * p->bl[j];
+    auto chunk = [&](long long values) { return (int)std::max(1LL, std::min((long long)MAPS, one ? values / one : 1)); };
+    p->sp_chunk = chunk((64LL << 20) / (long long)sizeof(double2));
+    if (one && (p->sp_chunk * one <= tb || dev_alloc(p, &p->sp_Tb, (size_t)(p->sp_chunk * one)))) {
+        p->sp_chunk = std::min(p->sp_chunk, chunk(tb));
+        if ((st = dev_alloc(p, &p->sp_Tb, (size_t)std::max(tb, p->sp_chunk * one)))) return st;
+    }
+    long long off = 0;
+    for (int j : p->sp_small) {
+        p->sp[j].tb_off = off;
+        off += (long long)p->sp_chunk * p->N * p->bl[j] * 2 * p->bl[j];
+    }
+    p->sp_tg_map = tg;
+    p->sp_v2f_map = v2f;
+    S2DW_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), s));
+    // gamma-DFT phases exp(i pi n g / N), [g*16 + n+N-1]
+    std::vector<double2> ph((size_t)p->N * 16, make_double2(0.0, 0.0));
+    for (int g = 0; g < p->N; g++)
+        for (int n = -(p->N - 1); n <= p->N - 1; n++) {
+            const long double x = 3.141592653589793238462643383279502884L * (long double)(n * g) / (long double)p->N;
+            ph[(size_t)g * 16 + n + p->N - 1] = make_double2((double)cosl(x), (double)sinl(x));
+        }
+    if ((st = dev_upload(p, &p->sp_ph, ph))) return st;
+    mem.keep = true;
+    p->sp_err = err;
+    p->sp_alloc = true;
+    return S2DWC_OK;
+}
+
+// Split form: the workspaces of split_alloc, those of up to 32 maps, and the
+// per-row exponent tables (which depend on the kernel tables and are rebuilt
+// after set_tables).
 int split_prepare(s2dwc_plan *p, int nmaps, cudaStream_t s)
 {
     int st;
     if (p->slm_general)
         return set_error(S2DWC_ERROR_ARG_INVALID,
                          "the split form needs Slm of the form s2dw_core_init_directionality produces (S/eta real)");
-    const int NP = p->NP, CH = split_chains(NP), MAPS = split_maps_per_pass(), MC = split_syn_mc(NP);
-    if (!p->sp_alloc) {
-        p->sp.resize(p->J + 1);
-        long long nd = 0, ns = 0, fdig = 0, fexp = 0, tg = 0, tb = 0, v2f = 0, vdig = 0;
-        for (int j = 0; j <= p->J; j++) {
-            auto &S = p->sp[j];
-            const int bl = p->bl[j], blo = p->blo[j], nl = bl - blo - 1;
-            const long long Vs = p->gs_stride[j];
-            S.c0 = (blo + 1) / 32;
-            S.nch = (bl - 1) / 32 - S.c0 + 1;
-            S.snch = (bl + MC - 1) / MC;
-            S.dexp_off = nd;
-            nd += (long long)bl * bl * NP;
-            S.sexp_off = ns;
-            ns += (long long)bl * bl;
-            S.fdig_off = fdig;
-            fdig += (split_fdig_bytes(bl, S.nch) + 255) / 256 * 256;
-            S.vdig_off = vdig;
-            vdig += (split_vdig_bytes(bl, S.snch) + 255) / 256 * 256;
-            S.fexp_off = fexp;
-            fexp += (long long)bl * 64;
-            S.tg_off = tg;
-            tg += (long long)p->N * bl * bl;
-            tb += (long long)p->N * bl * 2 * bl;
-            if ((long long)p->N * bl * 2 * bl * (long long)sizeof(double2) < (16LL << 20)) p->sp_small.push_back(j);
-            S.vstride = (long long)NP * bl * Vs;
-            S.v2f_off = v2f;
-            v2f += S.vstride;
-            // analysis tiles (m, chain tile), longest walks (smallest first row) first
-            std::vector<int2> tl;
-            const int np = (bl + CH - 1) / CH;
-            for (int m = 0; m < bl; m++)
-                for (int pt = 0; pt < np; pt++) tl.push_back(make_int2(m, pt));
-            std::stable_sort(tl.begin(), tl.end(), [CH](int2 a, int2 b) {
-                return std::max(a.x, a.y * CH) < std::max(b.x, b.y * CH);
-            });
-            S.ntiles = (int)tl.size();
-            if ((st = dev_upload(p, &S.tiles, tl))) return st;
-            // synthesis tiles (m, 128-row l tile), m-major so that the tiles of
-            // one m share its map digits in L2
-            tl.clear();
-            for (int m = 0; m < bl; m++)
-                for (int lt = 0; lt * 128 < nl; lt++) {
-                    const int lbase = blo + 1 + lt * 128;
-                    if (m <= std::min(lbase + 127, bl - 1)) tl.push_back(make_int2(m, lt));
-                }
-            S.sntiles = (int)tl.size();
-            if (tl.empty()) tl.push_back(make_int2(0, 0));
-            if ((st = dev_upload(p, &S.stiles, tl))) return st;
-        }
-        p->sp_pstride = std::max(1LL, p->offP.back() + (long long)std::max(0, p->bl[p->J] - p->blo[p->J] - 1) * p->bl[p->J]);
-        if ((st = dev_alloc(p, &p->sp_dexp, (size_t)nd)) || (st = dev_alloc(p, &p->sp_sexp, (size_t)ns)) ||
-            (st = dev_alloc(p, &p->sp_fexp, (size_t)fexp)) || (st = dev_alloc(p, &p->sp_vexp, (size_t)fexp)) ||
-            (st = dev_alloc(p, &p->sp_fdig, (size_t)fdig)) || (st = dev_alloc(p, &p->sp_vdig, (size_t)vdig)) ||
-            (st = dev_alloc(p, &p->sp_err, 1)))
-            return st;
-        // Tb of the small scales for a chunk of maps: about 64 MB, which stay
-        // in L2 between the beta and the alpha stage, or one map's Tb of every
-        // scale where a memory limit leaves no more
-        long long one = 0;
-        for (int j : p->sp_small) one += (long long)p->N * p->bl[j] * 2 * p->bl[j];
-        auto chunk = [&](long long values) { return (int)std::max(1LL, std::min((long long)MAPS, one ? values / one : 1)); };
-        p->sp_chunk = chunk((64LL << 20) / (long long)sizeof(double2));
-        if (one && (p->sp_chunk * one <= tb || dev_alloc(p, &p->sp_Tb, (size_t)(p->sp_chunk * one)))) {
-            cudaGetLastError();  // of a failed allocation
-            p->sp_chunk = std::min(p->sp_chunk, chunk(tb));
-            if ((st = dev_alloc(p, &p->sp_Tb, (size_t)tb))) return st;
-        }
-        long long off = 0;
-        for (int j : p->sp_small) {
-            p->sp[j].tb_off = off;
-            off += (long long)p->sp_chunk * p->N * p->bl[j] * 2 * p->bl[j];
-        }
-        p->sp_tg_map = tg;
-        p->sp_v2f_map = v2f;
-        S2DW_CUDA_TRY(cudaMemsetAsync(p->sp_err, 0, sizeof(int), s));
-        // gamma-DFT phases exp(i pi n g / N), [g*16 + n+N-1]
-        std::vector<double2> ph((size_t)p->N * 16, make_double2(0.0, 0.0));
-        for (int g = 0; g < p->N; g++)
-            for (int n = -(p->N - 1); n <= p->N - 1; n++) {
-                const long double x = 3.141592653589793238462643383279502884L * (long double)(n * g) / (long double)p->N;
-                ph[(size_t)g * 16 + n + p->N - 1] = make_double2((double)cosl(x), (double)sinl(x));
-            }
-        if ((st = dev_upload(p, &p->sp_ph, ph))) return st;
-        p->sp_alloc = true;
-    }
+    const int NP = p->NP, MAPS = split_maps_per_pass();
+    if (!p->sp_alloc && (st = split_alloc(p, s))) return st;
     const int need = std::max(1, std::min(MAPS, nmaps));
     if (need > p->sp_cap) {
         // the buffers may still be read by earlier work of this plan
@@ -1042,10 +1073,16 @@ int split_prepare(s2dwc_plan *p, int nmaps, cudaStream_t s)
         dev_release(p, &p->sp_V2f, (size_t)(p->sp_cap * p->sp_v2f_map));
         dev_release(p, &p->sp_part, (size_t)(p->sp_cap * p->sp_pstride));
         p->sp_cap = 0;
-        if ((st = dev_alloc(p, &p->sp_Tg, (size_t)(need * p->sp_tg_map))) ||
-            (st = dev_alloc(p, &p->sp_V2f, (size_t)(need * p->sp_v2f_map))) ||
-            (st = dev_alloc(p, &p->sp_part, (size_t)(need * p->sp_pstride))))
+        AllocGroup mem(p);
+        double2 *Tg, *V2f, *part;
+        if ((st = dev_alloc(p, &Tg, (size_t)(need * p->sp_tg_map))) ||
+            (st = dev_alloc(p, &V2f, (size_t)(need * p->sp_v2f_map))) ||
+            (st = dev_alloc(p, &part, (size_t)(need * p->sp_pstride))))
             return st;
+        mem.keep = true;
+        p->sp_Tg = Tg;
+        p->sp_V2f = V2f;
+        p->sp_part = part;
         p->sp_cap = need;
     }
     if (!p->sp_dexp_valid) {

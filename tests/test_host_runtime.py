@@ -1,0 +1,145 @@
+"""The host side of the library on a stand-in CUDA runtime (fake_cudart.cpp,
+preloaded into a child process): what a call leaves behind when the runtime
+refuses one of its steps, which launches it queues and how they are ordered.
+Nothing here needs a GPU and no kernel runs."""
+import ctypes
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include",
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", out], check=True)
+    return out
+
+
+def run(fake, name, *args):
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), name, *map(str, args)], capture_output=True, text=True,
+                       env=dict(os.environ, LD_PRELOAD=fake, OMP_NUM_THREADS="2", PYTHONPATH=os.path.dirname(HERE)))
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+# ---- in the child ----------------------------------------------------------
+def _fake():
+    f = ctypes.CDLL(None)
+    f.fake_log.restype = ctypes.c_char_p
+    f.fake_fail.argtypes = [ctypes.c_char_p, ctypes.c_int]
+    f.fake_pin.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    return f
+
+
+class Plan:
+    """s2dw_b200.device.Plan without torch, on host buffers."""
+
+    def __init__(self, B, N, form=0, alpha=2.0, tables=True):
+        from s2dw_b200._lib import check, lib
+        from s2dw_b200.workload import transform_setup
+
+        self.t = t = transform_setup(B, N, alpha)
+        self.B, self.J, self.bs = B, t["J"], t["bl_scoeff"]
+        self.L, self.check, self.h = lib(), check, ctypes.c_void_p()
+        check(self.L.s2dwc_plan_create(ctypes.byref(self.h), B, N, alpha, self.J, form, 0))
+        offs = (ctypes.c_longlong * (self.J + 2))()
+        check(self.L.s2dwc_plan_wav_offsets(self.h, offs))
+        self.size = offs[self.J + 1]
+        if tables:
+            self.set_tables(t["Slm"])
+
+    def set_tables(self, S):
+        dp = ctypes.POINTER(ctypes.c_double)
+        K, P = (np.asfortranarray(self.t[k]) for k in ("K_gamma", "Phi2"))
+        S = np.asfortranarray(S, dtype=np.complex128)
+        self.check(self.L.s2dwc_plan_set_tables(self.h, K.ctypes.data_as(dp), P.ctypes.data_as(dp), S.ctypes.data_as(dp),
+                                                self.bs))
+
+    def reserve(self, maps):
+        return self.L.s2dwc_plan_reserve(self.h, maps, None)
+
+    def bytes(self):
+        return self.L.s2dwc_plan_workspace_bytes(self.h)
+
+    def buffers(self, maps=1):
+        self.keep = [np.zeros(n * maps + 2) for n in (self.size, 2 * self.bs ** 2, 2 * self.B ** 2)]
+        return [ctypes.c_void_p(a.ctypes.data) for a in self.keep]
+
+    def close(self):
+        self.L.s2dwc_plan_destroy(self.h)
+
+
+def _launches(f):
+    """(stream, priority, programmatic, name, grid, block) of the kernels since the last call."""
+    out = []
+    for line in f.fake_log().decode().splitlines():
+        if line != "event":
+            s, prio, dep, rest = line.split(" ", 3)
+            name, grid, block = rest.rsplit(" ", 2)
+            out.append((int(s), int(prio), dep == "1", name, grid, block))
+    return out
+
+
+def failed_reserve():
+    f = _fake()
+
+    def batch(p):
+        w, s, x = p.buffers(4)
+        f.fake_log()
+        p.check(p.L.s2dwc_plan_analysis_batch(p.h, 4, w, s, x, None))
+        p.check(p.L.s2dwc_plan_synthesis_batch(p.h, 4, x, w, s, None))
+        return [k[3:] for k in _launches(f)]
+
+    p = Plan(64, 5, form=1)
+    base = p.bytes()
+    assert p.reserve(4) == 0
+    want, size = batch(p), p.bytes()
+    p.close()
+    assert len(want) > 0
+    # the plan memory limit refuses the first reserve
+    for extra in (1, 20000, (size - base) // 2, size - base - 1):
+        p = Plan(64, 5, form=1)
+        p.L.s2dwc_set_plan_memory_limit(base + extra)
+        st = p.reserve(4)
+        p.L.s2dwc_set_plan_memory_limit(0)
+        if st:
+            assert st == 4
+            assert p.reserve(4) == 0
+            assert p.bytes() == size and batch(p) == want, extra
+        p.close()
+    # so does the device, at any allocation
+    failed = 0
+    for n in range(1, 1000):
+        p = Plan(64, 5, form=1)
+        f.fake_fail(b"cudaMalloc", n)
+        st = p.reserve(4)
+        if f.fake_armed():  # fewer than n allocations: done
+            f.fake_fail(b"cudaMalloc", 1 << 30)
+            break
+        if st:
+            failed += 1
+            assert st == 4, n
+            assert p.reserve(4) == 0
+            assert p.bytes() == size and batch(p) == want, n
+        else:  # (the stages' workspace fell back to a smaller one)
+            assert p.bytes() < size
+            batch(p)
+        p.close()
+    assert failed > 8
+
+
+# ---- tests -----------------------------------------------------------------
+def test_a_failed_reserve_leaves_the_plan_as_it_was(fake):
+    """Split workspaces that do not fit: whichever allocation fails, the next
+    reserve succeeds, holds no more memory than on a fresh plan, and the batches
+    after it make a fresh plan's launches (every scale once in each grouped one)."""
+    run(fake, "failed_reserve")
+
+
+if __name__ == "__main__":
+    globals()[sys.argv[1]](*map(int, sys.argv[2:]))
