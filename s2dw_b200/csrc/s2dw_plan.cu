@@ -1554,10 +1554,16 @@ int s2dwc_plan_set_tables(s2dwc_plan *p, const double *K_gamma, const double *Ph
     DeviceGuard dg(p->device);
     if (general && !p->GA_b) {
         int st;
-        if ((st = dev_alloc(p, &p->kappaA_b, (size_t)(J + 1) * B * NP)) ||
-            (st = dev_alloc(p, &p->kappaS_b, (size_t)(J + 1) * B * NP)) ||
-            (st = dev_alloc(p, &p->GA_b, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT_b, (size_t)p->gtp_total)))
+        AllocGroup mem(p);
+        double *kA_b, *kS_b, *GA_b, *GT_b;
+        if ((st = dev_alloc(p, &kA_b, (size_t)(J + 1) * B * NP)) || (st = dev_alloc(p, &kS_b, (size_t)(J + 1) * B * NP)) ||
+            (st = dev_alloc(p, &GA_b, (size_t)p->gpk_total)) || (st = dev_alloc(p, &GT_b, (size_t)p->gtp_total)))
             return st;
+        mem.keep = true;
+        p->kappaA_b = kA_b;
+        p->kappaS_b = kS_b;
+        p->GA_b = GA_b;
+        p->GT_b = GT_b;
     }
     if (general) {
         std::vector<double> kAb, kSb;
@@ -1784,9 +1790,16 @@ int s2dwc_plan_stat_moments(s2dwc_plan *p, int nmaps, const double *d_wav, const
     int st;
     if (!p->st_part) {
         const size_t ny = (size_t)G * (p->J + 1);
-        if ((st = dev_alloc(p, &p->st_part, ny * STAT_P * STAT_W)) || (st = dev_alloc(p, &p->st_mean, ny * 2)) ||
-            (st = dev_alloc(p, &p->st_flags, ny)))
+        AllocGroup mem(p);
+        double *part, *mean;
+        int *flags;
+        if ((st = dev_alloc(p, &part, ny * STAT_P * STAT_W)) || (st = dev_alloc(p, &mean, ny * 2)) ||
+            (st = dev_alloc(p, &flags, ny)))
             return st;
+        mem.keep = true;
+        p->st_part = part;
+        p->st_mean = mean;
+        p->st_flags = flags;
     }
     const long long wtot = p->wav_off[p->J + 1];
     for (int g0 = 0; g0 < nmaps; g0 += G) {
@@ -2073,9 +2086,15 @@ static int host_prepare(int B, int N, double alpha, int J, int bl_scoeff, const 
         S2DW_CUDA_TRY(cudaStreamCreateWithFlags(&p->copy_stream, cudaStreamNonBlocking));
     }
     if (!p->hbWav) {
-        if ((st = dev_alloc(p, &p->hbWav, (size_t)std::max(1LL, p->wav_off[J + 1]))) ||
-            (st = dev_alloc(p, &p->hbFlm, (size_t)B * B)))
+        AllocGroup mem(p);
+        double *wav;
+        double2 *flm;
+        if ((st = dev_alloc(p, &wav, (size_t)std::max(1LL, p->wav_off[J + 1]))) ||
+            (st = dev_alloc(p, &flm, (size_t)B * B)))
             return st;
+        mem.keep = true;
+        p->hbWav = wav;
+        p->hbFlm = flm;
     }
     if (p->hbSc_n < bl_scoeff * bl_scoeff || !p->hbSc) {
         if ((st = dev_alloc(p, &p->hbSc, (size_t)std::max(1, bl_scoeff * bl_scoeff)))) return st;

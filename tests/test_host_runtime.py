@@ -39,26 +39,25 @@ def _fake():
 class Plan:
     """s2dw_b200.device.Plan without torch, on host buffers."""
 
-    def __init__(self, B, N, form=0, alpha=2.0, tables=True):
+    def __init__(self, B, N, form=0):
         from s2dw_b200._lib import check, lib
         from s2dw_b200.workload import transform_setup
 
-        self.t = t = transform_setup(B, N, alpha)
+        self.t = t = transform_setup(B, N, 2.0)
         self.B, self.J, self.bs = B, t["J"], t["bl_scoeff"]
         self.L, self.check, self.h = lib(), check, ctypes.c_void_p()
-        check(self.L.s2dwc_plan_create(ctypes.byref(self.h), B, N, alpha, self.J, form, 0))
+        check(self.L.s2dwc_plan_create(ctypes.byref(self.h), B, N, 2.0, self.J, form, 0))
         offs = (ctypes.c_longlong * (self.J + 2))()
         check(self.L.s2dwc_plan_wav_offsets(self.h, offs))
         self.size = offs[self.J + 1]
-        if tables:
-            self.set_tables(t["Slm"])
+        check(self.set_tables(t["Slm"]))
 
     def set_tables(self, S):
         dp = ctypes.POINTER(ctypes.c_double)
         K, P = (np.asfortranarray(self.t[k]) for k in ("K_gamma", "Phi2"))
         S = np.asfortranarray(S, dtype=np.complex128)
-        self.check(self.L.s2dwc_plan_set_tables(self.h, K.ctypes.data_as(dp), P.ctypes.data_as(dp), S.ctypes.data_as(dp),
-                                                self.bs))
+        return self.L.s2dwc_plan_set_tables(self.h, K.ctypes.data_as(dp), P.ctypes.data_as(dp), S.ctypes.data_as(dp),
+                                            self.bs)
 
     def reserve(self, maps):
         return self.L.s2dwc_plan_reserve(self.h, maps, None)
@@ -133,12 +132,67 @@ def failed_reserve():
     assert failed > 8
 
 
+def failed_buffers():
+    """Tables of a general Slm, moments' and host calls' buffers: every
+    allocation fails once, and the call works when it is repeated."""
+    f = _fake()
+    dp = ctypes.POINTER(ctypes.c_double)
+
+    def slm():
+        rng = np.random.default_rng(0)
+        return rng.standard_normal((24, 4)) + 1j * rng.standard_normal((24, 4))
+
+    def general(p):
+        return p.set_tables(slm())
+
+    def moments(p):
+        w, s, x = p.buffers()
+        m = ctypes.c_void_p(np.zeros((p.J + 1) * 6).ctypes.data)
+        return p.L.s2dwc_plan_stat_moments(p.h, 1, w, None, m, None)
+
+    def host(p):
+        t, B = p.t, p.B
+        K, S = np.asfortranarray(t["K_gamma"]), np.asfortranarray(t["Slm"])
+        out = [np.zeros(p.size) for _ in range(p.J + 1)]
+        sc, flm = np.zeros(2 * p.bs ** 2), np.zeros(2 * B * B)
+        ptrs = (dp * (p.J + 1))(*[o.ctypes.data_as(dp) for o in out])
+        return p.L.s2dwc_analysis_flm2wav_dynamic(ptrs, sc.ctypes.data_as(dp), flm.ctypes.data_as(dp), K.ctypes.data_as(dp),
+                                                  S.ctypes.data_as(dp), p.J, B, 4, p.bs, 2.0)
+
+    for call in (general, moments, host):
+        p = Plan(24, 4)
+        assert call(p) == 0
+        size = p.bytes()
+        p.close()
+        for n in range(1, 1000):
+            p = Plan(24, 4)
+            p.L.s2dwc_finalize()
+            held = f.fake_allocations()
+            f.fake_fail(b"cudaMalloc", n)
+            st = call(p)
+            if f.fake_armed():
+                f.fake_fail(b"cudaMalloc", 1 << 30)
+                break
+            assert st == 4
+            assert call is host or f.fake_allocations() == held
+            assert call(p) == 0, (call.__name__, n)
+            assert p.bytes() == size
+            p.close()
+        assert n > 3
+
+
 # ---- tests -----------------------------------------------------------------
 def test_a_failed_reserve_leaves_the_plan_as_it_was(fake):
     """Split workspaces that do not fit: whichever allocation fails, the next
     reserve succeeds, holds no more memory than on a fresh plan, and the batches
     after it make a fresh plan's launches (every scale once in each grouped one)."""
     run(fake, "failed_reserve")
+
+
+def test_a_failed_buffer_allocation_can_be_repeated(fake):
+    """No pointer of a group of buffers stays set while another of it is
+    missing: a kernel would get the null one on the next call."""
+    run(fake, "failed_buffers")
 
 
 if __name__ == "__main__":
