@@ -49,10 +49,11 @@ int set_error(int code, const char *fmt, ...);
 // Programmatic dependent launch: the kernels of a call that follow one another
 // on one stream are launched with it (`dep`), so that a kernel's CTAs are in
 // place, and its tables on their way, when its predecessor ends.  Every such
-// kernel calls pdl_start() first and pdl_wait() before it touches anything a
-// kernel before it reads or writes; launched without the attribute both do
-// nothing.  A kernel whose predecessor on the stream is not one of this call is
-// launched without it.
+// kernel calls pdl_start() and, before it touches anything a kernel before it
+// reads or writes, pdl_wait() (the alpha kernels, which have nothing to load
+// earlier, wait first; the other order measured the same); launched without the
+// attribute both do nothing.  A kernel whose predecessor on the stream is not one
+// of this call is launched without it.
 template <typename... P, typename... A>
 inline cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool dep,
                               A &&...args)
@@ -313,7 +314,6 @@ constexpr int STAGE_PFA = 6;
 constexpr int STAGE_MAX = 24;  // entries per launch
 struct StageArgs {
     int n, ncta, N, NP;
-    int late;              // length-1023 alpha rows: does not depend on the launch before
     int nq[S2DW_NPMAX];
     const double2 *tw;     // exp(-2 pi i k / 2048), k < 2048
     const double2 *ph;     // LwalkArgs::ph

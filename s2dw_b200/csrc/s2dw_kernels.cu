@@ -812,20 +812,6 @@ __global__ void __launch_bounds__(NT, (NT == 128 ? 3 : 2)) pfa2047_alpha_kernel(
     }
 }
 
-// Alpha launches of one stage do not depend on one another: a second one
-// (late) starts while the first still runs and waits for it at its end instead.
-// That is safe as an alpha kernel lets its successor start only after its own
-// wait: what came before the first launch is then complete.
-__device__ __forceinline__ void alpha_begin(const StageArgs &a)
-{
-    if (!a.late) pdl_wait();
-    pdl_start();
-}
-__device__ __forceinline__ void alpha_end(const StageArgs &a)
-{
-    if (a.late) pdl_wait();
-}
-
 // ---------------------------------------------------------------------------
 // Row pairs of an alpha stage into and out of shared memory: RP pairs (g, rr)
 // of the transform of odd length N = 2 bl - 1, value m of pair r at at(r, m).
@@ -1103,6 +1089,9 @@ __device__ __forceinline__ int pfc_out_pos(int k) { return k % 3 + 3 * (k % 11) 
 // the 33 length-31 DFTs with a column's real and imaginary parts in two lanes
 // (66 lanes; one thread per column took 168 registers and left 95 of 128 threads
 // waiting).
+// The launch follows the other scales' alpha launch of its stage.  Run beside it
+// (forked to a second stream) it took the same time: B = 512, N = 4 analysis 196
+// and 194 us, synthesis 222 and 222, B = 1024 810 and 813, 862 and 861.
 constexpr int PFC_THREADS = 96;
 
 template <int MODE>
@@ -1112,7 +1101,8 @@ __global__ void __launch_bounds__(PFC_THREADS, 6) pfa1023_kernel(const __grid_co
     extern __shared__ __align__(16) double2 smem[];
     int cta;
     const StageEnt &e = stage_entry(a, cta);
-    alpha_begin(a);
+    pdl_wait();
+    pdl_start();
     const int t = threadIdx.x;
     alpha_rows_in<MODE, PFC_N, 1, NT>(e, cta, [&](int, int m) -> double2 & { return smem[pfc_in_pos(m)]; });
     __syncthreads();
@@ -1132,7 +1122,6 @@ __global__ void __launch_bounds__(PFC_THREADS, 6) pfa1023_kernel(const __grid_co
     }
     __syncthreads();
     alpha_rows_out<MODE, PFC_N, 1, NT>(e, cta, [&](int, int k) -> double2 { return smem[pfc_out_pos(k)]; });
-    alpha_end(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1214,7 +1203,8 @@ __global__ void __launch_bounds__(ST_THREADS, BIG ? 4 : 6) alpha_kernel(const __
     extern __shared__ __align__(16) double2 smem[];
     int cta;
     const StageEnt &e = stage_entry(a, cta);
-    alpha_begin(a);
+    pdl_wait();
+    pdl_start();
     if (e.kind == STAGE_PFA) {
         switch (e.bl) {
         case 2: pfs_rows_run<3, 1, 1, MODE>(e, cta, smem); break;

@@ -647,14 +647,11 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
     std::memcpy(sa.nq, p->nq, sizeof(sa.nq));
     sa.tw = p->tw2048;
     sa.ph = p->ph;
-    bool grouped = false;  // the launch before on `s` is a group of this stage
     auto flush = [&]() -> int {
         if (sa.n == 0) return S2DWC_OK;
         KernelTimer kt(p, stage_kind(stg), s);
-        // the length-1023 rows come last and need not wait for the others
-        sa.late = grouped && !p->timing && stage_alone(sa.e[0]);
-        grouped = !stage_alone(sa.e[0]);
-        const int e = launch_stage(stg, sa, (dep || sa.late) && !p->timing, s);
+        const int e = launch_stage(stg, sa, dep && !p->timing, s);
+        dep = true;  // the stage's next launch follows this one
         sa.n = sa.ncta = 0;
         return e;
     };
@@ -670,7 +667,6 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
         const int mode = stage_mode(p, j, stg), rows = stage_rows(p, j, stg);
         const CztDev &c = p->czt[j][mode];
         if (!stage_small(p, j, stg)) {
-            grouped = false;
             CztArgs ca{};
             ca.mode = mode;
             ca.bl = p->bl[j];
