@@ -431,15 +431,25 @@ int launch_split(const SplitArgs &a, cudaStream_t s);
 // ---------------------------------------------------------------------------
 // Moments of the wavelet coefficients per scale (s2dw_stats.cu)
 // ---------------------------------------------------------------------------
-constexpr int STAT_P = 96;  // blocks per (map, scale) in the reduction passes
-constexpr int STAT_W = 8;   // partial sums per block: 2 of pass 1, 6 of pass 2
+constexpr int STAT_W = 8;       // partial sums per block: 2 of pass 1, 6 of pass 2
+// Maps per pair of passes and blocks per (map, scale) in them.  Without a mask many
+// maps fill the GPU with fewer blocks and gain from fewer passes: B=256, N=4, 16
+// maps 127 us with 48 blocks, 158 with 96, but 4 maps at B=512 147 and 117.
+struct StatSplit {
+    int maps, P;
+};
+__host__ __device__ constexpr StatSplit stat_split(int nmaps, bool mask)
+{
+    return mask ? StatSplit{16, 96} : nmaps <= 8 ? StatSplit{8, 96} : StatSplit{32, 48};
+}
+constexpr int STAT_BLOCKS = 16 * 96;  // the largest maps x P of them
 struct StatArgs {
-    int J, nmaps;
+    int J, nmaps, P;           // at most stat_split's maps, its P
     long long wtot;            // doubles per map in the packed layout
     long long off[S2DW_JMAX + 2];  // scale offsets (J+2 entries)
     const double *wav;         // map k at wav + k*wtot
     const double *mask;        // packed layout of one map, or null
-    double *part, *part2;      // nmaps*(J+1)*STAT_P x 2 and x 6 partial sums
+    double *part, *part2;      // nmaps*(J+1)*P x 2 and x 6 partial sums
     double *mean_nj;           // nmaps*(J+1)*2
     double *out;               // nmaps*(J+1)*6: mean, var, skew, kur, five, six
     int *flags;                // nmaps*(J+1): 1 zero variance, 2 fewer than two samples

@@ -131,7 +131,7 @@ struct s2dwc_plan {
     int *sp_err = nullptr;
     unsigned long long sp_wait_ns = 2000000000ull;  // bound on every split-kernel pipeline wait (2 s)
     int sp_min_batch = 1;  // split-form batches smaller than this run the FP64 path
-    // moments of the coefficients (built on first use): 16 maps per pass
+    // moments of the coefficients (built on first use)
     double *st_part = nullptr, *st_mean = nullptr;
     int *st_flags = nullptr;
     std::vector<void *> allocs;
@@ -1782,14 +1782,13 @@ int s2dwc_plan_stat_moments(s2dwc_plan *p, int nmaps, const double *d_wav, const
     if (!p || !d_wav || !d_moments) return set_error(S2DWC_ERROR_ARG_INVALID, "plan_stat_moments: null pointer");
     if (nmaps < 0) return set_error(S2DWC_ERROR_ARG_INVALID, "plan_stat_moments: nmaps=%d", nmaps);
     DeviceGuard dg(p->device);
-    constexpr int G = 16;
     int st;
     if (!p->st_part) {
-        const size_t ny = (size_t)G * (p->J + 1);
+        const size_t ny = 32 * (size_t)(p->J + 1);
         AllocGroup mem(p);
         double *part, *mean;
         int *flags;
-        if ((st = dev_alloc(p, &part, ny * STAT_P * STAT_W)) || (st = dev_alloc(p, &mean, ny * 2)) ||
+        if ((st = dev_alloc(p, &part, (size_t)(p->J + 1) * STAT_BLOCKS * STAT_W)) || (st = dev_alloc(p, &mean, ny * 2)) ||
             (st = dev_alloc(p, &flags, ny)))
             return st;
         mem.keep = true;
@@ -1798,16 +1797,18 @@ int s2dwc_plan_stat_moments(s2dwc_plan *p, int nmaps, const double *d_wav, const
         p->st_flags = flags;
     }
     const long long wtot = p->wav_off[p->J + 1];
-    for (int g0 = 0; g0 < nmaps; g0 += G) {
+    const StatSplit sp = stat_split(nmaps, d_mask != nullptr);
+    for (int g0 = 0; g0 < nmaps; g0 += sp.maps) {
         StatArgs a{};
         a.J = p->J;
-        a.nmaps = std::min(G, nmaps - g0);
+        a.nmaps = std::min(sp.maps, nmaps - g0);
+        a.P = sp.P;
         a.wtot = wtot;
         for (int j = 0; j <= p->J + 1; j++) a.off[j] = p->wav_off[j];
         a.wav = d_wav + (size_t)g0 * wtot;
         a.mask = d_mask;
         a.part = p->st_part;
-        a.part2 = p->st_part + (size_t)G * (p->J + 1) * STAT_P * 2;
+        a.part2 = p->st_part + (size_t)a.nmaps * (p->J + 1) * a.P * 2;
         a.mean_nj = p->st_mean;
         a.out = d_moments + (size_t)g0 * (p->J + 1) * 6;
         a.flags = p->st_flags;
@@ -1831,6 +1832,7 @@ int s2dwc_stat_moments(double *const *wav_scales, int J, int B, int N, double al
     StatArgs a{};
     a.J = J;
     a.nmaps = 1;
+    a.P = stat_split(1, mask_scales != nullptr).P;
     a.off[0] = 0;
     for (int j = 0; j <= J; j++) {
         int hi, lo;
@@ -1841,14 +1843,14 @@ int s2dwc_stat_moments(double *const *wav_scales, int J, int B, int N, double al
     const size_t ny = (size_t)J + 1;
     // one device block for everything this call needs, freed before return
     const size_t nw = (size_t)a.wtot, nm = mask_scales ? nw : 0;
-    const size_t bytes = 8 * (nw + nm + ny * STAT_P * STAT_W + ny * 2 + ny * 6) + 4 * ny + 256;
+    const size_t bytes = 8 * (nw + nm + ny * a.P * STAT_W + ny * 2 + ny * 6) + 4 * ny + 256;
     char *blk = nullptr;
     cudaError_t e = cudaMalloc(&blk, bytes);
     if (e != cudaSuccess)
         return set_error(S2DWC_ERROR_MEM_ALLOC_FAIL, "stat_moments: cudaMalloc of %zu bytes failed: %s", bytes,
                          cudaGetErrorString(e));
     std::unique_ptr<char, void (*)(char *)> guard(blk, [](char *q) { cudaFree(q); });
-    double *dw = reinterpret_cast<double *>(blk), *dm = dw + nw, *dpart = dm + nm, *dmean = dpart + ny * STAT_P * STAT_W,
+    double *dw = reinterpret_cast<double *>(blk), *dm = dw + nw, *dpart = dm + nm, *dmean = dpart + ny * a.P * STAT_W,
            *dout = dmean + ny * 2;
     int *dflags = reinterpret_cast<int *>(dout + ny * 6);
     for (int j = 0; j <= J; j++) {
@@ -1859,7 +1861,7 @@ int s2dwc_stat_moments(double *const *wav_scales, int J, int B, int N, double al
     a.wav = dw;
     a.mask = mask_scales ? dm : nullptr;
     a.part = dpart;
-    a.part2 = dpart + ny * STAT_P * 2;
+    a.part2 = dpart + ny * a.P * 2;
     a.mean_nj = dmean;
     a.out = dout;
     a.flags = dflags;

@@ -8,15 +8,15 @@
 // then the reference's normalisations (n-1 variance, standardised skewness,
 // excess kurtosis, fifth and excess sixth moments; zero variance -> zeros).
 // Every reduction runs in a fixed order (per-thread sums, shuffle and
-// shared-memory trees, then the STAT_P block partials in a warp's tree), so
+// shared-memory trees, then the blocks' partials in a warp's tree), so
 // results are bit-reproducible.
 //
-// Bound by HBM: two reads of the coefficients (and mask).  Each thread has
-// eight 8-byte loads in flight (four 16-byte ones where the arrays allow it),
-// and the partials are summed by a warp at the start of the pass that needs
-// them: 4 maps at B=512, N=4 with a mask (626 MB through the two passes, with
-// the mask's re-reads) took 245 us with one load in flight, 64 blocks per scale
-// and single threads summing the partials.
+// Bound by HBM: two reads of the coefficients (and mask).  Each thread has two or
+// four 16-byte loads in flight, whatever boundary the arrays start on, and the
+// partials are summed by a warp at the start of the pass that needs them.  Against
+// one 8-byte load in flight, 64 blocks per scale and single threads summing the
+// partials, B200 at B=512, N=4 (us): 4 maps with a mask 251 -> 138 (mask on another
+// 16-byte boundary 239 -> 144), without 167 -> 115; 16 maps 784 -> 464 and 459 -> 400.
 #include <cuda_runtime.h>
 
 #include "s2dw_internal.h"
@@ -54,101 +54,116 @@ __device__ __forceinline__ void block_sum(double (&v)[K])
         }
 }
 
-// Sum over the STAT_P block partials of pass 1's value k of row y, by one warp.
+// Sum over the P blocks' partials of pass 1's value k of row y, by one warp.
+template <int P>
 __device__ __forceinline__ double partial_sum(const StatArgs &a, int y, int k)
 {
     double s = 0.0;
-    for (int x = threadIdx.x & 31; x < STAT_P; x += 32) s += a.part[((size_t)y * STAT_P + x) * 2 + k];
+#pragma unroll
+    for (int x = threadIdx.x & 31; x < P; x += 32) s += a.part[((size_t)y * P + x) * 2 + k];
     return warp_sum(s);
 }
 
 // Grid (map, share, scale): the blocks of one share of a scale run together
 // over the maps, which read the same part of the mask (map-major, every map read
-// the mask from HBM: 92 us per pass for the 4 maps above).  Row y = map (J+1)
-// + scale of the partials, and the coefficient block.
+// the mask from HBM: 4 maps at B=512, N=4 180 us instead of 153; without a mask
+// 137 and 117).  Row y = map (J+1) + scale of the partials, and the coefficient
+// block.
 struct StatBlock {
     const double *w, *mk;
     long long n;
-    int y;
+    int y, x;
 };
+template <int MASK>
 __device__ __forceinline__ StatBlock stat_block(const StatArgs &a)
 {
     const int k = blockIdx.x, j = blockIdx.z;
     StatBlock b;
+    b.x = blockIdx.y;
     b.y = k * (a.J + 1) + j;
     b.w = a.wav + (size_t)k * a.wtot + a.off[j];
-    b.mk = a.mask ? a.mask + a.off[j] : nullptr;
+    b.mk = MASK ? a.mask + a.off[j] : nullptr;
     b.n = a.off[j + 1] - a.off[j];
     return b;
 }
 
-// Calls f(w, mask) for the block's share of the (map, scale) block's values,
-// eight per thread at a time.
-template <typename F>
+// Calls f(w, mask) for the block's share of the (map, scale) block's values, U
+// pairs per thread at a time, from the coefficients' first 16-byte boundary on: a
+// block holds an even number of values, and one that starts off a boundary has a
+// single first and last value.  The mask is read in pairs where its boundaries
+// are the same (MASK_PAIRS).
+enum StatMask { MASK_NONE, MASK_PAIRS, MASK_SINGLE };
+template <int MASK, int U, int P, typename F>
 __device__ __forceinline__ void stat_values(const StatBlock &b, F &&f)
 {
-    constexpr int U = 4;
-    const long long step = (long long)STAT_P * STAT_T;
-    const long long t = (long long)blockIdx.y * STAT_T + threadIdx.x;
-    if ((((uintptr_t)b.w | (uintptr_t)b.mk) & 15) == 0) {  // pairs (an even number of values)
-        const double2 *w = reinterpret_cast<const double2 *>(b.w), *m = reinterpret_cast<const double2 *>(b.mk);
-        const long long n = b.n / 2;
-        for (long long i0 = t; i0 < n; i0 += U * step) {
-            double2 x[U], y[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const long long i = i0 + u * step;
-                if (i < n) {
-                    x[u] = w[i];
-                    y[u] = m ? m[i] : make_double2(1.0, 1.0);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++)
-                if (i0 + u * step < n) {
-                    f(x[u].x, y[u].x);
-                    f(x[u].y, y[u].y);
-                }
-        }
-        return;
+    constexpr long long step = (long long)P * STAT_T;
+    const long long t = (long long)b.x * STAT_T + threadIdx.x;
+    const int odd = ((uintptr_t)b.w >> 3) & 1;
+    if (odd && t < 2) {
+        const long long i = t ? b.n - 1 : 0;
+        f(b.w[i], MASK ? b.mk[i] : 1.0);
     }
-    for (long long i = t; i < b.n; i += step) f(b.w[i], b.mk ? b.mk[i] : 1.0);
+    const double2 *w = reinterpret_cast<const double2 *>(b.w + odd);
+    const double *m = b.mk + odd;
+    const long long n = b.n / 2 - odd;
+    for (long long i0 = t; i0 < n; i0 += U * step) {
+        double2 x[U], y[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long i = i0 + u * step;
+            if (i < n) {
+                x[u] = w[i];
+                y[u] = MASK == MASK_NONE    ? make_double2(1.0, 1.0)
+                       : MASK == MASK_PAIRS ? reinterpret_cast<const double2 *>(m)[i]
+                                            : make_double2(m[2 * i], m[2 * i + 1]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (i0 + u * step < n) {
+                f(x[u].x, y[u].x);
+                f(x[u].y, y[u].y);
+            }
+    }
 }
 
+template <int MASK, int U, int P>
 __global__ void __launch_bounds__(STAT_T) stat_pass1(const __grid_constant__ StatArgs a)
 {
-    const StatBlock b = stat_block(a);
+    const StatBlock b = stat_block<MASK>(a);
     double v[2] = {0.0, 0.0};
-    stat_values(b, [&](double w, double m) {
-        if (fabs(m - 1.0) < TOL_ZERO) v[0] += w * m;
+    stat_values<MASK, U, P>(b, [&](double w, double m) {
+        if (!MASK || fabs(m - 1.0) < TOL_ZERO) v[0] += w * m;
         v[1] += m;
     });
     block_sum<2>(v);
     if (threadIdx.x == 0) {
-        double *p = a.part + ((size_t)b.y * STAT_P + blockIdx.y) * 2;
+        double *p = a.part + ((size_t)b.y * P + b.x) * 2;
         p[0] = v[0];
         p[1] = v[1];
     }
 }
 
 // mean and nj of row y, by one warp
+template <int P>
 __device__ __forceinline__ double2 stat_mean(const StatArgs &a, int y)
 {
     const int j = y % (a.J + 1);
-    const double s = partial_sum(a, y, 0), c = partial_sum(a, y, 1);
+    const double s = partial_sum<P>(a, y, 0), c = partial_sum<P>(a, y, 1);
     const double nj = a.mask ? rint(c) : (double)(a.off[j + 1] - a.off[j]);
     return make_double2(s / nj, nj);
 }
 
+template <int MASK, int U, int P>
 __global__ void __launch_bounds__(STAT_T) stat_pass2(const __grid_constant__ StatArgs a)
 {
     __shared__ double smu;
-    const StatBlock b = stat_block(a);
+    const StatBlock b = stat_block<MASK>(a);
     if (threadIdx.x < 32) {
-        const double2 m = stat_mean(a, b.y);
+        const double2 m = stat_mean<P>(a, b.y);
         if (threadIdx.x == 0) {
             smu = m.x;
-            if (blockIdx.y == 0) {
+            if (b.x == 0) {
                 a.mean_nj[2 * b.y] = m.x;
                 a.mean_nj[2 * b.y + 1] = m.y;
             }
@@ -157,8 +172,8 @@ __global__ void __launch_bounds__(STAT_T) stat_pass2(const __grid_constant__ Sta
     __syncthreads();
     const double mu = smu;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    stat_values(b, [&](double w, double m) {
-        if (!(fabs(m - 1.0) < TOL_ZERO)) return;
+    stat_values<MASK, U, P>(b, [&](double w, double m) {
+        if (MASK && !(fabs(m - 1.0) < TOL_ZERO)) return;
         const double s = w * m - mu;
         double p = s * s;
         v[0] += s;
@@ -174,7 +189,7 @@ __global__ void __launch_bounds__(STAT_T) stat_pass2(const __grid_constant__ Sta
     });
     block_sum<6>(v);
     if (threadIdx.x == 0) {
-        double *p = a.part2 + ((size_t)b.y * STAT_P + blockIdx.y) * 6;
+        double *p = a.part2 + ((size_t)b.y * P + b.x) * 6;
 #pragma unroll
         for (int k = 0; k < 6; k++) p[k] = v[k];
     }
@@ -182,6 +197,7 @@ __global__ void __launch_bounds__(STAT_T) stat_pass2(const __grid_constant__ Sta
 
 // moments per (map, scale), a warp each: out[y*6 + {mean, var, skew, kur,
 // five, six}], flags[y] = 1 zero variance, 2 fewer than two samples
+template <int P>
 __global__ void __launch_bounds__(128) stat_final(const __grid_constant__ StatArgs a)
 {
     const int y = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -190,7 +206,8 @@ __global__ void __launch_bounds__(128) stat_final(const __grid_constant__ StatAr
 #pragma unroll
     for (int k = 0; k < 6; k++) {
         double t = 0.0;
-        for (int x = threadIdx.x & 31; x < STAT_P; x += 32) t += a.part2[((size_t)y * STAT_P + x) * 6 + k];
+#pragma unroll
+        for (int x = threadIdx.x & 31; x < P; x += 32) t += a.part2[((size_t)y * P + x) * 6 + k];
         s[k] = warp_sum(t);
     }
     if (threadIdx.x & 31) return;
@@ -219,14 +236,23 @@ __global__ void __launch_bounds__(128) stat_final(const __grid_constant__ StatAr
 
 }  // namespace
 
+template <int MASK, int U, int P>
+static void launch_passes(const StatArgs &a, cudaStream_t s)
+{
+    const dim3 grid(a.nmaps, P, a.J + 1);
+    stat_pass1<MASK, U, P><<<grid, STAT_T, 0, s>>>(a);
+    stat_pass2<MASK, U, P><<<grid, STAT_T, 0, s>>>(a);
+    stat_final<P><<<(a.nmaps * (a.J + 1) + 3) / 4, 128, 0, s>>>(a);
+}
+
 int launch_stat_moments(const StatArgs &a, cudaStream_t s)
 {
-    const int ny = a.nmaps * (a.J + 1);
-    if (ny <= 0) return S2DWC_OK;
-    dim3 grid(a.nmaps, STAT_P, a.J + 1);
-    stat_pass1<<<grid, STAT_T, 0, s>>>(a);
-    stat_pass2<<<grid, STAT_T, 0, s>>>(a);
-    stat_final<<<(ny + 3) / 4, 128, 0, s>>>(a);
+    if (a.nmaps <= 0) return S2DWC_OK;
+    // (maps and scales have an even number of values: one boundary for all)
+    if (a.mask && (((uintptr_t)a.wav ^ (uintptr_t)a.mask) & 15) == 0) launch_passes<MASK_PAIRS, 4, 96>(a, s);
+    else if (a.mask) launch_passes<MASK_SINGLE, 4, 96>(a, s);
+    else if (a.P == 96) launch_passes<MASK_NONE, 4, 96>(a, s);
+    else launch_passes<MASK_NONE, 2, 48>(a, s);
     S2DW_CUDA_TRY(cudaGetLastError());
     return S2DWC_OK;
 }

@@ -100,3 +100,40 @@ def test_device_batched_moments_match_oracle():
         _, ref, _ = O.stat_moments(w, J, B, N, alpha, mask=mk)
         _close(m2[k], ref)
     plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wo,mo", [(0, None), (1, None), (1, 1), (1, 0), (0, 1)])
+@pytest.mark.parametrize("nmaps", [1, 9, 33])
+def test_device_moments_on_any_boundary(wo, mo, nmaps):
+    """Coefficients and mask that start on or 8 bytes off a 16-byte boundary (wo,
+    mo; no mask: None), and batches of every number of blocks per map and of more than one
+    pair of passes."""
+    import torch
+
+    from s2dw_b200.device import Plan
+
+    B, N, alpha = 12, 2, 2.0
+    J = core.s2dw_core_comp_Jmax(B, alpha)
+    plan = Plan(B, N, alpha, J)
+    off = plan.wav_offsets
+    rng = np.random.default_rng(nmaps)
+    w = rng.standard_normal((nmaps, plan.wav_size)) + 0.3
+    m = (rng.random(plan.wav_size) < 0.7).astype(np.float64)
+    d_w = torch.empty(w.size + wo, dtype=torch.float64, device="cuda")[wo:].view(w.shape)
+    d_w.copy_(torch.from_numpy(w))
+    d_m = None
+    if mo is not None:
+        d_m = torch.empty(m.size + mo, dtype=torch.float64, device="cuda")[mo:]
+        d_m.copy_(torch.from_numpy(m))
+    out = torch.empty((nmaps, J + 1, 6), dtype=torch.float64, device="cuda")
+    plan.stat_moments(d_w, out, d_m)
+    got = out.cpu().numpy()
+
+    def scales(x):
+        return [x[off[j]:off[j + 1]].reshape(N, 2 * plan.bl[j], -1).transpose(2, 1, 0).copy(order="F") for j in range(J + 1)]
+
+    for k in range(nmaps):
+        _, ref, _ = O.stat_moments(scales(w[k]), J, B, N, alpha, mask=None if mo is None else scales(m))
+        _close(got[k], ref)
+    plan.close()
