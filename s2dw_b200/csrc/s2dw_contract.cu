@@ -822,6 +822,15 @@ int lwalk_pairs(int B, int NP)
     return S;
 }
 
+// Whether the analysis walks once per scale (`only`, two pairs per thread) instead
+// of once for all: with NP = 7 and 8 the merged walk's accumulators leave one pair
+// per thread, whose table reads then weigh as much as its arithmetic.  Measured on
+// B200 (ms per analysis, one walk and one per scale): N = 14, B = 512 0.726,
+// 0.720; 640 2.54, 2.36; 1024 3.42, 2.89; 2048 19.0, 16.0; N = 16, B = 384 0.81,
+// 0.87; 640 2.90, 2.69; 1024 3.97, 3.28; 2048 22.5, 17.9.  (N = 12: 1024 2.73, 2.56,
+// but 512 0.56, 0.63.)  Up to B = 512 the scales share their stages' launches.
+bool lwalk_per_scale(int B, int NP) { return NP >= 7 && B > 512; }
+
 // Where the launch is bound by its longest walk (S = 1), the tiles that hold
 // pairs of the small scales (bl <= B/4) are two CTAs: one walks the small
 // scales' l and ends them (their many short ranges are cold code and flushes),

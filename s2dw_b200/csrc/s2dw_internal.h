@@ -241,6 +241,7 @@ struct MwalkArgs {
 };
 // Tile lists, ordered by decreasing work so that the longest walks start first.
 int lwalk_pairs(int B, int NP);
+bool lwalk_per_scale(int B, int NP);
 int lwalk_split(const std::vector<int> &bl, int S);
 void build_lwalk_tiles(const std::vector<int> &bl, int S, int jsplit, std::vector<int2> &t);
 int2 mwalk_shape(int B, int NP);

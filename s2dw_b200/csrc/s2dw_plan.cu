@@ -794,7 +794,8 @@ using ScaleHook = std::function<int(int, cudaStream_t)>;
 constexpr auto one_map = [](int) { return 0LL; };
 
 // Runs the analysis: the F table and the contraction of all scales on `s`,
-// then the beta and alpha stages of the scales' groups.
+// then the beta and alpha stages of the scales' groups (lwalk_per_scale: each
+// scale's contraction on its group's stream).
 // full_band_serial (host-buffer entry points): the groups from the last scale
 // to the first, the two full-band scales one after the other, so that the first
 // one's device-to-host copy overlaps the next one's kernels instead of both
@@ -811,17 +812,21 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         KernelTimer kt(p, S2DWC_KIND_OTHER, s);
         if ((st = launch_fprep(p->Fw, d_scoeff, d_flm, p->Om, p->B, p->Bp, p->bl_scoeff, s))) return st;
     }
-    LwalkArgs la = lwalk_args(p, p->Fw, p->wsC);
-    {
-        KernelTimer kt(p, S2DWC_KIND_LWALK, s);
-        if ((st = launch_lwalk(la, !p->timing, s))) return st;
-    }
-    if (p->slm_general) {  // the b part of a general Slm, accumulated into Tg
-        la.G = p->GA_b;
-        la.acc_imag = 1;
-        KernelTimer kt(p, S2DWC_KIND_LWALK, s);
-        if ((st = launch_lwalk(la, !p->timing, s))) return st;
-    }
+    // The contraction of all scales (-1) or of one, and the b part of a general
+    // Slm, accumulated into Tg.
+    auto walk = [&](int only, cudaStream_t q, bool dep) -> int {
+        LwalkArgs la = lwalk_args(p, p->Fw, p->wsC);
+        la.only = only;
+        for (int b = 0; b <= (p->slm_general ? 1 : 0); b++) {
+            if (b) la.G = p->GA_b;
+            la.acc_imag = b;
+            KernelTimer kt(p, S2DWC_KIND_LWALK, q);
+            if (int e = launch_lwalk(la, (b || dep) && !p->timing, q)) return e;
+        }
+        return S2DWC_OK;
+    };
+    const bool per_scale = lwalk_per_scale(p->B, p->NP);
+    if (!per_scale && (st = walk(-1, s, true))) return st;
     const bool serial = full_band_serial && !p->timing && (int)p->ev_done.size() == p->J + 1;
     auto groups = scale_groups(p, STAGE_ANA_BETA, STAGE_ANA_ALPHA, (bool)after);
     if (serial) std::reverse(groups.begin(), groups.end());
@@ -834,7 +839,9 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         auto Tg = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
         auto Tb = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
         auto wav = [&](int j) -> double * { return d_wav + p->wav_off[j]; };
-        if ((e = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj, sj == s))) return e;
+        for (int j : js)
+            if (per_scale && (e = walk(j, sj, false))) return e;
+        if ((e = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj, per_scale || sj == s))) return e;
         if ((e = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj, true))) return e;
         if (full) {
             S2DW_CUDA_TRY(cudaEventRecord(p->ev_done[j0], sj));
@@ -1660,7 +1667,8 @@ int s2dwc_plan_launch_count(const s2dwc_plan *p, int *analysis, int *synthesis)
             }
         return n;
     };
-    if (analysis) *analysis = stages(STAGE_ANA_BETA, STAGE_ANA_ALPHA) + 1 + g;
+    const int walks = lwalk_per_scale(p->B, p->NP) ? p->J + 1 : 1;
+    if (analysis) *analysis = stages(STAGE_ANA_BETA, STAGE_ANA_ALPHA) + 1 + g * walks;
     if (synthesis) *synthesis = stages(STAGE_SYN_ALPHA, STAGE_SYN_BETA) + g;
     return S2DWC_OK;
     S2DW_API_CATCH
