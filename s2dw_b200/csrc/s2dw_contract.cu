@@ -812,13 +812,19 @@ int launch_mwalk_t(const MwalkArgs &a, bool dep, cudaStream_t s)
 
 // Pairs per thread of the analysis kernel: the register limit, halved while
 // the tiles would give fewer than four CTAs per SM (the launch is then bound
-// by the longest walk, which fewer pairs per thread shorten).  Measured on
-// B200, N = 4: B = 512 S = 4 115 us, 2 99, 1 115; B = 256 68, 50, 39.
+// by the longest walk, which fewer pairs per thread shorten); with few n, whose
+// steps are short, four pairs need more CTAs than that.  Kernel on B200 (us, S = 1,
+// 2, 4, 8): N = 2 (NP = 1) B = 384 41, 45, 64, 89; 448 56, 53, 74, 103; 560 92, 72, 95,
+// 127; 640 129, 91, 107, 141; 700 165, 117, 119, 152; 768 207, 145, 144, 164; 900 326,
+// 226, 221, 223; 1024 461, 320, 308, 302.  N = 4 (NP = 2) 384 52, 60, 76; 448 72, 70, 87;
+// 560 123, 95, 105; 600 150, 114, 113; 640 174, 131, 127; 768 285, 211, 199.  N = 8 (NP =
+// 4) 384 82, 89; 448 121, 99; 560 216, 170.
 int lwalk_pairs(int B, int NP)
 {
     int S = lwalk_smax(NP);
     const long long tp = (B + 15) / 16;
-    while (S > 1 && tp * ((B + 8 * S - 1) / (8 * S)) < 592) S /= 2;
+    auto ctas = [&](int s) { return s == 4 && NP == 1 ? 940 : s == 4 && NP == 2 ? 700 : 592; };
+    while (S > 1 && tp * ((B + 8 * S - 1) / (8 * S)) < ctas(S)) S /= 2;
     return S;
 }
 
