@@ -718,16 +718,28 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
 
 // The scales as groups, each run on one stream: a scale with a transform of
 // more than 2048 points (or the 2048-point beta of bl = 1024) fills the GPU and
-// is a group of its own, the rest are one.  Without the former there is one
-// group and everything runs on the caller's stream.  `each`: also the scales
+// is a group of its own, and so is one whose first stage alone is two waves (of
+// 592 CTAs, four per SM) or more: its second stage then fills the gaps that the
+// last wave of another scale's first one leaves.  The rest are one group: without
+// the former there is one, and everything runs on the caller's stream.  Measured
+// on B200 (us, one group and two waves alone): N = 4, B = 400, alpha = 4 analysis 213,
+// 202 and synthesis 202, 193; alpha = 2 246, 229 and 230, 226; B = 512 198, 198 and 223,
+// 217; one wave alone B = 400 alpha = 4 201 and 200, B = 512 192 and 217, but N = 6 340
+// for 327 and 315 for 308.  `each`: also the scales
 // with an eighth of the coefficients or more by themselves (the host-buffer
 // entry points, whose copies follow the groups).
 std::vector<std::vector<int>> scale_groups(const s2dwc_plan *p, Stage a, Stage b, bool each)
 {
     std::vector<std::vector<int>> g;
     std::vector<int> rest;
+    auto waves = [&](int j) {
+        StageEnt e{};
+        int n = 0;
+        const int mode = stage_mode(p, j, a);
+        return stage_plan(mode, p->bl[j], p->czt[j][mode].M, stage_rows(p, j, a), &e, &n) ? n / 592 : 0;
+    };
     for (int j = 0; j <= p->J; j++) {
-        const bool alone = each && 8 * (p->wav_off[j + 1] - p->wav_off[j]) >= p->wav_off[p->J + 1];
+        const bool alone = (each && 8 * (p->wav_off[j + 1] - p->wav_off[j]) >= p->wav_off[p->J + 1]) || waves(j) >= 2;
         if (alone || !stage_small(p, j, a) || !stage_small(p, j, b)) g.push_back({j});
         else rest.push_back(j);
     }
