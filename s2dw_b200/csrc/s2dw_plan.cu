@@ -2262,7 +2262,10 @@ static bool all_pinned(const void *const *ptrs, int n)
 }
 
 // flm between the caller and the device on the legacy stream: queued (to the
-// device) or complete (to the host) on return.
+// device) or complete (to the host) on return.  Up to COPY_PLAIN bytes of pageable
+// memory the runtime's own copy is the shorter one (whole analysis at B=16, static
+// layout 165 us through the staging buffers, 151 without).
+constexpr size_t COPY_PLAIN = 64u << 10;
 static int copy_flm(s2dwc_plan *p, double *host, double2 *dev, bool to_device)
 {
     const size_t n = sizeof(double2) * (size_t)p->B * p->B;
@@ -2271,6 +2274,11 @@ static int copy_flm(s2dwc_plan *p, double *host, double2 *dev, bool to_device)
         S2DW_CUDA_TRY(cudaMemcpyAsync(to_device ? (void *)dev : host, to_device ? (void *)host : dev, n,
                                       to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, 0));
         if (!to_device) S2DW_CUDA_TRY(cudaStreamSynchronize(0));
+        return S2DWC_OK;
+    }
+    if (n <= COPY_PLAIN) {
+        S2DW_CUDA_TRY(cudaMemcpy(to_device ? (void *)dev : host, to_device ? (void *)host : dev, n,
+                                 to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
         return S2DWC_OK;
     }
     StagedCopy c(p, {{reinterpret_cast<char *>(host), reinterpret_cast<char *>(dev), n}}, 0);
@@ -2294,7 +2302,7 @@ static int analysis_host(double *wav_static, double *const *wav_scales, double *
     // The scales' device-to-host copies overlap the other scales' kernels,
     // with the full-band scales run one after another.  Pinned per-scale
     // outputs: each copy follows its scale's kernels on the scale's stream.
-    // Otherwise the staged copy (largest scale first) lets each scale's first
+    // Otherwise the staged copy (last scale first) lets each scale's first
     // chunk wait for that scale's kernels.
     const bool pinned = wav_scales && all_pinned(reinterpret_cast<const void *const *>(wav_scales), J + 1);
     ScaleHook after = [&](int j, cudaStream_t sj) -> int {
@@ -2385,11 +2393,11 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
     int st = host_prepare(B, N, alpha, J, bl_scoeff, K_gamma, Phi2, Slm, &p, hb, lk);
     if (st) return st;
     DeviceGuard dg(p->device);
-    // One copy stream brings the scales in, the last (largest) first, and
-    // each scale's kernels wait for their own copy only, so the largest
-    // scales' kernels overlap the remaining copies and the kernels left after
-    // the last copy are the small scales'.  Pinned per-scale inputs are
-    // queued at once; otherwise each scale's staged chunks (gathered from the
+    // One copy stream brings the scales in and each scale's kernels wait for
+    // their own copy only.  Pinned per-scale inputs are queued at once, the
+    // largest (first) scales first: their kernels overlap the remaining copies,
+    // and those left after the last copy are the small scales' and the
+    // contraction; otherwise each scale's staged chunks (gathered from the
     // static layout first, for that entry point) are queued just before the
     // scale's kernels.
     const bool pinned = wav_scales && all_pinned(reinterpret_cast<const void *const *>(wav_scales), J + 1);
@@ -2398,7 +2406,8 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
     std::unique_ptr<double[]> tmp;  // the static layout's per-scale blocks
     if (!wav_scales) tmp.reset(new double[std::max<long long>(p->wav_off[J + 1], 1)]);
     std::vector<HostSeg> segs;
-    for (int j = J; j >= 0; j--) {
+    for (int k = 0; k <= J; k++) {
+        const int j = pinned ? k : J - k;
         const size_t bytes = sizeof(double) * (size_t)(p->wav_off[j + 1] - p->wav_off[j]);
         if (pinned) {
             S2DW_CUDA_TRY(cudaMemcpyAsync(hb.wav + p->wav_off[j], wav_scales[j], bytes, cudaMemcpyHostToDevice,
