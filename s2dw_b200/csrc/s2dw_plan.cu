@@ -1142,20 +1142,34 @@ int split_prepare(s2dwc_plan *p, int nmaps, cudaStream_t s)
     return S2DWC_OK;
 }
 
+// The scales of a group of nk maps whose stages run together: those of sp_small.
+// One map above B = 256 leaves them only the smallest, as its larger scales finish
+// at different times and need not wait for one another (B=300, us per analysis
+// and synthesis: N=1 549, 430 together, 513, 387 apart; N=4 977, 647 and 964, 624;
+// B=400 N=1 939, 737 and 911, 702; but B=128 N=1 91, 91 together, 118, 106 with the four
+// largest apart, and 2 maps at B=300 N=1 561, 444 and 568, 427).
+std::vector<int> split_small(const s2dwc_plan *p, int nk)
+{
+    std::vector<int> sm;
+    for (int j : p->sp_small)
+        if (nk > 1 || p->B <= 256 || 64 * p->bl[j] < p->B) sm.push_back(j);
+    return sm;
+}
+
 // One group of maps of the split form: digits(j, stream) (digits and
 // contraction of scale j) and the transform stages, which follow it (analysis)
 // or go before it.  Each scale has its stream, forked from and joined back to
 // `s` (all on `s` in timing mode): large(j, stream) runs the stages of a large
-// scale there; small(stream) those of all small scales together on the first
+// scale there; small(stream) those of the scales `sm` together on the first
 // one's stream.
 template <typename D, typename L, typename S>
-int split_scales(s2dwc_plan *p, cudaStream_t s, bool analysis, D &&digits, L &&large, S &&small)
+int split_scales(s2dwc_plan *p, cudaStream_t s, bool analysis, const std::vector<int> &sm, D &&digits, L &&large, S &&small)
 {
     int st;
     const bool par = !p->timing;
     auto stream = [&](int j) { return par ? p->streams[j] : s; };
-    auto is_small = [&](int j) { return std::find(p->sp_small.begin(), p->sp_small.end(), j) != p->sp_small.end(); };
-    const int j0 = p->sp_small.empty() ? -1 : p->sp_small[0];  // the small scales' stream
+    auto is_small = [&](int j) { return std::find(sm.begin(), sm.end(), j) != sm.end(); };
+    const int j0 = sm.empty() ? -1 : sm[0];  // the small scales' stream
     if (par) {
         S2DW_CUDA_TRY(cudaEventRecord(p->ev_fork, s));
         for (int j = 0; j <= p->J; j++) S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j], p->ev_fork, 0));
@@ -1164,7 +1178,7 @@ int split_scales(s2dwc_plan *p, cudaStream_t s, bool analysis, D &&digits, L &&l
         if ((st = small(stream(j0)))) return st;
         if (par) {
             S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j0], p->streams[j0]));
-            for (int j : p->sp_small)
+            for (int j : sm)
                 if (j != j0) S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j], p->ev_join[j0], 0));
         }
     }
@@ -1176,7 +1190,7 @@ int split_scales(s2dwc_plan *p, cudaStream_t s, bool analysis, D &&digits, L &&l
     }
     if (analysis && j0 >= 0) {
         if (par)
-            for (int j : p->sp_small)
+            for (int j : sm)
                 if (j != j0) S2DW_CUDA_TRY(cudaStreamWaitEvent(p->streams[j0], p->ev_join[j], 0));
         if ((st = small(stream(j0)))) return st;
         if (par) S2DW_CUDA_TRY(cudaEventRecord(p->ev_join[j0], p->streams[j0]));
@@ -1188,9 +1202,9 @@ int split_scales(s2dwc_plan *p, cudaStream_t s, bool analysis, D &&digits, L &&l
 
 // Split-form analysis of `nmaps` maps (flm, wav and scoeff of map k at
 // k * B^2, k * wav_total and k * bl_scoeff^2): per group of up to 32 maps,
-// every scale on its own stream runs the map digits, the tensor-core
-// contraction into Tg of the whole group, then the beta and alpha transforms
-// map by map.
+// every scale on its own stream runs the map digits and the tensor-core
+// contraction into Tg of the whole group, then the beta and alpha transforms: a
+// large scale's map by map, the small scales' a chunk of maps per launch.
 int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoeff, const double2 *d_flm,
                        cudaStream_t s)
 {
@@ -1201,6 +1215,7 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
     const long long bs2 = (long long)p->bl_scoeff * p->bl_scoeff;
     for (int g0 = 0; g0 < nmaps; g0 += MAPS) {
         const int nk = std::min(MAPS, nmaps - g0);
+        const std::vector<int> sm = split_small(p, nk);
         auto digits = [&](int j, cudaStream_t sj) -> int {
             int st2;
             const int bl = p->bl[j];
@@ -1262,7 +1277,7 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
             return run_stage(p, STAGE_ANA_ALPHA, js, maps, Tb, wav, tb_map, wav_map, sj);
         };
         st = split_scales(
-            p, s, true, digits,
+            p, s, true, sm, digits,
             [&](int j, cudaStream_t sj) -> int {
                 for (int k = 0; k < nk; k++)
                     if (int e = stages({j}, k, 1, false, sj)) return e;
@@ -1270,7 +1285,7 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
             },
             [&](cudaStream_t sj) -> int {
                 for (int k = 0; k < nk; k += p->sp_chunk)
-                    if (int e = stages(p->sp_small, k, std::min(p->sp_chunk, nk - k), true, sj)) return e;
+                    if (int e = stages(sm, k, std::min(p->sp_chunk, nk - k), true, sj)) return e;
                 return S2DWC_OK;
             });
         if (st) return st;
@@ -1282,10 +1297,10 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
 }
 
 // Split-form synthesis of `nmaps` maps (layouts as run_analysis_split): per
-// group of up to 32 maps, every scale on its own stream runs the alpha and
-// beta transforms map by map into a batch of V tables, their digits and the
-// tensor-core contraction into per-map partial rows; then the scale sum of
-// each map, scales in order.
+// group of up to 32 maps, the alpha and beta transforms (a large scale's map by
+// map, the small scales' a chunk of maps per launch) into a batch of V tables, and
+// every scale's digits and tensor-core contraction into per-map partial rows on its
+// own stream; then the scale sum of each map, scales in order.
 int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *d_wav, const double2 *d_scoeff,
                         cudaStream_t s)
 {
@@ -1296,6 +1311,7 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
     const long long bs2 = (long long)p->bl_scoeff * p->bl_scoeff;
     for (int g0 = 0; g0 < nmaps; g0 += MAPS) {
         const int nk = std::min(MAPS, nmaps - g0);
+        const std::vector<int> sm = split_small(p, nk);
         auto digits = [&](int j, cudaStream_t sj) -> int {
             int st2;
             const int bl = p->bl[j];
@@ -1352,7 +1368,7 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
             return run_stage(p, STAGE_SYN_BETA, js, maps, V, V2f, v_map, v2f_map, sj);
         };
         st = split_scales(
-            p, s, false, digits,
+            p, s, false, sm, digits,
             [&](int j, cudaStream_t sj) -> int {
                 for (int k = 0; k < nk; k++)
                     if (int e = stages({j}, k, 1, false, sj)) return e;
@@ -1360,7 +1376,7 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
             },
             [&](cudaStream_t sj) -> int {
                 for (int k = 0; k < nk; k += p->sp_chunk)
-                    if (int e = stages(p->sp_small, k, std::min(p->sp_chunk, nk - k), true, sj)) return e;
+                    if (int e = stages(sm, k, std::min(p->sp_chunk, nk - k), true, sj)) return e;
                 return S2DWC_OK;
             });
         if (st) return st;
