@@ -2278,21 +2278,24 @@ static bool all_pinned(const void *const *ptrs, int n)
 }
 
 // flm between the caller and the device on the legacy stream: queued (to the
-// device) or complete (to the host) on return.  Up to COPY_PLAIN bytes of pageable
+// device) or complete (to the host) on return.  Of a small piece of pageable
 // memory the runtime's own copy is the shorter one (whole analysis at B=16, static
-// layout 165 us through the staging buffers, 151 without).
-constexpr size_t COPY_PLAIN = 64u << 10;
-static int copy_flm(s2dwc_plan *p, double *host, double2 *dev, bool to_device)
+// layout 179 us through the staging buffers, 156 without, B=64 290 and 268; synthesis
+// B=16 164 and 148, but B=64 232 and 244), and asking whether it is page-locked
+// costs ten: `pinned` says that the caller's other arrays are.
+constexpr size_t PLAIN_IN = 64u << 10, PLAIN_OUT = 16u << 10;
+static int copy_flm(s2dwc_plan *p, double *host, double2 *dev, bool to_device, bool pinned)
 {
     const size_t n = sizeof(double2) * (size_t)p->B * p->B;
     const void *ptr = host;
-    if (all_pinned(&ptr, 1)) {
+    const bool plain = n <= (to_device ? PLAIN_IN : PLAIN_OUT);
+    if ((pinned || !plain) && all_pinned(&ptr, 1)) {
         S2DW_CUDA_TRY(cudaMemcpyAsync(to_device ? (void *)dev : host, to_device ? (void *)host : dev, n,
                                       to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, 0));
         if (!to_device) S2DW_CUDA_TRY(cudaStreamSynchronize(0));
         return S2DWC_OK;
     }
-    if (n <= COPY_PLAIN) {
+    if (plain) {
         S2DW_CUDA_TRY(cudaMemcpy(to_device ? (void *)dev : host, to_device ? (void *)host : dev, n,
                                  to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
         return S2DWC_OK;
@@ -2314,13 +2317,15 @@ static int analysis_host(double *wav_static, double *const *wav_scales, double *
     int st = host_prepare(B, N, alpha, J, bl_scoeff, K_gamma, nullptr, Slm, &p, hb, lk);
     if (st) return st;
     DeviceGuard dg(p->device);
-    if ((st = copy_flm(p, const_cast<double *>(flm), hb.flm, true))) return st;
     // The scales' device-to-host copies overlap the other scales' kernels,
     // with the full-band scales run one after another.  Pinned per-scale
     // outputs: each copy follows its scale's kernels on the scale's stream.
     // Otherwise the staged copy (last scale first) lets each scale's first
     // chunk wait for that scale's kernels.
-    const bool pinned = wav_scales && all_pinned(reinterpret_cast<const void *const *>(wav_scales), J + 1);
+    const void *const *ws = reinterpret_cast<const void *const *>(wav_scales);
+    const bool pin0 = ws && all_pinned(ws, 1);
+    if ((st = copy_flm(p, const_cast<double *>(flm), hb.flm, true, pin0))) return st;
+    const bool pinned = pin0 && all_pinned(ws + 1, J);
     ScaleHook after = [&](int j, cudaStream_t sj) -> int {
         if (pinned)
             S2DW_CUDA_TRY(cudaMemcpyAsync(wav_scales[j], hb.wav + p->wav_off[j],
@@ -2410,10 +2415,12 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
     if (st) return st;
     DeviceGuard dg(p->device);
     // One copy stream brings the scales in and each scale's kernels wait for
-    // their own copy only.  Pinned per-scale inputs are queued at once, the
-    // largest (first) scales first: their kernels overlap the remaining copies,
-    // and those left after the last copy are the small scales' and the
-    // contraction; otherwise each scale's staged chunks (gathered from the
+    // their own copy only.  Pinned per-scale inputs are queued at once: above 32
+    // MB, where the copies are what the call waits for, the largest (first) scales
+    // first, so that their kernels overlap the remaining copies and those left after
+    // the last copy are the small scales' and the contraction (B=1024 N=4 6.66 ->
+    // 6.51 ms), below it last, as a short chain of two kernels (B=24 N=1 96 -> 85
+    // us).  Otherwise each scale's staged chunks (gathered from the
     // static layout first, for that entry point) are queued just before the
     // scale's kernels.
     const bool pinned = wav_scales && all_pinned(reinterpret_cast<const void *const *>(wav_scales), J + 1);
@@ -2422,8 +2429,9 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
     std::unique_ptr<double[]> tmp;  // the static layout's per-scale blocks
     if (!wav_scales) tmp.reset(new double[std::max<long long>(p->wav_off[J + 1], 1)]);
     std::vector<HostSeg> segs;
+    const bool first = pinned && sizeof(double) * (size_t)p->wav_off[J + 1] > STAGE_BYTES;
     for (int k = 0; k <= J; k++) {
-        const int j = pinned ? k : J - k;
+        const int j = first ? k : J - k;
         const size_t bytes = sizeof(double) * (size_t)(p->wav_off[j + 1] - p->wav_off[j]);
         if (pinned) {
             S2DW_CUDA_TRY(cudaMemcpyAsync(hb.wav + p->wav_off[j], wav_scales[j], bytes, cudaMemcpyHostToDevice,
@@ -2462,7 +2470,7 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
         cudaStreamSynchronize(p->copy_stream);  // no read of the caller's arrays outlives the call
         return st;
     }
-    return copy_flm(p, flm, hb.flm, false);
+    return copy_flm(p, flm, hb.flm, false, pinned);
 }
 
 int s2dwc_synthesis_wav2flm(double *flm, const double *wav, const double *scoeff, const double *K_gamma,
