@@ -2305,6 +2305,22 @@ static int copy_flm(s2dwc_plan *p, double *host, double2 *dev, bool to_device, b
     return to_device ? c.to_device_through(0) : c.to_host();
 }
 
+// No copy from or into the caller's arrays may outlive a host call: waits for all
+// of the plan's and the legacy stream's work unless the call ended well (and has
+// waited itself).
+struct HostCallEnd {
+    s2dwc_plan *p;
+    bool done = false;
+    ~HostCallEnd()
+    {
+        if (done) return;
+        cudaStreamSynchronize(0);
+        cudaStreamSynchronize(p->copy_stream);
+        for (auto st : p->streams) cudaStreamSynchronize(st);
+        cudaGetLastError();  // reported by the call
+    }
+};
+
 static int analysis_host(double *wav_static, double *const *wav_scales, double *scoeff, const double *flm,
                          const double *K_gamma, const double *Slm, int J, int B, int N, int bl_scoeff,
                          double alpha)
@@ -2317,6 +2333,7 @@ static int analysis_host(double *wav_static, double *const *wav_scales, double *
     int st = host_prepare(B, N, alpha, J, bl_scoeff, K_gamma, nullptr, Slm, &p, hb, lk);
     if (st) return st;
     DeviceGuard dg(p->device);
+    HostCallEnd end{p};
     // The scales' device-to-host copies overlap the other scales' kernels,
     // with the full-band scales run one after another.  Pinned per-scale
     // outputs: each copy follows its scale's kernels on the scale's stream.
@@ -2335,11 +2352,7 @@ static int analysis_host(double *wav_static, double *const *wav_scales, double *
             S2DW_CUDA_TRY(cudaEventRecord(p->ev_copy[j], sj));
         return S2DWC_OK;
     };
-    if ((st = run_analysis(p, hb.wav, hb.sc, hb.flm, 0, after, true))) {
-        // no copy into the caller's arrays may outlive the call
-        for (int j = 0; j <= J; j++) cudaStreamSynchronize(p->streams[j]);
-        return st;
-    }
+    if ((st = run_analysis(p, hb.wav, hb.sc, hb.flm, 0, after, true))) return st;
     if (!pinned) {
         std::unique_ptr<double[]> tmp;  // the static layout's per-scale blocks, uninitialised
         if (!wav_scales) tmp.reset(new double[std::max<long long>(p->wav_off[J + 1], 1)]);
@@ -2368,16 +2381,14 @@ static int analysis_host(double *wav_static, double *const *wav_scales, double *
         StagedCopy sc(p, segs, p->copy_stream);
         std::function<void(size_t)> seg_done;
         if (!wav_scales) seg_done = scatter;
-        if ((st = sc.start()) || (st = sc.to_host(wait.data(), seg_done))) {
-            cudaStreamSynchronize(p->copy_stream);
-            return st;
-        }
+        if ((st = sc.start()) || (st = sc.to_host(wait.data(), seg_done))) return st;
     }
     if (bl_scoeff > 0)
         S2DW_CUDA_TRY(cudaMemcpy(scoeff, hb.sc, sizeof(double2) * (size_t)bl_scoeff * bl_scoeff,
                                  cudaMemcpyDeviceToHost));
     S2DW_CUDA_TRY(cudaStreamSynchronize(0));
     S2DW_CUDA_TRY(cudaGetLastError());
+    end.done = true;
     return S2DWC_OK;
 }
 
@@ -2414,6 +2425,7 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
     int st = host_prepare(B, N, alpha, J, bl_scoeff, K_gamma, Phi2, Slm, &p, hb, lk);
     if (st) return st;
     DeviceGuard dg(p->device);
+    HostCallEnd end{p};
     // One copy stream brings the scales in and each scale's kernels wait for
     // their own copy only.  Pinned per-scale inputs are queued at once: above 32
     // MB, where the copies are what the call waits for, the largest (first) scales
@@ -2466,11 +2478,10 @@ static int synthesis_host(double *flm, const double *wav_static, const double *c
         S2DW_CUDA_TRY(cudaStreamWaitEvent(sj, p->ev_copy[j], 0));
         return S2DWC_OK;
     };
-    if ((st = run_synthesis(p, hb.flm, hb.wav, hb.sc, 0, copy_in, !pinned))) {
-        cudaStreamSynchronize(p->copy_stream);  // no read of the caller's arrays outlives the call
-        return st;
-    }
-    return copy_flm(p, flm, hb.flm, false, pinned);
+    if ((st = run_synthesis(p, hb.flm, hb.wav, hb.sc, 0, copy_in, !pinned))) return st;
+    st = copy_flm(p, flm, hb.flm, false, pinned);
+    end.done = st == S2DWC_OK;
+    return st;
 }
 
 int s2dwc_synthesis_wav2flm(double *flm, const double *wav, const double *scoeff, const double *K_gamma,

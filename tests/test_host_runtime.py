@@ -181,6 +181,54 @@ def failed_buffers():
         assert n > 3
 
 
+def failed_host_calls(alpha10):
+    """Host calls on page-locked and pageable arrays in which any one runtime
+    call fails: nothing of the caller's memory is still to be copied afterwards."""
+    from s2dw_b200._lib import check, lib
+    from s2dw_b200.workload import transform_setup
+
+    f = _fake()
+    B, N, alpha = 24, 2, alpha10 / 10
+    t = transform_setup(B, N, alpha)
+    J, bs = t["J"], t["bl_scoeff"]
+    dp = ctypes.POINTER(ctypes.c_double)
+    L = lib()
+    size = [L.s2dwc_wav_scale_size(j, B, N, alpha) for j in range(J + 1)]
+    K, S, P = np.asfortranarray(t["K_gamma"]), np.asfortranarray(t["Slm"]), np.ascontiguousarray(t["Phi2"])
+
+    def arrays(pin):
+        a = [np.zeros(n) for n in size] + [np.zeros(2 * B * B), np.zeros(2 * bs * bs)]
+        if pin:
+            for x in a:
+                f.fake_pin(x.ctypes.data, x.nbytes)
+        return a
+
+    def ptr(x):
+        return x.ctypes.data_as(dp)
+
+    for pin in (True, False):
+        a = arrays(pin)
+        w = (dp * (J + 1))(*[ptr(x) for x in a[:J + 1]])
+        flm, sc = a[-2:]
+        calls = [
+            lambda: L.s2dwc_analysis_flm2wav_dynamic(w, ptr(sc), ptr(flm), ptr(K), ptr(S), J, B, N, bs, alpha),
+            lambda: L.s2dwc_synthesis_wav2flm_dynamic(ptr(flm), w, ptr(sc), ptr(K), ptr(P), ptr(S), J, B, N, bs, alpha),
+        ]
+        for call in calls:
+            check(call())
+            assert f.fake_pending_copies() == 0
+            for name in (b"cudaLaunchKernel", b"cudaLaunchKernelExC", b"cudaMemcpyAsync", b"cudaMemcpy", b"cudaEventRecord",
+                         b"cudaStreamWaitEvent", b"cudaStreamSynchronize"):
+                for n in range(1, 400):
+                    f.fake_fail(name, n)
+                    st = call()
+                    if f.fake_armed():
+                        f.fake_fail(name, 1 << 30)
+                        break
+                    assert st != 0 and f.fake_pending_copies() == 0, (pin, name, n, st)
+                    check(call())
+
+
 # ---- tests -----------------------------------------------------------------
 def test_a_failed_reserve_leaves_the_plan_as_it_was(fake):
     """Split workspaces that do not fit: whichever allocation fails, the next
@@ -193,6 +241,11 @@ def test_a_failed_buffer_allocation_can_be_repeated(fake):
     """No pointer of a group of buffers stays set while another of it is
     missing: a kernel would get the null one on the next call."""
     run(fake, "failed_buffers")
+
+
+@pytest.mark.parametrize("alpha10", [20, 11])  # 1.1: no scale large enough for a stream of its own
+def test_no_copy_outlives_a_failed_host_call(fake, alpha10):
+    run(fake, "failed_host_calls", alpha10)
 
 
 if __name__ == "__main__":
