@@ -513,7 +513,8 @@ struct DeviceGuard {
     }
 };
 
-// Brackets one launch with CUDA events on its stream when timing is on.
+// Brackets one launch with CUDA events on its stream when timing is on (p null:
+// never).
 struct KernelTimer {
     s2dwc_plan *p;
     int kind;
@@ -521,7 +522,7 @@ struct KernelTimer {
     cudaEvent_t a = nullptr, b = nullptr;
     KernelTimer(s2dwc_plan *p_, int k, cudaStream_t s_) : p(p_), kind(k), s(s_)
     {
-        if (p->timing && cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess)
+        if (p && p->timing && cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess)
             cudaEventRecord(a, s);
     }
     ~KernelTimer()
@@ -635,9 +636,10 @@ bool stage_small(const s2dwc_plan *p, int j, Stage st)
 // their transforms allow: the large ones one launch each (per map), the rest
 // together.  in(j) and out(j): the first map's input and output of scale j;
 // im(j), om(j): values between maps.  dep: the launch before on `s` is one of
-// the same call (launch_dep).
+// the same call (launch_dep).  `timed`: the plan that records the launches' times,
+// or null.
 template <typename In, typename Out, typename Im, typename Om>
-int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In in, Out out, Im im, Om om,
+int run_stage(const s2dwc_plan *p, s2dwc_plan *timed, Stage stg, const std::vector<int> &js, int maps, In in, Out out, Im im, Om om,
               cudaStream_t s, bool dep = false)
 {
     int st;
@@ -649,8 +651,8 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
     sa.ph = p->ph;
     auto flush = [&]() -> int {
         if (sa.n == 0) return S2DWC_OK;
-        KernelTimer kt(p, stage_kind(stg), s);
-        const int e = launch_stage(stg, sa, dep && !p->timing, s);
+        KernelTimer kt(timed, stage_kind(stg), s);
+        const int e = launch_stage(stg, sa, dep && !(timed && timed->timing), s);
         dep = true;  // the stage's next launch follows this one
         sa.n = sa.ncta = 0;
         return e;
@@ -687,7 +689,7 @@ int run_stage(s2dwc_plan *p, Stage stg, const std::vector<int> &js, int maps, In
                 else ca.in_c = static_cast<const double2 *>(pi) + k * im(j);
                 if (rout) ca.out_r = static_cast<double *>(po) + k * om(j);
                 else ca.out_c = static_cast<double2 *>(po) + k * om(j);
-                KernelTimer kt(p, stage_kind(stg), s);
+                KernelTimer kt(timed, stage_kind(stg), s);
                 if ((st = launch_czt(ca, s))) return st;
             }
             continue;
@@ -853,8 +855,8 @@ int run_analysis(s2dwc_plan *p, double *d_wav, double2 *d_scoeff, const double2 
         auto wav = [&](int j) -> double * { return d_wav + p->wav_off[j]; };
         for (int j : js)
             if (per_scale && (e = walk(j, sj, false))) return e;
-        if ((e = run_stage(p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj, per_scale || sj == s))) return e;
-        if ((e = run_stage(p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj, true))) return e;
+        if ((e = run_stage(p, p, STAGE_ANA_BETA, js, 1, Tg, Tb, one_map, one_map, sj, per_scale || sj == s))) return e;
+        if ((e = run_stage(p, p, STAGE_ANA_ALPHA, js, 1, Tb, wav, one_map, one_map, sj, true))) return e;
         if (full) {
             S2DW_CUDA_TRY(cudaEventRecord(p->ev_done[j0], sj));
             prev_full = j0;
@@ -888,8 +890,8 @@ int run_synthesis(s2dwc_plan *p, double2 *d_flm, const double *d_wav, const doub
         auto wav = [&](int j) -> const double * { return d_wav + p->wav_off[j]; };
         auto V = [&](int j) -> double2 * { return p->wsA + p->offA[j]; };
         auto V2f = [&](int j) -> double2 * { return p->wsC + p->offC[j]; };
-        if ((e = run_stage(p, STAGE_SYN_ALPHA, js, 1, wav, V, one_map, one_map, sj))) return e;
-        return run_stage(p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj, true);
+        if ((e = run_stage(p, p, STAGE_SYN_ALPHA, js, 1, wav, V, one_map, one_map, sj))) return e;
+        return run_stage(p, p, STAGE_SYN_BETA, js, 1, V, V2f, one_map, one_map, sj, true);
     });
     if (st) return st;
     MwalkArgs ma = mwalk_args(p, d_flm, d_scoeff);
@@ -934,7 +936,7 @@ SerialLayout serial_layout(const s2dwc_plan *p)
 // scales one after another, so that each scale reuses the same Tg and Tb.
 // Every element a kernel reads here is written earlier in the same call, so
 // `ws` needs no initial contents.
-int run_analysis_serial(s2dwc_plan *p, unsigned char *ws, double *d_wav, double2 *d_scoeff,
+int run_analysis_serial(const s2dwc_plan *p, unsigned char *ws, double *d_wav, double2 *d_scoeff,
                         const double2 *d_flm, cudaStream_t s)
 {
     const SerialLayout L = serial_layout(p);
@@ -957,8 +959,8 @@ int run_analysis_serial(s2dwc_plan *p, unsigned char *ws, double *d_wav, double2
         auto tg = [&](int) { return Tg; };
         auto tb = [&](int) { return Tb; };
         auto wav = [&](int) { return d_wav + p->wav_off[j]; };
-        if ((st = run_stage(p, STAGE_ANA_BETA, js, 1, tg, tb, one_map, one_map, s))) return st;
-        if ((st = run_stage(p, STAGE_ANA_ALPHA, js, 1, tb, wav, one_map, one_map, s))) return st;
+        if ((st = run_stage(p, nullptr, STAGE_ANA_BETA, js, 1, tg, tb, one_map, one_map, s))) return st;
+        if ((st = run_stage(p, nullptr, STAGE_ANA_ALPHA, js, 1, tb, wav, one_map, one_map, s))) return st;
     }
     return S2DWC_OK;
 }
@@ -1273,8 +1275,8 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
             auto tg_map = [&](int j) { return (long long)p->N * p->bl[j] * p->bl[j]; };
             auto tb_map = [&](int j) { return 2 * tg_map(j); };
             auto wav_map = [&](int) { return wtot; };
-            if (int e = run_stage(p, STAGE_ANA_BETA, js, maps, Tg, Tb, tg_map, tb_map, sj)) return e;
-            return run_stage(p, STAGE_ANA_ALPHA, js, maps, Tb, wav, tb_map, wav_map, sj);
+            if (int e = run_stage(p, p, STAGE_ANA_BETA, js, maps, Tg, Tb, tg_map, tb_map, sj)) return e;
+            return run_stage(p, p, STAGE_ANA_ALPHA, js, maps, Tb, wav, tb_map, wav_map, sj);
         };
         st = split_scales(
             p, s, true, sm, digits,
@@ -1364,8 +1366,8 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
             auto wav_map = [&](int) { return wtot; };
             auto v_map = [&](int j) { return (long long)p->N * p->bl[j] * 2 * p->bl[j]; };
             auto v2f_map = [&](int j) { return p->sp[j].vstride; };
-            if (int e = run_stage(p, STAGE_SYN_ALPHA, js, maps, wav, V, wav_map, v_map, sj)) return e;
-            return run_stage(p, STAGE_SYN_BETA, js, maps, V, V2f, v_map, v2f_map, sj);
+            if (int e = run_stage(p, p, STAGE_SYN_ALPHA, js, maps, wav, V, wav_map, v_map, sj)) return e;
+            return run_stage(p, p, STAGE_SYN_BETA, js, maps, V, V2f, v_map, v2f_map, sj);
         };
         st = split_scales(
             p, s, false, sm, digits,
@@ -2046,8 +2048,7 @@ int s2dwc_plan_analysis_noalloc(const s2dwc_plan *p, double *d_wav, double *d_sc
     void *ws = nullptr;
     int st = noalloc_scratch(p->device, &ws);
     if (st) return st;
-    // run_stage only writes the plan's timing records, and only with timing on
-    return run_analysis_serial(const_cast<s2dwc_plan *>(p), static_cast<unsigned char *>(ws), d_wav, reinterpret_cast<double2 *>(d_scoeff),
+    return run_analysis_serial(p, static_cast<unsigned char *>(ws), d_wav, reinterpret_cast<double2 *>(d_scoeff),
                                reinterpret_cast<const double2 *>(d_flm), (cudaStream_t)stream);
     S2DW_API_CATCH
 }

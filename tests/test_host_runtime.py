@@ -229,6 +229,27 @@ def failed_host_calls(alpha10):
                     check(call())
 
 
+def noalloc_timing():
+    """s2dwc_plan_analysis_noalloc creates nothing, with the plan's timing on
+    too, and leaves its records alone."""
+    f = _fake()
+    p = Plan(24, 4)
+    w, s, x = p.buffers()
+    p.check(p.L.s2dwc_plan_analysis_noalloc(p.h, w, s, x, None))
+    f.fake_log()
+    p.check(p.L.s2dwc_plan_analysis_noalloc(p.h, w, s, x, None))
+    plain = f.fake_log().decode()
+    assert plain and "event" not in plain
+    p.L.s2dwc_plan_set_timing(p.h, 1)
+    p.check(p.L.s2dwc_plan_analysis_noalloc(p.h, w, s, x, None))
+    assert f.fake_log().decode() == plain
+    n, ms = ctypes.c_longlong(), ctypes.c_double()
+    for kind in range(7):
+        p.check(p.L.s2dwc_plan_timing(p.h, kind, ctypes.byref(n), ctypes.byref(ms)))
+        assert n.value == 0
+    p.close()
+
+
 # ---- tests -----------------------------------------------------------------
 def test_a_failed_reserve_leaves_the_plan_as_it_was(fake):
     """Split workspaces that do not fit: whichever allocation fails, the next
@@ -246,6 +267,10 @@ def test_a_failed_buffer_allocation_can_be_repeated(fake):
 @pytest.mark.parametrize("alpha10", [20, 11])  # 1.1: no scale large enough for a stream of its own
 def test_no_copy_outlives_a_failed_host_call(fake, alpha10):
     run(fake, "failed_host_calls", alpha10)
+
+
+def test_noalloc_creates_nothing_in_timing_mode(fake):
+    run(fake, "noalloc_timing")
 
 
 if __name__ == "__main__":
