@@ -146,16 +146,18 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
     const int rampEnd = min(max(p0 + 15, m0 + MT - 1), bend - 1);
     const int nchunks = (bend - lstart + LW_CH - 1) / LW_CH;
 
-    // Staging in a fixed pattern of 16-byte pieces per thread.  No bounds: the
-    // tables have rows to a multiple of 16 l and slack behind the last one;
-    // values of m or l past the band limit are read but belong to pairs that
-    // stay at zero and are not stored.
+    // Staging in a fixed pattern of 16-byte pieces per thread.  Rows of l past
+    // the last one repeat it; columns are not bounded: a row's values past m = B - 1
+    // are zeros up to Bp and, with tiles of more than 32 m, the next row's or the
+    // slack behind the last.  Both are read but belong to pairs that stay at zero
+    // and are not stored, or to steps that do not run.
+    auto lrow = [&](int l) { return (size_t)min(l, B - 1) * Bp; };
     auto stage_tables = [&](int c) {
         const int lc = lstart + c * LW_CH;
         double *b = lsm + (c % LW_ST) * L::BUF;
         {
             const int li = tid >> 3, pc = 2 * (tid & 7);
-            cp16(b + L::AP_OFF + li * 16 + pc, a.Acoef + (size_t)(lc + li) * Bp + p0 + pc);
+            cp16(b + L::AP_OFF + li * 16 + pc, a.Acoef + lrow(lc + li) + p0 + pc);
             // G rows (l, slot, q), packed: gpack_len(l) doubles each, the
             // rows of the 16 l of a chunk consecutive
             const int len = gpack_len(lc);
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
         for (int i = 0; i < (LW_CH * AP + THREADS - 1) / THREADS; i++) {
             const int f = tid + THREADS * i, li = f / AP, pc = 2 * (f % AP);
             if (LW_CH * AP % THREADS == 0 || f < LW_CH * AP)
-                cp16(b + L::AM_OFF + li * MT + pc, a.Acoef + (size_t)(lc + li) * Bp + m0 + pc);
+                cp16(b + L::AM_OFF + li * MT + pc, a.Acoef + lrow(lc + li) + m0 + pc);
         }
     };
     auto stage_f = [&](int c) {
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(THREADS, MINB) lwalk_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < LW_CH * MT / THREADS; i++) {
             const int f = tid + THREADS * i, li = f / MT, pc = f % MT;
-            cp16(b + L::F_OFF + 2 * (li * MT + pc), a.F + (size_t)(lc + li) * Bp + m0 + pc);
+            cp16(b + L::F_OFF + 2 * (li * MT + pc), a.F + lrow(lc + li) + m0 + pc);
         }
     };
     // the first chunks' tables are on their way while the start values are

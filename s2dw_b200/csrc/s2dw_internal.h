@@ -186,9 +186,9 @@ __host__ __device__ __forceinline__ long long gtpack_row(int mp, int R, int Lp)
     return R * ((long long)mp * Lp - 16 * skipped);
 }
 
-// Tables of the plan use a padded row stride Bp = roundup(B, 32); those that
-// the analysis kernel stages have rows to a multiple of 16 and 64 values of
-// slack, so that it reads whole tiles without bounds.
+// Tables of the plan use a padded row stride Bp = roundup(B, 32); Acoef and F have
+// 64 values of slack where tiles of more than 32 m read past the last row
+// (lwalk_slack).
 struct LwalkArgs {
     int B, Bp, N, NP, J;
     int nq[S2DW_NPMAX];
@@ -241,6 +241,7 @@ struct MwalkArgs {
 };
 // Tile lists, ordered by decreasing work so that the longest walks start first.
 int lwalk_pairs(int B, int NP);
+constexpr int lwalk_slack(int S) { return S > 4 ? 64 : 0; }
 bool lwalk_per_scale(int B, int NP);
 int lwalk_split(const std::vector<int> &bl, int S);
 void build_lwalk_tiles(const std::vector<int> &bl, int S, int jsplit, std::vector<int2> &t);

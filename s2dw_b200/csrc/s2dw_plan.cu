@@ -286,16 +286,16 @@ int plan_build(s2dwc_plan *p)
     // row-padded copies (stride Bp) of the tables read by 32-wide tiles
     const int Bp = (B + 31) / 32 * 32;
     p->Bp = Bp;
-    // a: rows to a multiple of 16 and 64 values of slack (LwalkArgs)
-    const int Br = (B + 15) / 16 * 16;
-    auto pad = [&](const std::vector<double> &v, bool a = false) {
-        std::vector<double> o(a ? (size_t)Br * Bp + 64 : (size_t)B * Bp, 0.0);
+    p->lw_pairs = lwalk_pairs(B, p->NP);
+    const int slack = lwalk_slack(p->lw_pairs);
+    auto pad = [&](const std::vector<double> &v, int slack = 0) {
+        std::vector<double> o((size_t)B * Bp + slack, 0.0);
         for (int l = 0; l < B; l++)
             std::copy(v.begin() + (size_t)l * B, v.begin() + (size_t)(l + 1) * B, o.begin() + (size_t)l * Bp);
         return o;
     };
     int st;
-    if ((st = dev_upload(p, &p->Om, pad(t.Om))) || (st = dev_upload(p, &p->Acoef, pad(t.Acoef, true))) ||
+    if ((st = dev_upload(p, &p->Om, pad(t.Om))) || (st = dev_upload(p, &p->Acoef, pad(t.Acoef, slack))) ||
         (st = dev_upload(p, &p->Stm, t.Stm)) || (st = dev_upload(p, &p->Ste, t.Ste)) ||
         (st = dev_upload(p, &p->Gam, pad(t.Gam))) || (st = dev_upload(p, &p->Bcoef, pad(t.Bcoef))) ||
         (st = dev_upload(p, &p->Em, t.Em)) || (st = dev_upload(p, &p->Ee, t.Ee)))
@@ -411,7 +411,7 @@ int plan_build(s2dwc_plan *p)
     p->gpk_total = gpack_row(32 * ((B + 31) / 32), 2 * p->NP);
     p->gtp_total = gtpack_row((B + 15) / 16 * 16, 2 * p->NP + 1, p->Lp);  // whole chunks of m'
     if ((st = dev_alloc(p, &p->GA, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT, (size_t)p->gtp_total)) ||
-        (st = dev_alloc(p, &p->Fw, (size_t)Br * Bp + 64)))
+        (st = dev_alloc(p, &p->Fw, (size_t)B * Bp + slack)))
         return st;
     if (p->form == S2DWC_FORM_SPLIT && ((st = dev_alloc(p, &p->Ga, (size_t)std::max(1LL, na))) ||
                                         (st = dev_alloc(p, &p->Gsyn, (size_t)std::max(1LL, ns)))))
@@ -430,7 +430,6 @@ int plan_build(s2dwc_plan *p)
     if ((st = dev_alloc(p, &p->wsA, (size_t)nA)) || (st = dev_alloc(p, &p->wsC, (size_t)nC))) return st;
     {
         std::vector<int2> tl;
-        p->lw_pairs = lwalk_pairs(B, p->NP);
         p->lw_split = lwalk_split(p->bl, p->lw_pairs);
         build_lwalk_tiles(p->bl, p->lw_pairs, p->lw_split, tl);
         if ((st = dev_upload(p, &p->lw_tiles, tl))) return st;
