@@ -722,8 +722,8 @@ __global__ void __launch_bounds__(THREADS, MINB) mwalk_kernel(const __grid_const
 // there is none, or m' > l.
 __global__ void gpack_kernel(GpackArgs a)
 {
-    const int kb = (a.B + 31) / 32, NP = a.NP;
-    const long long total = gpack_row(32 * kb, 2 * NP);
+    const int kb = (a.B + 15) / 16, NP = a.NP;
+    const long long total = gpack_row(16 * kb, 2 * NP);  // whole chunks of 16 l
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         // row block k holds 32 l of 2 NP rows of 32 (k + 1) values
@@ -739,7 +739,7 @@ __global__ void gpack_kernel(GpackArgs a)
             int j = slot;
             while (j <= a.J && !(a.blo[j] < l && l < a.bl[j])) j += 2;
             if (j <= a.J)
-                v = a.T[(size_t)l * a.Bp + x] * a.H[((size_t)l * NP + q) * a.B + x] *
+                v = a.T[(size_t)l * a.Bp + x] * a.H[hpack(l, NP, q, x)] *
                     a.kappa[((size_t)j * a.B + l) * NP + q];
         }
         a.out[i] = v;
@@ -762,7 +762,7 @@ __global__ void gtpack_kernel(GpackArgs a)
                 int j = r / NP;
                 while (j <= a.J && !(a.blo[j] < l && l < a.bl[j])) j += 2;
                 if (j <= a.J)
-                    v = a.T[(size_t)l * a.Bp + mp] * a.H[((size_t)l * NP + q) * a.B + mp] *
+                    v = a.T[(size_t)l * a.Bp + mp] * a.H[hpack(l, NP, q, mp)] *
                         a.kappa[((size_t)j * a.B + l) * NP + q];
             }
         }
@@ -994,7 +994,7 @@ int launch_mwalk(const MwalkArgs &a, bool dep, cudaStream_t s)
 int launch_gpack(const GpackArgs &a, bool transposed, cudaStream_t s)
 {
     if (!transposed) {
-        const long long total = gpack_row(32 * ((a.B + 31) / 32), 2 * a.NP);
+        const long long total = gpack_row(16 * ((a.B + 15) / 16), 2 * a.NP);
         gpack_kernel<<<(int)std::min<long long>((total + 255) / 256, 148 * 32), 256, 0, s>>>(a);
     } else {
         const dim3 grid(std::max(1, std::min(8, a.Lp / 256)), (a.B + 15) / 16 * 16);

@@ -175,6 +175,11 @@ __host__ __device__ __forceinline__ long long gpack_row(int l, int R)
     const long long k = l >> 5;
     return R * (512 * k * (k + 1) + 32 * (l & 31) * (k + 1));
 }
+// d^l_{m'n_q}(pi/2), m' <= l
+__host__ __device__ __forceinline__ size_t hpack(int l, int NP, int q, int mp)
+{
+    return (size_t)NP * l * (l + 1) / 2 + (size_t)q * (l + 1) + mp;
+}
 // (a tile of at most 32 l reads the chunks of up to 16 m' that start at or
 // below its last l, so 32 values before the chunk's own m' are kept)
 __host__ __device__ __forceinline__ int gtpack_start(int mp) { return mp < 32 ? 0 : 16 * ((mp >> 4) - 2); }
@@ -254,7 +259,7 @@ void build_mwalk_tiles(const std::vector<MwalkInterval> &iv, int2 shape, std::ve
 // T = Gam, kappa of the synthesis), built at set_tables time.
 struct GpackArgs {
     int B, Bp, NP, J, Lp;
-    const double *T, *H, *kappa, *Bcoef;  // H[(l*NP + q)*B + m'], kappa[(j*B + l)*NP + q]
+    const double *T, *H, *kappa, *Bcoef;  // H[hpack(l, NP, q, m')], kappa[(j*B + l)*NP + q]
     double *out;
     short bl[S2DW_JMAX + 1], blo[S2DW_JMAX + 1];
 };
@@ -276,7 +281,7 @@ struct CombineArgs {
 
 // Per-scale factor tables of the split form (see SplitArgs / SplitSynArgs),
 // built at set_tables time: out[((l-blo-1)*NP+q)*stride + x] = T[l*Bp+x] *
-// H[(l*NP+q)*B+x] * kappa[l*NP+q] for x <= l, x < bl; zero elsewhere.
+// H[hpack(l, NP, q, x)] * kappa[l*NP+q] for x <= l, x < bl; zero elsewhere.
 struct GprepArgs {
     int B, Bp, NP, bl, blo, stride;
     const double *T, *H, *kappa;
@@ -284,6 +289,7 @@ struct GprepArgs {
 };
 struct CztArgs {
     int mode, bl, N, NP, rows;
+    bool pfa;              // a prime-factor transform (czt and tw unset)
     int nq[S2DW_NPMAX];
     CztDev czt;
     TwDev tw;
@@ -323,9 +329,12 @@ struct StageArgs {
 };
 enum Stage { STAGE_ANA_BETA, STAGE_ANA_ALPHA, STAGE_SYN_ALPHA, STAGE_SYN_BETA };
 // Fills kind, lg and the CTA count of an entry whose mode, bl and transform
-// length M are given; false where the stage kernels have no transform of that
-// size (it then runs through launch_czt).
-bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta);
+// length M are given (pfa: prime-factor alpha stages where there are any); false
+// where the stage kernels have no transform of that size (it then runs through
+// launch_czt).
+bool stage_plan(int mode, int bl, int M, bool pfa, int rows, StageEnt *e, int *ncta);
+// Whether an alpha stage of this band limit has a prime-factor transform.
+bool pfa_size(int mode, int bl);
 int launch_stage(Stage st, const StageArgs &a, bool dep, cudaStream_t s);
 int launch_stage_beta(Stage st, const StageArgs &a, bool dep, cudaStream_t s);
 // The length-1023 alpha rows have a kernel of their own: a launch holds only
@@ -340,7 +349,6 @@ int launch_fprep(double2 *F, double2 *scoeff, const double2 *flm, const double *
                  cudaStream_t s);
 int launch_mwalk(const MwalkArgs &a, bool dep, cudaStream_t s);
 int launch_czt(const CztArgs &a, cudaStream_t s);
-void set_pfa(bool on);  // prime-factor alpha stages (default on; off: Bluestein)
 // Builds, once per device, the constant tables of the length-2047 and -511
 // alpha stages and the stages' twiddles
 // (the current device; synchronises).  Plan creation calls it, never a capture.

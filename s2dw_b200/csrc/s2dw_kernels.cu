@@ -34,7 +34,7 @@ __global__ void gprep_kernel(GprepArgs a)
         const int q = (int)(r % a.NP), l = a.blo + 1 + (int)(r / a.NP);
         double v = 0.0;
         if (x <= l && x < a.bl)
-            v = a.T[(size_t)l * a.Bp + x] * a.H[((size_t)l * a.NP + q) * a.B + x] * a.kappa[(size_t)l * a.NP + q];
+            v = a.T[(size_t)l * a.Bp + x] * a.H[hpack(l, a.NP, q, x)] * a.kappa[(size_t)l * a.NP + q];
         a.out[i] = v;
     }
 }
@@ -1395,9 +1395,6 @@ int stage_twiddles(const double2 **tw)
     return S2DWC_OK;
 }
 
-static bool g_pfa = true;  // prime-factor alpha stages
-void set_pfa(bool on) { g_pfa = on; }
-
 static bool g_alpha_prefetch = true;  // contiguous-input stages: persistent kernel with prefetched input
 
 // Persistent launch of the prefetching stages: as many CTAs as fit on the
@@ -1435,11 +1432,9 @@ void set_alpha_prefetch(bool on) { g_alpha_prefetch = on; }
 int launch_czt(const CztArgs &a, cudaStream_t s)
 {
     if (a.rows % a.bl) return set_error(S2DWC_ERROR_ARG_INVALID, "transform of %d rows at bl=%d", a.rows, a.bl);
-    if (g_pfa && a.bl == 2048) {
-        if (a.mode == CZT_ANA_ALPHA) return launch_pfa<CZT_ANA_ALPHA>(a, s);
-        if (a.mode == CZT_SYN_ALPHA) return launch_pfa<CZT_SYN_ALPHA>(a, s);
-    }
-    if (g_pfa && a.bl == 1024 && (a.mode == CZT_ANA_ALPHA || a.mode == CZT_SYN_ALPHA)) {
+    if (a.pfa && a.bl == 2048)
+        return a.mode == CZT_ANA_ALPHA ? launch_pfa<CZT_ANA_ALPHA>(a, s) : launch_pfa<CZT_SYN_ALPHA>(a, s);
+    if (a.pfa && a.bl == 1024) {
         int dev = 0;
         S2DW_CUDA_TRY(cudaGetDevice(&dev));
         if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
@@ -1468,11 +1463,18 @@ int launch_czt(const CztArgs &a, cudaStream_t s)
     return set_error(S2DWC_ERROR_SIZE_INVALID, "transform size %d unsupported", M);
 }
 
-bool stage_plan(int mode, int bl, int M, int rows, StageEnt *e, int *ncta)
+bool pfa_size(int mode, int bl)
+{
+    return (mode == CZT_ANA_ALPHA || mode == CZT_SYN_ALPHA) && bl >= 2 && bl <= 2048 && (bl & (bl - 1)) == 0 && bl != 64 &&
+           bl != 16;
+}
+
+bool stage_plan(int mode, int bl, int M, bool pfa, int rows, StageEnt *e, int *ncta)
 {
     const bool alpha = mode == CZT_ANA_ALPHA || mode == CZT_SYN_ALPHA;
     int per = 0;  // rows per CTA
-    if (alpha && g_pfa && bl <= 512 && bl >= 2 && (bl & (bl - 1)) == 0 && bl != 64 && bl != 16) {
+    if (pfa && pfa_size(mode, bl)) {
+        if (bl > 512) return false;
         e->kind = STAGE_PFA;
         e->lg = 0;
         per = bl == 512 ? 1 : bl == 256 ? PFD_RP : pfs_rows(2 * bl - 1);

@@ -42,6 +42,7 @@ struct s2dwc_plan {
     std::vector<int> ana_beta_mode, syn_beta_mode;
     std::map<int, TwDev> tw;
     const double2 *tw2048 = nullptr;  // StageArgs::tw, of the device
+    bool pfa = true;  // prime-factor alpha stages (S2DW_PFA=0 at creation: Bluestein everywhere)
     std::vector<double *> wq;  // quadrature weights per scale
     // caller tables folded into per-scale factor tables
     double *kappaA = nullptr, *kappaS = nullptr, *Phi2 = nullptr;
@@ -257,6 +258,7 @@ int plan_build(s2dwc_plan *p)
 {
     const int B = p->B, N = p->N, J = p->J;
     p->NP = positive_nset(N, p->nq);
+    if (const char *e = getenv("S2DW_PFA")) p->pfa = atoi(e) != 0;
     p->bl.resize(J + 1);
     p->blo.resize(J + 1);
     p->wav_off.assign(J + 2, 0);
@@ -300,11 +302,11 @@ int plan_build(s2dwc_plan *p)
         (st = dev_upload(p, &p->Gam, pad(t.Gam))) || (st = dev_upload(p, &p->Bcoef, pad(t.Bcoef))) ||
         (st = dev_upload(p, &p->Em, t.Em)) || (st = dev_upload(p, &p->Ee, t.Ee)))
         return st;
-    {  // d^l_{m'n}(pi/2) of the plan's n alone: [(l*NP + q)*B + m']
-        std::vector<double> h((size_t)B * p->NP * B);
+    {  // d^l_{m'n}(pi/2) of the plan's n alone
+        std::vector<double> h(hpack(B, p->NP, 0, 0));
         for (int l = 0; l < B; l++)
             for (int q = 0; q < p->NP; q++)
-                std::copy_n(t.H.begin() + ((size_t)l * hn + p->nq[q]) * B, B, h.begin() + ((size_t)l * p->NP + q) * B);
+                std::copy_n(t.H.begin() + ((size_t)l * hn + p->nq[q]) * B, l + 1, h.begin() + hpack(l, p->NP, q, 0));
         if ((st = dev_upload(p, &p->H, h))) return st;
     }
 
@@ -327,9 +329,23 @@ int plan_build(s2dwc_plan *p)
             // beta transforms as one power-of-two FFT of length L = 2 bl (a
             // DCT-III / DCT-II pair of that length) when 2 bl is a power of two
             const int L2 = 2 * b;
+            // two-level twiddles of the transforms that the stage kernels do not have
+            auto twiddles = [&](int mode, int M) -> int {
+                StageEnt e{};
+                int n = 0, st2;
+                if (p->tw.count(M) || stage_plan(mode, b, M, p->pfa, 1, &e, &n)) return S2DWC_OK;
+                std::vector<double2> hi, lo;
+                build_twiddles(M, hi, lo);
+                TwDev tw;
+                tw.M = M;
+                if ((st2 = dev_upload(p, &tw.hi, hi)) || (st2 = dev_upload(p, &tw.lo, lo))) return st2;
+                p->tw[M] = tw;
+                return S2DWC_OK;
+            };
             const bool fft_beta = L2 >= 16 && L2 <= 4096 && (L2 & (L2 - 1)) == 0;
             for (int md = 0; md < 4; md++) {
                 if (fft_beta && (md == CZT_ANA_BETA || md == CZT_SYN_BETA)) continue;
+                if (p->pfa && pfa_size(md, b)) continue;  // (no chirps)
                 CztSpec c = specs[md];
                 c.M = czt_size(c.K, c.Bout);
                 std::vector<double2> pre, post, Hf;
@@ -347,14 +363,7 @@ int plan_build(s2dwc_plan *p)
                     return st;
                 }
                 arr[md] = d;
-                if (!p->tw.count(c.M)) {
-                    std::vector<double2> hi, lo;
-                    build_twiddles(c.M, hi, lo);
-                    TwDev tw;
-                    tw.M = c.M;
-                    if ((st = dev_upload(p, &tw.hi, hi)) || (st = dev_upload(p, &tw.lo, lo))) return st;
-                    p->tw[c.M] = tw;
-                }
+                if ((st = twiddles(md, c.M))) return st;
             }
             if (fft_beta) {
                 std::vector<double2> twb;
@@ -366,14 +375,7 @@ int plan_build(s2dwc_plan *p)
                                      0, L2};
                     if ((st = dev_upload(p, &d.pre, twb))) return st;
                     arr[md] = d;
-                }
-                if (!p->tw.count(L2)) {
-                    std::vector<double2> hi, lo;
-                    build_twiddles(L2, hi, lo);
-                    TwDev tw;
-                    tw.M = L2;
-                    if ((st = dev_upload(p, &tw.hi, hi)) || (st = dev_upload(p, &tw.lo, lo))) return st;
-                    p->tw[L2] = tw;
+                    if ((st = twiddles(md, L2))) return st;
                 }
             }
             it = by_bl.emplace(b, arr).first;
@@ -408,7 +410,7 @@ int plan_build(s2dwc_plan *p)
     }
     p->mw_shape = mwalk_shape(B, p->NP);
     p->Lp = (B + 7) / 8 * 8 + 16 * p->mw_shape.x;
-    p->gpk_total = gpack_row(32 * ((B + 31) / 32), 2 * p->NP);
+    p->gpk_total = gpack_row(16 * ((B + 15) / 16), 2 * p->NP);
     p->gtp_total = gtpack_row((B + 15) / 16 * 16, 2 * p->NP + 1, p->Lp);  // whole chunks of m'
     if ((st = dev_alloc(p, &p->GA, (size_t)p->gpk_total)) || (st = dev_alloc(p, &p->GT, (size_t)p->gtp_total)) ||
         (st = dev_alloc(p, &p->Fw, (size_t)B * Bp + slack)))
@@ -628,7 +630,7 @@ bool stage_small(const s2dwc_plan *p, int j, Stage st)
     StageEnt e{};
     int n = 0;
     const int mode = stage_mode(p, j, st);
-    return stage_plan(mode, p->bl[j], p->czt[j][mode].M, 1, &e, &n);
+    return stage_plan(mode, p->bl[j], p->czt[j][mode].M, p->pfa, 1, &e, &n);
 }
 
 // One stage of scales `js` for `maps` maps on stream s, in as few launches as
@@ -662,7 +664,7 @@ int run_stage(const s2dwc_plan *p, s2dwc_plan *timed, Stage stg, const std::vect
         int n = 0;
         const int mode = stage_mode(p, j, stg);
         e.bl = p->bl[j];
-        return !(stage_plan(mode, p->bl[j], p->czt[j][mode].M, 1, &e, &n) && stage_alone(e));
+        return !(stage_plan(mode, p->bl[j], p->czt[j][mode].M, p->pfa, 1, &e, &n) && stage_alone(e));
     });
     for (int j : order) {
         const int mode = stage_mode(p, j, stg), rows = stage_rows(p, j, stg);
@@ -676,7 +678,8 @@ int run_stage(const s2dwc_plan *p, s2dwc_plan *timed, Stage stg, const std::vect
             std::memcpy(ca.nq, p->nq, sizeof(ca.nq));
             ca.rows = rows;
             ca.czt = c;
-            if ((st = plan_tw(p, c.M, &ca.tw))) return st;
+            ca.pfa = p->pfa && pfa_size(mode, p->bl[j]);
+            if (!ca.pfa && (st = plan_tw(p, c.M, &ca.tw))) return st;
             ca.out_stride = p->gs_stride[j];
             ca.wq = p->wq[j];
             ca.scale = syn_alpha_scale(p, j);
@@ -695,7 +698,7 @@ int run_stage(const s2dwc_plan *p, s2dwc_plan *timed, Stage stg, const std::vect
         }
         StageEnt e{};
         int n = 0;
-        stage_plan(mode, p->bl[j], c.M, rows * maps, &e, &n);
+        stage_plan(mode, p->bl[j], c.M, p->pfa, rows * maps, &e, &n);
         e.bl = p->bl[j];
         if ((sa.n == STAGE_MAX || (sa.n > 0 && stage_alone(sa.e[0]) != stage_alone(e))) && (st = flush())) return st;
         e.cta0 = sa.ncta;
@@ -737,7 +740,7 @@ std::vector<std::vector<int>> scale_groups(const s2dwc_plan *p, Stage a, Stage b
         StageEnt e{};
         int n = 0;
         const int mode = stage_mode(p, j, a);
-        return stage_plan(mode, p->bl[j], p->czt[j][mode].M, stage_rows(p, j, a), &e, &n) ? n / 592 : 0;
+        return stage_plan(mode, p->bl[j], p->czt[j][mode].M, p->pfa, stage_rows(p, j, a), &e, &n) ? n / 592 : 0;
     };
     for (int j = 0; j <= p->J; j++) {
         const bool alone = (each && 8 * (p->wav_off[j + 1] - p->wav_off[j]) >= p->wav_off[p->J + 1]) || waves(j) >= 2;
@@ -1476,10 +1479,6 @@ int s2dwc_plan_create(s2dwc_plan **plan, int B, int N, double alpha, int J, int 
         return set_error(S2DWC_ERROR_ARG_INVALID, "device %d out of range (%d devices)", device, ndev);
     DeviceGuard dg(device);
     {
-        const char *pf = getenv("S2DW_PFA");
-        set_pfa(pf ? atoi(pf) != 0 : true);
-    }
-    {
         const char *ap = getenv("S2DW_ALPHA_PREFETCH");
         set_alpha_prefetch(ap ? atoi(ap) != 0 : true);
     }
@@ -1689,7 +1688,7 @@ int s2dwc_plan_launch_count(const s2dwc_plan *p, int *analysis, int *synthesis)
                     e.bl = p->bl[j];
                     int c = 0;
                     const int mode = stage_mode(p, j, st);
-                    if (!stage_plan(mode, p->bl[j], p->czt[j][mode].M, 1, &e, &c)) n++;
+                    if (!stage_plan(mode, p->bl[j], p->czt[j][mode].M, p->pfa, 1, &e, &c)) n++;
                     else (stage_alone(e) ? alone : small)++;
                 }
                 n += (small + STAGE_MAX - 1) / STAGE_MAX + (alone + STAGE_MAX - 1) / STAGE_MAX;

@@ -250,6 +250,36 @@ def noalloc_timing():
     p.close()
 
 
+def alpha_stage_choice(B):
+    """The alpha stages' transforms are the plan's own choice (S2DW_PFA at its
+    creation), whatever plans come after it, and the tables are those it needs."""
+    f = _fake()
+
+    def create(pfa):
+        os.environ["S2DW_PFA"] = pfa
+        p = Plan(B, 2)
+        need = ctypes.c_longlong()
+        p.check(p.L.s2dwc_plan_footprint(B, 2, 2.0, p.J, 0, ctypes.byref(need)))
+        assert p.bytes() == need.value
+        return p
+
+    def launches(p):
+        w, s, x = p.buffers()
+        f.fake_log()
+        p.check(p.L.s2dwc_plan_analysis(p.h, w, s, x, None))
+        p.check(p.L.s2dwc_plan_synthesis(p.h, x, w, s, None))
+        return [k[3:] for k in _launches(f)]
+
+    blue = create("0")
+    first = launches(blue)
+    prime = create("1")
+    second = launches(prime)
+    assert launches(blue) == first != second
+    assert prime.bytes() < blue.bytes()
+    again = create("0")
+    assert launches(prime) == second and launches(again) == first
+
+
 # ---- tests -----------------------------------------------------------------
 def test_a_failed_reserve_leaves_the_plan_as_it_was(fake):
     """Split workspaces that do not fit: whichever allocation fails, the next
@@ -271,6 +301,11 @@ def test_no_copy_outlives_a_failed_host_call(fake, alpha10):
 
 def test_noalloc_creates_nothing_in_timing_mode(fake):
     run(fake, "noalloc_timing")
+
+
+@pytest.mark.parametrize("B", [128, 256, 1024])
+def test_alpha_stages_are_the_plan_s_choice(fake, B):
+    run(fake, "alpha_stage_choice", B)
 
 
 if __name__ == "__main__":
