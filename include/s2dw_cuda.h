@@ -271,9 +271,10 @@ int s2dwc_plan_set_split_min_batch(s2dwc_plan *plan, int nmaps);
  * this one, then take SMs ahead of work of lower priority: a server gives
  * its small, latency-bound transforms precedence over the full-band scales
  * of large ones.  Waits for the plan's streams to drain; call it between
- * transforms, outside stream capture.  A transform called on a stream of
- * another priority is forked from that stream to the plan's own and joined
- * back to it.  No counterpart in the reference. */
+ * transforms, outside stream capture.  A transform of either form called on a
+ * stream of another priority is forked from that stream to the plan's own and
+ * joined back to it (s2dwc_plan_analysis_noalloc and s2dwc_plan_stat_moments
+ * stay on the caller's stream).  No counterpart in the reference. */
 int s2dwc_plan_set_priority(s2dwc_plan *plan, int priority);
 
 /* Bound, in nanoseconds, on every wait of the split-form kernels' pipeline

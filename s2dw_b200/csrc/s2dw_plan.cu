@@ -70,7 +70,7 @@ struct s2dwc_plan {
     std::vector<MwalkInterval> mw_iv;
     double2 *ph = nullptr;                    // gamma-DFT phases, LwalkArgs::ph
     cudaEvent_t ev_fork = nullptr;
-    cudaStream_t prio_stream = nullptr;  // set_priority: where the FP64 form's transforms run
+    cudaStream_t prio_stream = nullptr;  // set_priority: where the transforms run
     int prio = 0;                        // its priority
     std::vector<cudaEvent_t> ev_join;
     // device buffers of the host-buffer entry points (allocated on first use)
@@ -1213,6 +1213,10 @@ int run_analysis_split(s2dwc_plan *p, int nmaps, double *d_wav, double2 *d_scoef
                        cudaStream_t s)
 {
     int st;
+    if (leaves_stream(p, s, st))
+        return st ? st : at_priority(p, s, [&](cudaStream_t q) {
+            return run_analysis_split(p, nmaps, d_wav, d_scoeff, d_flm, q);
+        });
     if ((st = split_prepare(p, nmaps, s))) return st;
     const int MAPS = split_maps_per_pass();
     const long long wtot = p->wav_off[p->J + 1], B2 = (long long)p->B * p->B;
@@ -1309,6 +1313,10 @@ int run_synthesis_split(s2dwc_plan *p, int nmaps, double2 *d_flm, const double *
                         cudaStream_t s)
 {
     int st;
+    if (leaves_stream(p, s, st))
+        return st ? st : at_priority(p, s, [&](cudaStream_t q) {
+            return run_synthesis_split(p, nmaps, d_flm, d_wav, d_scoeff, q);
+        });
     if ((st = split_prepare(p, nmaps, s))) return st;
     const int MAPS = split_maps_per_pass();
     const long long wtot = p->wav_off[p->J + 1], B2 = (long long)p->B * p->B;

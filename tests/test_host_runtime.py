@@ -280,6 +280,21 @@ def alpha_stage_choice(B):
     assert launches(prime) == second and launches(again) == first
 
 
+def priority(form):
+    f = _fake()
+    p = Plan(24, 4, form=form)
+    p.check(p.L.s2dwc_plan_set_priority(p.h, -3))
+    w, s, x = p.buffers(3)
+    p.check(p.reserve(3))
+    f.fake_log()
+    for maps in (1, 3):
+        p.check(p.L.s2dwc_plan_analysis_batch(p.h, maps, w, s, x, None))
+        p.check(p.L.s2dwc_plan_synthesis_batch(p.h, maps, x, w, s, None))
+    got = _launches(f)
+    assert len(got) > 6
+    assert all(k[1] == -3 for k in got), [k for k in got if k[1] != -3]
+
+
 # ---- tests -----------------------------------------------------------------
 def test_a_failed_reserve_leaves_the_plan_as_it_was(fake):
     """Split workspaces that do not fit: whichever allocation fails, the next
@@ -306,6 +321,12 @@ def test_noalloc_creates_nothing_in_timing_mode(fake):
 @pytest.mark.parametrize("B", [128, 256, 1024])
 def test_alpha_stages_are_the_plan_s_choice(fake, B):
     run(fake, "alpha_stage_choice", B)
+
+
+@pytest.mark.parametrize("form", [0, 1])
+def test_every_kernel_has_the_plan_s_priority(fake, form):
+    """On a stream of another priority, in both forms."""
+    run(fake, "priority", form)
 
 
 if __name__ == "__main__":
