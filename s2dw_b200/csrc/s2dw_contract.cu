@@ -29,18 +29,12 @@
 #include <type_traits>
 #include <vector>
 
+#include "s2dw_fft.cuh"
 #include "s2dw_internal.h"
 
 namespace s2dw {
 namespace {
 
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b)
-{
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 // z * i^k
 __device__ __forceinline__ double2 cipow(double2 z, int k)
 {

@@ -83,7 +83,6 @@ __device__ __forceinline__ void twiddle_powers16(double2 (&v)[16], double2 w)
     v[15] = cmul(v[15], cmul(w8, w7));
 }
 
-// One radix-16 pass (16 values per thread, thread t = butterfly j).
 // 32-byte accesses of the alpha stages (the two b columns of a b pair at
 // one (g, m)): one 256-bit access instead of two 128-bit ones halves the
 // L1 wavefronts of these row-strided loads and stores.  The streamed input
@@ -130,10 +129,6 @@ __device__ __forceinline__ double2 hf_at(const double2 *Hf, int k, int M)
 // (+ cos, - sin; the sin rows' input carries (-1)^b).  A sin row's V'(0)
 // multiplies d^l_{0m}(pi/2) d^l_{0n}(pi/2), which is zero for every l when m+n
 // is odd, so it is stored as 0.
-
-// Position b of the beta grid whose value sits at FFT index k in the
-// DCT-II / DCT-III reordering (k < bl: b = 2k; k >= bl: b = 2L-1-2k).
-__device__ __forceinline__ int beta_src(int k, int bl) { return k < bl ? 2 * k : 4 * bl - 1 - 2 * k; }
 
 // DCT-III input V_k of the analysis beta transform of row X (bl values).
 __device__ __forceinline__ double2 ana_beta_in(const double2 *X, int k, int bl, bool sn, const double2 *e)
@@ -342,7 +337,6 @@ __device__ __forceinline__ void pfa_dft(double2 (&x)[R])
     }
 }
 
-// DFTs of length R along the dimension of stride S of the 4-D layout.
 template <>
 __device__ __forceinline__ void pfa_cs<11>(int j, double &c, double &s)
 {

@@ -102,7 +102,8 @@ int positive_nset(int N, int *nq);
 constexpr int S2DW_NMAX = 16;
 constexpr int S2DW_NPMAX = S2DW_NMAX / 2;
 // Largest scale index J (scales j = 0..J): per-scale arrays passed to kernels
-// by value are sized by it (J+1 entries, under 2.2 KB of kernel arguments).
+// by value are sized by it (J+1 entries; MwalkArgs, the largest, is 3.4 KB of the
+// 4 KB that kernel arguments may be).
 constexpr int S2DW_JMAX = 127;
 
 struct RecTables {

@@ -613,6 +613,7 @@ __device__ __forceinline__ void pfa_load(const CztArgs &a, double2 *X, Pos pos)
 
 constexpr int PFA_N = 4095, PFA_THREADS = 256;
 
+// DFTs of length R along the dimension of stride S of the 4-D layout.
 template <int R, int S, int SIGN>
 __device__ __forceinline__ void pfa_stage(double2 *sm, int t)
 {
@@ -685,7 +686,7 @@ __global__ void __launch_bounds__(PFA_THREADS, 3) pfa_alpha_kernel(CztArgs a)
 // DFT; y_0 = x_0 + the convolution input's sum.  About 60 FP64 operations per
 // point against ~240 for the 4096-point Bluestein convolution.
 // ---------------------------------------------------------------------------
-constexpr int PFB_N = 2047;
+constexpr int PFB_N = 2047, PFB_THREADS = 128;
 constexpr int PFB_P = 25;              // pitch of d2 in the shared row
 constexpr int PFB_XS = PFB_P * 89;     // shared row size
 constexpr int PFB_SP = 103;            // pitch of a Rader column (positions i + 9 j, i < 8, j < 11)
@@ -724,11 +725,11 @@ __global__ void rader_init_kernel()
     g_rader_w[blockIdx.x][k % 8 + 8 * (k % 11)] = make_double2(re / 88.0, im / 88.0);
 }
 
-template <int MODE, int NT>
-__global__ void __launch_bounds__(NT, (NT == 128 ? 3 : 2)) pfa2047_alpha_kernel(CztArgs a)
+template <int MODE>
+__global__ void __launch_bounds__(PFB_THREADS, 3) pfa2047_alpha_kernel(CztArgs a)
 {
     static_assert(MODE == CZT_ANA_ALPHA || MODE == CZT_SYN_ALPHA, "alpha stages only");
-    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1;
+    constexpr int SIGN = MODE == CZT_ANA_ALPHA ? +1 : -1, NT = PFB_THREADS;
     extern __shared__ double2 smem[];
     // the row in layout d1 + 25 d2 (pitch 25: conflict-free shared-memory
     // access for the length-23 DFTs, two-way for the output gather); the 23
@@ -1340,7 +1341,7 @@ static int launch_pfa(const CztArgs &a, cudaStream_t s)
     return S2DWC_OK;
 }
 
-template <int MODE, int NT>
+template <int MODE>
 static int launch_pfa2047(const CztArgs &a, cudaStream_t s)
 {
     const size_t smem = sizeof(double2) * (PFB_XS + 23 * PFB_SP + 23);
@@ -1348,12 +1349,12 @@ static int launch_pfa2047(const CztArgs &a, cudaStream_t s)
     int dev = 0;
     S2DW_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 64 && !attr[dev]) {
-        S2DW_CUDA_TRY(cudaFuncSetAttribute(pfa2047_alpha_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        S2DW_CUDA_TRY(cudaFuncSetAttribute(pfa2047_alpha_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem));
         attr[dev] = true;
     }
     const dim3 grid(a.bl, a.rows / a.bl);  // (b pair, g)
-    pfa2047_alpha_kernel<MODE, NT><<<grid, NT, smem, s>>>(a);
+    pfa2047_alpha_kernel<MODE><<<grid, PFB_THREADS, smem, s>>>(a);
     S2DW_CUDA_TRY(cudaGetLastError());
     return S2DWC_OK;
 }
@@ -1439,8 +1440,8 @@ int launch_czt(const CztArgs &a, cudaStream_t s)
         S2DW_CUDA_TRY(cudaGetDevice(&dev));
         if (dev < 0 || dev >= 64 || !g_rader_ready[dev])
             return set_error(S2DWC_ERROR_NOT_INIT, "the length-2047 alpha tables are not built on device %d", dev);
-        return a.mode == CZT_ANA_ALPHA ? launch_pfa2047<CZT_ANA_ALPHA, 128>(a, s)
-                                       : launch_pfa2047<CZT_SYN_ALPHA, 128>(a, s);
+        return a.mode == CZT_ANA_ALPHA ? launch_pfa2047<CZT_ANA_ALPHA>(a, s)
+                                       : launch_pfa2047<CZT_SYN_ALPHA>(a, s);
     }
     // Stages whose input row is contiguous: persistent kernel with the next
     // row prefetched (synthesis alpha 4% faster than one row per CTA at
