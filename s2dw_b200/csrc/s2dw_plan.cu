@@ -2072,7 +2072,7 @@ struct HostCallBuffers {
 
 // Folds the caller's tables into the cached plan unless they equal, byte for
 // byte, the ones folded last: callers pass the same K_gamma and Slm on every
-// call, and refolding them costs 2(J+1) table kernels and a device
+// call, and refolding them costs two table kernels or more and a device
 // synchronisation per call.  Phi2 (synthesis only) is compared and uploaded
 // on its own; the analysis passes none and leaves the plan's copy as is.
 static int host_fold_tables(s2dwc_plan *p, const double *K_gamma, const double *Phi2, const double *Slm,
