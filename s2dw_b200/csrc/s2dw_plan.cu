@@ -723,12 +723,12 @@ int run_stage(const s2dwc_plan *p, s2dwc_plan *timed, Stage stg, const std::vect
 // The scales as groups, each run on one stream: a scale with a transform of
 // more than 2048 points (or the 2048-point beta of bl = 1024) fills the GPU and
 // is a group of its own, and so is one whose first stage alone is two waves (of
-// 592 CTAs, four per SM) or more: its second stage then fills the gaps that the
-// last wave of another scale's first one leaves.  The rest are one group: without
+// 592 CTAs, four per SM) or more, or one wave if it is a full-band scale: its second
+// stage then fills the gaps that the last wave of another scale's first one leaves.  The rest are one group: without
 // the former there is one, and everything runs on the caller's stream.  Measured
-// on B200 (us, one group and two waves alone): N = 4, B = 400, alpha = 4 analysis 213,
-// 202 and synthesis 202, 193; alpha = 2 246, 229 and 230, 226; B = 512 198, 198 and 223,
-// 217; one wave alone B = 400 alpha = 4 201 and 200, B = 512 192 and 217, but N = 6 340
+// on B200 (us, one group and this rule): N = 4, B = 400, alpha = 4 analysis 213, 202 and
+// synthesis 202, 194; alpha = 2 249, 231 and 232, 216; B = 512 199, 193 and 225, 212; N =
+// 2, B = 450 177, 159 and 129, 122; any scale of one wave alone N = 6, B = 400 330
 // for 327 and 315 for 308.  `each`: also the scales
 // with an eighth of the coefficients or more by themselves (the host-buffer
 // entry points, whose copies follow the groups).
@@ -743,7 +743,8 @@ std::vector<std::vector<int>> scale_groups(const s2dwc_plan *p, Stage a, Stage b
         return stage_plan(mode, p->bl[j], p->czt[j][mode].M, p->pfa, stage_rows(p, j, a), &e, &n) ? n / 592 : 0;
     };
     for (int j = 0; j <= p->J; j++) {
-        const bool alone = (each && 8 * (p->wav_off[j + 1] - p->wav_off[j]) >= p->wav_off[p->J + 1]) || waves(j) >= 2;
+        const bool alone = (each && 8 * (p->wav_off[j + 1] - p->wav_off[j]) >= p->wav_off[p->J + 1]) ||
+                           waves(j) >= (p->bl[j] == p->bl[0] ? 1 : 2);
         if (alone || !stage_small(p, j, a) || !stage_small(p, j, b)) g.push_back({j});
         else rest.push_back(j);
     }
