@@ -1090,9 +1090,10 @@ __device__ __forceinline__ int pfc_out_pos(int k) { return k % 3 + 3 * (k % 11) 
 // the 33 length-31 DFTs with a column's real and imaginary parts in two lanes
 // (66 lanes; one thread per column took 168 registers and left 95 of 128 threads
 // waiting).
-// The launch follows the other scales' alpha launch of its stage.  Run beside it
-// (forked to a second stream) it took the same time: B = 512, N = 4 analysis 196
-// and 194 us, synthesis 222 and 222, B = 1024 810 and 813, 862 and 861.
+// The launch follows the other scales' alpha launch of its stage (where they share
+// a group).  Run beside it, forked to a second stream, it took the same time: B =
+// 512, N = 4 analysis 196 and 194 us, synthesis 222 and 222, B = 1024 810 and 813, 862
+// and 861.
 constexpr int PFC_THREADS = 96;
 
 template <int MODE>
