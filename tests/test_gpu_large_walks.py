@@ -70,3 +70,45 @@ def test_walks_per_scale_of_a_general_slm():
     top = np.abs(wav["ab"]).max()
     assert np.abs(wav["ab"] - wav["a"] - wav["jb"]).max() <= 1e-12 * top
     assert np.abs(wav["jb"]).max() > 0.1 * top
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,N,alpha", [(520, 14, 4.0), (450, 2, 2.0), (512, 4, 2.0)])
+def test_scales_on_their_own_streams_in_host_calls_and_graphs(B, N, alpha):
+    """Walks per scale and full-band scales as groups of their own: the host entry
+    points, whose groups follow their copies, and a CUDA graph of both directions give the
+    device calls' values bit for bit."""
+    import torch
+
+    from s2dw_b200 import core
+    from s2dw_b200.device import Plan
+    from s2dw_b200.workload import gaussian_flm, transform_setup
+
+    t = transform_setup(B, N, alpha)
+    J, bs = t["J"], t["bl_scoeff"]
+    f = gaussian_flm(B, seed=5)
+    plan = Plan(B, N, alpha, J)
+    plan.set_tables(t["K_gamma"], t["Phi2"], t["Slm"], bs)
+    flm = torch.from_numpy(np.ascontiguousarray(f.T)).cuda()
+    wav = torch.empty(plan.wav_size, dtype=torch.float64, device="cuda")
+    sc = torch.empty(bs * bs, dtype=torch.complex128, device="cuda")
+    out = torch.empty_like(flm)
+    plan.analysis(flm, wav, sc)
+    plan.synthesis(wav, sc, out)
+    torch.cuda.synchronize()
+    host, hsc = core.s2dw_core_analysis_flm2wav_dynamic(f, t["K_gamma"], t["Slm"], J, B, N, bs, alpha)
+    for j in range(J + 1):
+        np.testing.assert_array_equal(plan.scale_view(wav, j).cpu().numpy().transpose(2, 1, 0), host[j])
+    back = core.s2dw_core_synthesis_wav2flm_dynamic(host, hsc, t["K_gamma"], t["Phi2"], t["Slm"], J, B, N, bs, alpha)
+    np.testing.assert_array_equal(back, out.cpu().numpy().T)
+    w2, s2, o2 = torch.zeros_like(wav), torch.zeros_like(sc), torch.zeros_like(out)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        plan.analysis(flm, w2, s2)
+        plan.synthesis(w2, s2, o2)
+    for _ in range(2):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(w2, wav) and torch.equal(o2, out)
+    del g
+    plan.close()
